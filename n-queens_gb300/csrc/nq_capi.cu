@@ -840,7 +840,7 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
         const HostTask& t = htasks[i];
         hr[i] = make_uint4(t.root[0], t.root[1], t.root[2], t.root[3]);
         hi[i] = make_uint2(t.info, t.job);
-        for (int d = 0; d <= t.T; d++) hs[(size_t)i * b->sw + d] = make_uint2(t.sched[2 * d], t.sched[2 * d + 1]);
+        for (int d = 0; d <= t.T; d++) hs[(size_t)i * b->sw + d] = make_uint2(t.sched[2 * d] ^ W_NOLOOK, t.sched[2 * d + 1]);
       }
       if ((e = cudaMemcpyAsync((uint4*)b->root.p + m_rec, hr.data(), m_host * sizeof(uint4), cudaMemcpyHostToDevice, st)) != cudaSuccess) break;
       if ((e = cudaMemcpyAsync((uint2*)b->info.p + m_rec, hi.data(), m_host * sizeof(uint2), cudaMemcpyHostToDevice, st)) != cudaSuccess) break;

@@ -309,6 +309,10 @@ NQ_HD Op unpack_compact(uint32_t w, int N, bool term) {
   o.tall = 0;
   return o;
 }
+// Device form of the words: the look-ahead flag inverted, so the DFS step folds it into the look-ahead
+// mask with one three-input op and one test ((mask | word & NOLOOK) != 0).
+constexpr uint32_t C_NOLOOK = C_FC;
+constexpr uint32_t W_NOLOOK = W_FC;
 // True when the op packs into a wide word: LA in the top s bits clear of the flags (s <= 24).
 NQ_HD bool wide_fits(const Op& o) { return o.s <= 24 && (uint64_t)o.la < (1ull << o.s); }
 NQ_HD uint32_t pack_wide_x(const Op& o) {

@@ -18,8 +18,11 @@
 //   shifts and no field extraction (nq_common.cuh).  The current frame is in
 //   registers; saved frames (only those with candidates left, as the
 //   reference's packed stack) sit in shared memory, interleaved by lane so
-//   every access is conflict-free, above a sentinel frame that leaves a
-//   finished lane with no free column.
+//   every access is conflict-free, above a sentinel frame whose candidates
+//   all die, which a finished lane works on until the next check.
+//   Bound by the issue slots and the integer pipes: N=18 takes 35.7 warp
+//   instructions a step of 32 lanes (16.7 on the ALU pipe, 14.0 on FMA, 8.5
+//   shared-memory wavefronts) at 77 % issue.
 //   Counts are summed per lane in u64 and flushed per job with one atomicAdd
 //   per warp (shuffle tree) at exit or per task when the job id changes.
 #include <type_traits>
@@ -32,17 +35,13 @@ namespace nq {
 constexpr unsigned FULL = 0xFFFFFFFFu;
 
 // DFS steps each lane takes between two checks for finished lanes (flush +
-// refill).  A lane that runs dry mid-round idles for the rest of the round; a
-// check costs two ballots, so checking less often wins until that idle time
-// dominates.
-#ifndef NQ_STEPS_PER_CHECK
-#define NQ_STEPS_PER_CHECK 32
-#endif
-#ifndef NQ_STEP_UNROLL
-#define NQ_STEP_UNROLL 16
-#endif
-constexpr int kStepsPerCheck = NQ_STEPS_PER_CHECK;
-constexpr int kStepUnroll = NQ_STEP_UNROLL;
+// refill), unrolled.  A lane that runs dry mid-round idles for the rest of the
+// round; a check costs two ballots, so checking less often wins until that
+// idle time dominates.  At most 31: the sentinel frame holds 31 candidates.
+// N=19 / N=17, ms: 30 steps unrolled 30 75.1 / 1.92, 15 76.1 / 1.93, 10 76.5 /
+// 1.91, 6 77.4 / 1.97; 20 steps 76.7 / 2.01; 15 steps 75.6 / 1.99.
+constexpr int kStepsPerCheck = 30;
+constexpr int kStepUnroll = kStepsPerCheck;
 
 template <bool WIDE> struct WordT { using type = uint32_t; };
 template <> struct WordT<true> { using type = uint2; };
@@ -86,8 +85,8 @@ __device__ __forceinline__ int prepare_one(int N, const uint4* __restrict__ rec,
     typename WordT<WIDE>::type* s = sched + t * sw;
     bool fits = true;
     for (int d = 0; d <= T; d++) {
-      if constexpr (WIDE) { fits = fits && wide_fits(ops[d]); s[d] = make_uint2(pack_wide_x(ops[d]), ops[d].ra); }
-      else { fits = fits && compact_fits(ops[d], N); s[d] = pack_compact(ops[d]); }
+      if constexpr (WIDE) { fits = fits && wide_fits(ops[d]); s[d] = make_uint2(pack_wide_x(ops[d]) ^ W_NOLOOK, ops[d].ra); }
+      else { fits = fits && compact_fits(ops[d], N); s[d] = pack_compact(ops[d]) ^ C_NOLOOK; }
     }
     if (!fits) {                      // never seen (N=6..21, presets 4-7): fail loudly rather than miscount
       atomicOr(err, DERR_FORMAT);
@@ -133,12 +132,12 @@ cudaError_t launch_prepare(int N, int64_t m, const uint4* records, const TaskArr
 struct Dec { uint32_t s, la, ra, fc, term, tall; };
 // compact word of depth k of a task of board N and terminal depth T
 __device__ __forceinline__ Dec decode(uint32_t w, uint32_t N, uint32_t k, uint32_t T) {
-  const Op o = unpack_compact(w, (int)N, k == T);
+  const Op o = unpack_compact(w ^ C_NOLOOK, (int)N, k == T);
   return Dec{o.s, o.la, o.ra, o.fc, o.term, o.tall};
 }
 __device__ __forceinline__ Dec decode(uint2 w, uint32_t, uint32_t, uint32_t) {
   const uint32_t s = w.x & W_S;
-  return Dec{s, s ? (w.x >> (32 - s)) : 0u, w.y, w.x & W_FC, w.x & W_TERM, w.x & W_TALL};
+  return Dec{s, s ? (w.x >> (32 - s)) : 0u, w.y, ~w.x & W_NOLOOK, w.x & W_TERM, w.x & W_TALL};
 }
 
 // ---------------------------------------------------------------------------
@@ -372,24 +371,16 @@ __device__ __forceinline__ void flush_job(const DfsArgs& a, unsigned job, unsign
   if (v) atomicAdd(a.job_totals + (job - a.job_base), v);
 }
 
-// Saved frames per lane: at most one per depth 0..T'-1 above the sentinel.
-__host__ __device__ constexpr int stack_slots(int maxt) { return maxt + 1; }
+// Shared memory per lane: frames at depths 0..maxt above the sentinel's slot, and schedule words
+// 0..maxt with the sentinel's word behind them.
+__host__ __device__ constexpr int stack_slots(int maxt) { return maxt + 2; }
+__host__ __device__ constexpr int word_slots(int maxt) { return maxt + 2; }
 
 size_t dfs_smem_bytes(bool wide, int block, int maxt) {
-  return (size_t)block * ((size_t)stack_slots(maxt) * sizeof(uint4) + (size_t)(maxt + 1) * (wide ? 8 : 4));
+  return (size_t)block * ((size_t)stack_slots(maxt) * sizeof(uint4) + (size_t)word_slots(maxt) * (wide ? 8 : 4));
 }
 
-// One lane's DFS state and its step.  Every lane runs the same predicated
-// sequence each step: resume a saved frame if the current one is exhausted,
-// take the lowest candidate, build the child with the depth's schedule word,
-// apply the look-ahead, then count (terminal depth) or descend.  '+' and '-'
-// replace '|' and '&~' where the bits are disjoint (a candidate is never in ld
-// or rd, and always one of the free columns), so those ops issue on the FMA
-// pipe as well as the ALU pipe.  Per-task counts are u32 (BIG: u64, where a
-// queue item may count 2^32 solutions).
-// Shared-memory accesses of the step, as predicated PTX so the pop and the push
-// are single predicated instructions rather than branches around them.
-// Addresses are 32-bit shared-window addresses.
+// Shared-memory accesses of the step at 32-bit shared-window addresses.
 __device__ __forceinline__ uint32_t lds_word(uint32_t a, uint32_t) {
   uint32_t w;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"(a));
@@ -401,6 +392,25 @@ __device__ __forceinline__ uint2 lds_word(uint32_t a, uint2) {
   return w;
 }
 
+// The sentinel frame under a lane's stack feeds a lane that has run out of work: its word (all ones)
+// shifts by 31 and fills every column of ld, so each of its 31 candidates dies.  kStepsPerCheck <= 31
+// steps therefore never pop below it, and the step tests neither the stack's depth nor the lane's
+// activity.
+constexpr uint32_t kSentinelAvail = 0xFFFFFFFEu;   // bits 1..31: ld + bit stays odd (ld = 1), so bit 31 of nld is set
+constexpr uint32_t kSentinelWord = 0xFFFFFFFFu;
+static_assert(kStepsPerCheck <= 31 && kStepsPerCheck % kStepUnroll == 0, "the sentinel holds 31 candidates");
+
+// One lane's DFS state and its step.  Every lane runs the same predicated sequence each step: resume a
+// saved frame if the current one is exhausted, take the lowest candidate, save the frame with the rest,
+// build the child with the depth's schedule word and make it the current frame -- with no candidates if
+// the look-ahead rejects it or its row is the last (counted there), so the next step resumes the saved
+// frame.  The frame is stored whether or not candidates are left (the slot above the stack is free) and
+// only the stack pointer moves by the test: the store costs the same wavefronts either way, and no
+// select is left but the child's candidates.  Selecting between parent and child instead (four selects
+// and a predicate passed into the store) took 18.1 ALU instructions a step against 16.7: N=19 84.6 ms,
+// this form 75.1 ms; N=17 2.08 ms, 1.92 ms.  '+' and '-' replace '|' and '&~' where the bits are disjoint (a candidate is never in ld or
+// rd, and always one of the free columns), so those ops issue on the FMA pipe as well as the ALU pipe.
+// Per-task counts are u32 (BIG: u64, where a queue item may count 2^32 solutions).
 template <bool WIDE, bool BIG>
 struct Lane {
   // A frame is {ld, rd, fr, avail}: fr holds the columns still free at the frame's
@@ -408,10 +418,9 @@ struct Lane {
   // needs no field of its own) and avail the candidates, a subset of fr.
   uint32_t ld = 0, rd = 0, fr = 0, avail = 0;
   uint32_t sp = 0;      // shared address of the next free frame of this lane's stack
-  uint32_t sbase = 0;   // shared address of its first frame: the stack is empty when sp == sbase
   uint32_t sw0 = 0;     // shared address of the word of the depth where popc(fr) == 0 (word d sits at
                         // sw0 - popc(fr) * row, row = BLOCK words, since popc(fr) = R - d, R = popc(root fr))
-  uint32_t tf = 0;      // popc(fr) at the subtask's terminal depth: R - terminal depth
+  uint32_t tf = ~0u;    // popc(fr) at the subtask's terminal depth: R - terminal depth
   uint32_t ram = 0;     // compact words: the bits where RA << s may sit (compact_ra_mask)
   typename std::conditional<BIG, unsigned long long, uint32_t>::type cnt = 0;
 
@@ -420,51 +429,36 @@ struct Lane {
     using W = typename WordT<WIDE>::type;
     constexpr uint32_t F = BLOCK * (uint32_t)sizeof(uint4);
     constexpr uint32_t ROW = BLOCK * (uint32_t)sizeof(W);
-    // pop (the current frame is exhausted and a saved one is left): the condition is formed in a
-    // predicate register inside the block, so no 0/1 value is materialised for it (2 % faster at N=19)
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %3, 0;\n\tsetp.ne.and.u32 p, %4, %5, p;\n\t"
-                 "@p sub.u32 %4, %4, %6;\n\t@p ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
-                 : "+r"(ld), "+r"(rd), "+r"(fr), "+r"(avail), "+r"(sp) : "r"(sbase), "n"(F));
+    // resume: the condition is formed in a predicate register inside the block, so no 0/1 value is
+    // materialised for it
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.u32 p, %3, 0;\n\t"
+                 "@p sub.u32 %4, %4, %5;\n\t@p ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+                 : "+r"(ld), "+r"(rd), "+r"(fr), "+r"(avail), "+r"(sp) : "n"(F));
     const uint32_t pf = __popc(fr);                  // R - depth
-    const bool act = avail != 0;
     const uint32_t bit = avail & (0u - avail);
-    avail -= bit;
+    const uint32_t rest = avail - bit;
     const W w = lds_word(sw0 - pf * ROW, W{});
-    uint32_t nld, nrd;
-    bool term, fc, tall = false;
-    if constexpr (WIDE) {
-      // the same funnel shift for nld; RA, which may sit anywhere, is or-ed after the right shift
-      asm("shf.l.wrap.b32 %0, %1, %2, %1;" : "=r"(nld) : "r"(w.x), "r"(ld + bit));
-      uint32_t y;
-      asm("shf.r.wrap.b32 %0, %1, 0, %2;" : "=r"(y) : "r"(rd + bit), "r"(w.x));
-      nrd = y | w.y;
-      term = (w.x & W_TERM) != 0u; fc = (w.x & W_FC) != 0u; tall = (w.x & W_TALL) != 0u;
-    } else {
-      // nld = (x << s) | LA in one funnel shift of the word (LA in its top s bits, s in its low 5);
-      // nrd = ((y | RA << s) >> s) = (y >> s) | RA, RA << s or-ed in from the word's bits N-1..N
-      asm("shf.l.wrap.b32 %0, %1, %2, %1;" : "=r"(nld) : "r"(w), "r"(ld + bit));
-      uint32_t y;
-      asm("lop3.b32 %0, %1, %2, %3, 0xF8;" : "=r"(y) : "r"(rd + bit), "r"(w), "r"(ram));   // a | (b & c)
-      asm("shf.r.wrap.b32 %0, %1, 0, %2;" : "=r"(nrd) : "r"(y), "r"(w));
-      term = pf == tf; fc = (w & C_FC) != 0u;
-    }
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" :: "r"(sp), "r"(ld), "r"(rd), "r"(fr), "r"(rest) : "memory");
+    if (rest != 0u) sp += F;
+    // nld = (x << s) | LA in one funnel shift of the word (LA in its top s bits, s in its low 5)
+    uint32_t wx, nld, nrd, y = rd + bit;
+    if constexpr (WIDE) wx = w.x; else wx = w;
+    asm("shf.l.wrap.b32 %0, %1, %2, %1;" : "=r"(nld) : "r"(wx), "r"(ld + bit));
+    // compact: nrd = ((y | RA << s) >> s) = (y >> s) | RA, RA << s or-ed in from the word's bits N-1..N;
+    // wide: RA, which may sit anywhere, is or-ed after the right shift
+    if constexpr (!WIDE) asm("lop3.b32 %0, %1, %2, %3, 0xF8;" : "=r"(y) : "r"(rd + bit), "r"(wx), "r"(ram));   // a | (b & c)
+    asm("shf.r.wrap.b32 %0, %1, 0, %2;" : "=r"(nrd) : "r"(y), "r"(wx));
+    if constexpr (WIDE) nrd |= w.y;
     const uint32_t free_cols = fr - bit;             // the child row's free columns
     const uint32_t nf = free_cols & ~(nld | nrd);
     const uint32_t ahead = free_cols & ~((nld + nld) | __umulhi(nrd, 0x80000000u));   // nrd >> 1
-    // terminal depth: count the child (the SQd2B rule is LA bit 0 of the word);
-    // otherwise descend unless the child row or, with look-ahead, the row after is full.
-    // A lane with nothing left holds the sentinel frame (no free column), so nf == 0
-    // there; only the tall rule of wide words needs the lane's activity itself.
-    const bool live = nf != 0u;
-    bool hit = live && term;
-    if constexpr (WIDE) hit = (act && live && term) || (act && term && tall);
-    cnt += hit ? 1u : 0u;
-    const bool desc = (WIDE ? act : true) && live && !term && !(fc && ahead == 0u);
-    const uint32_t push = (desc && avail != 0u) ? 1u : 0u;
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p st.shared.v4.u32 [%1], {%2, %3, %4, %5};\n\t}"
-                 :: "r"(push), "r"(sp), "r"(ld), "r"(rd), "r"(fr), "r"(avail) : "memory");
-    sp += push ? F : 0u;
-    if (desc) { ld = nld; rd = nrd; fr = free_cols; avail = nf; }
+    const uint32_t keep = ahead | (wx & (WIDE ? W_NOLOOK : C_NOLOOK));
+    // terminal depth: count the child if its row has a free square (the SQd2B rule is LA bit 0 of the word);
+    // otherwise descend unless the child row or, with look-ahead, the row after is full
+    const bool term = pf == tf;
+    if (term && nf != 0u) cnt += 1u;
+    ld = nld; rd = nrd; fr = free_cols;
+    avail = (nf != 0u && keep != 0u && !term) ? nf : 0u;
   }
 };
 
@@ -477,19 +471,26 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt_mask = (1u << lane) - 1u;
   const W* __restrict__ gsched = reinterpret_cast<const W*>(a.sched);
-  Lane<WIDE, BIG> L;
-  L.sbase = L.sp = (uint32_t)__cvta_generic_to_shared(stk);
-  const uint32_t sch_sh = (uint32_t)__cvta_generic_to_shared(sch);
   constexpr uint32_t ROW = BLOCK * (uint32_t)sizeof(W);
-  L.sw0 = sch_sh;                     // a lane without work reads word 0 (fr == 0: no candidate survives)
+  auto put_word = [&](uint32_t k, W w) { sch[k * BLOCK] = w; };
+  auto sentinel_word = [] { W w; if constexpr (WIDE) w = make_uint2(kSentinelWord, 0u); else w = kSentinelWord; return w; };
+  Lane<WIDE, BIG> L;
+  const uint32_t sch_sh = (uint32_t)__cvta_generic_to_shared(sch);
+  // stack pointer above the sentinel: a lane is idle when no frame but the sentinel is left
+  const uint32_t top = (uint32_t)__cvta_generic_to_shared(stk) + BLOCK * (uint32_t)sizeof(uint4);
+  L.sp = top;
+  L.sw0 = sch_sh;                     // a lane without work reads word 0 (the sentinel's fr is 0)
+  stk[0] = make_uint4(1u, 0u, 0u, kSentinelAvail);
+  put_word(0, sentinel_word());
   uint32_t wexp = 0, job = a.job_base, task = 0;
   bool have = false, exhausted = false;
   unsigned long long acc = 0;
   uint32_t acc_job = a.job_base;
 
   for (;;) {
-    const bool idle = (L.avail | (L.sp - L.sbase)) == 0u;
+    const bool idle = L.avail == 0u && L.sp == top;
     if (__ballot_sync(FULL, idle)) {          // some lane finished: flush, refill, maybe exit
+      if (idle) stk[0].w = kSentinelAvail;    // the steps since it finished have used some of its candidates
       if (idle && have) {
         const unsigned long long v = (unsigned long long)L.cnt << wexp;
         if (a.per_task) {
@@ -521,33 +522,39 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
             L.cnt = (d0 == 0) ? info_root(in.x) : 0u;
             wexp = info_wexp(in.x);
             job = in.y;
-            L.sp = L.sbase;
             if (T == INFO_NO_DFS || info_status(in.x) != TS_OK || T < d0) {
-              L.avail = 0; L.fr = 0; L.sw0 = sch_sh;
-            } else if ((int)(T - d0) > a.maxt) {    // frames at depths 0..T'-1, words 0..T'
+              // no DFS work: the lane stays on its sentinel
+            } else if ((int)(T - d0) > a.maxt) {    // frames at depths 0..T', words 0..T'
               atomicOr(a.err, DERR_DEPTH);
-              L.avail = 0; L.fr = 0; L.sw0 = sch_sh;
             } else {
               // root: the free columns of the board, R of them; depth d has R - d (one queen per depth,
               // T' + 1 <= R of them), so word d is found from popc(fr) alone
               const uint32_t fr = ((1u << info_N(in.x)) - 1u) & ~r.z;
               const uint32_t R = __popc(fr);
-              L.ld = r.x; L.rd = r.y; L.fr = fr; L.avail = r.w & fr;
-              L.tf = R - (T - d0); L.sw0 = sch_sh + R * ROW; L.ram = compact_ra_mask((int)info_N(in.x));
               const W* src = gsched + (size_t)task * a.sw + d0;
-              for (uint32_t k = 0; k <= T - d0; k++) sch[k * BLOCK] = src[k];
-              // the sentinel under the stack, popped after the last real frame: depth 0 (fr has R
-              // columns, so the word it reads is word 0) with every diagonal blocked, so no
-              // candidate survives
-              stk[0] = make_uint4(~0u, ~0u, fr, 0u);
-              L.sp = L.sbase + BLOCK * (uint32_t)sizeof(uint4);
+              uint32_t n = T - d0;                 // terminal depth
+              bool leaf = false;
+              if constexpr (WIDE) {
+                // a tall last row has one free column: its parent row is the terminal one by the compact
+                // words' rule (count the child if its row has a free square)
+                if (src[n].x & W_TALL) { leaf = n == 0u; n -= leaf ? 0u : 1u; }
+              }
+              if (leaf) {
+                L.cnt += __popc(r.w & fr);
+              } else if (n + 2u <= R) {            // fewer free columns than rows: no solution, no work
+                L.ld = r.x; L.rd = r.y; L.fr = fr; L.avail = r.w & fr;
+                L.tf = R - n; L.sw0 = sch_sh + R * ROW; L.ram = compact_ra_mask((int)info_N(in.x));
+                for (uint32_t k = 0; k <= n; k++) put_word(k, src[k]);
+                put_word(n + 1u, sentinel_word());
+                stk[0] = make_uint4(1u, 0u, (1u << (R - n - 1u)) - 1u, kSentinelAvail);   // popc(fr) finds its word
+              }
             }
           } else {
             exhausted = true;
           }
         }
       }
-      if (__all_sync(FULL, exhausted && (L.avail | (L.sp - L.sbase)) == 0u)) break;
+      if (__all_sync(FULL, exhausted && L.avail == 0u && L.sp == top)) break;
       asm volatile("" ::: "memory");   // refill stores to the schedule before the steps' loads
     }
 #pragma unroll kStepUnroll
