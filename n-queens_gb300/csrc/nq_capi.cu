@@ -52,20 +52,23 @@ const char* derr_text(uint32_t e) {
   return "ok";
 }
 
-// Expand tasks until the queue holds at least 13 items per resident DFS lane
-// (the DFS kernel keeps about 768 lanes per SM), at most 3 levels.  Each level
-// multiplies the queue by about 7 (measured: 6.2x at N=16 to 8x at N=20).
-// Task lists of a million or more are split at least once: their largest
-// tasks set the tail (GB300, N=21: D=0 7466 ms, D=1 6983 ms, D=2 6914 ms).
-// This rule picks the depth the autotuner found fastest on GB300 for
-// N=16..21 (2, 2, 1, 1, 1-2, 1-2).
-int choose_split(int64_t m, int sms) {
-  const double target = 13.0 * 768.0 * (double)sms;
-  int D = 0;
-  double est = (double)m;
-  while (D < 3 && est < target) { est *= 7.0; D++; }
-  // ~7 subtasks per task must stay within the u32 subtask queue
-  return (D == 0 && m >= 1000000 && m <= 400000000) ? 1 : D;
+// Levels every task is expanded by before the DFS.  `rows`: rows left below the shallowest start (N - 2 -
+// start row), which sets a task's work (about 7x per row).  Lanes of a warp share their work at the end of
+// the queue, so splitting only has to even out the warps and give a short list more items than lanes:
+// us of a whole call on GB300 at D = 0 / 1 / 2 / 3, m tasks:
+//   8 rows (N=12):    m=4300   81 / 83 / 85 / 110
+//   10 rows (N=14):   m=13233 125 / 117 / 121 / 182
+//   11 rows (N=15):   m=21270 187 / 168 / 179 / 293
+//   12 rows (N=16):   m=4000  190 / 177 / 182 / 286   m=33046   602 / 448 / 407 / 585
+//   13 rows (N=18):   m=16000 900 / 738 / 527 / 668   m=200000 5634 / 4121 / 4407 / 5657
+//   14 rows (N=19):   m=50000 10.1 / 5.5 / 4.8 / 5.3 ms   m=897071 80.7 / 74.1 / 78.8 ms
+//   15 rows (N=20):   m=4000  9.1 / 5.5 / 3.2 / 2.6 ms
+// Each level makes about 7 times the items (measured: 6.2x at N=16 to 8x at N=20), and an item costs its
+// loading; lists of 10^5 tasks and more are balanced at D = 1.
+int choose_split(int64_t m, int rows) {
+  if (rows <= 9) return 0;
+  if (rows <= 11 || m > 100000) return m > 400000000 ? 0 : 1;   // ~7 subtasks a task stay within the u32 subtask queue
+  return rows >= 15 && m < 8192 ? 3 : 2;
 }
 
 // Records per chunk of a whole-board count (nq_count): one chunk up to N=21
@@ -107,8 +110,8 @@ int run_records(nq_handle* h, int N, const uint4* d_rec, int64_t m, int start_mi
   unsigned long long* sctr = (unsigned long long*)(c + ctl::kSplit);   // split: [0] subtasks, [1] allocation cursor
   unsigned int* tmax = (unsigned int*)(c + ctl::kTmax);                 // deepest schedule of the launch
   NQ_CUDA(h, cudaEventRecord(h->ev[0], st));
-  NQ_CUDA(h, launch_prepare(N, m, d_rec, ta, 0, 0, err, st, tmax));
-  const int D = h->split >= 0 ? h->split : choose_split(m, h->sms);
+  NQ_CUDA(h, launch_prepare(N, m, d_rec, ta, 0, 0, err, st, tmax, d_per_task));
+  const int D = h->split >= 0 ? h->split : choose_split(m, maxt);
   DfsLaunch L;
   L.tasks = ta; L.m = m; L.order = nullptr; L.cursor = cursor; L.job_totals = totals;
   L.per_task = d_per_task; L.err = err; L.maxt = maxt; L.block = h->block; L.grid = h->grid;
@@ -641,7 +644,7 @@ struct nq_batch {
   bool wide = true;                        // 8-byte schedule words (completion tasks); compact otherwise
   std::vector<int64_t> job_off, job_m;     // task range per job
   std::vector<int64_t> sub_off, sub_m;     // subtask range per job
-  std::vector<int> job_maxt, job_split;
+  std::vector<int> job_maxt, job_rows, job_split;   // job_rows: rows left, as choose_split takes them
   std::vector<uint64_t> fixed_total;       // counts settled at build time (small tasks, full boards)
   uint64_t* h_out = nullptr;               // pinned: totals per job + cursor/err
   cudaGraphExec_t graph = nullptr;
@@ -735,7 +738,7 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
   b->h = h;
   b->jobs.assign(jobs, jobs + njobs);
   b->block = h->block;
-  b->job_off.assign(njobs, 0); b->job_m.assign(njobs, 0); b->job_maxt.assign(njobs, 1); b->fixed_total.assign(njobs, 0);
+  b->job_off.assign(njobs, 0); b->job_m.assign(njobs, 0); b->job_maxt.assign(njobs, 1); b->job_rows.assign(njobs, 1); b->fixed_total.assign(njobs, 0);
   // Build: count jobs (N >= 6) become constellation records prepared on the
   // device; count jobs with N <= 5 and completion jobs become host tasks.
   struct Seg { int job, N; int64_t rec_off, m; };
@@ -766,7 +769,7 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
       Seg sg{j, J.N, (int64_t)recs.size(), (int64_t)v.size()};
       for (auto& g : v) recs.push_back(nq_record{(uint32_t)g.ld, (uint32_t)g.rd, (uint32_t)g.col, g.startijkl});
       segs.push_back(sg);
-      b->job_maxt[j] = maxt_for(J.N, it->second.smin);
+      b->job_rows[j] = b->job_maxt[j] = maxt_for(J.N, it->second.smin);
       maxt = std::max(maxt, b->job_maxt[j]);
     } else if (J.kind == NQ_JOB_COUNT || J.kind == NQ_JOB_COMPLETION) {
       int rows[8], cols[8];
@@ -779,6 +782,7 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
       if (s == 2) b->fixed_total[j] = 1;
       job_host_begin[j] = before; job_host_end[j] = (int64_t)htasks.size();
       b->job_maxt[j] = std::max(1, mt);
+      b->job_rows[j] = mt + 2;             // mt + 1 free rows
       maxt = std::max(maxt, b->job_maxt[j]);
     } else {
       nq_batch_destroy(b);
@@ -864,7 +868,7 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
     unsigned long long* sc = (unsigned long long*)sctr.p;   // [2j] subtasks of job j, [2*njobs+1] cursor
     if ((e = cudaMemsetAsync(sc, 0, (size_t)(njobs + 1) * 16, st)) != cudaSuccess) { sctr.release(); break; }
     for (int j = 0; j < njobs && e == cudaSuccess; j++) {
-      b->job_split[j] = (jobs[j].N <= 12) ? 0 : (h->split >= 0 ? h->split : choose_split(b->job_m[j], h->sms));
+      b->job_split[j] = (jobs[j].N <= 12) ? 0 : (h->split >= 0 ? h->split : choose_split(b->job_m[j], b->job_rows[j]));
       e = launch_split(0, b->job_split[j], b->job_off[j], b->job_m[j], ta, (uint32_t*)b->nsub.p, nullptr, nullptr,
                        sc + 2 * j, nullptr, nullptr, 0, st);
     }
@@ -911,7 +915,7 @@ int64_t nq_job_device_bytes(const nq_job* job, int sms, int split_depth) {
   if (J.N < 1 || J.N > kMaxN || J.k < 0 || J.k > 8) return NQ_EINVAL;
   int64_t m = 0;
   size_t word = 0;
-  int maxt = 1;
+  int maxt = 1, rows_left = 1;
   if (J.kind == NQ_JOB_COUNT && J.N >= 6) {
     // the generator's record count, as nq_batch_create builds the job (compact schedule words)
     const int p = J.preset > 0 ? J.preset : preset_for(J.N);
@@ -921,7 +925,7 @@ int64_t nq_job_device_bytes(const nq_job* job, int sms, int split_depth) {
     m = (int64_t)v.size();
     int smin = 64;
     for (const GenRecord& r : v) smin = std::min<int>(smin, (int)(r.startijkl >> 20));
-    maxt = maxt_for(J.N, smin);
+    rows_left = maxt = maxt_for(J.N, smin);
     word = sizeof(uint32_t);
   } else if (J.kind == NQ_JOB_COUNT || J.kind == NQ_JOB_COMPLETION) {
     int rows[8], cols[8];
@@ -932,12 +936,13 @@ int64_t nq_job_device_bytes(const nq_job* job, int sms, int split_depth) {
     if (build_completion_tasks(J.N, k, rows, cols, 4096, 0, t, &mt) < 0) return NQ_EINVAL;
     m = (int64_t)t.size();
     maxt = std::max(1, mt);
+    rows_left = mt + 2;
     word = sizeof(uint2);
   } else {
     return NQ_EINVAL;
   }
   // split queue: each level multiplies the items by at most ~8 (measured 6.2-8x)
-  const int D = (J.N <= 12) ? 0 : (split_depth >= 0 ? split_depth : choose_split(m, sms));
+  const int D = (J.N <= 12) ? 0 : (split_depth >= 0 ? split_depth : choose_split(m, rows_left));
   int64_t ns = m;
   for (int d = 0; d < D; d++) ns *= 8;
   const int64_t per_task = 16 /*record*/ + 16 /*root*/ + 8 /*info*/ + 4 /*split count*/ + (int64_t)(maxt + 1) * (int64_t)word;

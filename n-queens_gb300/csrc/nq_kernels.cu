@@ -9,8 +9,9 @@
 // dfs_kernel: persistent, explicit-stack bitboard DFS replacing
 //   kernel_dfs_iter_gpu_maxd14..21 (356Py:618-1747) and dfs_iter
 //   (356Py:1837-1967).  Every lane runs its own task; a lane whose task is
-//   done takes the next one from a global queue (one atomicAdd per warp and
-//   refill round, ranks by ballot).  Each step every busy lane
+//   done takes the next one from the warp's pool, which the warp fills from a
+//   global queue, and when the queue is empty part of a task of a busy lane
+//   of its warp.  Each step every busy lane
 //   expands exactly one candidate queen, so lanes stay converged on the same
 //   short instruction sequence whatever their task, depth or SQ* variant:
 //   the variant lives in the schedule word read from shared memory, not in
@@ -25,6 +26,7 @@
 //   shared-memory wavefronts) at 77 % issue.
 //   Counts are summed per lane in u64 and flushed per job with one atomicAdd
 //   per warp (shuffle tree) at exit or per task when the job id changes.
+#include <algorithm>
 #include <type_traits>
 
 #include "nq_common.cuh"
@@ -43,6 +45,16 @@ constexpr unsigned FULL = 0xFFFFFFFFu;
 constexpr int kStepsPerCheck = 30;
 constexpr int kStepUnroll = kStepsPerCheck;
 
+// A warp takes 32 queue items at a time (one atomic and one coalesced load round for the 32), less towards
+// the end of the queue: 1/8 of its even share of what is left, at least 8, so the warps end together.
+// Taking the items one by one instead took 74.1 ms at N=19, 1.715 at N=17 (73.2 and 1.675 with the pool);
+// a share of 1/4 1.71 at N=17; at least 1: 0.375 ms at N=16 against 0.365, 16: 1.725 at N=17.
+constexpr float kChunkShare = 8.0f;
+constexpr unsigned kMinChunk = 8;
+// A frame is given to a lane without work when it is at least this many levels above the terminal depth
+// (fewer: not worth the exchange; 3 and 7 measured the same from N=16 on, 7 is 25 % slower at N=14).
+constexpr int kGiveRows = 5;
+
 template <bool WIDE> struct WordT { using type = uint32_t; };
 template <> struct WordT<true> { using type = uint2; };
 
@@ -52,9 +64,11 @@ template <> struct WordT<true> { using type = uint2; };
 template <bool WIDE>
 __device__ __forceinline__ int prepare_one(int N, const uint4* __restrict__ rec, uint4* __restrict__ root,
                                            uint2* __restrict__ info, typename WordT<WIDE>::type* __restrict__ sched,
-                                           int sw, int64_t offset, uint32_t job, unsigned int* err, int64_t i) {
+                                           int sw, int64_t offset, uint32_t job, unsigned int* err, int64_t i,
+                                           unsigned long long* __restrict__ per_task) {
   const uint4 r = rec[i];
   const int64_t t = offset + i;
+  if (per_task) per_task[t] = 0;      // the DFS adds each queue item's share
   uint32_t status = TS_OK;
   Root rt = {0, 0, 0, 0};
   uint32_t root_count = 0;
@@ -102,9 +116,9 @@ __global__ void __launch_bounds__(256) prepare_kernel(int N, int64_t m, const ui
                                                       uint4* __restrict__ root, uint2* __restrict__ info,
                                                       typename WordT<WIDE>::type* __restrict__ sched, int sw,
                                                       int64_t offset, uint32_t job, unsigned int* err,
-                                                      unsigned int* tmax) {
+                                                      unsigned int* tmax, unsigned long long* __restrict__ per_task) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int T = (i < m) ? prepare_one<WIDE>(N, rec, root, info, sched, sw, offset, job, err, i) : -1;
+  const int T = (i < m) ? prepare_one<WIDE>(N, rec, root, info, sched, sw, offset, job, err, i, per_task) : -1;
   if (tmax) {                         // deepest schedule of the launch, for sizing the DFS stack
     const unsigned v = __reduce_max_sync(FULL, (unsigned)(T < 0 ? 0 : T));
     if ((threadIdx.x & 31u) == 0 && v) atomicMax(tmax, v);
@@ -113,16 +127,17 @@ __global__ void __launch_bounds__(256) prepare_kernel(int N, int64_t m, const ui
 
 
 cudaError_t launch_prepare(int N, int64_t m, const uint4* records, const TaskArrays& out, int64_t offset,
-                           uint32_t job, unsigned int* err, cudaStream_t st, unsigned int* tmax) {
+                           uint32_t job, unsigned int* err, cudaStream_t st, unsigned int* tmax,
+                           unsigned long long* per_task) {
   if (m <= 0) return cudaSuccess;
   const int B = 256;
   const unsigned G = (unsigned)((m + B - 1) / B);
   if (out.wide)
     prepare_kernel<true><<<G, B, 0, st>>>(N, m, records, out.root, out.info, (uint2*)out.sched, out.sw, offset, job, err,
-                                          tmax);
+                                          tmax, per_task);
   else
     prepare_kernel<false><<<G, B, 0, st>>>(N, m, records, out.root, out.info, (uint32_t*)out.sched, out.sw, offset, job,
-                                           err, tmax);
+                                           err, tmax, per_task);
   return cudaGetLastError();
 }
 
@@ -365,6 +380,8 @@ struct DfsArgs {
   unsigned long long* per_task;
   unsigned int* err;
   int maxt;
+  unsigned chunk;             // queue items a warp takes first: 32, or its share of a queue smaller than the grid
+  float share;                // the later chunks' share of the items left
 };
 
 __device__ __forceinline__ void flush_job(const DfsArgs& a, unsigned job, unsigned long long v) {
@@ -462,99 +479,181 @@ struct Lane {
   }
 };
 
+__device__ __forceinline__ void sts_frame(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" :: "r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ uint4 lds_frame(uint32_t a) {
+  uint4 f;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(f.x), "=r"(f.y), "=r"(f.z), "=r"(f.w) : "r"(a) : "memory");
+  return f;
+}
+// position of the r-th set bit of m (r < popc(m))
+__device__ __forceinline__ uint32_t nth_set(uint32_t m, uint32_t r) {
+  uint32_t pos = 0;
+#pragma unroll
+  for (uint32_t w = 16; w; w >>= 1) {
+    const uint32_t c = __popc(m & ((1u << w) - 1u));
+    if (r >= c) { r -= c; m >>= w; pos += w; }
+  }
+  return pos;
+}
+
 template <bool WIDE, int BLOCK, bool BIG>
 __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
   using W = typename WordT<WIDE>::type;
   extern __shared__ __align__(16) unsigned char smem[];
-  uint4* stk = reinterpret_cast<uint4*>(smem) + threadIdx.x;                                   // stride BLOCK
   W* sch = reinterpret_cast<W*>(smem + (size_t)stack_slots(a.maxt) * BLOCK * sizeof(uint4)) + threadIdx.x;  // stride BLOCK
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt_mask = (1u << lane) - 1u;
   const W* __restrict__ gsched = reinterpret_cast<const W*>(a.sched);
   constexpr uint32_t ROW = BLOCK * (uint32_t)sizeof(W);
+  constexpr uint32_t F = BLOCK * (uint32_t)sizeof(uint4);
   auto put_word = [&](uint32_t k, W w) { sch[k * BLOCK] = w; };
   auto sentinel_word = [] { W w; if constexpr (WIDE) w = make_uint2(kSentinelWord, 0u); else w = kSentinelWord; return w; };
   Lane<WIDE, BIG> L;
   const uint32_t sch_sh = (uint32_t)__cvta_generic_to_shared(sch);
-  // stack pointer above the sentinel: a lane is idle when no frame but the sentinel is left
-  const uint32_t top = (uint32_t)__cvta_generic_to_shared(stk) + BLOCK * (uint32_t)sizeof(uint4);
+  const uint32_t bottom = (uint32_t)__cvta_generic_to_shared(smem) + threadIdx.x * (uint32_t)sizeof(uint4);
+  // stack pointer above the sentinel: a lane is idle when no frame but the sentinel is left.  The sentinel
+  // is the lane's first slot until a frame above it is given away (below).
+  uint32_t top = bottom + F;
   L.sp = top;
   L.sw0 = sch_sh;                     // a lane without work reads word 0 (the sentinel's fr is 0)
-  stk[0] = make_uint4(1u, 0u, 0u, kSentinelAvail);
+  L.tf = 1;
   put_word(0, sentinel_word());
+  // where popc(fr) == tf - 1 the lane's word is the sentinel's
+  auto arm = [&]() { sts_frame(top - F, 1u, 0u, (1u << (L.tf - 1u)) - 1u, kSentinelAvail); };
   uint32_t wexp = 0, job = a.job_base, task = 0;
-  bool have = false, exhausted = false;
+  bool have = false, exhausted = false, drained = false;   // exhausted, drained: warp-uniform, as the pool's counters
+  unsigned chunk = a.chunk, pool_n = 0, pool_at = 0;
+  uint4 p_root = make_uint4(0, 0, 0, 0);
+  uint32_t p_task = 0, p_info = 0, p_job = 0;
   unsigned long long acc = 0;
   uint32_t acc_job = a.job_base;
 
   for (;;) {
     const bool idle = L.avail == 0u && L.sp == top;
     if (__ballot_sync(FULL, idle)) {          // some lane finished: flush, refill, maybe exit
-      if (idle) stk[0].w = kSentinelAvail;    // the steps since it finished have used some of its candidates
+      if (idle) arm();                        // the steps since it finished have used some of its candidates
       if (idle && have) {
         const unsigned long long v = (unsigned long long)L.cnt << wexp;
-        if (a.per_task) {
-          if (a.sinfo) atomicAdd(a.per_task + task, v);
-          else a.per_task[task] = v;
-        }
+        if (a.per_task && v) atomicAdd(a.per_task + task, v);
         if (job != acc_job) { flush_job(a, acc_job, acc); acc = 0; acc_job = job; }
         acc += v;
         have = false;
       }
-      const bool want = idle && !exhausted;
-      const unsigned need = __ballot_sync(FULL, want);
-      if (need) {
-        const int leader = __ffs(need) - 1;
-        unsigned long long base = 0;
-        if ((int)lane == leader) base = atomicAdd(a.cursor, (unsigned long long)__popc(need));
-        base = __shfl_sync(FULL, base, leader);
-        if (want) {
-          const uint64_t slot = (uint64_t)base + (uint64_t)__popc(need & lt_mask);
-          if (slot < (uint64_t)a.m) {
+      // Refill from the warp's pool of queue items: lane i holds item i of the last chunk taken, loaded by
+      // the whole warp at once, so a lane that needs work costs seven shuffles, not an atomic and two
+      // dependent rounds of loads.
+      bool want = idle && !exhausted;
+      for (unsigned need = __ballot_sync(FULL, want); need; need = __ballot_sync(FULL, want)) {
+        if (pool_n == 0u) {
+          if (drained) { exhausted = true; break; }
+          unsigned long long base = 0;
+          if (lane == 0) base = atomicAdd(a.cursor, (unsigned long long)chunk);
+          base = __shfl_sync(FULL, base, 0);
+          const unsigned long long left = base < (unsigned long long)a.m ? (unsigned long long)a.m - base : 0ull;
+          pool_n = left < chunk ? (unsigned)left : chunk;
+          pool_at = 0;
+          // the next chunk is a share of what is left, so the warps end together; where the first chunks
+          // cover the queue there is no next one
+          drained = a.chunk < 32u || left <= chunk;
+          chunk = min(32u, max(kMinChunk, (unsigned)((float)left * a.share)));
+          if (pool_n == 0u) { exhausted = true; break; }
+          if (lane < pool_n) {
+            const uint64_t slot = base + lane;
             const uint64_t q = a.order ? (uint64_t)a.order[slot] : slot;
-            uint4 r;
-            uint32_t d0;
-            if (a.sinfo) { const uint2 si = a.sinfo[q]; task = si.x; d0 = si.y; r = a.sroot[q]; }
-            else { task = (uint32_t)q; d0 = 0; r = a.root[q]; }
-            const uint2 in = a.info[task];
-            const uint32_t T = info_T(in.x);
-            have = true;
-            L.cnt = (d0 == 0) ? info_root(in.x) : 0u;
-            wexp = info_wexp(in.x);
-            job = in.y;
-            if (T == INFO_NO_DFS || info_status(in.x) != TS_OK || T < d0) {
-              // no DFS work: the lane stays on its sentinel
-            } else if ((int)(T - d0) > a.maxt) {    // frames at depths 0..T', words 0..T'
-              atomicOr(a.err, DERR_DEPTH);
-            } else {
-              // root: the free columns of the board, R of them; depth d has R - d (one queen per depth,
-              // T' + 1 <= R of them), so word d is found from popc(fr) alone
-              const uint32_t fr = ((1u << info_N(in.x)) - 1u) & ~r.z;
-              const uint32_t R = __popc(fr);
-              const W* src = gsched + (size_t)task * a.sw + d0;
-              uint32_t n = T - d0;                 // terminal depth
-              bool leaf = false;
-              if constexpr (WIDE) {
-                // a tall last row has one free column: its parent row is the terminal one by the compact
-                // words' rule (count the child if its row has a free square)
-                if (src[n].x & W_TALL) { leaf = n == 0u; n -= leaf ? 0u : 1u; }
-              }
-              if (leaf) {
-                L.cnt += __popc(r.w & fr);
-              } else if (n + 2u <= R) {            // fewer free columns than rows: no solution, no work
-                L.ld = r.x; L.rd = r.y; L.fr = fr; L.avail = r.w & fr;
-                L.tf = R - n; L.sw0 = sch_sh + R * ROW; L.ram = compact_ra_mask((int)info_N(in.x));
-                for (uint32_t k = 0; k <= n; k++) put_word(k, src[k]);
-                put_word(n + 1u, sentinel_word());
-                stk[0] = make_uint4(1u, 0u, (1u << (R - n - 1u)) - 1u, kSentinelAvail);   // popc(fr) finds its word
-              }
-            }
+            uint32_t d0 = 0;
+            if (a.sinfo) { const uint2 si = a.sinfo[q]; p_task = si.x; d0 = si.y; p_root = a.sroot[q]; }
+            else { p_task = (uint32_t)q; p_root = a.root[q]; }
+            const uint2 in = a.info[p_task];
+            p_info = in.x | (d0 << 16); p_job = in.y;
+          }
+        }
+        const unsigned give = min((unsigned)__popc(need), pool_n);
+        const unsigned rank = __popc(need & lt_mask);
+        const int src = (int)(pool_at + rank);
+        uint4 r;
+        r.x = __shfl_sync(FULL, p_root.x, src); r.y = __shfl_sync(FULL, p_root.y, src);
+        r.z = __shfl_sync(FULL, p_root.z, src); r.w = __shfl_sync(FULL, p_root.w, src);
+        const uint32_t i_task = __shfl_sync(FULL, p_task, src), i_info = __shfl_sync(FULL, p_info, src);
+        const uint32_t i_job = __shfl_sync(FULL, p_job, src);
+        pool_at += give; pool_n -= give;
+        if (want && rank < give) {
+          want = false;
+          const uint32_t d0 = i_info >> 16, T = info_T(i_info);
+          task = i_task; job = i_job;
+          have = true;
+          L.cnt = (d0 == 0) ? info_root(i_info) : 0u;
+          wexp = info_wexp(i_info);
+          if (T == INFO_NO_DFS || info_status(i_info) != TS_OK || T < d0) {
+            // no DFS work: the lane stays on its sentinel
+          } else if ((int)(T - d0) > a.maxt) {    // frames at depths 0..T', words 0..T'
+            atomicOr(a.err, DERR_DEPTH);
           } else {
-            exhausted = true;
+            // root: the free columns of the board, R of them; depth d has R - d (one queen per depth,
+            // T' + 1 <= R of them), so word d is found from popc(fr) alone
+            const uint32_t fr = ((1u << info_N(i_info)) - 1u) & ~r.z;
+            const uint32_t R = __popc(fr);
+            const W* src_w = gsched + (size_t)task * a.sw + d0;
+            uint32_t n = T - d0;                 // terminal depth
+            bool leaf = false;
+            if constexpr (WIDE) {
+              // a tall last row has one free column: its parent row is the terminal one by the compact
+              // words' rule (count the child if its row has a free square)
+              if (src_w[n].x & W_TALL) { leaf = n == 0u; n -= leaf ? 0u : 1u; }
+            }
+            if (leaf) {
+              L.cnt += __popc(r.w & fr);
+            } else if (n + 2u <= R) {            // fewer free columns than rows: no solution, no work
+              L.ld = r.x; L.rd = r.y; L.fr = fr; L.avail = r.w & fr;
+              L.tf = R - n; L.sw0 = sch_sh + R * ROW; L.ram = compact_ra_mask((int)info_N(i_info));
+              for (uint32_t k = 0; k <= n; k++) put_word(k, src_w[k]);
+              put_word(n + 1u, sentinel_word());
+              arm();
+            }
           }
         }
       }
-      if (__all_sync(FULL, exhausted && L.avail == 0u && L.sp == top)) break;
+      if (exhausted) {
+        // The queue is empty: a lane without work takes the bottom saved frame (the largest subtree left) of
+        // a busy lane of its warp, or all but one candidate of that lane's current frame.  It reads the
+        // giver's schedule words in place: only loading a queue item overwrites words, and none is left.
+        // Without this the last items of a warp left 7 of 32 lanes idle at N=17 (1.92 ms, 1.715 with it),
+        // N=16 0.404 -> 0.352, N=18 10.9 -> 10.4, N=19 75.1 -> 74.1.
+        const unsigned starved = __ballot_sync(FULL, !have);
+        if (starved) {
+          const bool saved = L.sp != top;
+          const uint32_t rest = L.avail & (L.avail - 1u);
+          const uint32_t gfr = saved ? lds_frame(top).z : L.fr;
+          const bool can = have && (saved ? (L.avail != 0u || L.sp != top + F) : rest != 0u) &&
+                           __popc(gfr) >= (int)L.tf + kGiveRows;
+          const unsigned givers = __ballot_sync(FULL, can);
+          if (givers) {
+            const int n = min(__popc(starved), __popc(givers));
+            const bool gives = can && __popc(givers & lt_mask) < n;
+            const int srank = __popc(starved & lt_mask);
+            const bool takes = !have && srank < n;
+            if (gives && !saved) { sts_frame(top, L.ld, L.rd, L.fr, rest); L.avail ^= rest; }
+            __syncwarp();
+            const int src = takes ? (int)nth_set(givers, (uint32_t)srank) : (int)lane;
+            const uint32_t from = __shfl_sync(FULL, top, src), gsw0 = __shfl_sync(FULL, L.sw0, src);
+            const uint32_t gtf = __shfl_sync(FULL, L.tf, src), gram = __shfl_sync(FULL, L.ram, src);
+            const uint32_t gw = __shfl_sync(FULL, wexp, src), gjob = __shfl_sync(FULL, job, src);
+            const uint32_t gtask = __shfl_sync(FULL, task, src);
+            if (takes) {
+              const uint4 f = lds_frame(from);
+              L.ld = f.x; L.rd = f.y; L.fr = f.z; L.avail = f.w;
+              L.sw0 = gsw0; L.tf = gtf; L.ram = gram; L.cnt = 0;
+              wexp = gw; job = gjob; task = gtask; have = true;
+              top = bottom + F; L.sp = top;
+              arm();
+            }
+            __syncwarp();
+            if (gives && saved) { top += F; arm(); }   // the sentinel takes the given frame's place
+          }
+        }
+      }
+      if (__all_sync(FULL, exhausted && !have)) break;
       asm volatile("" ::: "memory");   // refill stores to the schedule before the steps' loads
     }
 #pragma unroll kStepUnroll
@@ -606,6 +705,9 @@ static cudaError_t launch_dfs_t(const DfsLaunch& L, cudaStream_t st) {
   a.sroot = L.sroot; a.sinfo = L.sinfo;
   a.m = L.m; a.order = L.order; a.cursor = L.cursor; a.job_totals = L.job_totals; a.job_base = L.job_base;
   a.per_task = L.per_task; a.err = L.err; a.maxt = L.maxt;
+  const int64_t warps = (int64_t)grid * (BLOCK / 32);
+  a.chunk = (unsigned)std::min<int64_t>(32, (L.m + warps - 1) / warps);
+  a.share = 1.0f / (kChunkShare * (float)warps);
   dfs_kernel<WIDE, BLOCK, BIG><<<grid, BLOCK, smem, st>>>(a);
   return cudaGetLastError();
 }

@@ -86,7 +86,8 @@ extern "C" int nq_exec_solutions_noalloc(int N, const nq_record* d_records, int6
     ta.sched = (void*)(c + kCtrlBytes + kRootBytes + kInfoBytes);
     ta.sw = maxt + 1;
     ta.wide = false;
-    if (launch_prepare(N, m, (const uint4*)d_records, ta, 0, 0, err, st) != cudaSuccess) return NQ_ECUDA;
+    if (launch_prepare(N, m, (const uint4*)d_records, ta, 0, 0, err, st, nullptr,
+                       (unsigned long long*)d_solutions) != cudaSuccess) return NQ_ECUDA;
     DfsLaunch L;
     L.tasks = ta; L.m = m; L.cursor = cursor; L.job_totals = totals;
     L.per_task = (unsigned long long*)d_solutions; L.err = err; L.maxt = maxt; L.block = 128; L.grid = 0;

@@ -105,3 +105,25 @@ def test_short_lists_per_record(nq, oracle_mod, N, m, split):
             assert total == int(want.sum())
     finally:
         eng.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not gpu_available(), reason="needs a CUDA GPU")
+@pytest.mark.parametrize("grid", [1, 3, 0])
+@pytest.mark.parametrize("m", [1, 31, 1000])
+def test_shared_work_counts_every_solution_once(nq, oracle_mod, m, grid):
+    """Few large items: lanes of a warp give parts of them to each other (grid 1 and 3: the pool is refilled in
+    chunks too).  Every record's count, in which several lanes take part, equals the oracle's."""
+    N = 15
+    o, rec = _oracle_records(nq, oracle_mod, N, 4)
+    at = np.sort(np.random.default_rng(m).choice(len(rec), m, replace=False))
+    want = oracle_mod.exec_solutions(N, oracle_mod.Records(o.ld[at], o.rd[at], o.col[at], o.startijkl[at]))
+    eng = nq.Engine(0, auto_tune=False)
+    try:
+        for split in (0, 2):
+            eng.set_config(64, grid, split)
+            total, sol = eng.exec_records(N, np.ascontiguousarray(rec[at]), want_solutions=True)
+            assert np.array_equal(sol, want), (m, grid, split)
+            assert total == int(want.sum())
+    finally:
+        eng.close()
