@@ -115,6 +115,7 @@ struct nq_handle {
     if (bytes <= h_ctrl_cap) return NQ_OK;
     if (h_ctrl) cudaFreeHost(h_ctrl);
     h_ctrl = nullptr; h_ctrl_cap = 0;
+    bytes = std::max<size_t>(bytes, 4096);
     cudaError_t e = cudaMallocHost((void**)&h_ctrl, bytes);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMallocHost");
     h_ctrl_cap = bytes;

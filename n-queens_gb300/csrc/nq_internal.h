@@ -74,4 +74,17 @@ int dfs_blocks_per_sm(bool wide, int block, int maxt);
 cudaError_t int_peak(int kind, int iters, int grid, uint32_t* out, cudaStream_t st);
 size_t dfs_smem_bytes(bool wide, int block, int maxt);
 
+#ifdef __CUDACC__
+// position of the r-th set bit of m (r < popc(m))
+__device__ __forceinline__ uint32_t nth_set(uint32_t m, uint32_t r) {
+  uint32_t pos = 0;
+#pragma unroll
+  for (uint32_t w = 16; w; w >>= 1) {
+    const uint32_t c = __popc(m & ((1u << w) - 1u));
+    if (r >= c) { r -= c; m >>= w; pos += w; }
+  }
+  return pos;
+}
+#endif
+
 }  // namespace nq

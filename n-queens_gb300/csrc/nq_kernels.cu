@@ -487,17 +487,6 @@ __device__ __forceinline__ uint4 lds_frame(uint32_t a) {
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(f.x), "=r"(f.y), "=r"(f.z), "=r"(f.w) : "r"(a) : "memory");
   return f;
 }
-// position of the r-th set bit of m (r < popc(m))
-__device__ __forceinline__ uint32_t nth_set(uint32_t m, uint32_t r) {
-  uint32_t pos = 0;
-#pragma unroll
-  for (uint32_t w = 16; w; w >>= 1) {
-    const uint32_t c = __popc(m & ((1u << w) - 1u));
-    if (r >= c) { r -= c; m >>= w; pos += w; }
-  }
-  return pos;
-}
-
 template <bool WIDE, int BLOCK, bool BIG>
 __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
   using W = typename WordT<WIDE>::type;

@@ -13,15 +13,16 @@
 //     x2, x4 or x8 or dropped as a non-canonical copy (symmetryops, :65-125).
 // Unique = c2 + c4 + c8, total = 2 c2 + 4 c4 + 8 c8.
 //
-// The host expands the first rows of every (part, bound1) start into tasks;
-// the kernel is persistent, queue-fed and explicit-stack like the
-// constellation DFS (one candidate per lane per step, predicated pop/push,
-// the row carried in `down`'s high bits), keeping each lane's board (one bit
-// per row) in shared memory for the leaf classification.
+// The first rows of every (part, bound1) start are expanded on the device, a
+// row per launch, into the task queue (unique_init_kernel,
+// unique_expand_kernel).  unique_kernel is persistent, queue-fed and
+// explicit-stack like the constellation DFS (one candidate per lane per step,
+// predicated pop/push, the row carried in `down`'s high bits, work shared in a
+// warp at the end of the queue), keeping each lane's board (one bit per row)
+// in shared memory for the leaf classification.
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <vector>
 
 #include "../../include/nqueens_gb300.h"
 #include "nq_common.cuh"
@@ -32,8 +33,10 @@ namespace nq {
 namespace {
 
 constexpr unsigned FULLM = 0xFFFFFFFFu;
-constexpr int kBoardWords = 8;   // rows of the board prefix carried by a task
+constexpr int kBoardRows = 8;    // rows of the board prefix carried by a task
 constexpr int kUniqueSteps = 16;   // steps per lane between checks for finished lanes
+constexpr int kReadBackN = 14;     // boards from here on size the stacks to the tasks' rows
+constexpr uint32_t kGiveRows = 5;   // rows below a frame worth giving away
 
 // One start configuration (symmetry part and its bounds).
 struct UConf {
@@ -41,12 +44,19 @@ struct UConf {
   uint32_t bound1, bound2, endbit, lastmask, sidemask, topbit;
 };
 
-// A task: the search state at `row` plus the board rows above it.
-struct UTask {
+// A task: the search state at `row` plus the board rows above it (one byte each, the queen's column), 32 bytes.
+struct __align__(16) UTask {
   uint32_t left, down, right, avail;
   uint32_t row, conf;
-  uint32_t board[kBoardWords];
+  uint32_t board[kBoardRows / 4];
 };
+__device__ __forceinline__ uint32_t board_bit(const UTask& t, uint32_t r) {   // row r's queen as a bit
+  return 1u << ((t.board[r >> 2] >> (8u * (r & 3u))) & 31u);
+}
+__device__ __forceinline__ void board_set(UTask& t, uint32_t r, uint32_t bit) {
+  const uint32_t v = (31u - (uint32_t)__clz((int)bit)) << (8u * (r & 3u));
+  if (r < 4u) t.board[0] |= v; else t.board[1] |= v;
+}
 
 // symmetryops (07Py_bit_symmetry.py:65-125): 2, 4 or 8 for a canonical
 // solution, 0 for a rotated copy.  `b(k)` reads board row k.
@@ -101,15 +111,29 @@ __host__ __device__ __forceinline__ uint32_t row_filter(uint32_t bitmap, uint32_
   return bitmap;
 }
 
+// Control block: counts, queue cursor, states after each expanded row.
+constexpr int kLevels = kBoardRows - 2;   // expanded rows at most: from row 1, and a task carries the rows above its own
+struct UCtl {
+  unsigned long long c2, c4, c8;
+  unsigned int cursor, pad;
+  unsigned int n[kLevels + 1];
+};
+// The queue is the last level with states in it that its buffer holds (levels alternate between two
+// buffers; a level that was large enough, or whose states all died, leaves the next one empty).
+__host__ __device__ __forceinline__ int queue_level(const UCtl* c, unsigned cap) {
+  int f = 0;
+  for (int l = 1; l <= kLevels; l++)
+    if (c->n[l] && c->n[l] <= cap) f = l;
+  return f;
+}
+
 struct UArgs {
-  const UTask* tasks;
+  const UTask* tasks[2];
   const UConf* confs;
-  int64_t m;
   int N;
   int maxf;                     // stack frames per lane: N - 2 - (smallest task row)
-  unsigned int* cursor;
-  unsigned long long* counts;   // c2, c4, c8
-  unsigned int* err;
+  unsigned cap;                 // tasks a buffer holds
+  UCtl* ctl;
 };
 
 // Predicated shared-memory stores (32-bit shared-window addresses), so the push is
@@ -121,6 +145,15 @@ __device__ __forceinline__ void sts_frame_if(uint32_t p, uint32_t a, uint32_t x,
 __device__ __forceinline__ void sts_word_if(uint32_t p, uint32_t a, uint32_t x) {
   asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q st.shared.u32 [%1], %2;\n\t}"
                :: "r"(p), "r"(a), "r"(x) : "memory");
+}
+
+__device__ __forceinline__ uint32_t lds_word_u(uint32_t a) {
+  uint32_t w;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"(a) : "memory");
+  return w;
+}
+__device__ __forceinline__ void lds_frame_u(uint32_t a, uint32_t& x, uint32_t& y, uint32_t& z, uint32_t& w) {
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(x), "=r"(y), "=r"(z), "=r"(w) : "r"(a) : "memory");
 }
 
 // One lane per task, one candidate per step, all lanes on the same predicated
@@ -137,7 +170,8 @@ __global__ void __launch_bounds__(BLOCK) unique_kernel(const UArgs a) {
   // a lane pushes at most one frame per row from its task's row to N - 3
   uint4* stk = reinterpret_cast<uint4*>(smem) + threadIdx.x;                            // maxf frames, stride BLOCK
   uint32_t* brd = reinterpret_cast<uint32_t*>(smem + (size_t)a.maxf * BLOCK * sizeof(uint4)) + threadIdx.x;  // N rows
-  const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(stk);
+  const uint32_t bottom = (uint32_t)__cvta_generic_to_shared(stk);
+  uint32_t sbase = bottom;            // moves up when the lane gives its bottom frame away
   const uint32_t bbase = (uint32_t)__cvta_generic_to_shared(brd);
   const unsigned lane = threadIdx.x & 31u;
   const uint32_t mask = (1u << N) - 1u;
@@ -145,32 +179,74 @@ __global__ void __launch_bounds__(BLOCK) unique_kernel(const UArgs a) {
   uint32_t left = 0, down = 0, right = 0, avail = 0, sp = sbase;
   UConf cf = {0, 0, 0, 0, 0, 0, 0};
   uint32_t lowmask = ~0u, b2 = ~0u;      // row rules of the task's part
+  // part 1: rows above bound1 avoid column 1; part 2: they avoid the side
+  // columns, and row bound2 is gated on the side columns used so far
+  auto load_conf = [&](const UConf& c) {
+    cf = c;
+    lowmask = (cf.part == 1) ? ~2u : ~cf.sidemask;
+    b2 = (cf.part == 1) ? ~0u : cf.bound2;
+  };
   unsigned long long c2 = 0, c4 = 0, c8 = 0;
   bool exhausted = false;
+  const int level = queue_level(a.ctl, a.cap);
+  const UTask* __restrict__ tasks = a.tasks[level & 1];
+  const unsigned m = a.ctl->n[level];
+  // where the queue is smaller than the lanes, each warp takes its share and shares it among its lanes
+  const unsigned warps = gridDim.x * (BLOCK / 32);
+  const unsigned take = min(32u, (m + warps - 1u) / warps);
+  uint32_t conf_ix = 0;
   for (;;) {
     const bool idle = (avail | (sp - sbase)) == 0u;
     if (__ballot_sync(FULLM, idle)) {
+      if (idle) sbase = sp = bottom;
       const bool want = idle && !exhausted;
       const unsigned need = __ballot_sync(FULLM, want);
       if (need) {
-        const int leader = __ffs(need) - 1;
+        const unsigned n_take = min((unsigned)__popc(need), take);
         unsigned base = 0;
-        if ((int)lane == leader) base = atomicAdd(a.cursor, (unsigned)__popc(need));
-        base = __shfl_sync(FULLM, base, leader);
-        if (want) {
-          const uint64_t slot = (uint64_t)base + (uint64_t)__popc(need & ((1u << lane) - 1u));
-          if (slot < (uint64_t)a.m) {
-            const UTask t = a.tasks[slot];
-            cf = a.confs[t.conf];
-            // part 1: rows above bound1 avoid column 1; part 2: they avoid the side
-            // columns, and row bound2 is gated on the side columns used so far
-            lowmask = (cf.part == 1) ? ~2u : ~cf.sidemask;
-            b2 = (cf.part == 1) ? ~0u : cf.bound2;
-            left = t.left; down = (t.down & mask) | (t.row << 27); right = t.right; avail = t.avail; sp = sbase;
-            for (uint32_t r = 0; r < t.row && r < (uint32_t)kBoardWords; r++) brd[r * BLOCK] = t.board[r];
-          } else {
-            exhausted = true;
+        if (lane == 0 && n_take) base = atomicAdd(&a.ctl->cursor, n_take);
+        base = __shfl_sync(FULLM, base, 0);
+        const unsigned rank = __popc(need & ((1u << lane) - 1u));
+        if (want && rank < n_take && base + rank < m) {
+          const UTask t = tasks[base + rank];
+          conf_ix = t.conf;
+          load_conf(a.confs[conf_ix]);
+          left = t.left; down = (t.down & mask) | (t.row << 27); right = t.right; avail = t.avail;
+          for (uint32_t r = 0; r < t.row && r < (uint32_t)kBoardRows; r++) brd[r * BLOCK] = board_bit(t, r);
+        }
+        exhausted = take < 32u || base + n_take >= m;   // warp-uniform
+      }
+      if (exhausted) {
+        // The queue is empty: a lane without work takes the bottom saved frame of a busy lane of its warp,
+        // or all but one candidate of its current frame, with the rows of the board above it.
+        const bool busy = avail != 0u || sp != sbase;
+        const unsigned starved = __ballot_sync(FULLM, !busy);
+        const bool saved = sp != sbase;
+        const uint32_t rest = avail & (avail - 1u);
+        const uint32_t gdown = saved ? lds_word_u(sbase + 4u) : down;
+        const bool can = busy && (saved ? (avail != 0u || sp != sbase + F) : rest != 0u) &&
+                         (gdown >> 27) + kGiveRows <= last_row;
+        const unsigned givers = starved ? __ballot_sync(FULLM, can) : 0u;
+        if (givers) {
+          const unsigned lt = (1u << lane) - 1u;
+          const int n = min(__popc(starved), __popc(givers));
+          const bool gives = can && __popc(givers & lt) < n;
+          const int srank = __popc(starved & lt);
+          const bool takes = !busy && srank < n;
+          if (gives && !saved) { sts_frame_if(1u, sbase, left, down, right, rest); avail ^= rest; }
+          __syncwarp();
+          const int src = takes ? (int)nth_set(givers, (uint32_t)srank) : (int)lane;
+          const uint32_t from = __shfl_sync(FULLM, sbase, src), fconf = __shfl_sync(FULLM, conf_ix, src);
+          const uint32_t fbrd = __shfl_sync(FULLM, bbase, src);
+          if (takes) {
+            lds_frame_u(from, left, down, right, avail);
+            conf_ix = fconf;
+            load_conf(a.confs[conf_ix]);
+            const uint32_t rows = down >> 27;
+            for (uint32_t r = 0; r < rows; r++) brd[r * BLOCK] = lds_word_u(fbrd + r * RB);
           }
+          __syncwarp();
+          if (gives && saved) sbase += F;
         }
       }
       if (__all_sync(FULLM, exhausted && (avail | (sp - sbase)) == 0u)) break;
@@ -223,80 +299,105 @@ __global__ void __launch_bounds__(BLOCK) unique_kernel(const UArgs a) {
     c8 += __shfl_xor_sync(FULLM, c8, o);
   }
   if (lane == 0) {
-    if (c2) atomicAdd(a.counts + 0, c2);
-    if (c4) atomicAdd(a.counts + 1, c4);
-    if (c8) atomicAdd(a.counts + 2, c8);
+    if (c2) atomicAdd(&a.ctl->c2, c2);
+    if (c4) atomicAdd(&a.ctl->c4, c4);
+    if (c8) atomicAdd(&a.ctl->c8, c8);
   }
 }
 
-// Host: every (part, bound1) start of 07Py_bit_symmetry.py NQueens() (:171-200),
-// expanded breadth-first over its first rows until there are enough tasks.
-int build_unique_tasks(int N, int64_t min_tasks, std::vector<UConf>& confs, std::vector<UTask>& tasks) {
-  const uint32_t mask = (1u << N) - 1u;
-  // Search states are kept in the task layout itself (avail is filled in at the
-  // end), so the last level becomes the task list without another copy.
-  std::vector<UTask> cur;
-  // part 1: corner queen
-  for (int b1 = 2; b1 < N - 1; b1++) {
-    UConf c = {1, (uint32_t)b1, 0, 0, 0, 0, 1u << (N - 1)};
-    confs.push_back(c);
-    const uint32_t bit = 1u << b1;
-    UTask s{};
+// ---------------------------------------------------------------------------
+// Task queue: every (part, bound1) start of 07Py_bit_symmetry.py NQueens()
+// (:171-200), expanded a whole row at a time (tasks of one row are of similar
+// size) until there are enough tasks, they reach the last row, or their rows
+// no longer fit the board prefix.  Bound by launch latency: about 2 us a row
+// at N=12; the same expansion on one host thread and its upload took 0.8 ms at
+// N=12, 6 ms at N=14 and 25 ms at N=16.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ UConf make_conf(int N, int i) {
+  const uint32_t topbit = 1u << (N - 1);
+  const int n1 = N - 3;                                 // part 1: bound1 = 2..N-2
+  if (i < n1) return UConf{1, (uint32_t)(i + 2), 0, 0, 0, 0, topbit};
+  const int k = i - n1;                                 // part 2: bound1 = 1.., bound2 = N-1-bound1
+  const uint32_t sidemask = topbit | 1u;
+  uint32_t lastmask = sidemask;
+  for (int q = 0; q < k; q++) lastmask = (lastmask << 1) | lastmask | (lastmask >> 1);
+  return UConf{2, (uint32_t)(k + 1), (uint32_t)(N - 2 - k), topbit >> (k + 1), lastmask, sidemask, topbit};
+}
+
+__device__ __forceinline__ uint32_t candidates(const UTask& t, uint32_t mask, const UConf& c) {
+  return row_filter(mask & ~(t.left | t.down | t.right), t.row, t.down, c);
+}
+
+__global__ void __launch_bounds__(64) unique_init_kernel(int N, int nconf, UConf* confs, UTask* tasks, UCtl* ctl) {
+  const int i = threadIdx.x;
+  if (i < (int)(sizeof(UCtl) / 4)) reinterpret_cast<unsigned int*>(ctl)[i] = 0;
+  __syncthreads();
+  if (i >= nconf) return;
+  const UConf c = make_conf(N, i);
+  confs[i] = c;
+  const uint32_t bit = 1u << c.bound1;
+  UTask s{};
+  s.conf = (uint32_t)i;
+  if (c.part == 1) {
     s.left = (2u | bit) << 1; s.down = 1u | bit; s.right = (2u | bit) >> 1; s.row = 2;
-    s.board[0] = 1; s.board[1] = bit; s.conf = (uint32_t)confs.size() - 1;
-    cur.push_back(s);
+    board_set(s, 0, 1u); board_set(s, 1, bit);
+  } else {
+    s.left = bit << 1; s.down = bit; s.right = bit >> 1; s.row = 1;
+    board_set(s, 0, bit);
   }
-  // part 2: no corner queen
-  {
-    const uint32_t topbit = 1u << (N - 1);
-    uint32_t endbit = topbit >> 1, lastmask = topbit | 1u;
-    const uint32_t sidemask = topbit | 1u;
-    for (int b1 = 1, b2 = N - 2; b1 > 0 && b2 < N - 1 && b1 < b2; b1++, b2--) {
-      UConf c = {2, (uint32_t)b1, (uint32_t)b2, endbit, lastmask, sidemask, topbit};
-      confs.push_back(c);
-      const uint32_t bit = 1u << b1;
-      UTask s{};
-      s.left = bit << 1; s.down = bit; s.right = bit >> 1; s.row = 1; s.board[0] = bit;
-      s.conf = (uint32_t)confs.size() - 1;
-      cur.push_back(s);
-      endbit >>= 1;
-      lastmask = (lastmask << 1) | lastmask | (lastmask >> 1);
-    }
-  }
-  // expand whole rows breadth-first (tasks of one row are of similar size) while
-  // the tasks stay above the last row and fit the board prefix
-  std::vector<UTask> nxt;
-  while ((int64_t)cur.size() < min_tasks) {
-    bool grew = false;
-    nxt.clear();
-    nxt.reserve(cur.size() * (size_t)N);
-    for (const UTask& s : cur) {
-      if ((int)s.row + 1 >= N - 1 || s.row + 1 >= (uint32_t)kBoardWords) { nxt.push_back(s); continue; }
-      uint32_t bm = row_filter(mask & ~(s.left | s.down | s.right), s.row, s.down, confs[s.conf]);
-      while (bm) {
+  s.avail = candidates(s, (1u << N) - 1u, c);
+  if (s.avail) tasks[atomicAdd(&ctl->n[0], 1u)] = s;
+}
+
+// Level l -> l + 1: one thread per state; its children with candidates left are counted, the warp reserves
+// their slots with one atomic, and they are written.  States that must not be expanded move on as they are.
+// n[l] <= 2^32: a level below the target (at most 2^21 states) has at most 27 children a state.
+__global__ void __launch_bounds__(128) unique_expand_kernel(int N, int level, unsigned target, unsigned cap, const UConf* __restrict__ confs,
+                                                            const UTask* __restrict__ in, UTask* __restrict__ out,
+                                                            UCtl* ctl) {
+  const unsigned n = ctl->n[level];
+  if (n >= target) return;
+  const uint32_t mask = (1u << N) - 1u;
+  const unsigned lane = threadIdx.x & 31u;
+  for (unsigned i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
+    const unsigned i = i0 + threadIdx.x;
+    UTask s{};
+    UConf c{};
+    bool keep = false;
+    unsigned cnt = 0;
+    auto each_child = [&](auto&& f) {
+      for (uint32_t bm = s.avail; bm;) {
         const uint32_t bit = bm & (0u - bm);
         bm ^= bit;
         UTask t = s;
-        t.board[s.row] = bit;
         t.left = (s.left | bit) << 1; t.down = s.down | bit; t.right = (s.right | bit) >> 1; t.row = s.row + 1;
-        nxt.push_back(t);
-        grew = true;
+        t.avail = candidates(t, mask, c);
+        if (t.avail) f(t, bit);
       }
+    };
+    if (i < n) {
+      s = in[i];
+      c = confs[s.conf];
+      keep = (int)s.row + 1 >= N - 1 || s.row + 1 >= (uint32_t)kBoardRows;
+      if (keep) cnt = 1;
+      else each_child([&](const UTask&, uint32_t) { cnt++; });
     }
-    cur.swap(nxt);
-    if (!grew) break;
+    unsigned incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned v = __shfl_up_sync(FULLM, incl, o);
+      if ((int)lane >= o) incl += v;
+    }
+    unsigned base = 0;
+    if (lane == 31 && incl) base = atomicAdd(&ctl->n[level + 1], incl);
+    base = __shfl_sync(FULLM, base, 31) + incl - cnt;
+    if (base + cnt > cap) continue;      // the level does not fit: the queue stays the level before it
+    if (keep) out[base] = s;
+    else if (cnt) each_child([&](UTask& t, uint32_t bit) {
+      board_set(t, s.row, bit);
+      out[base++] = t;
+    });
   }
-  // each state's candidate set; states without one are dropped (in place)
-  size_t k = 0;
-  for (size_t q = 0; q < cur.size(); q++) {
-    UTask& t = cur[q];
-    t.avail = row_filter(mask & ~(t.left | t.down | t.right), t.row, t.down, confs[t.conf]);
-    if (t.avail) cur[k++] = t;
-  }
-  cur.resize(k);
-  if (tasks.empty()) tasks.swap(cur);
-  else tasks.insert(tasks.end(), cur.begin(), cur.end());
-  return 0;
 }
 
 }  // namespace
@@ -312,48 +413,51 @@ extern "C" int nq_count_unique(nq_handle* h, int N, uint64_t* unique, uint64_t* 
   NQ_CUDA(h, cudaSetDevice(h->device));
   const int dev = h->device, sms = h->sms;
   cudaStream_t st = h->stream;
-  std::vector<UConf> confs;
-  std::vector<UTask> tasks;
-  // About 8 tasks per resident lane (the kernel keeps ~512 lanes per SM): fewer
-  // leave a tail at N=20 (+35 % with 4 per lane), more cost host time (N=19:
-  // 0.66 s with 32 per lane against 0.48 s, the same kernel time).
-  build_unique_tasks(N, (int64_t)sms * 2048 * 2, confs, tasks);
-  const int64_t m = (int64_t)tasks.size();
-  uint32_t min_row = (uint32_t)N;
-  for (const UTask& t : tasks) min_row = std::min(min_row, t.row);
-  const int maxf = std::max(1, N - 2 - (int)min_row);
+  const int nconf = (N - 3) + (N - 2) / 2;      // part 1: bound1 2..N-2; part 2: bound1 < N - 1 - bound1
+  // Rows are expanded until the queue holds `target` tasks, unless the next row does not fit the buffer.
+  // Lanes share work within a warp only, so the warps' sums have to even out: us of a whole count on GB300
+  // with a target of 512 / 1024 / 4096 tasks per SM, N=15 303 / 303 / 227, N=16 921 / 936 / 736, N=17 11323 /
+  // 4154 / 4204, N=18 56174 / 59898 / 27268 (5 10^5 tasks against 4.9 10^6).
+  const unsigned target = (unsigned)sms * (N <= 15 ? 1024u : N <= 17 ? 4096u : 13824u);
+  const size_t cap = (size_t)target * 5;
+  NQ_CUDA(h, h->utasks.ensure(2 * cap * sizeof(UTask)));
+  NQ_CUDA(h, h->uconfs.ensure((size_t)nconf * sizeof(UConf)));
+  NQ_CUDA(h, h->uctl.ensure(sizeof(UCtl)));
+  UCtl* ctl = (UCtl*)h->uctl.p;
+  UConf* confs = (UConf*)h->uconfs.p;
+  UTask* buf[2] = {(UTask*)h->utasks.p, (UTask*)h->utasks.p + cap};
+  unique_init_kernel<<<1, 64, 0, st>>>(N, nconf, confs, buf[0], ctl);
+  const int levels = N <= 9 ? 1 : std::min(kLevels, N - 3);   // N <= 9: a launch costs more than it balances
+  for (int l = 0; l < levels; l++)
+    unique_expand_kernel<<<l < 2 ? 1 : l == 2 ? sms : 4 * sms, 128, 0, st>>>(N, l, target, (unsigned)cap, confs, buf[l & 1],
+                                                                            buf[(l + 1) & 1], ctl);
+  NQ_CUDA(h, cudaGetLastError());
+  if (int s = h->ensure_pinned(sizeof(UCtl))) return s;
+  // Stacks sized to the tasks' rows need the level reached (one read-back); boards whose search takes less
+  // than the wait run with the largest stacks.
+  int row = 1;
+  if (N >= kReadBackN) {
+    NQ_CUDA(h, cudaMemcpyAsync(h->h_ctrl, ctl, sizeof(UCtl), cudaMemcpyDeviceToHost, st));
+    NQ_CUDA(h, cudaStreamSynchronize(st));
+    row = 1 + queue_level((const UCtl*)h->h_ctrl, (unsigned)cap);
+  }
+  const int maxf = std::max(1, N - 2 - row);
   constexpr int B = 128;
   const size_t smem = (size_t)B * ((size_t)maxf * sizeof(uint4) + (size_t)N * sizeof(uint32_t));
-  NQ_CUDA(h, h->utasks.ensure(std::max<size_t>(1, (size_t)m * sizeof(UTask))));
-  NQ_CUDA(h, h->uconfs.ensure(std::max<size_t>(1, confs.size() * sizeof(UConf))));
-  NQ_CUDA(h, h->uctl.ensure(64));
-  unsigned char* ctl = (unsigned char*)h->uctl.p;
-  NQ_CUDA(h, cudaMemsetAsync(ctl, 0, 64, st));
-  if (m > 0) NQ_CUDA(h, cudaMemcpyAsync(h->utasks.p, tasks.data(), (size_t)m * sizeof(UTask), cudaMemcpyHostToDevice, st));
-  if (!confs.empty())
-    NQ_CUDA(h, cudaMemcpyAsync(h->uconfs.p, confs.data(), confs.size() * sizeof(UConf), cudaMemcpyHostToDevice, st));
-  if (m > 0) {
-    int optin = 0;   // the cap is process-wide: set it to the device maximum, never to one launch's size
-    NQ_CUDA(h, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    NQ_CUDA(h, cudaFuncSetAttribute(unique_kernel<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-    int per = 0;
-    NQ_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, unique_kernel<B>, B, smem));
-    if (per <= 0) return h->fail(NQ_ECUDA, "count_unique: N=%d does not fit on an SM", N);
-    UArgs a;
-    a.tasks = (const UTask*)h->utasks.p; a.confs = (const UConf*)h->uconfs.p; a.m = m; a.N = N; a.maxf = maxf;
-    a.counts = (unsigned long long*)ctl; a.cursor = (unsigned int*)(ctl + 32);
-    a.err = (unsigned int*)(ctl + 36);
-    unique_kernel<B><<<sms * per, B, smem, st>>>(a);
-    NQ_CUDA(h, cudaGetLastError());
-  }
-  // the host task vectors stay alive until the stream has consumed them (synchronised below)
-  if (int s = h->ensure_pinned(64)) return s;
-  NQ_CUDA(h, cudaMemcpyAsync(h->h_ctrl, ctl, 64, cudaMemcpyDeviceToHost, st));
+  int optin = 0;   // the cap is process-wide: set it to the device maximum, never to one launch's size
+  NQ_CUDA(h, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  NQ_CUDA(h, cudaFuncSetAttribute(unique_kernel<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+  int per = 0;
+  NQ_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, unique_kernel<B>, B, smem));
+  if (per <= 0) return h->fail(NQ_ECUDA, "count_unique: N=%d does not fit on an SM", N);
+  UArgs a;
+  a.tasks[0] = buf[0]; a.tasks[1] = buf[1]; a.confs = confs; a.N = N; a.maxf = maxf; a.cap = (unsigned)cap; a.ctl = ctl;
+  unique_kernel<B><<<sms * per, B, smem, st>>>(a);
+  NQ_CUDA(h, cudaGetLastError());
+  NQ_CUDA(h, cudaMemcpyAsync(h->h_ctrl, ctl, sizeof(UCtl), cudaMemcpyDeviceToHost, st));
   NQ_CUDA(h, cudaStreamSynchronize(st));
-  const unsigned long long* hc = (const unsigned long long*)h->h_ctrl;
-  const uint32_t herr = ((const uint32_t*)h->h_ctrl)[9];
-  if (herr) return h->fail(NQ_EINVAL, "count_unique: device error word %u", herr);
-  *unique = hc[0] + hc[1] + hc[2];
-  *total = 2 * hc[0] + 4 * hc[1] + 8 * hc[2];
+  const UCtl* hc = (const UCtl*)h->h_ctrl;
+  *unique = hc->c2 + hc->c4 + hc->c8;
+  *total = 2 * hc->c2 + 4 * hc->c4 + 8 * hc->c8;
   return NQ_OK;
 }
