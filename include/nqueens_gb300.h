@@ -120,7 +120,8 @@ int nq_last_run_info(const nq_handle *h, int *split_depth, int64_t *queued);
  * scratch is one fixed __device__ array of about 15 MiB inside the library,
  * held by every GPU that loads it until exit.  Limit: m <= 131072 records and
  * schedules up to 24 depths (N - start_min <= 25); larger inputs are rejected
- * with NQ_EINVAL, never truncated.  No task splitting.  The first call on each
+ * with NQ_EINVAL, never truncated.  Tasks are split as far as the array holds
+ * the queue; one that does not fit is counted unsplit.  The first call on each
  * device looks the array's address up (cudaGetSymbolAddress) with that device
  * current; with lazy module loading that first call is also when the array
  * and the kernels are loaded onto the device, so make it once at start-up --

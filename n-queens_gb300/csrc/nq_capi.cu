@@ -52,25 +52,6 @@ const char* derr_text(uint32_t e) {
   return "ok";
 }
 
-// Levels every task is expanded by before the DFS.  `rows`: rows left below the shallowest start (N - 2 -
-// start row), which sets a task's work (about 7x per row).  Lanes of a warp share their work at the end of
-// the queue, so splitting only has to even out the warps and give a short list more items than lanes:
-// us of a whole call on GB300 at D = 0 / 1 / 2 / 3, m tasks:
-//   8 rows (N=12):    m=4300   81 / 83 / 85 / 110
-//   10 rows (N=14):   m=13233 125 / 117 / 121 / 182
-//   11 rows (N=15):   m=21270 187 / 168 / 179 / 293
-//   12 rows (N=16):   m=4000  190 / 177 / 182 / 286   m=33046   602 / 448 / 407 / 585
-//   13 rows (N=18):   m=16000 900 / 738 / 527 / 668   m=200000 5634 / 4121 / 4407 / 5657
-//   14 rows (N=19):   m=50000 10.1 / 5.5 / 4.8 / 5.3 ms   m=897071 80.7 / 74.1 / 78.8 ms
-//   15 rows (N=20):   m=4000  9.1 / 5.5 / 3.2 / 2.6 ms
-// Each level makes about 7 times the items (measured: 6.2x at N=16 to 8x at N=20), and an item costs its
-// loading; lists of 10^5 tasks and more are balanced at D = 1.
-int choose_split(int64_t m, int rows) {
-  if (rows <= 9) return 0;
-  if (rows <= 11 || m > 100000) return m > 400000000 ? 0 : 1;   // ~7 subtasks a task stay within the u32 subtask queue
-  return rows >= 15 && m < 8192 ? 3 : 2;
-}
-
 // Records per chunk of a whole-board count (nq_count): one chunk up to N=21
 // (2.0 M records), four at N=22 (28.7 M), about 32 MB of host records each.
 constexpr int64_t kChunkRecords = 8 << 20;
@@ -87,66 +68,82 @@ int maxt_for(int N, int start_min) {
 namespace {
 
 
-// records (device) -> counts on st; totals land in ctrl[0].  Launches
-// prepare, then (when splitting) the split count pass, one read-back of the
-// control block (subtask count and deepest schedule), the split write pass,
-// and the DFS with a stack sized to the deepest subtask.
+// Lists up to this length run without a read-back between the launches: the DFS takes the queue's length
+// from the device and stacks for the deepest task the start rows allow.  Longer ones read the queue's length
+// and the deepest schedule first (about 15 us), which buys a tighter stack (more resident warps).
+constexpr int64_t kNoReadBack = 16384;
+constexpr int64_t kQueueBytes = 256 << 20;   // queue buffer a short list may bound its queue by
+
+// records (device) -> counts on st; totals land in ctrl[0].  One launch prepares and splits, one counts.
+// maxt: the deepest schedule of any record (rows left below the shallowest start).
 int run_records(nq_handle* h, int N, const uint4* d_rec, int64_t m, int start_min, unsigned long long* d_per_task,
                 cudaStream_t st) {
   const int maxt = maxt_for(N, start_min);
-  const int sw = maxt + 1;
-  NQ_CUDA(h, cudaSetDevice(h->device));
-  NQ_CUDA(h, h->root.ensure((size_t)m * sizeof(uint4)));
-  NQ_CUDA(h, h->info.ensure((size_t)m * sizeof(uint2)));
-  NQ_CUDA(h, h->sched.ensure((size_t)m * sw * sizeof(uint32_t)));
-  NQ_CUDA(h, h->ctrl.ensure(ctl::kBytes));
-  unsigned char* c = (unsigned char*)h->ctrl.p;
-  NQ_CUDA(h, cudaMemsetAsync(c, 0, ctl::kBytes, st));
-  TaskArrays ta;
-  ta.root = (uint4*)h->root.p; ta.info = (uint2*)h->info.p; ta.sched = h->sched.p; ta.sw = sw; ta.wide = false;
-  unsigned long long* totals = (unsigned long long*)(c + ctl::kTotal);
-  unsigned long long* cursor = (unsigned long long*)(c + ctl::kCursor);
-  unsigned int* err = (unsigned int*)(c + ctl::kErr);
-  unsigned long long* sctr = (unsigned long long*)(c + ctl::kSplit);   // split: [0] subtasks, [1] allocation cursor
-  unsigned int* tmax = (unsigned int*)(c + ctl::kTmax);                 // deepest schedule of the launch
-  NQ_CUDA(h, cudaEventRecord(h->ev[0], st));
-  NQ_CUDA(h, launch_prepare(N, m, d_rec, ta, 0, 0, err, st, tmax, d_per_task));
   const int D = h->split >= 0 ? h->split : choose_split(m, maxt);
-  DfsLaunch L;
-  L.tasks = ta; L.m = m; L.order = nullptr; L.cursor = cursor; L.job_totals = totals;
-  L.per_task = d_per_task; L.err = err; L.maxt = maxt; L.block = h->block; L.grid = h->grid;
-  if (D > 0) {
-    NQ_CUDA(h, h->nsub.ensure((size_t)m * sizeof(uint32_t)));
-    NQ_CUDA(h, launch_split(0, D, 0, m, ta, (uint32_t*)h->nsub.p, nullptr, nullptr, sctr, nullptr, totals, 0, st));
-  }
-  // One read-back: the split size and the deepest schedule T.  Subtasks start
-  // at depth D with an empty stack, so the DFS needs T - D frames and T - D + 1
-  // schedule words per lane; the kernel still rejects any task deeper than that.
+  NQ_CUDA(h, cudaSetDevice(h->device));
+  NQ_CUDA(h, h->info.ensure((size_t)m * sizeof(uint2)));
+  NQ_CUDA(h, h->sched.ensure((size_t)m * (maxt + 1) * sizeof(uint32_t)));
+  NQ_CUDA(h, h->ctrl.ensure(ctl::kBytes));
   if (int s = h->ensure_pinned(ctl::kBytes)) return s;
-  NQ_CUDA(h, cudaMemcpyAsync(h->h_ctrl, c, ctl::kBytes, cudaMemcpyDeviceToHost, st));
-  NQ_CUDA(h, cudaStreamSynchronize(st));
-  const unsigned char* hc = (const unsigned char*)h->h_ctrl;
-  const int t_deep = (int)*(const uint32_t*)(hc + ctl::kTmax);
-  L.maxt = std::max(1, std::min(maxt, t_deep - D));
+  unsigned char* c = (unsigned char*)h->ctrl.p;
+  PrepareSplit P;
+  P.N = N; P.m = m; P.rec = d_rec; P.info = (uint2*)h->info.p; P.sched = (uint32_t*)h->sched.p; P.sw = maxt + 1;
+  P.err = (unsigned int*)(c + ctl::kErr); P.tmax = (unsigned int*)(c + ctl::kTmax);
+  P.per_task = d_per_task; P.qn = (unsigned long long*)(c + ctl::kSplit); P.total = (unsigned long long*)(c + ctl::kTotal);
+  // Queue capacity: a bound (each level places a queen in one of at most N - 2, N - 3, ... columns) where that
+  // is small, else 8 a level (measured: 6.2 to 8), built again if it was too small.
+  uint64_t bound = (uint64_t)m, guess = (uint64_t)m + 1024;
+  for (int d = 0; d < D; d++) { bound *= (uint64_t)(N - 2 - d); guess *= 8; }
+  const bool read_back = m > kNoReadBack || h->queue_order == 1 || (D > 0 && bound * 24 > (uint64_t)kQueueBytes);
   if (D > 0) {
-    const int64_t ns = (int64_t)*(const uint64_t*)(hc + ctl::kSplit);
-    if (ns > (int64_t)0xFFFFFFFF) return h->fail(NQ_ENOMEM, "split: %lld subtasks", (long long)ns);
-    NQ_CUDA(h, h->sroot.ensure((size_t)std::max<int64_t>(ns, 1) * sizeof(uint4)));
-    NQ_CUDA(h, h->sinfo.ensure((size_t)std::max<int64_t>(ns, 1) * sizeof(uint2)));
-    NQ_CUDA(h, launch_split(1, D, 0, m, ta, (uint32_t*)h->nsub.p, (uint4*)h->sroot.p, (uint2*)h->sinfo.p, sctr,
-                            d_per_task, totals, 0, st));
-    L.sroot = (const uint4*)h->sroot.p; L.sinfo = (const uint2*)h->sinfo.p; L.m = ns;
+    const uint64_t q = std::max(read_back ? std::min(bound, guess) : bound, (uint64_t)(h->sroot.cap / sizeof(uint4)));
+    NQ_CUDA(h, h->sroot.ensure((size_t)q * sizeof(uint4)));
+    NQ_CUDA(h, h->sinfo.ensure((size_t)q * sizeof(uint2)));
+  } else {
+    NQ_CUDA(h, h->root.ensure((size_t)m * sizeof(uint4)));
+    P.root = (uint4*)h->root.p;
   }
-  L.big = counts_need_u64(N, L.m);
+  DfsLaunch L;
+  L.tasks.root = (uint4*)h->root.p; L.tasks.info = P.info; L.tasks.sched = P.sched; L.tasks.sw = P.sw; L.tasks.wide = false;
+  L.cursor = (unsigned long long*)(c + ctl::kCursor); L.job_totals = P.total;
+  L.per_task = d_per_task; L.err = P.err; L.block = h->block; L.grid = h->grid;
+  L.m = m;
+  NQ_CUDA(h, cudaEventRecord(h->ev[0], st));
+  for (;;) {
+    P.sroot = (uint4*)h->sroot.p; P.sinfo = (uint2*)h->sinfo.p;
+    P.qcap = std::min(h->sroot.cap / sizeof(uint4), h->sinfo.cap / sizeof(uint2));
+    NQ_CUDA(h, cudaMemsetAsync(c, 0, ctl::kBytes, st));
+    NQ_CUDA(h, launch_prepare_split(D, m, P, st));
+    if (D > 0) { L.sroot = P.sroot; L.sinfo = P.sinfo; }
+    if (!read_back) {
+      if (D > 0) { L.m_dev = P.qn; L.qcap = P.qcap; }
+      L.maxt = std::max(1, maxt - D);
+      break;
+    }
+    // Subtasks start at depth D with an empty stack, so the DFS needs T - D frames and T - D + 1 schedule
+    // words per lane; the kernel still rejects any task deeper than that.
+    NQ_CUDA(h, cudaMemcpyAsync(h->h_ctrl, c, ctl::kBytes, cudaMemcpyDeviceToHost, st));
+    NQ_CUDA(h, cudaStreamSynchronize(st));
+    const unsigned char* hc = (const unsigned char*)h->h_ctrl;
+    L.maxt = std::max(1, std::min(maxt, (int)*(const uint32_t*)(hc + ctl::kTmax) - D));
+    if (D == 0) break;
+    const uint64_t ns = *(const uint64_t*)(hc + ctl::kSplit);
+    if (ns > 0xFFFFFFFFull) return h->fail(NQ_ENOMEM, "split: %llu subtasks", (unsigned long long)ns);
+    L.m = (int64_t)ns;
+    if (ns <= P.qcap) break;
+    NQ_CUDA(h, h->sroot.ensure((size_t)ns * sizeof(uint4)));
+    NQ_CUDA(h, h->sinfo.ensure((size_t)ns * sizeof(uint2)));
+  }
+  L.big = counts_need_u64(N, D > 0 && !read_back ? m : L.m);
   if (h->queue_order == 1) {
     NQ_CUDA(h, h->okeys.ensure((size_t)std::max<int64_t>(L.m, 1)));
     NQ_CUDA(h, h->oorder.ensure((size_t)std::max<int64_t>(L.m, 1) * sizeof(uint32_t)));
     NQ_CUDA(h, h->ohist.ensure(512 * sizeof(unsigned int)));
-    NQ_CUDA(h, launch_order(L.m, L.sroot, L.sinfo, ta, (uint8_t*)h->okeys.p, (unsigned int*)h->ohist.p,
+    NQ_CUDA(h, launch_order(L.m, L.sroot, L.sinfo, L.tasks, (uint8_t*)h->okeys.p, (unsigned int*)h->ohist.p,
                             (uint32_t*)h->oorder.p, st));
     L.order = (const uint32_t*)h->oorder.p;
   }
-  h->last_split = D; h->last_queue = L.m;
+  h->last_split = D; h->last_queue = L.m; h->queue_on_device = L.m_dev != nullptr;
   NQ_CUDA(h, cudaEventRecord(h->ev[1], st));
   NQ_CUDA(h, launch_dfs(L, st));
   NQ_CUDA(h, cudaEventRecord(h->ev[2], st));
@@ -159,6 +156,7 @@ int read_ctrl(nq_handle* h, cudaStream_t st, uint64_t* total) {
   NQ_CUDA(h, cudaStreamSynchronize(st));
   const unsigned char* hc = (const unsigned char*)h->h_ctrl;
   const uint32_t e = *(const uint32_t*)(hc + ctl::kErr);
+  if (h->queue_on_device) h->last_queue = (int64_t)*(const uint64_t*)(hc + ctl::kSplit);
   if (e) return h->fail(derr_to_status(e), "device: %s", derr_text(e));
   if (total) *total = *(const uint64_t*)(hc + ctl::kTotal);
   return NQ_OK;
@@ -389,11 +387,7 @@ int nq_sync(nq_handle* h) {
   // waits for this handle's last count only (its event), not for other handles, batches or streams
   NQ_CUDA(h, cudaEventSynchronize(h->done));
   h->pending = false;
-  uint32_t e = 0;
-  NQ_CUDA(h, cudaMemcpyAsync(&e, (unsigned char*)h->ctrl.p + ctl::kErr, 4, cudaMemcpyDeviceToHost, h->stream));
-  NQ_CUDA(h, cudaStreamSynchronize(h->stream));
-  if (e) return h->fail(derr_to_status(e), "device: %s", derr_text(e));
-  return NQ_OK;
+  return read_ctrl(h, h->stream, nullptr);
 }
 
 int nq_debug_task_schedule(int N, nq_record rec, uint32_t root[4], uint32_t* info, uint32_t* words, int cap) {

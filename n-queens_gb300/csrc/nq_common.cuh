@@ -227,9 +227,10 @@ struct Op { uint32_t s, la, ra, fc, term, tall; };
 // candidate dies (or, at a terminal parent, counts nothing): pruning there
 // changes no count.  A tall terminal counts its candidates without looking
 // at a further row, so a child with a tall word is never pruned.
-NQ_HD void extend_lookahead(Op* ops, int T) {
+NQ_HD bool lookahead_sound(const Op& child) { return child.s == 1 && !child.tall; }
+inline void extend_lookahead(Op* ops, int T) {
   for (int d = 0; d < T; d++)
-    if (ops[d + 1].s == 1 && !ops[d + 1].tall) ops[d].fc = 1;
+    if (lookahead_sound(ops[d + 1])) ops[d].fc = 1;
 }
 
 // Walk the SQ* state machine from the task's root frame and emit one Op per
@@ -240,12 +241,16 @@ NQ_HD void extend_lookahead(Op* ops, int T) {
 // empty, or -2 on a schedule longer than max_depth / without a terminal.
 struct Root { uint32_t ld, rd, col, avail; };
 
-NQ_HD int walk_schedule(int N, const TaskHead& t, Root* root, uint32_t* root_count, Op* ops, int max_depth) {
+// The ops are emitted in order, emit(depth, op), each when the next one is known (it decides the look-ahead
+// and may add to LA), so no array of them is kept: on the device the walk stays in registers.
+template <class Emit>
+NQ_HD int walk_schedule(int N, const TaskHead& t, Root* root, uint32_t* root_count, int max_depth, Emit&& emit) {
   const uint32_t n3 = 1u << (N - 3), n4 = 1u << (N - 4);
   root->ld = t.ld; root->rd = t.rd; root->col = t.col; root->avail = t.free_;
   *root_count = 0;
   if (root->avail == 0) return -1;                       // dfs_iter: `if not free: continue`
   int fid = t.fid, row = t.start;
+  Op prev = {1, 0, 0, 0, 0, 0};
   for (int d = 0;; d++) {
     FidRow fr = fid_row(fid);
     if (fr.ptn == 4 && row == t.mark1) { fid = fr.next; fr = fid_row(fid); }   // P5: re-push with next fid
@@ -254,13 +259,13 @@ NQ_HD int walk_schedule(int N, const TaskHead& t, Root* root, uint32_t* root_cou
         *root_count = (fid == 14) ? ((root->avail >> 1) ? 1u : 0u) : 1u;
         return -1;
       }
-      ops[d - 1].term = 1;
+      prev.term = 1;
       // The terminal-parent frame never descends, so its LA bits only feed the
       // child row's free set: LA bit 0 there removes column 0, which is the
       // SQd2B base rule "count only if a square other than column 0 is free"
       // (356Py:1855-1860).
-      if (fid == 14) ops[d - 1].la |= 1u;
-      extend_lookahead(ops, d - 1);
+      if (fid == 14) prev.la |= 1u;
+      emit(d - 1, prev);
       return d - 1;
     }
     if (d >= max_depth || row > 31) return -2;
@@ -278,15 +283,27 @@ NQ_HD int walk_schedule(int N, const TaskHead& t, Root* root, uint32_t* root_cou
         // this frame is a jmark frame: column 0 is forbidden in it and ld gets bit 0.
         // Both happen when the frame is created: fold into the parent's LA.
         if (d == 0) { root->avail &= ~1u; root->ld |= 1u; if (root->avail == 0) return -1; }
-        else ops[d - 1].la |= 1u;
+        else prev.la |= 1u;
         nfid = fr.next;
       }
       op.fc = (fr.av == 1 && row + 1 < t.endmark) ? 1u : 0u;
     }
-    ops[d] = op;
+    if (d > 0) {
+      if (lookahead_sound(op)) prev.fc = 1;
+      emit(d - 1, prev);
+    }
+    prev = op;
     fid = nfid;
     row += (int)op.s;
   }
+}
+// The same into an array of max_depth ops.
+struct OpArray {
+  Op* ops;
+  NQ_HD void operator()(int d, const Op& o) const { ops[d] = o; }
+};
+NQ_HD int walk_schedule(int N, const TaskHead& t, Root* root, uint32_t* root_count, Op* ops, int max_depth) {
+  return walk_schedule(N, t, root, root_count, max_depth, OpArray{ops});
 }
 
 // True when the op packs into a compact word without overlapping fields.

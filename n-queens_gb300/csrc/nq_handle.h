@@ -99,6 +99,7 @@ struct nq_handle {
   bool pending = false;
   int last_split = 0;        // split depth and queue length of the last run
   int64_t last_queue = 0;
+  bool queue_on_device = false;   // its length stands in the control block, not yet in last_queue
   // events around the last run's kernels (same stream as the launches)
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
 

@@ -15,6 +15,27 @@ constexpr uint32_t DERR_NOTERM = 4u;     // a schedule never reaches a base fram
 constexpr uint32_t DERR_BADN = 8u;       // N outside 6..27 in a task
 constexpr uint32_t DERR_FORMAT = 16u;    // a schedule op does not fit the compact word's fields
 
+// Levels every task is expanded by before the DFS.  `rows`: rows left below the shallowest start (N - 2 -
+// start row), which sets a task's work (about 7x per row).  Lanes of a warp share their work at the end of
+// the queue, so splitting only has to even out the warps and give a short list more items than lanes:
+// us of a whole call on GB300 at D = 0 / 1 / 2 / 3, m tasks:
+//   8 rows (N=12):    m=4300   60 / 59 / 60 / 70
+//   9 rows (N=13):    m=7731   75 / 72 / 68 / 79
+//   10 rows (N=14):   m=1000   73 / 65 / 61 / 76       m=13233 100 / 87 / 86 / 129
+//   12 rows (N=16):   m=4000  178 / 149 / 138 / 175    m=33046 593 / 441 / 381 / 471
+//   13 rows (N=18):   m=16000 898 / 761 / 493 / 550    m=200000 5761 / 4056 / 4326 / 5343
+//   14 rows (N=19):   m=100   915 / 247 / 144 / 180    m=4000 1747 / 1115 / 789 / 658
+//                     m=50000 10.5 / 5.4 / 4.7 / 5.2 ms   m=897071 79.1 / 74.3 / 78.8 ms
+//   15 rows (N=20):   m=1000  4.9 / 2.1 / 1.7 / 1.0 ms    m=16000 21.8 / 14.6 / 8.4 / 7.9 ms
+// Each level makes about 7 times the items (measured: 6.2x at N=16 to 8x at N=20), and an item costs its
+// loading; lists of 10^5 tasks and more are balanced at D = 1.
+inline int choose_split(int64_t m, int rows) {
+  if (rows <= 8) return 0;
+  if (m > 100000) return m > 400000000 ? 0 : 1;   // ~7 subtasks a task stay within the u32 subtask queue
+  if (rows >= 15 ? m < 20000 : rows == 14 && m >= 512 && m < 8192) return 3;
+  return 2;
+}
+
 // Prepared task arrays (structure of arrays, one entry per task).
 struct TaskArrays {
   uint4* root = nullptr;      // {ld, rd, col, avail} of the root frame
@@ -28,7 +49,9 @@ struct DfsLaunch {
   TaskArrays tasks;
   const uint4* sroot = nullptr;         // split queue: subtask frames ...
   const uint2* sinfo = nullptr;         // ... and {task, depth}; nullptr: the queue holds tasks
-  int64_t m = 0;                        // queue length
+  int64_t m = 0;                        // queue length ...
+  const unsigned long long* m_dev = nullptr;   // ... or where it stands on the device; above qcap the DFS does nothing
+  unsigned long long qcap = 0;
   const uint32_t* order = nullptr;      // optional queue order (task index per slot)
   unsigned long long* cursor = nullptr; // queue cursor (device, zeroed before launch; 64-bit, so it never wraps)
   unsigned long long* job_totals = nullptr;  // weighted totals, slot (job id - job_base) (device)
@@ -44,11 +67,32 @@ struct DfsLaunch {
 // Prepare: records {ld, rd, col, startijkl} (the reference's 16-byte task
 // record) -> task arrays.  job/offset place the tasks of one job inside a
 // larger queue.
-// per_task (optional): set to 0 for every task.
 // tmax (optional): atomicMax of the schedule depth T over the launch's tasks.
 cudaError_t launch_prepare(int N, int64_t m, const uint4* records, const TaskArrays& out, int64_t offset,
-                           uint32_t job, unsigned int* err, cudaStream_t st, unsigned int* tmax = nullptr,
-                           unsigned long long* per_task = nullptr);
+                           uint32_t job, unsigned int* err, cudaStream_t st, unsigned int* tmax = nullptr);
+
+// Prepare and split a single-N list (compact words) in one launch: tasks, and for D = 1..3 the queue of their
+// depth-D frames (qn counts them, also past qcap, where nothing is written any more) and the counts settled
+// above depth D.  D = 0 writes the tasks' roots instead, which are the queue.
+struct PrepareSplit {
+  int N = 0;
+  int64_t m = 0;                        // records ...
+  const unsigned int* m_dev = nullptr;  // ... or where their number stands on the device (the launch covers m_max)
+  const uint4* rec = nullptr;
+  uint4* root = nullptr;                // D = 0
+  uint2* info = nullptr;
+  uint32_t* sched = nullptr;
+  int sw = 0;
+  unsigned int* err = nullptr;
+  unsigned int* tmax = nullptr;         // optional
+  unsigned long long* per_task = nullptr;    // optional; set for every task
+  uint4* sroot = nullptr;               // D > 0
+  uint2* sinfo = nullptr;
+  unsigned long long qcap = 0;
+  unsigned long long* qn = nullptr;     // zeroed before
+  unsigned long long* total = nullptr;
+};
+cudaError_t launch_prepare_split(int D, int64_t m_max, const PrepareSplit& a, cudaStream_t st);
 
 cudaError_t launch_dfs(const DfsLaunch& L, cudaStream_t st);
 

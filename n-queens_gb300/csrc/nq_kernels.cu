@@ -1,10 +1,11 @@
 // nq_kernels.cu -- sm_103a kernels of the constellation DFS.
 //
-// prepare_kernel: one thread per constellation record.  It runs the task
-//   decision tree of build_soa_for_range (356Py_savesp_narrow.py:1971-2169)
-//   and walks the SQ* state machine once (356Py:689-756 does this per thread
-//   inside the reference kernel) to write the task's root frame, info word
-//   and per-depth schedule.
+// prepare_kernel, prepare_split_kernel: one thread per constellation record.
+//   It runs the task decision tree of build_soa_for_range
+//   (356Py_savesp_narrow.py:1971-2169) and walks the SQ* state machine once
+//   (356Py:689-756 does this per thread inside the reference kernel) to write
+//   the task's root frame, info word and per-depth schedule, and for a single
+//   list the queue of its depth-D frames.
 //
 // dfs_kernel: persistent, explicit-stack bitboard DFS replacing
 //   kernel_dfs_iter_gpu_maxd14..21 (356Py:618-1747) and dfs_iter
@@ -61,20 +62,15 @@ template <> struct WordT<true> { using type = uint2; };
 // ---------------------------------------------------------------------------
 // prepare
 // ---------------------------------------------------------------------------
-template <bool WIDE>
-__device__ __forceinline__ int prepare_one(int N, const uint4* __restrict__ rec, uint4* __restrict__ root,
-                                           uint2* __restrict__ info, typename WordT<WIDE>::type* __restrict__ sched,
-                                           int sw, int64_t offset, uint32_t job, unsigned int* err, int64_t i,
-                                           unsigned long long* __restrict__ per_task) {
-  const uint4 r = rec[i];
-  const int64_t t = offset + i;
-  if (per_task) per_task[t] = 0;      // the DFS adds each queue item's share
+// Device words of one record's task, its info word and root; returns T or -1.  emit(depth, word).
+template <bool WIDE, class Emit>
+__device__ __forceinline__ int prepare_task(int N, const uint4 r, int sw, Root& rt, uint32_t& info, unsigned int* err, Emit&& emit) {
   uint32_t status = TS_OK;
-  Root rt = {0, 0, 0, 0};
+  rt = {0, 0, 0, 0};
   uint32_t root_count = 0;
   int T = -1;
   int wexp = 0;
-  Op ops[kMaxDepth];
+  bool fits = true;
   if (N < 6 || N > kMaxN) {
     status = TS_BADN;
   } else {
@@ -83,32 +79,26 @@ __device__ __forceinline__ int prepare_one(int N, const uint4* __restrict__ rec,
     status = h.status;
     if (status == TS_OK) {
       const int lim = sw < kMaxDepth ? sw : kMaxDepth;
-      T = walk_schedule(N, h, &rt, &root_count, ops, lim);
+      T = walk_schedule(N, h, &rt, &root_count, lim, [&](int d, const Op& o) {
+        if constexpr (WIDE) { fits = fits && wide_fits(o); emit(d, make_uint2(pack_wide_x(o) ^ W_NOLOOK, o.ra)); }
+        else { fits = fits && compact_fits(o, N); emit(d, pack_compact(o) ^ C_NOLOOK); }
+      });
       if (T == -2) status = (lim < kMaxDepth) ? TS_DEPTH : TS_NOTERM;
+      else if (T >= 0 && !fits) status = TS_FORMAT;   // never seen (N=6..21, presets 4-7): fail loudly rather than miscount
     }
   }
   if (status != TS_OK) {
     atomicOr(err, status == TS_BAD_SHIFT ? DERR_SHIFT : status == TS_DEPTH ? DERR_DEPTH
-                : status == TS_NOTERM ? DERR_NOTERM : DERR_BADN);
+                : status == TS_NOTERM ? DERR_NOTERM : status == TS_FORMAT ? DERR_FORMAT : DERR_BADN);
     T = -1; rt = {0, 0, 0, 0}; root_count = 0;
   }
-  const uint32_t Tw = (T < 0) ? INFO_NO_DFS : (uint32_t)T;
-  root[t] = make_uint4(rt.ld, rt.rd, rt.col, T < 0 ? 0u : rt.avail);
-  info[t] = make_uint2(info_pack(Tw, (uint32_t)wexp, root_count, (uint32_t)N, status), job);
-  if (T >= 0) {
-    typename WordT<WIDE>::type* s = sched + t * sw;
-    bool fits = true;
-    for (int d = 0; d <= T; d++) {
-      if constexpr (WIDE) { fits = fits && wide_fits(ops[d]); s[d] = make_uint2(pack_wide_x(ops[d]) ^ W_NOLOOK, ops[d].ra); }
-      else { fits = fits && compact_fits(ops[d], N); s[d] = pack_compact(ops[d]) ^ C_NOLOOK; }
-    }
-    if (!fits) {                      // never seen (N=6..21, presets 4-7): fail loudly rather than miscount
-      atomicOr(err, DERR_FORMAT);
-      info[t] = make_uint2(info_pack(INFO_NO_DFS, (uint32_t)wexp, 0u, (uint32_t)N, TS_FORMAT), job);
-      return -1;
-    }
-  }
+  info = info_pack((T < 0) ? INFO_NO_DFS : (uint32_t)T, (uint32_t)wexp, root_count, (uint32_t)N, status);
   return T;
+}
+
+__device__ __forceinline__ void max_depth_of(unsigned int* tmax, int T) {
+  const unsigned v = __reduce_max_sync(FULL, (unsigned)(T < 0 ? 0 : T));
+  if ((threadIdx.x & 31u) == 0 && v) atomicMax(tmax, v);
 }
 
 template <bool WIDE>
@@ -116,28 +106,32 @@ __global__ void __launch_bounds__(256) prepare_kernel(int N, int64_t m, const ui
                                                       uint4* __restrict__ root, uint2* __restrict__ info,
                                                       typename WordT<WIDE>::type* __restrict__ sched, int sw,
                                                       int64_t offset, uint32_t job, unsigned int* err,
-                                                      unsigned int* tmax, unsigned long long* __restrict__ per_task) {
+                                                      unsigned int* tmax) {
+  using W = typename WordT<WIDE>::type;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int T = (i < m) ? prepare_one<WIDE>(N, rec, root, info, sched, sw, offset, job, err, i, per_task) : -1;
-  if (tmax) {                         // deepest schedule of the launch, for sizing the DFS stack
-    const unsigned v = __reduce_max_sync(FULL, (unsigned)(T < 0 ? 0 : T));
-    if ((threadIdx.x & 31u) == 0 && v) atomicMax(tmax, v);
+  int T = -1;
+  if (i < m) {
+    const int64_t t = offset + i;
+    Root rt;
+    uint32_t in;
+    T = prepare_task<WIDE>(N, rec[i], sw, rt, in, err, [&](int d, W w) { sched[t * sw + d] = w; });
+    root[t] = make_uint4(rt.ld, rt.rd, rt.col, T < 0 ? 0u : rt.avail);
+    info[t] = make_uint2(in, job);
   }
+  if (tmax) max_depth_of(tmax, T);    // deepest schedule of the launch, for sizing the DFS stack
 }
 
-
 cudaError_t launch_prepare(int N, int64_t m, const uint4* records, const TaskArrays& out, int64_t offset,
-                           uint32_t job, unsigned int* err, cudaStream_t st, unsigned int* tmax,
-                           unsigned long long* per_task) {
+                           uint32_t job, unsigned int* err, cudaStream_t st, unsigned int* tmax) {
   if (m <= 0) return cudaSuccess;
   const int B = 256;
   const unsigned G = (unsigned)((m + B - 1) / B);
   if (out.wide)
     prepare_kernel<true><<<G, B, 0, st>>>(N, m, records, out.root, out.info, (uint2*)out.sched, out.sw, offset, job, err,
-                                          tmax, per_task);
+                                          tmax);
   else
     prepare_kernel<false><<<G, B, 0, st>>>(N, m, records, out.root, out.info, (uint32_t*)out.sched, out.sw, offset, job,
-                                           err, tmax, per_task);
+                                           err, tmax);
   return cudaGetLastError();
 }
 
@@ -153,6 +147,102 @@ __device__ __forceinline__ Dec decode(uint32_t w, uint32_t N, uint32_t k, uint32
 __device__ __forceinline__ Dec decode(uint2 w, uint32_t, uint32_t, uint32_t) {
   const uint32_t s = w.x & W_S;
   return Dec{s, s ? (w.x >> (32 - s)) : 0u, w.y, ~w.x & W_NOLOOK, w.x & W_TERM, w.x & W_TALL};
+}
+
+// ---------------------------------------------------------------------------
+// prepare + split of a single-N list in one launch: each thread prepares its
+// record, counts the task's depth-D frames, takes its warp's slots with one
+// atomic and writes them, the words of depths 0..D-1 still in registers.  The
+// queue's length stays on the device (the DFS reads it there), so a short list
+// needs no read-back between the launches.  Tasks that end above depth D and
+// tasks without a DFS are settled here.  D = 0: the tasks themselves are the
+// queue.  Bound by latency and the record walk (about 300 instructions a
+// record); the three launches it replaces kept 28 ops a record in local memory
+// and read tasks back from memory twice.
+// ---------------------------------------------------------------------------
+template <int K, int D, class F>
+__device__ __forceinline__ void frames_at(uint32_t ld, uint32_t rd, uint32_t col, uint32_t avail, const uint32_t* w,
+                                          uint32_t N, uint32_t T, uint32_t& direct, F&& f) {
+  if constexpr (K == D) {
+    f(make_uint4(ld, rd, col, avail));
+  } else {
+    const Dec o = decode(w[K], N, (uint32_t)K, T);
+    const uint32_t bm = (1u << N) - 1u;
+    while (avail) {
+      const uint32_t bit = avail & (0u - avail);
+      avail ^= bit;
+      const uint32_t nld = ((ld | bit) << o.s) | o.la, nrd = ((rd | bit) >> o.s) | o.ra, ncol = col | bit;
+      uint32_t nf = bm & ~(nld | nrd | ncol);
+      if (o.fc && (bm & ~((nld << 1) | (nrd >> 1) | ncol)) == 0u) nf = 0;
+      if (o.term) { direct += nf != 0u ? 1u : 0u; continue; }   // SQd2B: LA bit 0
+      if (nf) frames_at<K + 1, D>(nld, nrd, ncol, nf, w, N, T, direct, f);
+    }
+  }
+}
+
+template <int D>
+__global__ void __launch_bounds__(256) prepare_split_kernel(const PrepareSplit a) {
+  const int64_t m = a.m_dev ? (int64_t)*a.m_dev : a.m;
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if ((int64_t)blockIdx.x * blockDim.x >= m) return;
+  const unsigned lane = threadIdx.x & 31u;
+  Root rt = {0, 0, 0, 0};
+  uint32_t in = 0, w[D > 0 ? D : 1] = {0};
+  int T = -1;
+  if (t < m) {
+    T = prepare_task<false>(a.N, a.rec[t], a.sw, rt, in, a.err, [&](int d, uint32_t x) {
+      a.sched[t * a.sw + d] = x;
+#pragma unroll
+      for (int k = 0; k < D; k++)
+        if (d == k) w[k] = x;
+    });
+    a.info[t] = make_uint2(in, 0u);
+    if (D == 0) {
+      a.root[t] = make_uint4(rt.ld, rt.rd, rt.col, T < 0 ? 0u : rt.avail);
+      if (a.per_task) a.per_task[t] = 0;      // the DFS adds the task's counts
+    }
+  }
+  if (a.tmax) max_depth_of(a.tmax, T);
+  if constexpr (D > 0) {
+    uint32_t n = 0, direct = 0;
+    if (T >= 0) frames_at<0, D>(rt.ld, rt.rd, rt.col, rt.avail, w, (uint32_t)a.N, (uint32_t)T, direct, [&](uint4) { n++; });
+    else if (t < m && info_status(in) == TS_OK) direct = info_root(in);
+    uint32_t incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(FULL, incl, o);
+      if ((int)lane >= o) incl += v;
+    }
+    unsigned long long base = 0;
+    if (lane == 31 && incl) base = atomicAdd(a.qn, (unsigned long long)incl);
+    base = __shfl_sync(FULL, base, 31) + (incl - n);
+    if (n && base + n <= a.qcap) {            // a queue that does not fit is sized by qn and built again
+      uint32_t dummy = 0;
+      frames_at<0, D>(rt.ld, rt.rd, rt.col, rt.avail, w, (uint32_t)a.N, (uint32_t)T, dummy, [&](uint4 f) {
+        a.sroot[base] = f;
+        a.sinfo[base++] = make_uint2((uint32_t)t, (uint32_t)D);
+      });
+    }
+    const unsigned long long dv = (unsigned long long)direct << info_wexp(in);
+    if (t < m && a.per_task) a.per_task[t] = dv;
+    unsigned long long v = dv;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
+    if (lane == 0 && v) atomicAdd(a.total, v);
+  }
+}
+
+cudaError_t launch_prepare_split(int D, int64_t m_max, const PrepareSplit& a, cudaStream_t st) {
+  if (m_max <= 0) return cudaSuccess;
+  const unsigned B = 256, G = (unsigned)((m_max + B - 1) / B);
+  switch (D) {
+    case 0: prepare_split_kernel<0><<<G, B, 0, st>>>(a); break;
+    case 1: prepare_split_kernel<1><<<G, B, 0, st>>>(a); break;
+    case 2: prepare_split_kernel<2><<<G, B, 0, st>>>(a); break;
+    case 3: prepare_split_kernel<3><<<G, B, 0, st>>>(a); break;
+    default: return cudaErrorInvalidValue;
+  }
+  return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
@@ -372,7 +462,9 @@ struct DfsArgs {
   int sw;
   const uint4* sroot;         // subtask frames and {task, depth} (split queue)
   const uint2* sinfo;
-  int64_t m;                  // queue length
+  int64_t m;                  // queue length, ...
+  const unsigned long long* m_dev;   // ... or where it stands on the device (above qcap: the queue did not fit, no work)
+  unsigned long long qcap;
   const uint32_t* order;
   unsigned long long* cursor;
   unsigned long long* job_totals;
@@ -380,8 +472,6 @@ struct DfsArgs {
   unsigned long long* per_task;
   unsigned int* err;
   int maxt;
-  unsigned chunk;             // queue items a warp takes first: 32, or its share of a queue smaller than the grid
-  float share;                // the later chunks' share of the items left
 };
 
 __device__ __forceinline__ void flush_job(const DfsArgs& a, unsigned job, unsigned long long v) {
@@ -513,7 +603,13 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
   auto arm = [&]() { sts_frame(top - F, 1u, 0u, (1u << (L.tf - 1u)) - 1u, kSentinelAvail); };
   uint32_t wexp = 0, job = a.job_base, task = 0;
   bool have = false, exhausted = false, drained = false;   // exhausted, drained: warp-uniform, as the pool's counters
-  unsigned chunk = a.chunk, pool_n = 0, pool_at = 0;
+  unsigned long long m = a.m;
+  if (a.m_dev) { m = *a.m_dev; if (m > a.qcap) m = 0; }
+  // queue items a warp takes first: 32, or its share of a queue smaller than the grid
+  const unsigned warps = gridDim.x * (BLOCK / 32);
+  const unsigned chunk0 = m >= 32ull * warps ? 32u : ((unsigned)m + warps - 1u) / warps;
+  const float share = 1.0f / (kChunkShare * (float)warps);
+  unsigned chunk = chunk0, pool_n = 0, pool_at = 0;
   uint4 p_root = make_uint4(0, 0, 0, 0);
   uint32_t p_task = 0, p_info = 0, p_job = 0;
   unsigned long long acc = 0;
@@ -540,13 +636,13 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
           unsigned long long base = 0;
           if (lane == 0) base = atomicAdd(a.cursor, (unsigned long long)chunk);
           base = __shfl_sync(FULL, base, 0);
-          const unsigned long long left = base < (unsigned long long)a.m ? (unsigned long long)a.m - base : 0ull;
+          const unsigned long long left = base < m ? m - base : 0ull;
           pool_n = left < chunk ? (unsigned)left : chunk;
           pool_at = 0;
           // the next chunk is a share of what is left, so the warps end together; where the first chunks
           // cover the queue there is no next one
-          drained = a.chunk < 32u || left <= chunk;
-          chunk = min(32u, max(kMinChunk, (unsigned)((float)left * a.share)));
+          drained = chunk0 < 32u || left <= chunk;
+          chunk = min(32u, max(kMinChunk, (unsigned)((float)left * share)));
           if (pool_n == 0u) { exhausted = true; break; }
           if (lane < pool_n) {
             const uint64_t slot = base + lane;
@@ -692,18 +788,15 @@ static cudaError_t launch_dfs_t(const DfsLaunch& L, cudaStream_t st) {
   DfsArgs a;
   a.root = L.tasks.root; a.info = L.tasks.info; a.sched = L.tasks.sched; a.sw = L.tasks.sw;
   a.sroot = L.sroot; a.sinfo = L.sinfo;
-  a.m = L.m; a.order = L.order; a.cursor = L.cursor; a.job_totals = L.job_totals; a.job_base = L.job_base;
+  a.m = L.m; a.m_dev = L.m_dev; a.qcap = L.qcap; a.order = L.order; a.cursor = L.cursor; a.job_totals = L.job_totals; a.job_base = L.job_base;
   a.per_task = L.per_task; a.err = L.err; a.maxt = L.maxt;
-  const int64_t warps = (int64_t)grid * (BLOCK / 32);
-  a.chunk = (unsigned)std::min<int64_t>(32, (L.m + warps - 1) / warps);
-  a.share = 1.0f / (kChunkShare * (float)warps);
   dfs_kernel<WIDE, BLOCK, BIG><<<grid, BLOCK, smem, st>>>(a);
   return cudaGetLastError();
 }
 
 
 cudaError_t launch_dfs(const DfsLaunch& L, cudaStream_t st) {
-  if (L.m <= 0) return cudaSuccess;
+  if (L.m <= 0 && !L.m_dev) return cudaSuccess;
   if (L.maxt < 1 || L.maxt > kMaxDepth) return cudaErrorInvalidValue;
 #define NQ_DFS_BLOCK(B)                                                                        \
   if (L.tasks.wide) return L.big ? launch_dfs_t<true, B, true>(L, st) : launch_dfs_t<true, B, false>(L, st); \

@@ -6,9 +6,10 @@
 // budget), or a latency-critical loop where an allocation's implicit device
 // synchronisation would stall every other stream.  This entry point runs the
 // same prepare and DFS kernels as nq_exec_solutions_device, but its scratch
-// (control words, task roots, task info, per-depth schedules) lives in one
-// file-scope __device__ array of fixed size, which every GPU that loads the
-// library holds until the process exits.  Nothing here allocates.
+// (control words, task info, per-depth schedules, and the split queue in what
+// is left) lives in one file-scope __device__ array of fixed size, which every
+// GPU that loads the library holds until the process exits.  Nothing here
+// allocates.
 //
 // Limits: at most kMaxRecords records per call (N <= 17 at the default
 // presets) and schedules of at most kMaxWords depths.  All calls share the
@@ -26,7 +27,7 @@ namespace {
 
 constexpr int64_t kMaxRecords = 131072;
 constexpr int kMaxWords = 24;                        // schedule words per task (depths 0..23)
-constexpr size_t kCtrlBytes = 256;                   // totals, queue cursor, error word
+constexpr size_t kCtrlBytes = 256;                   // totals, queue cursor, error word, queue length
 constexpr size_t kRootBytes = (size_t)kMaxRecords * sizeof(uint4);
 constexpr size_t kInfoBytes = (size_t)kMaxRecords * sizeof(uint2);
 constexpr size_t kSchedBytes = (size_t)kMaxRecords * kMaxWords * sizeof(uint32_t);
@@ -77,27 +78,50 @@ extern "C" int nq_exec_solutions_noalloc(int N, const nq_record* d_records, int6
   unsigned long long* totals = (unsigned long long*)c;
   unsigned long long* cursor = (unsigned long long*)(c + 8);
   unsigned int* err = (unsigned int*)(c + 16);
-  // the array keeps the previous call's contents: clear what must start at zero
-  if (cudaMemsetAsync(c, 0, 24, st) != cudaSuccess) return NQ_ECUDA;
-  if (m > 0) {
-    TaskArrays ta;
-    ta.root = (uint4*)(c + kCtrlBytes);
-    ta.info = (uint2*)(c + kCtrlBytes + kRootBytes);
-    ta.sched = (void*)(c + kCtrlBytes + kRootBytes + kInfoBytes);
-    ta.sw = maxt + 1;
-    ta.wide = false;
-    if (launch_prepare(N, m, (const uint4*)d_records, ta, 0, 0, err, st, nullptr,
-                       (unsigned long long*)d_solutions) != cudaSuccess) return NQ_ECUDA;
+  if (m == 0) {
+    if (cudaMemsetAsync(d_total, 0, 8, st) != cudaSuccess) return NQ_ECUDA;
+    return cudaStreamSynchronize(st) == cudaSuccess ? NQ_OK : NQ_ECUDA;
+  }
+  // info and schedules first, then the roots (unsplit) or as many queue items as fit
+  PrepareSplit P;
+  P.N = N; P.m = m; P.rec = (const uint4*)d_records; P.sw = maxt + 1; P.err = err; P.total = totals;
+  P.per_task = (unsigned long long*)d_solutions; P.qn = (unsigned long long*)(c + 24);
+  size_t used = kCtrlBytes;
+  P.info = (uint2*)(c + used);
+  used += ((size_t)m * sizeof(uint2) + 15) & ~(size_t)15;
+  P.sched = (uint32_t*)(c + used);
+  used += ((size_t)m * P.sw * sizeof(uint32_t) + 15) & ~(size_t)15;
+  P.qcap = (kScratchBytes - used) / (sizeof(uint4) + sizeof(uint2));
+  // Split as deep as the usual rule says while the queue should fit (8 items a level); one that does not
+  // after all leaves the DFS without work, and the call runs again unsplit (the scratch always holds that).
+  // 20,011 records of N=16: unsplit 417 us, one level 324 us.
+  int D = choose_split(m, maxt);
+  while (D > 0 && ((uint64_t)m << (3 * D)) > P.qcap) D--;
+  uint64_t hc[4];
+  for (;; D = 0) {
+    // the array keeps the previous call's contents: clear what must start at zero
+    if (cudaMemsetAsync(c, 0, 32, st) != cudaSuccess) return NQ_ECUDA;
     DfsLaunch L;
-    L.tasks = ta; L.m = m; L.cursor = cursor; L.job_totals = totals;
-    L.per_task = (unsigned long long*)d_solutions; L.err = err; L.maxt = maxt; L.block = 128; L.grid = 0;
+    if (D == 0) {
+      P.root = (uint4*)(c + used);
+      L.m = m;
+    } else {
+      P.sroot = (uint4*)(c + used);
+      P.sinfo = (uint2*)(P.sroot + P.qcap);
+      L.sroot = P.sroot; L.sinfo = P.sinfo; L.m_dev = P.qn; L.qcap = P.qcap;
+    }
+    if (launch_prepare_split(D, m, P, st) != cudaSuccess) return NQ_ECUDA;
+    L.tasks.root = P.root; L.tasks.info = P.info; L.tasks.sched = P.sched; L.tasks.sw = P.sw; L.tasks.wide = false;
+    L.cursor = cursor; L.job_totals = totals;
+    L.per_task = (unsigned long long*)d_solutions; L.err = err; L.maxt = maxt - D < 1 ? 1 : maxt - D; L.block = 128; L.grid = 0;
     L.big = counts_need_u64(N, m);
     if (launch_dfs(L, st) != cudaSuccess) return NQ_ECUDA;
+    if (cudaMemcpyAsync(d_total, totals, 8, cudaMemcpyDeviceToDevice, st) != cudaSuccess) return NQ_ECUDA;
+    if (cudaMemcpyAsync(hc, c, 32, cudaMemcpyDeviceToHost, st) != cudaSuccess) return NQ_ECUDA;
+    if (cudaStreamSynchronize(st) != cudaSuccess) return NQ_ECUDA;
+    if (D == 0 || hc[3] <= P.qcap) break;
   }
-  if (cudaMemcpyAsync(d_total, totals, 8, cudaMemcpyDeviceToDevice, st) != cudaSuccess) return NQ_ECUDA;
-  uint32_t herr = 0;
-  if (cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, st) != cudaSuccess) return NQ_ECUDA;
-  if (cudaStreamSynchronize(st) != cudaSuccess) return NQ_ECUDA;
+  const uint32_t herr = (uint32_t)hc[2];
   if (herr & DERR_DEPTH) return NQ_ESTACK;
   if (herr & DERR_SHIFT) return NQ_EPRESET;
   if (herr) return NQ_EINVAL;
