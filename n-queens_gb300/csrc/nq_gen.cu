@@ -1,0 +1,151 @@
+// nq_gen.cu -- task lists built on the device.
+//
+// query_kernel: the queue of one completion query, from its root frame to
+//   thousands of frames, in one block; query_level_kernel expands it by
+//   another level over the whole GPU.
+//
+// All of them count a state's children, take the warp's slots with one atomic
+// and write them; list order is not kept (a count does not depend on it).
+// Bound by launch latency at small boards: a level takes 2-3 us.
+#include <cuda_runtime.h>
+
+#include "nq_common.cuh"
+#include "nq_internal.h"
+
+namespace nq {
+namespace {
+
+constexpr unsigned FULL = 0xFFFFFFFFu;
+
+// First slot of this thread's `n` entries in a list with counter `c` (all lanes of the warp call it).
+__device__ __forceinline__ unsigned take_slots(unsigned* c, unsigned n) {
+  const unsigned lane = threadIdx.x & 31u;
+  unsigned incl = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned v = __shfl_up_sync(FULL, incl, o);
+    if ((int)lane >= o) incl += v;
+  }
+  unsigned base = 0;
+  if (lane == 31 && incl) base = atomicAdd(c, incl);
+  return __shfl_sync(FULL, base, 31) + incl - n;
+}
+
+// ---------------------------------------------------------------------------
+// completion queries
+// ---------------------------------------------------------------------------
+struct QWord { uint32_t s, la, ra, fc; };
+__device__ __forceinline__ QWord qword(uint32_t w, uint32_t N) {
+  const Op o = unpack_compact(w ^ C_NOLOOK, (int)N, false);
+  return QWord{o.s, o.la, o.ra, o.fc};
+}
+__device__ __forceinline__ QWord qword(uint2 w, uint32_t) {
+  const uint32_t s = w.x & W_S;
+  return QWord{s, s ? (w.x >> (32 - s)) : 0u, w.y, ~w.x & W_NOLOOK};
+}
+
+template <class F>
+__device__ __forceinline__ void each_child(const uint4 f, const QWord o, uint32_t bm, F&& fn) {
+  for (uint32_t av = f.w; av;) {
+    const uint32_t bit = av & (0u - av);
+    av ^= bit;
+    const uint32_t nl = ((f.x | bit) << o.s) | o.la, nr = ((f.y | bit) >> o.s) | o.ra, nc = f.z | bit;
+    const uint32_t nf = bm & ~(nl | nr | nc);
+    if (nf && !(o.fc && (bm & ~((nl << 1) | (nr >> 1) | nc)) == 0u)) fn(make_uint4(nl, nr, nc, nf));
+  }
+}
+
+// The frames of one query, breadth-first from its root until there are `target` of them, the next level may
+// not fit, or they stand at the terminal depth: into (sroot, sinfo) from `slot` on.  Returns their number;
+// one block, buffers of `cap` frames.
+template <class W>
+__device__ unsigned expand_query(const uint4 root, uint32_t N, uint32_t T, const W* words, unsigned target, unsigned cap,
+                                 uint4* buf0, uint4* buf1, unsigned& depth) {
+  __shared__ unsigned cnt;
+  const uint32_t bm = (1u << N) - 1u;
+  uint4 *in = buf0, *out = buf1;
+  if (threadIdx.x == 0) in[0] = root;
+  unsigned n = root.w ? 1u : 0u, d = 0;
+  __syncthreads();
+  while (d < T && n && n < target && n * N <= cap) {
+    if (threadIdx.x == 0) cnt = 0;
+    __syncthreads();
+    const QWord o = qword(words[d], N);
+    for (unsigned q0 = 0; q0 < n; q0 += blockDim.x) {
+      const unsigned q = q0 + threadIdx.x;
+      const uint4 f = q < n ? in[q] : make_uint4(0, 0, 0, 0);
+      unsigned c = 0;
+      each_child(f, o, bm, [&](uint4) { c++; });
+      unsigned at = take_slots(&cnt, c);
+      if (c) each_child(f, o, bm, [&](uint4 g) { out[at++] = g; });
+    }
+    __syncthreads();
+    n = cnt;
+    uint4* t = in; in = out; out = t;
+    d++;
+    __syncthreads();
+  }
+  depth = d;
+  if (in != buf0)                       // callers read buf0
+    for (unsigned q = threadIdx.x; q < n; q += blockDim.x) buf0[q] = in[q];
+  __syncthreads();
+  return n;
+}
+
+template <bool WIDE>
+__global__ void __launch_bounds__(1024) query_kernel(const __grid_constant__ QueryParam p, QueryBuffers b) {
+  using W = typename QueryWord<WIDE>::type;
+  __shared__ W words[kMaxDepth];
+  if (threadIdx.x <= p.T) {
+    const uint2 w = p.words[threadIdx.x];
+    if constexpr (WIDE) words[threadIdx.x] = w; else words[threadIdx.x] = w.x;
+    ((W*)b.sched)[threadIdx.x] = words[threadIdx.x];
+  }
+  if (threadIdx.x < QueryCtl::kWords) b.ctl[threadIdx.x] = 0;
+  if (threadIdx.x == 0) b.info[0] = make_uint2(info_pack(p.T, 0, 0, p.N, TS_OK), 0u);
+  __syncthreads();
+  unsigned d;
+  const unsigned n = expand_query<W>(p.root, p.N, p.T, words, p.target, b.cap[0], b.sroot[0], b.tmp, d);
+  for (unsigned q = threadIdx.x; q < n; q += blockDim.x) b.sinfo[0][q] = make_uint2(0u, d);
+  if (threadIdx.x == 0) b.ctl[QueryCtl::kQueue] = n;
+}
+
+// The query's queue by another level (frames at the terminal depth move on).
+template <bool WIDE>
+__global__ void __launch_bounds__(128) query_level_kernel(uint32_t N, uint32_t T, QueryBuffers b, int level) {
+  using W = typename QueryWord<WIDE>::type;
+  const unsigned n = b.ctl[QueryCtl::kQueue + level];
+  const unsigned cap = b.cap[level + 1];
+  const uint4* __restrict__ in = b.sroot[level];
+  uint4* __restrict__ out = b.sroot[level + 1];
+  uint2* __restrict__ info = b.sinfo[level + 1];
+  const uint32_t bm = (1u << N) - 1u;
+  for (unsigned q0 = blockIdx.x * blockDim.x; q0 < n; q0 += gridDim.x * blockDim.x) {
+    const unsigned q = q0 + threadIdx.x;
+    uint4 f = make_uint4(0, 0, 0, 0);
+    uint32_t d = 0;
+    if (q < n) { f = in[q]; d = b.sinfo[level][q].y; }
+    const bool keep = q < n && d >= T;
+    const QWord o = keep ? QWord{1, 0, 0, 0} : qword(((const W*)b.sched)[d], N);
+    unsigned c = keep ? 1u : 0u;
+    if (!keep) each_child(f, o, bm, [&](uint4) { c++; });
+    unsigned at = take_slots((unsigned*)&b.ctl[QueryCtl::kQueue + level + 1], c);
+    if (at + c > cap) continue;
+    if (keep) { out[at] = f; info[at] = make_uint2(0u, d); }
+    else if (c) each_child(f, o, bm, [&](uint4 g) { out[at] = g; info[at++] = make_uint2(0u, d + 1u); });
+  }
+}
+
+}  // namespace
+
+cudaError_t launch_query(const QueryParam& p, const QueryBuffers& b, bool wide, int levels, int sms, cudaStream_t st) {
+  if (wide) query_kernel<true><<<1, 1024, 0, st>>>(p, b);
+  else query_kernel<false><<<1, 1024, 0, st>>>(p, b);
+  for (int l = 0; l < levels; l++) {
+    if (wide) query_level_kernel<true><<<4 * sms, 128, 0, st>>>(p.N, p.T, b, l);
+    else query_level_kernel<false><<<4 * sms, 128, 0, st>>>(p.N, p.T, b, l);
+  }
+  return cudaGetLastError();
+}
+
+}  // namespace nq

@@ -60,6 +60,11 @@ struct nq_handle {
   std::string err;
   nq::DevBuf rec, root, info, sched, per_task, ctrl, nsub, sroot, sinfo;
   nq::DevBuf utasks, uconfs, uctl;       // unique counter (nq_count_unique)
+  // completion queries: a stream and buffers of their own, so a query may run beside an asynchronous count
+  cudaStream_t q_stream = nullptr;
+  nq::DevBuf qbuf;
+  uint64_t* h_query = nullptr;           // pinned read-back of a query's control block
+  std::mutex q_mu;
   nq::DevBuf okeys, oorder, ohist;       // queue order (nq_set_queue_order)
   int queue_order = 0;                   // 0: generator / split order, 1: largest estimated subtree first
   int64_t chunk_records = 0;             // records per chunk of nq_count (0: the library default)

@@ -223,8 +223,7 @@ int gen_constellations(int N, int preset, std::vector<GenRecord>& out, int threa
 // ---------------------------------------------------------------------------
 // completion queries
 // ---------------------------------------------------------------------------
-int build_completion_tasks(int N, int k, const int* rows, const int* cols, int min_tasks, uint32_t job,
-                           std::vector<HostTask>& out, int* max_T) {
+int completion_root(int N, int k, const int* rows, const int* cols, uint32_t root[4], Op* ops, int* n_rows) {
   if (N < 1 || N > kMaxN || k < 0 || k > N) return -1;
   int fixed_col[32];
   for (int r = 0; r < N; r++) fixed_col[r] = -1;
@@ -241,11 +240,11 @@ int build_completion_tasks(int N, int k, const int* rows, const int* cols, int m
   int F[32], n = 0;
   for (int r = 0; r < N; r++)
     if (fixed_col[r] < 0) F[n++] = r;
+  *n_rows = n;
   if (n == 0) return 2;   // every row holds a pre-placed queen and none attack: exactly one placement
   const uint32_t bm = (N >= 32) ? 0xFFFFFFFFu : ((1u << N) - 1u);
   // root frame at row F[0]
   uint32_t ld = 0, rd = 0, col = 0;
-  Op ops[kMaxDepth + 1];
   if (n > kMaxDepth) return -1;
   for (int d = 0; d < n; d++) ops[d] = Op{1, 0, 0, 0, 0, 0};
   for (int q = 0; q < k; q++) {
@@ -275,10 +274,22 @@ int build_completion_tasks(int N, int k, const int* rows, const int* cols, int m
   extend_lookahead(ops, T);
   for (int d = 0; d < n; d++)
     if (!wide_fits(ops[d])) return -1;
+  root[0] = ld; root[1] = rd; root[2] = col; root[3] = bm & ~(ld | rd | col);
+  return 0;
+}
+
+int build_completion_tasks(int N, int k, const int* rows, const int* cols, int min_tasks, uint32_t job,
+                           std::vector<HostTask>& out, int* max_T) {
+  uint32_t root[4];
+  Op ops[kMaxDepth + 1];
+  int n = 0;
+  if (const int s = completion_root(N, k, rows, cols, root, ops, &n)) return s;
+  const int T = n - 1;
+  const uint32_t bm = (1u << N) - 1u;
 
   // Expand the first levels breadth-first until there are enough tasks.
   struct F4 { uint32_t ld, rd, col, avail; };
-  std::vector<F4> cur{F4{ld, rd, col, bm & ~(ld | rd | col)}}, nxt;
+  std::vector<F4> cur{F4{root[0], root[1], root[2], root[3]}}, nxt;
   int depth = 0;
   while (depth < T && (int)cur.size() < min_tasks) {
     nxt.clear();

@@ -36,6 +36,10 @@ int start_constellations(int N, std::vector<int>& starts);
 int expand_starts(int N, int preset, const std::vector<int>& starts, size_t s0, size_t s1,
                   std::vector<GenRecord>& out, int threads);
 
+// The root frame {ld, rd, col, avail} and per-depth ops (the last one tall, n = free rows of them) of the
+// completions of k pre-placed queens; return values as build_completion_tasks.
+int completion_root(int N, int k, const int* rows, const int* cols, uint32_t root[4], Op* ops, int* n);
+
 // Tasks whose counts sum to the number of N-queens solutions containing the
 // k pre-placed queens (rows[q], cols[q]); no symmetry weight.  Returns 0 with
 // tasks appended, 1 when the count is 0 without any task (attacking queens or

@@ -36,6 +36,9 @@ inline int choose_split(int64_t m, int rows) {
   return 2;
 }
 
+template <bool WIDE> struct QueryWord { using type = uint32_t; };
+template <> struct QueryWord<true> { using type = uint2; };
+
 // Prepared task arrays (structure of arrays, one entry per task).
 struct TaskArrays {
   uint4* root = nullptr;      // {ld, rd, col, avail} of the root frame
@@ -95,6 +98,30 @@ struct PrepareSplit {
 cudaError_t launch_prepare_split(int D, int64_t m_max, const PrepareSplit& a, cudaStream_t st);
 
 cudaError_t launch_dfs(const DfsLaunch& L, cudaStream_t st);
+
+// A completion query as one task: root frame, terminal depth and device words (wide; compact queries use x).
+struct QueryParam {
+  uint4 root;
+  uint32_t N, T;
+  unsigned target;              // frames that are enough
+  uint2 words[28];
+};
+// Its control block (u64 words): total, queue cursor, error word, queue length after each level.
+struct QueryCtl {
+  static constexpr unsigned kTotal = 0, kCursor = 1, kErr = 2, kQueue = 3, kWords = 6;
+};
+struct QueryBuffers {
+  unsigned long long* ctl;
+  uint2* info;                  // one task
+  void* sched;
+  uint4* tmp;                   // cap[0] frames
+  uint4* sroot[3];              // the queue from one block, and after one and two levels over the whole GPU
+  uint2* sinfo[3];
+  unsigned cap[3];              // items each holds; cap[1] = cap[0] * N, so only the last can be too small
+};
+// Writes the task, its queue and the control block, the queue expanded by `levels` (0..2) more levels.  A
+// queue longer than its buffer leaves ctl[kQueue + levels] above cap[levels]: the DFS does nothing.
+cudaError_t launch_query(const QueryParam& p, const QueryBuffers& b, bool wide, int levels, int sms, cudaStream_t st);
 
 // Split tasks t0..t0+m-1 to depth D (0..3; 0 queues the tasks themselves).
 // pass 0: nsub[t] and ctr[0] += subtasks; pass 1: writes subtasks at the

@@ -56,8 +56,7 @@ constexpr unsigned kMinChunk = 8;
 // (fewer: not worth the exchange; 3 and 7 measured the same from N=16 on, 7 is 25 % slower at N=14).
 constexpr int kGiveRows = 5;
 
-template <bool WIDE> struct WordT { using type = uint32_t; };
-template <> struct WordT<true> { using type = uint2; };
+template <bool WIDE> using WordT = QueryWord<WIDE>;
 
 // ---------------------------------------------------------------------------
 // prepare
