@@ -55,6 +55,7 @@ const char* derr_text(uint32_t e) {
 // Records per chunk of a whole-board count (nq_count): one chunk up to N=21
 // (2.0 M records), four at N=22 (28.7 M), about 32 MB of host records each.
 constexpr int64_t kChunkRecords = 8 << 20;
+constexpr size_t kStage = 4096;      // pinned read-back block: uploads are staged behind its first bytes
 
 int maxt_for(int N, int start_min) {
   // Terminal-parent depth T <= N - 3 - start; one frame of margin.
@@ -75,26 +76,27 @@ constexpr int64_t kNoReadBack = 16384;
 constexpr int64_t kQueueBytes = 256 << 20;   // queue buffer a short list may bound its queue by
 
 // records (device) -> counts on st; totals land in ctrl[0].  One launch prepares and splits, one counts.
-// maxt: the deepest schedule of any record (rows left below the shallowest start).
+// start_min bounds the records' schedules; t_max, where the caller knows it, is the deepest one's T.
+// m_dev: the list's length stands there (u32) and m bounds it.
 int run_records(nq_handle* h, int N, const uint4* d_rec, int64_t m, int start_min, unsigned long long* d_per_task,
-                cudaStream_t st) {
+                cudaStream_t st, int t_max = kMaxDepth, const unsigned int* m_dev = nullptr) {
   const int maxt = maxt_for(N, start_min);
   const int D = h->split >= 0 ? h->split : choose_split(m, maxt);
   NQ_CUDA(h, cudaSetDevice(h->device));
   NQ_CUDA(h, h->info.ensure((size_t)m * sizeof(uint2)));
   NQ_CUDA(h, h->sched.ensure((size_t)m * (maxt + 1) * sizeof(uint32_t)));
-  NQ_CUDA(h, h->ctrl.ensure(ctl::kBytes));
+  NQ_CUDA(h, h->ctrl.ensure(ctl::kAll));
   if (int s = h->ensure_pinned(ctl::kBytes)) return s;
   unsigned char* c = (unsigned char*)h->ctrl.p;
   PrepareSplit P;
-  P.N = N; P.m = m; P.rec = d_rec; P.info = (uint2*)h->info.p; P.sched = (uint32_t*)h->sched.p; P.sw = maxt + 1;
+  P.N = N; P.m = m; P.m_dev = m_dev; P.rec = d_rec; P.info = (uint2*)h->info.p; P.sched = (uint32_t*)h->sched.p; P.sw = maxt + 1;
   P.err = (unsigned int*)(c + ctl::kErr); P.tmax = (unsigned int*)(c + ctl::kTmax);
   P.per_task = d_per_task; P.qn = (unsigned long long*)(c + ctl::kSplit); P.total = (unsigned long long*)(c + ctl::kTotal);
   // Queue capacity: a bound (each level places a queen in one of at most N - 2, N - 3, ... columns) where that
   // is small, else 8 a level (measured: 6.2 to 8), built again if it was too small.
   uint64_t bound = (uint64_t)m, guess = (uint64_t)m + 1024;
   for (int d = 0; d < D; d++) { bound *= (uint64_t)(N - 2 - d); guess *= 8; }
-  const bool read_back = m > kNoReadBack || h->queue_order == 1 || (D > 0 && bound * 24 > (uint64_t)kQueueBytes);
+  const bool read_back = (m > kNoReadBack && !m_dev) || h->queue_order == 1 || (D > 0 && bound * 24 > (uint64_t)kQueueBytes);
   if (D > 0) {
     const uint64_t q = std::max(read_back ? std::min(bound, guess) : bound, (uint64_t)(h->sroot.cap / sizeof(uint4)));
     NQ_CUDA(h, h->sroot.ensure((size_t)q * sizeof(uint4)));
@@ -116,8 +118,8 @@ int run_records(nq_handle* h, int N, const uint4* d_rec, int64_t m, int start_mi
     NQ_CUDA(h, launch_prepare_split(D, m, P, st));
     if (D > 0) { L.sroot = P.sroot; L.sinfo = P.sinfo; }
     if (!read_back) {
-      if (D > 0) { L.m_dev = P.qn; L.qcap = P.qcap; }
-      L.maxt = std::max(1, maxt - D);
+      if (D > 0 || m_dev) { L.m_dev = P.qn; L.qcap = D > 0 ? P.qcap : ~0ull; }
+      L.maxt = std::max(1, std::min(maxt, t_max) - D);
       break;
     }
     // Subtasks start at depth D with an empty stack, so the DFS needs T - D frames and T - D + 1 schedule
@@ -126,8 +128,8 @@ int run_records(nq_handle* h, int N, const uint4* d_rec, int64_t m, int start_mi
     NQ_CUDA(h, cudaStreamSynchronize(st));
     const unsigned char* hc = (const unsigned char*)h->h_ctrl;
     L.maxt = std::max(1, std::min(maxt, (int)*(const uint32_t*)(hc + ctl::kTmax) - D));
-    if (D == 0) break;
-    const uint64_t ns = *(const uint64_t*)(hc + ctl::kSplit);
+    const uint64_t ns = *(const uint64_t*)(hc + ctl::kSplit);     // D = 0: the list's length
+    if (D == 0) { L.m = (int64_t)ns; break; }
     if (ns > 0xFFFFFFFFull) return h->fail(NQ_ENOMEM, "split: %llu subtasks", (unsigned long long)ns);
     L.m = (int64_t)ns;
     if (ns <= P.qcap) break;
@@ -151,8 +153,8 @@ int run_records(nq_handle* h, int N, const uint4* d_rec, int64_t m, int start_mi
 }
 
 int read_ctrl(nq_handle* h, cudaStream_t st, uint64_t* total) {
-  if (int s = h->ensure_pinned(ctl::kBytes)) return s;
-  NQ_CUDA(h, cudaMemcpyAsync(h->h_ctrl, h->ctrl.p, ctl::kBytes, cudaMemcpyDeviceToHost, st));
+  if (int s = h->ensure_pinned(ctl::kAll)) return s;
+  NQ_CUDA(h, cudaMemcpyAsync(h->h_ctrl, h->ctrl.p, ctl::kAll, cudaMemcpyDeviceToHost, st));
   NQ_CUDA(h, cudaStreamSynchronize(st));
   const unsigned char* hc = (const unsigned char*)h->h_ctrl;
   const uint32_t e = *(const uint32_t*)(hc + ctl::kErr);
@@ -240,7 +242,7 @@ void nq_destroy(nq_handle* h) {
   cudaSetDevice(h->device);
   if (h->stream) cudaStreamSynchronize(h->stream);
   h->rec.release(); h->root.release(); h->info.release(); h->sched.release(); h->per_task.release(); h->ctrl.release();
-  h->nsub.release(); h->sroot.release(); h->sinfo.release();
+  h->sroot.release(); h->sinfo.release(); h->gen.release(); h->starts.release();
   h->okeys.release(); h->oorder.release(); h->ohist.release();
   h->utasks.release(); h->uconfs.release(); h->uctl.release();
   if (h->h_ctrl) cudaFreeHost(h->h_ctrl);
@@ -533,8 +535,13 @@ namespace {
 // gen_constellations_stream_to_bin, 356Py_savesp_narrow.py:2988-3084): each
 // chunk of starts is expanded into records on the host threads while the
 // previous chunk's DFS runs on the GPU.
+int count_generated(nq_handle* h, int N, int p, const std::vector<int>& starts, size_t s_begin, size_t s_end,
+                    uint64_t* total);
+
 int count_start_range(nq_handle* h, int N, int p, const std::vector<int>& starts, size_t s_begin, size_t s_end,
                       uint64_t* total) {
+  // a chunk size set by the caller bounds the host list, deeper presets make more records than a buffer holds
+  if (h->chunk_records == 0 && p <= 8) return count_generated(h, N, p, starts, s_begin, s_end, total);
   const int64_t chunk = h->chunk_records > 0 ? h->chunk_records : kChunkRecords;
   size_t next = s_begin;
   double per_start = 0.0;                  // records per start constellation seen so far
@@ -582,6 +589,76 @@ int count_start_range(nq_handle* h, int N, int p, const std::vector<int>& starts
     acc += t; chunks++; records += m;
     cur.swap(nxt);
   }
+  h->last_chunks = chunks;
+  h->last_records = records;
+  *total = acc;
+  return NQ_OK;
+}
+
+// The same with the records generated on the device (presets 4..8): chunks of start constellations whose
+// records are bounded by the buffers, one launch a queen, then the usual run over the list that never left
+// the device.  The host generator above spends 0.9 ms on its threads alone at N=9..13 (a count of N=13 took
+// 1.3 ms, 0.1 of it on the GPU) and 8 ms on N=19's 897,071 records.
+constexpr uint64_t kGenRecords = 8 << 20;         // records a chunk may have (bound), 128 MiB a buffer
+constexpr int64_t kGenNoReadBack = 65536;         // bound up to which the list's length stays on the device
+
+// At most this many records from one start constellation: it holds 3 or 4 queens, and its first free row has
+// N - 3 or N - 4 columns left, the next one fewer, ...
+uint64_t start_bound(int N, int preset, int start) {
+  const uint32_t col = 1u | (1u << (N - 1)) | ((1u << (N - 1)) >> geti(start)) | ((1u << (N - 1)) >> getj(start));
+  uint64_t b = 1;
+  int c = N - __builtin_popcount(col);
+  for (int q = getj(start) == N - 1 ? 3 : 4; q < preset; q++) b *= (uint64_t)std::max(0, c--);
+  return b;
+}
+
+int count_generated(nq_handle* h, int N, int p, const std::vector<int>& starts, size_t s_begin, size_t s_end,
+                    uint64_t* total) {
+  cudaStream_t st = h->stream;
+  NQ_CUDA(h, cudaSetDevice(h->device));
+  NQ_CUDA(h, h->ctrl.ensure(ctl::kAll));
+  unsigned char* c = (unsigned char*)h->ctrl.p;
+  unsigned int* gn = (unsigned int*)(c + ctl::kGen);
+  const int levels = gen_levels(p);
+  uint64_t acc = 0;
+  int64_t chunks = 0, records = 0;
+  for (size_t s0 = s_begin; s0 < s_end;) {
+    size_t s1 = s0;
+    uint64_t bound = 0;
+    do { bound += std::max<uint64_t>(1, start_bound(N, p, starts[s1++])); }
+    while (s1 < s_end && bound + start_bound(N, p, starts[s1]) <= kGenRecords);
+    const size_t n = s1 - s0;
+    if (bound > 0x7FFFFFFFull) return h->fail(NQ_ENOMEM, "generator: too many records from one start constellation");
+    const size_t cap = std::max<size_t>((size_t)bound, n);
+    NQ_CUDA(h, h->rec.ensure(cap * sizeof(uint4)));
+    NQ_CUDA(h, h->gen.ensure(cap * sizeof(uint4)));
+    NQ_CUDA(h, h->starts.ensure(n * sizeof(int)));
+    if (int e = h->ensure_pinned(kStage + n * sizeof(int))) return e;
+    std::memcpy((unsigned char*)h->h_ctrl + kStage, &starts[s0], n * sizeof(int));
+    NQ_CUDA(h, cudaMemcpyAsync(h->starts.p, (unsigned char*)h->h_ctrl + kStage, n * sizeof(int), cudaMemcpyHostToDevice, st));
+    NQ_CUDA(h, cudaMemsetAsync(c, 0, ctl::kAll, st));
+    uint4* buf[2] = {(uint4*)h->rec.p, (uint4*)h->gen.p};
+    NQ_CUDA(h, launch_generate(N, p, (unsigned)n, (const int*)h->starts.p, buf[0], buf[1], (unsigned)cap, gn,
+                               (unsigned int*)(c + ctl::kGenErr), h->sms, st));
+    const uint4* rec = buf[levels & 1];
+    const int t_max = std::max(1, N - p - 2);        // a queen a depth, one column left in the base row
+    const bool on_device = (int64_t)bound <= kGenNoReadBack && h->queue_order == 0;
+    int64_t m = (int64_t)bound;
+    if (!on_device) {
+      NQ_CUDA(h, cudaMemcpyAsync(h->h_ctrl, c, ctl::kAll, cudaMemcpyDeviceToHost, st));
+      NQ_CUDA(h, cudaStreamSynchronize(st));
+      m = *(const uint32_t*)((const unsigned char*)h->h_ctrl + ctl::kGen + 4 * levels);
+    }
+    if (m > 0)
+      if (int e = run_records(h, N, rec, m, p - 3, nullptr, st, t_max, on_device ? gn + levels : nullptr)) return e;
+    uint64_t t = 0;
+    if (int e = read_ctrl(h, st, &t)) return e;
+    const unsigned char* hc = (const unsigned char*)h->h_ctrl;
+    if (*(const uint32_t*)(hc + ctl::kGenErr)) return h->fail(NQ_EPRESET, "generator: preset %d too deep for N=%d", p, N);
+    acc += t; chunks++; records += *(const uint32_t*)(hc + ctl::kGen + 4 * levels);
+    s0 = s1;
+  }
+  if (records == 0) chunks = 0;
   h->last_chunks = chunks;
   h->last_records = records;
   *total = acc;

@@ -1,5 +1,8 @@
 // nq_gen.cu -- task lists built on the device.
 //
+// gen_kernels: the records of a range of start constellations (the preset-
+//   queen expansion of gen_constellations, 14Bit_codon_GPU/
+//   356Py_savesp_narrow.py:2759-2835), one launch a queen.
 // query_kernel: the queue of one completion query, from its root frame to
 //   thousands of frames, in one block; query_level_kernel expands it by
 //   another level over the whole GPU.
@@ -29,6 +32,77 @@ __device__ __forceinline__ unsigned take_slots(unsigned* c, unsigned n) {
   unsigned base = 0;
   if (lane == 31 && incl) base = atomicAdd(c, incl);
   return __shfl_sync(FULL, base, 31) + incl - n;
+}
+
+// ---------------------------------------------------------------------------
+// constellation records.  A state is the record {ld, rd, col, row<<20 | ijkl}
+// with its queens in bits 27-30 of the last word; masks keep their low 32 bits,
+// which is all a record holds and all the next row's free set reads (columns
+// are bits 0..N-1, N <= 27, and rd starts below bit N).  The reference drops
+// states it has seen (subconst cache, and the signatures up to preset 5): over
+// all N <= 27 and presets 4-6 no state occurs twice (enumerated), and from
+// preset 7 on the reference does not look, so nothing is looked up here.
+// ---------------------------------------------------------------------------
+constexpr unsigned kQueens = 27;
+
+__device__ __forceinline__ uint4 settle(uint32_t ld, uint32_t rd, uint32_t col, int row, int queens, uint32_t ijkl) {
+  while (row == getk((int)ijkl) || row == getl((int)ijkl)) { ld <<= 1; rd >>= 1; row++; }   // rows of the side queens
+  return make_uint4(ld, rd, col, ((uint32_t)row << 20) | ijkl | ((uint32_t)queens << kQueens));
+}
+
+__global__ void __launch_bounds__(128) gen_start_kernel(int N, unsigned n, const int* __restrict__ starts,
+                                                        uint4* __restrict__ out, unsigned* gn) {
+  const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q == 0) gn[0] = n;
+  if (q >= n) return;
+  const int sc = starts[q], i = geti(sc), j = getj(sc), k = getk(sc), l = getl(sc);
+  const uint32_t L = 1u << (N - 1), Lj = L >> j, Li = L >> i;
+  const uint32_t ld = ((i > 0) ? (L >> (i - 1)) : 0u) | (1u << (N - k));
+  const uint32_t rd = (L >> (i + 1)) | (1u << (l - 1));
+  out[q] = settle(ld, rd, 1u | L | Li | Lj, 1, (j == N - 1) ? 3 : 4, (uint32_t)sc);
+}
+
+// One queen more for every state below the preset; the others move on (last: as records).
+__global__ void __launch_bounds__(128) gen_level_kernel(int N, int preset, bool last, const uint4* __restrict__ in,
+                                                        uint4* __restrict__ out, unsigned cap, unsigned* gn, int level,
+                                                        unsigned* err) {
+  const unsigned n = gn[level];
+  for (unsigned q0 = blockIdx.x * blockDim.x; q0 < n; q0 += gridDim.x * blockDim.x) {
+    const unsigned q = q0 + threadIdx.x;
+    uint4 s = make_uint4(0, 0, 0, 0);
+    uint32_t fr = 0;
+    bool keep = false;
+    int row = 0, queens = 0;
+    uint32_t ijkl = 0;
+    if (q < n) {
+      s = in[q];
+      ijkl = s.w & 0xFFFFFu; row = (int)(s.w >> 20) & 31; queens = (int)(s.w >> kQueens);
+      keep = queens >= preset;
+      if (!keep) {
+        const int sh = N - 1 - row;
+        if (sh < 0) atomicOr(err, DERR_SHIFT);           // the reference raises on a negative shift here
+        else {
+          const uint32_t L = 1u << (N - 1), Lj = L >> getj((int)ijkl);
+          const uint32_t LD = Lj | (L >> getl((int)ijkl)), RD = Lj | (1u << getk((int)ijkl));
+          fr = ~(s.x | s.y | s.z | (LD >> sh) | (RD << sh)) & ((1u << N) - 1u);
+        }
+      }
+    }
+    unsigned at = take_slots(&gn[level + 1], keep ? 1u : (unsigned)__popc(fr));
+    const uint32_t mask = last ? (1u << kQueens) - 1u : ~0u;
+    if (keep) {
+      if (at < cap) out[at] = make_uint4(s.x, s.y, s.z, s.w & mask);
+    } else {
+      while (fr) {
+        const uint32_t bit = fr & (0u - fr);
+        fr ^= bit;
+        uint4 c = settle((s.x | bit) << 1, (s.y | bit) >> 1, s.z | bit, row + 1, queens + 1, ijkl);
+        c.w &= mask;
+        if (at < cap) out[at] = c;
+        at++;
+      }
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -137,6 +211,20 @@ __global__ void __launch_bounds__(128) query_level_kernel(uint32_t N, uint32_t T
 }
 
 }  // namespace
+
+cudaError_t launch_generate(int N, int preset, unsigned n_starts, const int* starts, uint4* buf0, uint4* buf1, unsigned cap,
+                            unsigned* gn, unsigned* err, int sms, cudaStream_t st) {
+  if (n_starts == 0) return cudaSuccess;
+  const int levels = gen_levels(preset);
+  uint4* buf[2] = {buf0, buf1};
+  gen_start_kernel<<<(n_starts + 127) / 128, 128, 0, st>>>(N, n_starts, starts, buf[0], gn);
+  for (int l = 0; l < levels; l++) {
+    const unsigned need = l == 0 ? (n_starts + 127) / 128 : 8u * (unsigned)sms;
+    gen_level_kernel<<<need < 8u * (unsigned)sms ? need : 8u * (unsigned)sms, 128, 0, st>>>(
+        N, preset, l + 1 == levels, buf[l & 1], buf[(l + 1) & 1], cap, gn, l, err);
+  }
+  return cudaGetLastError();
+}
 
 cudaError_t launch_query(const QueryParam& p, const QueryBuffers& b, bool wide, int levels, int sms, cudaStream_t st) {
   if (wide) query_kernel<true><<<1, 1024, 0, st>>>(p, b);

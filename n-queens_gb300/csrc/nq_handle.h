@@ -45,9 +45,11 @@ struct Ctrl {
 
 // Control block of a single-N run (device, zeroed before each run):
 //   job total (u64), queue cursor (u64), error word (u32), deepest schedule (u32),
-//   split counters (u64 subtasks, u64 allocation cursor).
+//   split counters (u64 queue length, u64 unused); behind them, zeroed when a list is
+//   generated on the device: the states of each level (u32 x 7) and its error word (u32).
 namespace ctl {
 constexpr size_t kTotal = 0, kCursor = 8, kErr = 16, kTmax = 20, kSplit = 24, kBytes = 40;
+constexpr size_t kGen = 40, kGenErr = 68, kAll = 72;
 }
 
 }  // namespace nq
@@ -58,7 +60,8 @@ struct nq_handle {
   cudaStream_t stream = nullptr;
   int block = 64, grid = 0, split = -1;    // split: -1 automatic, 0..3 fixed depth
   std::string err;
-  nq::DevBuf rec, root, info, sched, per_task, ctrl, nsub, sroot, sinfo;
+  nq::DevBuf rec, root, info, sched, per_task, ctrl, sroot, sinfo;
+  nq::DevBuf gen, starts;                // device generator: the other state buffer, the start list
   nq::DevBuf utasks, uconfs, uctl;       // unique counter (nq_count_unique)
   // completion queries: a stream and buffers of their own, so a query may run beside an asynchronous count
   cudaStream_t q_stream = nullptr;

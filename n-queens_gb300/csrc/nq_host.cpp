@@ -4,9 +4,8 @@
 //    their preset-queen expansion (14Bit_codon_GPU/356Py_savesp_narrow.py:
 //    2714-2926).  The start-constellation set is built sequentially (the
 //    rotation check depends on insertion order, 356Py:2850-2880); the preset
-//    expansion of each start constellation is independent (its subconst
-//    cache and signature set are cleared per constellation, 356Py:2886-2889)
-//    and runs on all host threads.  Output order: ascending packed ijkl, then
+//    expansion of each start constellation is independent and runs on the host
+//    threads.  Output order: ascending packed ijkl, then
 //    the reference's expansion order within a constellation.
 // 2. build_completion_tasks: DFS tasks for boards with pre-placed queens (no
 //    reference counterpart: the reference only counts whole boards).  Rows
@@ -17,7 +16,6 @@
 //    the host until there are enough tasks to fill the GPU.
 #include <algorithm>
 #include <atomic>
-#include <cstring>
 #include <thread>
 #include <vector>
 
@@ -44,68 +42,20 @@ inline int canon(int x, int N) {   // jasmin, 356Py:2739-2756
   return x;
 }
 
-inline uint64_t hmix(uint64_t x) {
-  x ^= x >> 31; x *= 0x7fb5d329728ea185ULL; x ^= x >> 27; x *= 0x81dadef4bc2dd44dULL; x ^= x >> 33;
-  return x;
-}
-
-// Open-addressing set of fixed-width keys with O(1) clear (generation stamps).
-template <int W>
-struct KeySet {
-  std::vector<uint64_t> keys;
-  std::vector<uint32_t> stamp;
-  uint32_t gen = 1;
-  size_t count = 0, mask = 0;
-  KeySet() { resize(1 << 12); }
-  void resize(size_t cap) {
-    std::vector<uint64_t> ok;
-    std::vector<uint32_t> os;
-    ok.swap(keys); os.swap(stamp);
-    keys.assign(cap * W, 0); stamp.assign(cap, 0); mask = cap - 1; count = 0;
-    for (size_t s = 0; s < os.size(); s++)
-      if (os[s] == gen) insert(&ok[s * W]);
-  }
-  void clear() { gen++; count = 0; if (gen == 0) { std::fill(stamp.begin(), stamp.end(), 0); gen = 1; } }
-  // true when the key was absent (and is now present)
-  bool insert(const uint64_t* k) {
-    if ((count + 1) * 2 > stamp.size()) resize(stamp.size() * 2);
-    uint64_t h = 0x243f6a8885a308d3ULL;
-    for (int w = 0; w < W; w++) h = hmix(h ^ k[w]);
-    size_t p = h & mask;
-    while (stamp[p] == gen) {
-      if (std::memcmp(&keys[p * W], k, W * sizeof(uint64_t)) == 0) return false;
-      p = (p + 1) & mask;
-    }
-    std::memcpy(&keys[p * W], k, W * sizeof(uint64_t));
-    stamp[p] = gen; count++;
-    return true;
-  }
-};
-
+// The reference looks every expanded state up (set_pre_queens_cached's subconst cache, 356Py:2773-2784, and
+// the signatures up to preset 5, :2820-2824) and drops repeats.  No state occurs twice: enumerated for every
+// N of 5..27 and presets 4, 5 and 6 (15.7 M states at N=27), and from preset 7 on the reference does not look.
+// So nothing is looked up here; the list is the same, record for record.
 struct Expander {
   int N, preset, k, l;
   uint64_t board_mask;
-  KeySet<6> cache;     // (ld, rd, col, LD, RD, row | queens<<8)
-  KeySet<4> sigs;      // (ld, rd, col, row)
   std::vector<GenRecord>* out;
   uint32_t base;
   int err = 0;
 
-  void cached(uint64_t ld, uint64_t rd, uint64_t col, int row, int queens, uint64_t LD, uint64_t RD) {
-    if (err) return;
-    if (preset < 7) {   // set_pre_queens_cached bypasses its cache for preset >= 7 (356Py:2773-2784)
-      const uint64_t key[6] = {ld, rd, col, LD, RD, (uint64_t)row | ((uint64_t)queens << 8)};
-      if (!cache.insert(key)) return;
-    }
-    expand(ld, rd, col, row, queens, LD, RD);
-  }
   void expand(uint64_t ld, uint64_t rd, uint64_t col, int row, int queens, uint64_t LD, uint64_t RD) {
-    if (row == k || row == l) { cached(ld << 1, rd >> 1, col, row + 1, queens, LD, RD); return; }
+    while (row == k || row == l) { ld <<= 1; rd >>= 1; row++; }     // rows of the side queens
     if (queens == preset) {
-      if (preset <= 5) {  // signature prune only up to preset 5 (356Py:2820-2824)
-        const uint64_t s[4] = {ld, rd, col, (uint64_t)row};
-        if (!sigs.insert(s)) return;
-      }
       out->push_back(GenRecord{ld, rd, col, ((uint32_t)row << 20) | base});
       return;
     }
@@ -115,17 +65,25 @@ struct Expander {
     while (fr) {
       const uint64_t bit = fr & (0 - fr);
       fr &= fr - 1;
-      cached((ld | bit) << 1, (rd | bit) >> 1, col | bit, row + 1, queens + 1, LD, RD);
+      expand((ld | bit) << 1, (rd | bit) >> 1, col | bit, row + 1, queens + 1, LD, RD);
       if (err) return;
     }
   }
 };
 
-bool rotated_present(const std::vector<uint8_t>& S, int i, int j, int k, int l, int N) {
+// Set of packed ijkl values of board N (below N << 15).
+struct IjklSet {
+  std::vector<uint64_t> w;
+  explicit IjklSet(int N) : w((size_t)N << 9, 0) {}
+  bool has(int x) const { return (w[(size_t)x >> 6] >> (x & 63)) & 1; }
+  void add(int x) { w[(size_t)x >> 6] |= 1ull << (x & 63); }
+};
+
+bool rotated_present(const IjklSet& S, int i, int j, int k, int l, int N) {
   const int r1 = ((N - 1 - k) << 15) + ((N - 1 - l) << 10) + (j << 5) + i;
   const int r2 = ((N - 1 - j) << 15) + ((N - 1 - i) << 10) + ((N - 1 - l) << 5) + (N - 1 - k);
   const int r3 = (l << 15) + (k << 10) + ((N - 1 - i) << 5) + (N - 1 - j);
-  return S[r1] || S[r2] || S[r3];
+  return S.has(r1) || S.has(r2) || S.has(r3);
 }
 
 }  // namespace
@@ -134,11 +92,11 @@ int start_constellations(int N, std::vector<int>& starts) {
   starts.clear();
   if (N < 5 || N > kMaxN) return -1;
   const int halfN = (N + 1) / 2, N1 = N - 1, N2 = N - 2;
-  // S: the set of start constellations (random access for the rotation check),
-  // with its members also listed so nothing scans all 2^20 packed ijkl values.
-  std::vector<uint8_t> S(1u << 20, 0);
-  std::vector<int> members;
-  auto add = [&](int x) { if (!S[x]) { S[x] = 1; members.push_back(x); } };
+  // S: the set of start constellations, for the rotation check; C: their canonical
+  // forms (jasmin), read out in ascending packed order (4 KB a board row each, so both
+  // stay in the cache; byte flags and a sort took 178 us at N=16, these 108)
+  IjklSet S(N), C(N);
+  auto add = [&](int x) { if (!S.has(x)) { S.add(x); C.add(canon(x, N)); } };
   if (N % 2 == 1) {   // centre column of odd boards (356Py:2857-2867)
     const int c = N / 2;
     for (int l = c + 1; l < N1; l++)
@@ -157,11 +115,8 @@ int start_constellations(int N, std::vector<int>& starts) {
       }
   for (int j = 1; j < N2; j++)      // queen in a corner (356Py:2880)
     for (int l = j + 1; l < N1; l++) add(to_ijkl(0, j, 0, l));
-  // canonical forms (jasmin), distinct, in ascending packed order
-  starts.reserve(members.size());
-  for (int x : members) starts.push_back(canon(x, N));
-  std::sort(starts.begin(), starts.end());
-  starts.erase(std::unique(starts.begin(), starts.end()), starts.end());
+  for (size_t q = 0; q < C.w.size(); q++)
+    for (uint64_t b = C.w[q]; b; b &= b - 1) starts.push_back((int)(q << 6) | __builtin_ctzll(b));
   return 0;
 }
 
@@ -189,14 +144,16 @@ int expand_starts(int N, int preset, const std::vector<int>& starts, size_t s0, 
       const uint64_t ld = ((i > 0) ? (L >> (i - 1)) : 0) | (1ull << (N - k));
       const uint64_t rd = (L >> (i + 1)) | (1ull << (l - 1));
       const uint64_t col = 1 | L | Li | Lj;
-      e.cache.clear(); e.sigs.clear();
       e.k = k; e.l = l; e.out = &parts[q]; e.base = (uint32_t)to_ijkl(i, j, k, l);
-      e.cached(ld, rd, col, 1, (j == N1) ? 3 : 4, Lj | Ll, Lj | (1ull << k));
+      e.expand(ld, rd, col, 1, (j == N1) ? 3 : 4, Lj | Ll, Lj | (1ull << k));
       if (e.err) { err = 1; break; }
     }
   };
   if (threads <= 0) threads = (int)std::max(1u, std::thread::hardware_concurrency());
-  threads = (int)std::min<size_t>((size_t)threads, std::max<size_t>(1, ns / 8));
+  // about 15 ns a record and 60 us a thread: a thread for every 20000 records (about (N - 4)^(preset - 4) a start)
+  double est = (double)ns;
+  for (int q = 4; q < preset; q++) est *= (double)std::max(1, N - q);
+  threads = (int)std::min<double>((double)std::min<size_t>((size_t)threads, std::max<size_t>(1, ns / 8)), std::max(1.0, est / 20000.0));
   if (threads <= 1) worker();
   else {
     std::vector<std::thread> th;

@@ -183,6 +183,7 @@ template <int D>
 __global__ void __launch_bounds__(256) prepare_split_kernel(const PrepareSplit a) {
   const int64_t m = a.m_dev ? (int64_t)*a.m_dev : a.m;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (D == 0 && t == 0) *a.qn = (unsigned long long)m;
   if ((int64_t)blockIdx.x * blockDim.x >= m) return;
   const unsigned lane = threadIdx.x & 31u;
   Root rt = {0, 0, 0, 0};
