@@ -634,8 +634,12 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
         if (pool_n == 0u) {
           if (drained) { exhausted = true; break; }
           unsigned long long base = 0;
-          if (lane == 0) base = atomicAdd(a.cursor, (unsigned long long)chunk);
-          base = __shfl_sync(FULL, base, 0);
+          if (chunk0 < 32u) {                    // the shares cover the queue: no cursor
+            base = (unsigned long long)(blockIdx.x * (BLOCK / 32) + (threadIdx.x >> 5)) * chunk0;
+          } else {
+            if (lane == 0) base = atomicAdd(a.cursor, (unsigned long long)chunk);
+            base = __shfl_sync(FULL, base, 0);
+          }
           const unsigned long long left = base < m ? m - base : 0ull;
           pool_n = left < chunk ? (unsigned)left : chunk;
           pool_at = 0;
