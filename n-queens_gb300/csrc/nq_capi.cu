@@ -83,13 +83,13 @@ int run_records(nq_handle* h, int N, const uint4* d_rec, int64_t m, int start_mi
   const int maxt = maxt_for(N, start_min);
   const int D = h->split >= 0 ? h->split : choose_split(m, maxt);
   NQ_CUDA(h, cudaSetDevice(h->device));
-  NQ_CUDA(h, h->info.ensure((size_t)m * sizeof(uint2)));
+  NQ_CUDA(h, h->info.ensure((size_t)m * sizeof(uint32_t)));
   NQ_CUDA(h, h->sched.ensure((size_t)m * (maxt + 1) * sizeof(uint32_t)));
   NQ_CUDA(h, h->ctrl.ensure(ctl::kAll));
   if (int s = h->ensure_pinned(ctl::kBytes)) return s;
   unsigned char* c = (unsigned char*)h->ctrl.p;
   PrepareSplit P;
-  P.N = N; P.m = m; P.m_dev = m_dev; P.rec = d_rec; P.info = (uint2*)h->info.p; P.sched = (uint32_t*)h->sched.p; P.sw = maxt + 1;
+  P.N = N; P.m = m; P.m_dev = m_dev; P.rec = d_rec; P.info = (uint32_t*)h->info.p; P.sched = (uint32_t*)h->sched.p; P.sw = maxt + 1;
   P.err = (unsigned int*)(c + ctl::kErr); P.tmax = (unsigned int*)(c + ctl::kTmax);
   P.per_task = d_per_task; P.qn = (unsigned long long*)(c + ctl::kSplit); P.total = (unsigned long long*)(c + ctl::kTotal);
   // Queue capacity: a bound (each level places a queen in one of at most N - 2, N - 3, ... columns) where that
@@ -189,11 +189,21 @@ int query_task(int N, int k, const int* rows, const int* cols, QueryParam* p, bo
   }
   p->root = make_uint4(root[0], root[1], root[2], root[3]);
   p->N = (uint32_t)N; p->T = (uint32_t)(n - 2); p->target = 0;
-  *wide = N < 6;                       // compact words keep RA's bits N-1..N apart from the shift in bits 0-4
+  *wide = false;
   for (int d = 0; d <= n - 2; d++) *wide = *wide || !compact_fits(ops[d], N);
+  p->words_wide = *wide ? 1u : 0u;
   for (int d = 0; d <= n - 2; d++)
     p->words[d] = *wide ? make_uint2(pack_wide_x(ops[d]) ^ W_NOLOOK, ops[d].ra) : make_uint2(pack_compact(ops[d]) ^ C_NOLOOK, 0u);
   return 1;
+}
+
+// A compact query's words in the wide form.
+void widen_query(QueryParam* p) {
+  for (uint32_t d = 0; d <= p->T; d++) {
+    const Op o = unpack_compact(p->words[d].x ^ C_NOLOOK, (int)p->N, false);
+    p->words[d] = make_uint2(pack_wide_x(o) ^ W_NOLOOK, o.ra);
+  }
+  p->words_wide = 1;
 }
 
 }  // namespace
@@ -612,6 +622,12 @@ uint64_t start_bound(int N, int preset, int start) {
   return b;
 }
 
+uint64_t board_bound(int N, int p, const std::vector<int>& starts) {
+  uint64_t b = 0;
+  for (int s : starts) b += std::max<uint64_t>(1, start_bound(N, p, s));
+  return b;
+}
+
 int count_generated(nq_handle* h, int N, int p, const std::vector<int>& starts, size_t s_begin, size_t s_end,
                     uint64_t* total) {
   cudaStream_t st = h->stream;
@@ -742,25 +758,21 @@ struct nq_batch {
   std::vector<nq_job> jobs;
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr;
-  DevBuf rec, root, info, sched, ctrl, nsub, sroot, sinfo;
-  int64_t m = 0;        // tasks
-  int64_t ms = 0;       // queued subtasks (every job's split output, job after job)
+  DevBuf info, sched, ctrl, sroot, sinfo;  // tasks (jobs of one board share them), and the queue
+  int64_t m = 0;        // sources of all jobs (records, query frames)
+  int64_t ms = 0;       // queued items (every job's split output, job after job)
   int maxt = 1, sw = 2, grid = 0, block = 128;
   bool big = false;                        // some job's queue items may count 2^32: u64 per-lane counters
-  bool wide = true;                        // 8-byte schedule words (completion tasks); compact otherwise
-  std::vector<int64_t> job_off, job_m;     // task range per job
-  std::vector<int64_t> sub_off, sub_m;     // subtask range per job
-  std::vector<int> job_maxt, job_rows, job_split;   // job_rows: rows left, as choose_split takes them
+  bool wide = false;                       // 8-byte schedule words (a query with far-reaching steps); compact otherwise
+  std::vector<int64_t> sub_off, sub_m;     // queue range per job
+  std::vector<int> job_maxt;
   std::vector<uint64_t> fixed_total;       // counts settled at build time (small tasks, full boards)
   uint64_t* h_out = nullptr;               // pinned: totals per job + cursor/err
+  unsigned char* stage = nullptr;          // pinned: the build's uploads
   cudaGraphExec_t graph = nullptr;
   bool submitted = false;
   int64_t device_bytes = 0;
-  int64_t h2d_bytes = 0;                   // host->device bytes of the build (records, host-built tasks)
-  cudaError_t set_ordered() {
-    for (DevBuf* d : {&rec, &root, &info, &sched, &ctrl, &nsub, &sroot, &sinfo}) d->ordered = stream;
-    return cudaSuccess;
-  }
+  int64_t h2d_bytes = 0;                   // host->device bytes of the build (start lists, queries, job table)
 };
 
 namespace {
@@ -774,7 +786,7 @@ int batch_enqueue(nq_batch* b, int use_graph) {
     cudaError_t e = cudaMemsetAsync(c, 0, cb, st);
     if (e != cudaSuccess) return e;
     TaskArrays ta;
-    ta.root = (uint4*)b->root.p; ta.info = (uint2*)b->info.p; ta.sched = b->sched.p; ta.sw = b->sw; ta.wide = b->wide;
+    ta.info = (uint32_t*)b->info.p; ta.sched = b->sched.p; ta.sw = b->sw; ta.wide = b->wide;
     DfsLaunch L;
     L.tasks = ta; L.sroot = (const uint4*)b->sroot.p; L.sinfo = (const uint2*)b->sinfo.p;
     L.m = b->ms; L.cursor = (unsigned long long*)(c + (size_t)nj * 8);
@@ -826,15 +838,20 @@ void nq_batch_destroy(nq_batch* b) {
   cudaSetDevice(b->h->device);
   if (b->stream) cudaStreamSynchronize(b->stream);
   if (b->graph) cudaGraphExecDestroy(b->graph);
-  b->rec.release(); b->root.release(); b->info.release(); b->sched.release(); b->ctrl.release();
-  b->nsub.release(); b->sroot.release(); b->sinfo.release();
+  for (DevBuf* d : {&b->info, &b->sched, &b->ctrl, &b->sroot, &b->sinfo}) d->release();
   if (b->stream) cudaStreamSynchronize(b->stream);   // this batch's own frees only
   b->h->pin_put(b->h_out);
+  b->h->pin_put(b->stage);
   if (b->done) cudaEventDestroy(b->done);
   if (b->stream) cudaStreamDestroy(b->stream);
   delete b;
 }
 
+// Build, one synchronisation in all: the boards' records are generated on the device and prepared, each
+// query is expanded by one block (small boards' start lists, queries and tables are the only uploads), every
+// list's split is counted, the queue is allocated, and the jobs' items are written job after job.  Jobs of
+// one board share its tasks and its counted list; each has its own items.  Building 64 mixed jobs of N=9..16
+// on the host (generator, breadth-first searches, staging, two split launches a job) took 19 ms.
 int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out) {
   if (!h || !out || njobs <= 0 || !jobs) return h ? h->fail(NQ_EINVAL, "batch: bad arguments") : NQ_EINVAL;
   *out = nullptr;
@@ -844,173 +861,231 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
   b->h = h;
   b->jobs.assign(jobs, jobs + njobs);
   b->block = h->block;
-  b->job_off.assign(njobs, 0); b->job_m.assign(njobs, 0); b->job_maxt.assign(njobs, 1); b->job_rows.assign(njobs, 1); b->fixed_total.assign(njobs, 0);
-  // Build: count jobs (N >= 6) become constellation records prepared on the
-  // device; count jobs with N <= 5 and completion jobs become host tasks.
-  struct Seg { int job, N; int64_t rec_off, m; };
-  std::vector<Seg> segs;
-  std::vector<nq_record> recs;
-  std::vector<HostTask> htasks;
-  std::vector<int64_t> job_host_begin(njobs, -1), job_host_end(njobs, -1);
-  // The generator is deterministic in (N, preset): jobs that repeat a pair reuse
-  // its records (each job still gets its own task segment and job id).
-  struct Gen { std::vector<GenRecord> v; int smin; };
-  std::map<std::pair<int, int>, Gen> generated;
-  int maxt = 1;
+  b->job_maxt.assign(njobs, 1); b->fixed_total.assign(njobs, 0);
+  b->sub_off.assign(njobs, 0); b->sub_m.assign(njobs, 0);
+  auto bad = [&](int status, const char* what, int j) {
+    nq_batch_destroy(b);
+    return h->fail(status, "batch job %d: %s", j, what);
+  };
+  // ---- the lists: one per board (N, preset) and one per query
+  struct List { int N = 0, rows = 0, T = 0; uint64_t cap = 0; bool query = false; int D = 0; uint32_t src0 = 0, task0 = 0; };
+  struct Board { int p; uint32_t list; std::vector<int> starts; std::vector<GenRecord> recs; size_t starts_at = 0; };
+  std::vector<List> lists;
+  std::vector<Board> boards;
+  std::vector<BatchQuery> queries;
+  std::vector<int> job_list(njobs, -1);
+  std::map<std::pair<int, int>, uint32_t> board_list;
+  uint64_t sources = 0;                          // all jobs' sources, roughly
   for (int j = 0; j < njobs; j++) {
     const nq_job& J = jobs[j];
-    if (J.N < 1 || J.N > kMaxN || J.k < 0 || J.k > 8) { nq_batch_destroy(b); return h->fail(NQ_EINVAL, "batch job %d: bad N or k", j); }
+    if (J.N < 1 || J.N > kMaxN || J.k < 0 || J.k > 8) return bad(NQ_EINVAL, "bad N or k", j);
+    if (J.kind != NQ_JOB_COUNT && J.kind != NQ_JOB_COMPLETION) return bad(NQ_EINVAL, "unknown kind", j);
     if (J.kind == NQ_JOB_COUNT && J.N >= 6) {
       const int p = J.preset > 0 ? J.preset : preset_for(J.N);
-      auto it = generated.find({J.N, p});
-      if (it == generated.end()) {
-        Gen g;
-        const int s = gen_constellations(J.N, p, g.v, 0);
-        if (s != 0) { nq_batch_destroy(b); return h->fail(s == -2 ? NQ_EPRESET : NQ_EINVAL, "batch job %d: generator failed", j); }
-        g.smin = 64;
-        for (auto& r : g.v) g.smin = std::min<int>(g.smin, (int)(r.startijkl >> 20));
-        it = generated.emplace(std::make_pair(J.N, p), std::move(g)).first;
+      if (p < 4) return bad(NQ_EPRESET, "generator failed (preset below 4)", j);
+      auto it = board_list.find({J.N, p});
+      if (it == board_list.end()) {
+        Board bd;
+        bd.p = p; bd.list = (uint32_t)lists.size();
+        if (start_constellations(J.N, bd.starts) != 0) return bad(NQ_EINVAL, "generator failed", j);
+        List l;
+        l.N = J.N; l.cap = board_bound(J.N, p, bd.starts); l.rows = maxt_for(J.N, p - 3);
+        if (p > 8 || l.cap > kGenRecords) {      // more than the device generator's buffers: the host's list
+          const int s = gen_constellations(J.N, p, bd.recs, 0);
+          if (s != 0) return bad(s == -2 ? NQ_EPRESET : NQ_EINVAL, "generator failed", j);
+          std::vector<int>().swap(bd.starts);
+          l.cap = bd.recs.size();
+        }
+        it = board_list.emplace(std::make_pair(J.N, p), bd.list).first;
+        lists.push_back(l);
+        boards.push_back(std::move(bd));
       }
-      const std::vector<GenRecord>& v = it->second.v;
-      Seg sg{j, J.N, (int64_t)recs.size(), (int64_t)v.size()};
-      for (auto& g : v) recs.push_back(nq_record{(uint32_t)g.ld, (uint32_t)g.rd, (uint32_t)g.col, g.startijkl});
-      segs.push_back(sg);
-      b->job_rows[j] = b->job_maxt[j] = maxt_for(J.N, it->second.smin);
-      maxt = std::max(maxt, b->job_maxt[j]);
-    } else if (J.kind == NQ_JOB_COUNT || J.kind == NQ_JOB_COMPLETION) {
+      job_list[j] = (int)it->second;
+      sources += lists[it->second].cap / 2;      // the bound is about twice the records
+    } else {
       int rows[8], cols[8];
       const int k = (J.kind == NQ_JOB_COUNT) ? 0 : J.k;
       for (int q = 0; q < k; q++) { rows[q] = J.rows[q]; cols[q] = J.cols[q]; }
-      int mt = 0;
-      const int64_t before = (int64_t)htasks.size();
-      const int s = build_completion_tasks(J.N, k, rows, cols, 4096, (uint32_t)j, htasks, &mt);
-      if (s < 0) { nq_batch_destroy(b); return h->fail(NQ_EINVAL, "batch job %d: bad pre-placed queens", j); }
-      if (s == 2) b->fixed_total[j] = 1;
-      job_host_begin[j] = before; job_host_end[j] = (int64_t)htasks.size();
-      b->job_maxt[j] = std::max(1, mt);
-      b->job_rows[j] = mt + 2;             // mt + 1 free rows
-      maxt = std::max(maxt, b->job_maxt[j]);
-    } else {
-      nq_batch_destroy(b);
-      return h->fail(NQ_EINVAL, "batch job %d: unknown kind %d", j, J.kind);
+      BatchQuery q{};
+      bool wide = false;
+      const int s = query_task(J.N, k, rows, cols, &q.p, &wide, &b->fixed_total[j]);
+      if (s < 0) return bad(NQ_EINVAL, "bad pre-placed queens", j);
+      if (s == 0) continue;
+      b->wide = b->wide || wide;
+      List l;
+      l.N = J.N; l.T = (int)q.p.T; l.rows = l.T + 2; l.query = true;
+      q.list = (uint32_t)lists.size();
+      job_list[j] = (int)lists.size();
+      lists.push_back(l);
+      queries.push_back(q);
     }
   }
-  if (maxt >= kMaxDepth) { nq_batch_destroy(b); return h->fail(NQ_ESTACK, "batch: schedule too deep"); }
-  b->maxt = maxt; b->sw = maxt + 1;
-  b->wide = !htasks.empty();             // constellation-only batches keep the compact 4-byte words
-  const int64_t m_rec = (int64_t)recs.size(), m_host = (int64_t)htasks.size();
-  b->m = m_rec + m_host;
-  for (auto& sg : segs) { b->job_off[sg.job] = sg.rec_off; b->job_m[sg.job] = sg.m; }
-  for (int j = 0; j < njobs; j++)
-    if (job_host_begin[j] >= 0) { b->job_off[j] = m_rec + job_host_begin[j]; b->job_m[j] = job_host_end[j] - job_host_begin[j]; }
-  const size_t cb = Ctrl::bytes(njobs);
-  cudaError_t e;
-  if ((e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking)) != cudaSuccess ||
-      (e = cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming)) != cudaSuccess ||
-      (e = b->set_ordered()) != cudaSuccess ||
-      (e = ((b->h_out = (uint64_t*)h->pin_get(cb)) ? cudaSuccess : cudaErrorMemoryAllocation)) != cudaSuccess ||
-      (e = b->ctrl.ensure(cb)) != cudaSuccess ||
-      (e = b->root.ensure((size_t)std::max<int64_t>(b->m, 1) * sizeof(uint4))) != cudaSuccess ||
-      (e = b->info.ensure((size_t)std::max<int64_t>(b->m, 1) * sizeof(uint2))) != cudaSuccess ||
-      (e = b->sched.ensure((size_t)std::max<int64_t>(b->m, 1) * b->sw * (b->wide ? sizeof(uint2) : sizeof(uint32_t)))) !=
-          cudaSuccess ||
-      (e = b->rec.ensure((size_t)std::max<int64_t>(m_rec, 1) * sizeof(nq_record))) != cudaSuccess) {
-    int st = h->cuda_fail(e, "batch allocation");
-    nq_batch_destroy(b);
-    return st;
+  const unsigned target = queries.size() > 64 ? kQueryTarget / 4 : kQueryTarget;
+  for (BatchQuery& q : queries) {
+    q.p.target = std::min(target, kQueryCap / q.p.N);
+    lists[q.list].cap = (uint64_t)q.p.target * q.p.N;
+    sources += 4 * q.p.target;
+    if (b->wide != (q.p.words_wide != 0)) widen_query(&q.p);
   }
-  b->device_bytes = (int64_t)(b->root.cap + b->info.cap + b->sched.cap + b->rec.cap + b->ctrl.cap);
-  TaskArrays ta;
-  ta.root = (uint4*)b->root.p; ta.info = (uint2*)b->info.p; ta.sched = b->sched.p; ta.sw = b->sw; ta.wide = b->wide;
-  unsigned char* c = (unsigned char*)b->ctrl.p;
-  unsigned int* derr = (unsigned int*)(c + (size_t)njobs * 8 + 8);
-  cudaStream_t st = b->stream;
+  // ---- offsets, split depths, table sizes
+  const size_t nl = lists.size(), nb = boards.size(), nq = queries.size();
+  std::vector<unsigned long long> ends(nl);
+  uint64_t src = 0, ntask = 0, words = 1, rec_cap = 0, gen_cap = 0;
+  size_t n_starts = 0;
+  for (size_t i = 0; i < nl; i++) {
+    List& l = lists[i];
+    l.src0 = (uint32_t)src; l.task0 = (uint32_t)ntask;
+    src += (l.cap + 31) & ~31ull;                // warps stay within a list
+    ends[i] = src;
+    ntask += l.query ? 1 : l.cap;
+    words = std::max<uint64_t>(words, l.query ? l.T + 1 : l.rows + 1);
+    const int levels = l.query ? query_levels(l.rows) : choose_split((int64_t)std::max(sources, l.cap), l.rows);
+    l.D = l.N <= 12 ? 0 : h->split >= 0 ? h->split : l.query && sources > 100000 ? std::min(levels, 1) : levels;
+  }
+  for (Board& bd : boards) {
+    bd.starts_at = n_starts;
+    n_starts += bd.starts.size();
+    rec_cap = std::max(rec_cap, lists[bd.list].cap);
+    if (!bd.starts.empty()) gen_cap = std::max(gen_cap, lists[bd.list].cap);
+  }
+  if (src > 0xFFFFFFFFull || words > (uint64_t)kMaxDepth) { nq_batch_destroy(b); return h->fail(NQ_ENOMEM, "batch: too many tasks"); }
+  b->sw = (int)words;
+  const size_t word = b->wide ? sizeof(uint2) : sizeof(uint32_t), cb = Ctrl::bytes(njobs);
+  auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+  const size_t o_lists = up(nl * 8), o_starts = o_lists + up(nl * sizeof(BatchList)), o_q = o_starts + up(n_starts * sizeof(int));
+  const size_t o_jends = o_q + up(nq * sizeof(BatchQuery)), o_jobs = o_jends + up((size_t)njobs * 8);
+  const size_t tab_bytes = o_jobs + up((size_t)njobs * sizeof(BatchJob));
+  // state: list states, generated levels and deepest schedule per board, error words of generator and prepare
+  const size_t o_gn = up(nl * sizeof(ListState)), o_tmax = o_gn + up(nb * 32), o_err = o_tmax + up(nb * 4);
+  const size_t state_bytes = o_err + 8;
+  cudaError_t e = cudaSuccess;
+  cudaStream_t st = nullptr;
+  DevBuf tab, state, rec, gen, frames, tmp, off;
   int status = NQ_OK;
-  DevBuf jt;                                   // deepest schedule per job (constellation jobs)
-  jt.ordered = st;
-  std::vector<uint32_t> job_deep(njobs, 0);
   do {
-    if ((e = cudaMemsetAsync(c, 0, cb, st)) != cudaSuccess) break;
-    if ((e = jt.ensure((size_t)njobs * sizeof(uint32_t))) != cudaSuccess) break;
-    if ((e = cudaMemsetAsync(jt.p, 0, (size_t)njobs * sizeof(uint32_t), st)) != cudaSuccess) break;
-    if (m_rec && (e = cudaMemcpyAsync(b->rec.p, recs.data(), (size_t)m_rec * sizeof(nq_record), cudaMemcpyHostToDevice, st)) != cudaSuccess) break;
-    b->h2d_bytes = m_rec * (int64_t)sizeof(nq_record) +
-                   m_host * (int64_t)(sizeof(uint4) + sizeof(uint2) + (size_t)b->sw * sizeof(uint2));
-    for (auto& sg : segs)
-      if ((e = launch_prepare(sg.N, sg.m, (const uint4*)b->rec.p + sg.rec_off, ta, sg.rec_off, (uint32_t)sg.job, derr, st,
-                              (unsigned int*)jt.p + sg.job)) != cudaSuccess) break;
-    if (e != cudaSuccess) break;
-    if ((e = cudaMemcpyAsync(job_deep.data(), jt.p, (size_t)njobs * sizeof(uint32_t), cudaMemcpyDeviceToHost, st)) !=
-        cudaSuccess) break;
-    if (m_host) {
-      std::vector<uint4> hr(m_host);
-      std::vector<uint2> hi(m_host);
-      std::vector<uint2> hs((size_t)m_host * b->sw, make_uint2(0, 0));
-      for (int64_t i = 0; i < m_host; i++) {
-        const HostTask& t = htasks[i];
-        hr[i] = make_uint4(t.root[0], t.root[1], t.root[2], t.root[3]);
-        hi[i] = make_uint2(t.info, t.job);
-        for (int d = 0; d <= t.T; d++) hs[(size_t)i * b->sw + d] = make_uint2(t.sched[2 * d] ^ W_NOLOOK, t.sched[2 * d + 1]);
+    if ((e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming)) != cudaSuccess) break;
+    st = b->stream;
+    for (DevBuf* d : {&b->info, &b->sched, &b->ctrl, &b->sroot, &b->sinfo, &tab, &state, &rec, &gen, &frames, &tmp, &off})
+      d->ordered = st;
+    b->h_out = (uint64_t*)h->pin_get(std::max(cb, state_bytes));
+    b->stage = (unsigned char*)h->pin_get(tab_bytes);
+    if (!b->h_out || !b->stage) { e = cudaErrorMemoryAllocation; break; }
+    if ((e = b->ctrl.ensure(cb)) != cudaSuccess || (e = tab.ensure(tab_bytes)) != cudaSuccess ||
+        (e = state.ensure(state_bytes)) != cudaSuccess || (e = b->info.ensure(std::max<uint64_t>(ntask, 1) * 4)) != cudaSuccess ||
+        (e = b->sched.ensure(std::max<uint64_t>(ntask, 1) * words * word)) != cudaSuccess ||
+        (e = frames.ensure(std::max<uint64_t>(src, 1) * sizeof(uint4))) != cudaSuccess ||
+        (e = off.ensure(std::max<uint64_t>(src, 1) * 4)) != cudaSuccess ||
+        (nb && (e = rec.ensure(std::max<uint64_t>(rec_cap, 1) * sizeof(uint4))) != cudaSuccess) ||
+        (gen_cap && (e = gen.ensure(gen_cap * sizeof(uint4))) != cudaSuccess) ||
+        (nq && (e = tmp.ensure(src * sizeof(uint4))) != cudaSuccess)) break;
+    unsigned char *dt = (unsigned char*)tab.p, *ds = (unsigned char*)state.p;
+    // ---- upload the lists, start lists and queries
+    BatchList* hl = (BatchList*)(b->stage + o_lists);
+    if (nl) std::memcpy(b->stage, ends.data(), nl * 8);
+    for (size_t i = 0; i < nl; i++) hl[i] = BatchList{lists[i].src0, lists[i].task0, lists[i].query ? 1u : 0u, (uint32_t)lists[i].D};
+    for (const Board& bd : boards)
+      if (!bd.starts.empty())
+        std::memcpy(b->stage + o_starts + bd.starts_at * sizeof(int), bd.starts.data(), bd.starts.size() * sizeof(int));
+    BatchQuery* hq = (BatchQuery*)(b->stage + o_q);
+    for (size_t i = 0; i < nq; i++) {
+      hq[i] = queries[i];
+      hq[i].src0 = lists[queries[i].list].src0; hq[i].task = lists[queries[i].list].task0;
+    }
+    if ((e = cudaMemcpyAsync(dt, b->stage, o_jends, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+        (e = cudaMemsetAsync(ds, 0, state_bytes, st)) != cudaSuccess) break;
+    b->h2d_bytes = (int64_t)o_jends;
+    ListState* dstate = (ListState*)ds;
+    unsigned int* derr = (unsigned int*)(ds + o_err);
+    TaskArrays ta;
+    ta.info = (uint32_t*)b->info.p; ta.sched = b->sched.p; ta.sw = b->sw; ta.wide = b->wide;
+    // ---- boards: generate (or upload) the records, prepare them into the board's tasks
+    for (size_t i = 0; i < nb && e == cudaSuccess; i++) {
+      const Board& bd = boards[i];
+      const List& l = lists[bd.list];
+      const uint4* drec = (const uint4*)rec.p;
+      const unsigned int* dn = nullptr;
+      std::vector<nq_record> packed;
+      if (!bd.starts.empty()) {
+        const int levels = gen_levels(bd.p);
+        uint4* buf[2] = {(uint4*)rec.p, (uint4*)gen.p};
+        unsigned int* gn = (unsigned int*)(ds + o_gn + i * 32);
+        e = launch_generate(l.N, bd.p, (unsigned)bd.starts.size(), (const int*)(dt + o_starts) + bd.starts_at, buf[0], buf[1],
+                            (unsigned)l.cap, gn, derr, h->sms, st);
+        drec = buf[levels & 1];
+        dn = gn + levels;
+      } else if (l.cap) {
+        packed.resize(l.cap);
+        for (size_t r = 0; r < l.cap; r++)
+          packed[r] = nq_record{(uint32_t)bd.recs[r].ld, (uint32_t)bd.recs[r].rd, (uint32_t)bd.recs[r].col, bd.recs[r].startijkl};
+        e = cudaMemcpyAsync(rec.p, packed.data(), l.cap * sizeof(nq_record), cudaMemcpyHostToDevice, st);
+        b->h2d_bytes += (int64_t)(l.cap * sizeof(nq_record));
       }
-      if ((e = cudaMemcpyAsync((uint4*)b->root.p + m_rec, hr.data(), m_host * sizeof(uint4), cudaMemcpyHostToDevice, st)) != cudaSuccess) break;
-      if ((e = cudaMemcpyAsync((uint2*)b->info.p + m_rec, hi.data(), m_host * sizeof(uint2), cudaMemcpyHostToDevice, st)) != cudaSuccess) break;
-      if ((e = cudaMemcpyAsync((uint2*)b->sched.p + (size_t)m_rec * b->sw, hs.data(), hs.size() * sizeof(uint2),
-                               cudaMemcpyHostToDevice, st)) != cudaSuccess) break;
-      if ((e = cudaStreamSynchronize(st)) != cudaSuccess) break;   // host staging vectors go out of scope
+      ta.root = (uint4*)frames.p + ((int64_t)l.src0 - (int64_t)l.task0);      // task t's root is its list's source
+      if (e == cudaSuccess)
+        e = launch_prepare(l.N, (int64_t)l.cap, dn, drec, ta, l.task0, derr + 1, st, (unsigned int*)(ds + o_tmax) + i, &dstate[bd.list].n);
+      if (e == cudaSuccess && !packed.empty()) e = cudaStreamSynchronize(st);   // the host list goes out of scope
     }
-    if ((e = cudaMemcpyAsync(b->h_out, c, cb, cudaMemcpyDeviceToHost, st)) != cudaSuccess) break;
-    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) break;
-    const uint32_t de = ((const uint32_t*)(b->h_out + njobs))[2];
-    if (de) { status = h->fail(derr_to_status(de), "batch prepare: %s", derr_text(de)); break; }
-    // Split each job on its own (tiny boards are not split), so every job's
-    // subtasks form one contiguous queue range: pass 0 counts per job, then
-    // pass 1 writes job after job behind one allocation cursor.
-    b->job_split.assign(njobs, 0);
-    b->sub_off.assign(njobs, 0); b->sub_m.assign(njobs, 0);
-    if ((e = b->nsub.ensure((size_t)std::max<int64_t>(b->m, 1) * sizeof(uint32_t))) != cudaSuccess) break;
-    DevBuf sctr;
-    sctr.ordered = st;
-    if ((e = sctr.ensure((size_t)(njobs + 1) * 16)) != cudaSuccess) break;
-    unsigned long long* sc = (unsigned long long*)sctr.p;   // [2j] subtasks of job j, [2*njobs+1] cursor
-    if ((e = cudaMemsetAsync(sc, 0, (size_t)(njobs + 1) * 16, st)) != cudaSuccess) { sctr.release(); break; }
-    for (int j = 0; j < njobs && e == cudaSuccess; j++) {
-      b->job_split[j] = (jobs[j].N <= 12) ? 0 : (h->split >= 0 ? h->split : choose_split(b->job_m[j], b->job_rows[j]));
-      e = launch_split(0, b->job_split[j], b->job_off[j], b->job_m[j], ta, (uint32_t*)b->nsub.p, nullptr, nullptr,
-                       sc + 2 * j, nullptr, nullptr, 0, st);
-    }
-    std::vector<unsigned long long> cnts((size_t)(njobs + 1) * 2, 0);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(cnts.data(), sc, cnts.size() * 8, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) { sctr.release(); break; }
-    int64_t total_sub = 0;
-    for (int j = 0; j < njobs; j++) { b->sub_off[j] = total_sub; b->sub_m[j] = (int64_t)cnts[2 * j]; total_sub += b->sub_m[j]; }
-    for (int j = 0; j < njobs; j++) b->big = b->big || (b->sub_m[j] > 0 && counts_need_u64(jobs[j].N, b->sub_m[j]));
-    b->ms = total_sub;
-    // Stacks sized to the deepest subtask: a job's subtasks start at depth
-    // job_split[j], so they need (deepest T) - job_split[j] frames.
+    if (e != cudaSuccess) break;
+    ta.root = nullptr;
+    if ((e = launch_batch_queries((int)nq, (const BatchQuery*)(dt + o_q), (uint4*)frames.p, (uint4*)tmp.p, dstate, ta, st)) !=
+        cudaSuccess) break;
+    // ---- count every list's items, read the sizes back
+    ListArgs a;
+    a.n = (int)nl; a.total = src; a.ends = (const unsigned long long*)dt; a.lists = (const BatchList*)(dt + o_lists);
+    a.state = dstate; a.src = (const uint4*)frames.p; a.info = ta.info; a.sched = ta.sched; a.sw = ta.sw; a.off = (uint32_t*)off.p;
+    if ((e = launch_list_count(a, b->wide, st)) != cudaSuccess) break;
+    if ((e = cudaMemcpyAsync(b->h_out, ds, state_bytes, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(st)) != cudaSuccess) break;
+    const unsigned char* hs = (const unsigned char*)b->h_out;
+    const unsigned int* herr = (const unsigned int*)(hs + o_err);
+    if (herr[0]) { status = h->fail(NQ_EPRESET, "batch: generator failed (preset too deep)"); break; }
+    if (herr[1]) { status = h->fail(derr_to_status(herr[1]), "batch prepare: %s", derr_text(herr[1])); break; }
+    const ListState* hst = (const ListState*)hs;
+    // Stacks sized to the deepest item: items start `depth` + D down, so they need (deepest T) less that.
+    std::vector<int> deep(nl, 1);
+    for (size_t i = 0; i < nb; i++)
+      deep[boards[i].list] = std::max(1, (int)((const unsigned int*)(hs + o_tmax))[i] - lists[boards[i].list].D);
+    for (const BatchQuery& q : queries)
+      deep[q.list] = std::max(1, lists[q.list].T - (int)hst[q.list].depth - lists[q.list].D);
+    unsigned long long* je = (unsigned long long*)(b->stage + o_jends);
+    BatchJob* jt = (BatchJob*)(b->stage + o_jobs);
+    int nj = 0;
+    uint64_t items = 0, jsrc = 0;
     b->maxt = 1;
     for (int j = 0; j < njobs; j++) {
-      const int deep = (job_host_begin[j] >= 0) ? b->job_maxt[j] : (int)job_deep[j];
-      b->job_maxt[j] = std::max(1, std::min(b->job_maxt[j], deep - b->job_split[j]));
-      b->maxt = std::max(b->maxt, b->job_maxt[j]);
+      b->sub_off[j] = (int64_t)items;
+      const int li = job_list[j];
+      if (li < 0) continue;
+      const ListState& s = hst[li];
+      b->fixed_total[j] += s.settled;
+      b->sub_m[j] = (int64_t)s.items;
+      b->job_maxt[j] = deep[li];
+      b->m += s.n;
+      if (s.items == 0) continue;
+      b->maxt = std::max(b->maxt, deep[li]);
+      b->big = b->big || counts_need_u64(jobs[j].N, (int64_t)s.items);
+      jsrc += s.n;
+      je[nj] = jsrc;
+      jt[nj++] = BatchJob{items, (uint32_t)(li ? ends[li - 1] : 0ull), (uint32_t)li, (uint32_t)j, 0};
+      items += s.items;
     }
-    if ((e = b->sroot.ensure((size_t)std::max<int64_t>(total_sub, 1) * sizeof(uint4))) != cudaSuccess ||
-        (e = b->sinfo.ensure((size_t)std::max<int64_t>(total_sub, 1) * sizeof(uint2))) != cudaSuccess) { sctr.release(); break; }
-    // settled counts of small tasks land in the control block's totals (zeroed above)
-    for (int j = 0; j < njobs && e == cudaSuccess; j++)
-      e = launch_split(1, b->job_split[j], b->job_off[j], b->job_m[j], ta, (uint32_t*)b->nsub.p, (uint4*)b->sroot.p,
-                       (uint2*)b->sinfo.p, sc + 2 * njobs, nullptr, (unsigned long long*)c, 0, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(b->h_out, c, cb, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    sctr.release();
-    if (e != cudaSuccess) break;
-    for (int j = 0; j < njobs; j++) b->fixed_total[j] += b->h_out[j];
-    b->device_bytes = (int64_t)(b->root.cap + b->info.cap + b->sched.cap + b->rec.cap + b->ctrl.cap + b->nsub.cap +
-                                b->sroot.cap + b->sinfo.cap);
+    b->ms = (int64_t)items;
+    if ((e = b->sroot.ensure(std::max<uint64_t>(items, 1) * sizeof(uint4))) != cudaSuccess ||
+        (e = b->sinfo.ensure(std::max<uint64_t>(items, 1) * sizeof(uint2))) != cudaSuccess) break;
+    // ---- write the jobs' items
+    if (nj) {
+      if ((e = cudaMemcpyAsync(dt + o_jends, b->stage + o_jends, tab_bytes - o_jends, cudaMemcpyHostToDevice, st)) != cudaSuccess) break;
+      b->h2d_bytes += (int64_t)(tab_bytes - o_jends);
+      a.n = nj; a.total = jsrc; a.ends = (const unsigned long long*)(dt + o_jends);
+      if ((e = launch_list_write(a, (const BatchJob*)(dt + o_jobs), (uint4*)b->sroot.p, (uint2*)b->sinfo.p, b->wide, st)) !=
+          cudaSuccess) break;
+    }
   } while (0);
-  jt.release();
+  if (st) for (DevBuf* d : {&tab, &state, &rec, &gen, &frames, &tmp, &off}) d->release();   // after the launches above, on the stream
   if (e != cudaSuccess) status = h->cuda_fail(e, "batch build");
   if (status != NQ_OK) { nq_batch_destroy(b); return status; }
+  b->device_bytes = (int64_t)(b->info.cap + b->sched.cap + b->ctrl.cap + b->sroot.cap + b->sinfo.cap);
   *out = b;
   return NQ_OK;
 }
@@ -1019,40 +1094,49 @@ int64_t nq_job_device_bytes(const nq_job* job, int sms, int split_depth) {
   if (!job || sms < 1 || split_depth < -1 || split_depth > 3) return NQ_EINVAL;
   const nq_job& J = *job;
   if (J.N < 1 || J.N > kMaxN || J.k < 0 || J.k > 8) return NQ_EINVAL;
-  int64_t m = 0;
-  size_t word = 0;
-  int maxt = 1, rows_left = 1;
+  int64_t m = 0, tasks = 1;
+  int rows = 1;
+  int levels = 0;
   if (J.kind == NQ_JOB_COUNT && J.N >= 6) {
-    // the generator's record count, as nq_batch_create builds the job (compact schedule words)
+    // the record bound nq_batch_create builds the job with
     const int p = J.preset > 0 ? J.preset : preset_for(J.N);
-    std::vector<GenRecord> v;
-    const int s = gen_constellations(J.N, p, v, 0);
-    if (s != 0) return s == -2 ? NQ_EPRESET : NQ_EINVAL;
-    m = (int64_t)v.size();
-    int smin = 64;
-    for (const GenRecord& r : v) smin = std::min<int>(smin, (int)(r.startijkl >> 20));
-    rows_left = maxt = maxt_for(J.N, smin);
-    word = sizeof(uint32_t);
+    if (p < 4) return NQ_EPRESET;
+    std::vector<int> starts;
+    if (start_constellations(J.N, starts) != 0) return NQ_EINVAL;
+    m = (int64_t)board_bound(J.N, p, starts);
+    if (p > 8 || (uint64_t)m > kGenRecords) {
+      std::vector<GenRecord> v;
+      const int s = gen_constellations(J.N, p, v, 0);
+      if (s != 0) return s == -2 ? NQ_EPRESET : NQ_EINVAL;
+      m = (int64_t)v.size();
+    }
+    tasks = m;
+    rows = maxt_for(J.N, p - 3);
+    levels = choose_split(m / 2, rows);
   } else if (J.kind == NQ_JOB_COUNT || J.kind == NQ_JOB_COMPLETION) {
-    int rows[8], cols[8];
+    int r[8], c[8];
     const int k = (J.kind == NQ_JOB_COUNT) ? 0 : J.k;
-    for (int q = 0; q < k; q++) { rows[q] = J.rows[q]; cols[q] = J.cols[q]; }
-    std::vector<HostTask> t;
-    int mt = 0;
-    if (build_completion_tasks(J.N, k, rows, cols, 4096, 0, t, &mt) < 0) return NQ_EINVAL;
-    m = (int64_t)t.size();
-    maxt = std::max(1, mt);
-    rows_left = mt + 2;
-    word = sizeof(uint2);
+    for (int q = 0; q < k; q++) { r[q] = J.rows[q]; c[q] = J.cols[q]; }
+    QueryParam p;
+    bool wide = false;
+    uint64_t fixed = 0;
+    const int s = query_task(J.N, k, r, c, &p, &wide, &fixed);
+    if (s < 0) return NQ_EINVAL;
+    if (s > 0) {
+      m = (int64_t)std::min(kQueryTarget, kQueryCap / (unsigned)J.N) * J.N;
+      rows = (int)p.T + 2;
+      levels = query_levels(rows);
+    }
   } else {
     return NQ_EINVAL;
   }
   // split queue: each level multiplies the items by at most ~8 (measured 6.2-8x)
-  const int D = (J.N <= 12) ? 0 : (split_depth >= 0 ? split_depth : choose_split(m, rows_left));
+  const int D = (J.N <= 12) ? 0 : (split_depth >= 0 ? split_depth : levels);
   int64_t ns = m;
   for (int d = 0; d < D; d++) ns *= 8;
-  const int64_t per_task = 16 /*record*/ + 16 /*root*/ + 8 /*info*/ + 4 /*split count*/ + (int64_t)(maxt + 1) * (int64_t)word;
-  return m * per_task + ns * (16 + 8) + (int64_t)Ctrl::bytes(1) + 4096;
+  const int64_t per_source = 16 /*record*/ + 16 /*generator*/ + 16 /*frame*/ + 4 /*slot*/;
+  return m * per_source + tasks * (4 /*info*/ + (int64_t)(rows + 1) * 8 /*widest words*/) + ns * (16 + 8) +
+         (int64_t)Ctrl::bytes(1) + 8192;
 }
 
 int nq_batch_set_grid(nq_batch* b, int grid) {
@@ -1118,7 +1202,7 @@ int nq_batch_run_plain(nq_batch* b, uint64_t* totals) {
     if (b->sub_m[j] > 0) {
       NQ_CUDA(h, cudaMemsetAsync(c, 0, 24, b->stream));
       TaskArrays ta;
-      ta.root = (uint4*)b->root.p; ta.info = (uint2*)b->info.p; ta.sched = b->sched.p; ta.sw = b->sw; ta.wide = b->wide;
+      ta.info = (uint32_t*)b->info.p; ta.sched = b->sched.p; ta.sw = b->sw; ta.wide = b->wide;
       // One job per launch over its subtask range; its tasks carry job id j, which lands in slot 0.
       DfsLaunch L;
       L.tasks = ta; L.sroot = (const uint4*)b->sroot.p + b->sub_off[j]; L.sinfo = (const uint2*)b->sinfo.p + b->sub_off[j];
@@ -1164,7 +1248,7 @@ int nq_count_completions(nq_handle* h, int N, int k, const int* rows, const int*
     for (int l = 0; l <= levels; l++) items += b.cap[l];
     NQ_CUDA(h, h->qbuf.ensure(1024 + (kQueryCap + items) * sizeof(uint4) + items * sizeof(uint2)));
     unsigned char* c = (unsigned char*)h->qbuf.p;
-    b.ctl = (unsigned long long*)c; b.info = (uint2*)(c + 128); b.sched = c + 256;
+    b.ctl = (unsigned long long*)c; b.info = (uint32_t*)(c + 128); b.sched = c + 256;
     b.tmp = (uint4*)(c + 1024);
     b.sroot[0] = b.tmp + kQueryCap;
     b.sinfo[0] = (uint2*)(b.sroot[0] + items);

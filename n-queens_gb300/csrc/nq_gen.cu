@@ -176,12 +176,34 @@ __global__ void __launch_bounds__(1024) query_kernel(const __grid_constant__ Que
     ((W*)b.sched)[threadIdx.x] = words[threadIdx.x];
   }
   if (threadIdx.x < QueryCtl::kWords) b.ctl[threadIdx.x] = 0;
-  if (threadIdx.x == 0) b.info[0] = make_uint2(info_pack(p.T, 0, 0, p.N, TS_OK), 0u);
+  if (threadIdx.x == 0) b.info[0] = info_pack(p.T, 0, 0, p.N, TS_OK);
   __syncthreads();
   unsigned d;
   const unsigned n = expand_query<W>(p.root, p.N, p.T, words, p.target, b.cap[0], b.sroot[0], b.tmp, d);
   for (unsigned q = threadIdx.x; q < n; q += blockDim.x) b.sinfo[0][q] = make_uint2(0u, d);
   if (threadIdx.x == 0) b.ctl[QueryCtl::kQueue] = n;
+}
+
+// A batch's queries: task and frames of each.
+template <bool WIDE>
+__global__ void __launch_bounds__(512) batch_query_kernel(const BatchQuery* __restrict__ qs, uint4* src, uint4* tmp,
+                                                          ListState* state, uint32_t* info, void* sched, int sw) {
+  using W = typename QueryWord<WIDE>::type;
+  __shared__ W words[kMaxDepth];
+  const BatchQuery& q = qs[blockIdx.x];
+  if (threadIdx.x <= q.p.T) {
+    const uint2 w = q.p.words[threadIdx.x];
+    if constexpr (WIDE) words[threadIdx.x] = w; else words[threadIdx.x] = w.x;
+    ((W*)sched)[(size_t)q.task * sw + threadIdx.x] = words[threadIdx.x];
+  }
+  __syncthreads();
+  unsigned d;
+  const unsigned n = expand_query<W>(q.p.root, q.p.N, q.p.T, words, q.p.target, q.p.target * q.p.N, src + q.src0, tmp + q.src0, d);
+  if (threadIdx.x == 0) {
+    info[q.task] = info_pack(q.p.T, 0, 0, q.p.N, TS_OK);
+    state[q.list].n = n;
+    state[q.list].depth = d;
+  }
 }
 
 // The query's queue by another level (frames at the terminal depth move on).
@@ -233,6 +255,14 @@ cudaError_t launch_query(const QueryParam& p, const QueryBuffers& b, bool wide, 
     if (wide) query_level_kernel<true><<<4 * sms, 128, 0, st>>>(p.N, p.T, b, l);
     else query_level_kernel<false><<<4 * sms, 128, 0, st>>>(p.N, p.T, b, l);
   }
+  return cudaGetLastError();
+}
+
+cudaError_t launch_batch_queries(int n, const BatchQuery* q, uint4* src, uint4* tmp, ListState* state, const TaskArrays& ta,
+                                 cudaStream_t st) {
+  if (n == 0) return cudaSuccess;
+  if (ta.wide) batch_query_kernel<true><<<n, 512, 0, st>>>(q, src, tmp, state, ta.info, ta.sched, ta.sw);
+  else batch_query_kernel<false><<<n, 512, 0, st>>>(q, src, tmp, state, ta.info, ta.sched, ta.sw);
   return cudaGetLastError();
 }
 

@@ -7,13 +7,14 @@
 //    expansion of each start constellation is independent and runs on the host
 //    threads.  Output order: ascending packed ijkl, then
 //    the reference's expansion order within a constellation.
-// 2. build_completion_tasks: DFS tasks for boards with pre-placed queens (no
-//    reference counterpart: the reference only counts whole boards).  Rows
-//    holding a pre-placed queen are skipped with a multi-row step, and the
-//    queens' diagonals are carried in ld/rd from the root or injected when
-//    they enter the bitboard, as the reference does for its corner queens
-//    (blockK/blockL, 356Py:2586-2589).  The first free rows are expanded on
-//    the host until there are enough tasks to fill the GPU.
+// 2. completion_root: the root frame and per-depth ops of a board with pre-
+//    placed queens (no reference counterpart: the reference only counts whole
+//    boards).  Rows holding a pre-placed queen are skipped with a multi-row
+//    step, and the queens' diagonals are carried in ld/rd from the root or
+//    injected when they enter the bitboard, as the reference does for its
+//    corner queens (blockK/blockL, 356Py:2586-2589).  The device expands it
+//    (nq_gen.cu); build_completion_tasks expands it on the host for the
+//    diagnostic nq_debug_completion_tasks.
 #include <algorithm>
 #include <atomic>
 #include <thread>

@@ -42,7 +42,7 @@ template <> struct QueryWord<true> { using type = uint2; };
 // Prepared task arrays (structure of arrays, one entry per task).
 struct TaskArrays {
   uint4* root = nullptr;      // {ld, rd, col, avail} of the root frame
-  uint2* info = nullptr;      // {info word (T, wexp, root count, N, status), job id}
+  uint32_t* info = nullptr;   // info word (T, wexp, root count, N, status)
   void* sched = nullptr;      // per-task schedule words, stride `sw` words
   int sw = 0;                 // schedule words per task (>= T+1 of every task)
   bool wide = false;          // uint2 words (mixed batches) instead of uint32
@@ -51,7 +51,7 @@ struct TaskArrays {
 struct DfsLaunch {
   TaskArrays tasks;
   const uint4* sroot = nullptr;         // split queue: subtask frames ...
-  const uint2* sinfo = nullptr;         // ... and {task, depth}; nullptr: the queue holds tasks
+  const uint2* sinfo = nullptr;         // ... and {task, depth | job << 5}; nullptr: the queue holds tasks (job 0)
   int64_t m = 0;                        // queue length ...
   const unsigned long long* m_dev = nullptr;   // ... or where it stands on the device; above qcap the DFS does nothing
   unsigned long long qcap = 0;
@@ -68,11 +68,11 @@ struct DfsLaunch {
 };
 
 // Prepare: records {ld, rd, col, startijkl} (the reference's 16-byte task
-// record) -> task arrays.  job/offset place the tasks of one job inside a
-// larger queue.
-// tmax (optional): atomicMax of the schedule depth T over the launch's tasks.
-cudaError_t launch_prepare(int N, int64_t m, const uint4* records, const TaskArrays& out, int64_t offset,
-                           uint32_t job, unsigned int* err, cudaStream_t st, unsigned int* tmax = nullptr);
+// record) -> task arrays at `offset`.  m_dev: the records' number stands on the
+// device and m bounds it.  tmax: atomicMax of the schedule depth T over the
+// launch's tasks; n_out: their number.
+cudaError_t launch_prepare(int N, int64_t m, const unsigned int* m_dev, const uint4* records, const TaskArrays& out,
+                           int64_t offset, unsigned int* err, cudaStream_t st, unsigned int* tmax, unsigned int* n_out);
 
 // Prepare and split a single-N list (compact words) in one launch: tasks, and for D = 1..3 the queue of their
 // depth-D frames (qn counts them, also past qcap, where nothing is written any more) and the counts settled
@@ -83,7 +83,7 @@ struct PrepareSplit {
   const unsigned int* m_dev = nullptr;  // ... or where their number stands on the device (the launch covers m_max)
   const uint4* rec = nullptr;
   uint4* root = nullptr;                // D = 0
-  uint2* info = nullptr;
+  uint32_t* info = nullptr;
   uint32_t* sched = nullptr;
   int sw = 0;
   unsigned int* err = nullptr;
@@ -111,6 +111,7 @@ struct QueryParam {
   uint4 root;
   uint32_t N, T;
   unsigned target;              // frames that are enough
+  uint32_t words_wide;          // the words' form
   uint2 words[28];
 };
 // Its control block (u64 words): total, queue cursor, error word, queue length after each level.
@@ -119,7 +120,7 @@ struct QueryCtl {
 };
 struct QueryBuffers {
   unsigned long long* ctl;
-  uint2* info;                  // one task
+  uint32_t* info;               // one task
   void* sched;
   uint4* tmp;                   // cap[0] frames
   uint4* sroot[3];              // the queue from one block, and after one and two levels over the whole GPU
@@ -130,13 +131,36 @@ struct QueryBuffers {
 // queue longer than its buffer leaves ctl[kQueue + levels] above cap[levels]: the DFS does nothing.
 cudaError_t launch_query(const QueryParam& p, const QueryBuffers& b, bool wide, int levels, int sms, cudaStream_t st);
 
-// Split tasks t0..t0+m-1 to depth D (0..3; 0 queues the tasks themselves).
-// pass 0: nsub[t] and ctr[0] += subtasks; pass 1: writes subtasks at the
-// allocation cursor ctr[1], initialises per_task (nullable) and adds counts
-// settled above depth D to job_totals.
-cudaError_t launch_split(int pass, int D, int64_t t0, int64_t m, const TaskArrays& ta, uint32_t* nsub, uint4* sroot,
-                         uint2* sinfo, unsigned long long* ctr, unsigned long long* per_task,
-                         unsigned long long* job_totals, uint32_t job_base, cudaStream_t st);
+// Batches.  A list holds sources: the tasks of a board's records (depth 0), or the frames a query was expanded
+// to.  Jobs of one board share a list.
+struct BatchList {
+  uint32_t src0;                // its first source in src
+  uint32_t task0;               // its first task, or the query's one
+  uint32_t query, D;            // D: levels to expand the sources by
+};
+struct ListState {              // on the device, zeroed before the build
+  unsigned int n, depth;        // sources, their depth
+  unsigned long long items, settled;   // queue items, weighted counts settled above them
+};
+struct BatchJob { unsigned long long base; uint32_t off0, list, job, pad; };   // items from base on; off0: the list's first source in off
+struct ListArgs {
+  int n;                        // ranges (lists, or jobs)
+  unsigned long long total;     // sources in them, padded to warps
+  const unsigned long long* ends;
+  const BatchList* lists;
+  ListState* state;
+  const uint4* src;
+  const uint32_t* info;
+  const void* sched;
+  int sw;
+  uint32_t* off;                // per source: its first item in the list's queue
+};
+cudaError_t launch_list_count(const ListArgs& a, bool wide, cudaStream_t st);
+cudaError_t launch_list_write(const ListArgs& a, const BatchJob* jobs, uint4* sroot, uint2* sinfo, bool wide, cudaStream_t st);
+// The queries' tasks and frames (state n and depth), one block each; frames in src and tmp (cap = target * N).
+struct BatchQuery { QueryParam p; uint32_t list, src0, task, pad; };
+cudaError_t launch_batch_queries(int n, const BatchQuery* q, uint4* src, uint4* tmp, ListState* state, const TaskArrays& ta,
+                                 cudaStream_t st);
 
 // Queue order, largest estimated subtree first: order[0..m) receives the queue
 // indices (subtasks when sinfo is set, else tasks); keys: m bytes of scratch,

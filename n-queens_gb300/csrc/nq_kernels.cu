@@ -101,13 +101,15 @@ __device__ __forceinline__ void max_depth_of(unsigned int* tmax, int T) {
 }
 
 template <bool WIDE>
-__global__ void __launch_bounds__(256) prepare_kernel(int N, int64_t m, const uint4* __restrict__ rec,
-                                                      uint4* __restrict__ root, uint2* __restrict__ info,
+__global__ void __launch_bounds__(256) prepare_kernel(int N, int64_t m, const unsigned* __restrict__ m_dev,
+                                                      const uint4* __restrict__ rec, uint4* __restrict__ root,
+                                                      uint32_t* __restrict__ info,
                                                       typename WordT<WIDE>::type* __restrict__ sched, int sw,
-                                                      int64_t offset, uint32_t job, unsigned int* err,
-                                                      unsigned int* tmax) {
+                                                      int64_t offset, unsigned int* err, unsigned int* tmax, unsigned int* n_out) {
   using W = typename WordT<WIDE>::type;
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (m_dev) m = *m_dev;
+  if (i == 0) *n_out = (unsigned int)m;
   int T = -1;
   if (i < m) {
     const int64_t t = offset + i;
@@ -115,37 +117,37 @@ __global__ void __launch_bounds__(256) prepare_kernel(int N, int64_t m, const ui
     uint32_t in;
     T = prepare_task<WIDE>(N, rec[i], sw, rt, in, err, [&](int d, W w) { sched[t * sw + d] = w; });
     root[t] = make_uint4(rt.ld, rt.rd, rt.col, T < 0 ? 0u : rt.avail);
-    info[t] = make_uint2(in, job);
+    info[t] = in;
   }
-  if (tmax) max_depth_of(tmax, T);    // deepest schedule of the launch, for sizing the DFS stack
+  max_depth_of(tmax, T);              // deepest schedule of the launch, for sizing the DFS stack
 }
 
-cudaError_t launch_prepare(int N, int64_t m, const uint4* records, const TaskArrays& out, int64_t offset,
-                           uint32_t job, unsigned int* err, cudaStream_t st, unsigned int* tmax) {
+cudaError_t launch_prepare(int N, int64_t m, const unsigned int* m_dev, const uint4* records, const TaskArrays& out,
+                           int64_t offset, unsigned int* err, cudaStream_t st, unsigned int* tmax, unsigned int* n_out) {
   if (m <= 0) return cudaSuccess;
   const int B = 256;
   const unsigned G = (unsigned)((m + B - 1) / B);
   if (out.wide)
-    prepare_kernel<true><<<G, B, 0, st>>>(N, m, records, out.root, out.info, (uint2*)out.sched, out.sw, offset, job, err,
-                                          tmax);
+    prepare_kernel<true><<<G, B, 0, st>>>(N, m, m_dev, records, out.root, out.info, (uint2*)out.sched, out.sw, offset, err,
+                                          tmax, n_out);
   else
-    prepare_kernel<false><<<G, B, 0, st>>>(N, m, records, out.root, out.info, (uint32_t*)out.sched, out.sw, offset, job,
-                                           err, tmax);
+    prepare_kernel<false><<<G, B, 0, st>>>(N, m, m_dev, records, out.root, out.info, (uint32_t*)out.sched, out.sw, offset,
+                                           err, tmax, n_out);
   return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
 // Schedule word decoding shared by the split and DFS kernels
 // ---------------------------------------------------------------------------
-struct Dec { uint32_t s, la, ra, fc, term, tall; };
-// compact word of depth k of a task of board N and terminal depth T
+struct Dec { uint32_t s, la, ra, fc; bool term; };
+// word of depth k of a task of board N and terminal depth T
 __device__ __forceinline__ Dec decode(uint32_t w, uint32_t N, uint32_t k, uint32_t T) {
   const Op o = unpack_compact(w ^ C_NOLOOK, (int)N, k == T);
-  return Dec{o.s, o.la, o.ra, o.fc, o.term, o.tall};
+  return Dec{o.s, o.la, o.ra, o.fc, k == T};
 }
-__device__ __forceinline__ Dec decode(uint2 w, uint32_t, uint32_t, uint32_t) {
+__device__ __forceinline__ Dec decode(uint2 w, uint32_t, uint32_t k, uint32_t T) {
   const uint32_t s = w.x & W_S;
-  return Dec{s, s ? (w.x >> (32 - s)) : 0u, w.y, ~w.x & W_NOLOOK, w.x & W_TERM, w.x & W_TALL};
+  return Dec{s, s ? (w.x >> (32 - s)) : 0u, w.y, ~w.x & W_NOLOOK, k == T};
 }
 
 // ---------------------------------------------------------------------------
@@ -159,9 +161,8 @@ __device__ __forceinline__ Dec decode(uint2 w, uint32_t, uint32_t, uint32_t) {
 // record); the three launches it replaces kept 28 ops a record in local memory
 // and read tasks back from memory twice.
 // ---------------------------------------------------------------------------
-template <int K, int D, class F>
-__device__ __forceinline__ void frames_at(uint32_t ld, uint32_t rd, uint32_t col, uint32_t avail, const uint32_t* w,
-                                          uint32_t N, uint32_t T, uint32_t& direct, F&& f) {
+template <int K, int D, class W, class F>
+__device__ __forceinline__ void frames_at(uint32_t ld, uint32_t rd, uint32_t col, uint32_t avail, const W* w, uint32_t N, uint32_t T, uint32_t& direct, F&& f) {
   if constexpr (K == D) {
     f(make_uint4(ld, rd, col, avail));
   } else {
@@ -196,7 +197,7 @@ __global__ void __launch_bounds__(256) prepare_split_kernel(const PrepareSplit a
       for (int k = 0; k < D; k++)
         if (d == k) w[k] = x;
     });
-    a.info[t] = make_uint2(in, 0u);
+    a.info[t] = in;
     if (D == 0) {
       a.root[t] = make_uint4(rt.ld, rt.rd, rt.col, T < 0 ? 0u : rt.avail);
       if (a.per_task) a.per_task[t] = 0;      // the DFS adds the task's counts
@@ -246,127 +247,103 @@ cudaError_t launch_prepare_split(int D, int64_t m_max, const PrepareSplit& a, cu
 }
 
 // ---------------------------------------------------------------------------
-// split: expand every task to depth D (1..3) so the DFS queue holds many
-// small subtasks instead of few large ones (the reference's measured
-// bottleneck is the tail of large tasks, 14Bit_codon_GPU/README.md:4344-4404).
-// Pass 0 counts each task's depth-D frames into nsub[t] and the grand total
-// into ctr[0]; pass 1 writes them (warp-aggregated allocation on ctr[1]) and
-// settles, without subtasks, tasks that end above depth D and tasks whose
-// root is already terminal: their weighted count goes to per_task[t] (which
-// pass 1 initialises for every task) and to the job totals.
+// split of a batch's source lists (the records of a board, the frames of a
+// query) in one launch each way: list_count_kernel counts every source's
+// frames D levels down and gives them slots in its list's queue;
+// list_write_kernel writes them for every job, jobs of one board from the same
+// list, so each job's items are one range of the batch's queue.  Counts
+// settled above that depth are summed per list.  Lists are padded to warps.
 // ---------------------------------------------------------------------------
-template <bool WIDE, int D>
-__global__ void __launch_bounds__(256) split_kernel(int pass, int64_t t0, int64_t m, const uint4* __restrict__ root,
-                                                    const uint2* __restrict__ info,
-                                                    const typename WordT<WIDE>::type* __restrict__ sched, int sw,
-                                                    uint32_t* __restrict__ nsub, uint4* __restrict__ sroot,
-                                                    uint2* __restrict__ sinfo, unsigned long long* ctr,
-                                                    unsigned long long* __restrict__ per_task,
-                                                    unsigned long long* job_totals, uint32_t job_base) {
-  const int64_t tr = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t t = t0 + tr;          // absolute task index
-  const unsigned lane = threadIdx.x & 31u;
-  const bool active = tr < m;
-  uint32_t count = 0;                 // depth-D frames of this task
-  unsigned long long direct = 0;      // unweighted count settled here
-  uint32_t wexp = 0, job = job_base;
-  uint32_t base = 0;
-  if (pass == 1) {
-    // reserve this warp's slots: exclusive scan of the per-task counts
-    const uint32_t mine = active ? nsub[t] : 0u;
-    uint32_t incl = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t v = __shfl_up_sync(FULL, incl, o);
-      if ((int)lane >= o) incl += v;
-    }
-    const uint32_t tot = __shfl_sync(FULL, incl, 31);
-    unsigned long long wb = 0;
-    if (lane == 31 && tot) wb = atomicAdd(ctr + 1, (unsigned long long)tot);
-    wb = __shfl_sync(FULL, wb, 31);
-    base = (uint32_t)wb + incl - mine;
+__device__ __forceinline__ int find_range(const unsigned long long* __restrict__ ends, int n, unsigned long long i) {
+  int lo = 0, hi = n - 1;              // the first range whose end is above i
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (i < ends[mid]) hi = mid; else lo = mid + 1;
   }
-  if (active) {
-    const uint2 in = info[t];
-    const uint32_t T = info_T(in.x);
-    wexp = info_wexp(in.x);
-    job = in.y;
-    if (T == INFO_NO_DFS || info_status(in.x) != TS_OK) {
-      direct = info_status(in.x) == TS_OK ? info_root(in.x) : 0u;
-    } else if (D == 0) {
-      if (pass == 1) { sroot[base] = root[t]; sinfo[base] = make_uint2((uint32_t)t, 0u); }
-      count = 1;
-    } else {
-      const uint32_t bm = (1u << info_N(in.x)) - 1u;
-      const typename WordT<WIDE>::type* w = sched + (size_t)t * sw;
-      uint4 st[D + 1];
-      st[0] = root[t];
-      int k = 0;
-      while (k >= 0) {
-        uint4& f = st[k];
-        if (f.w == 0u) { --k; continue; }
-        const uint32_t bit = f.w & (0u - f.w);
-        f.w ^= bit;
-        const Dec o = decode(w[k], info_N(in.x), (uint32_t)k, T);
-        const uint32_t nld = ((f.x | bit) << o.s) | o.la;
-        const uint32_t nrd = ((f.y | bit) >> o.s) | o.ra;
-        const uint32_t ncol = f.z | bit;
-        uint32_t nf = bm & ~(nld | nrd | ncol);
-        if (o.fc && (bm & ~((nld << 1) | (nrd >> 1) | ncol)) == 0u) nf = 0;
-        if (o.term) { direct += (nf != 0u || o.tall) ? 1u : 0u; continue; }   // SQd2B: LA bit 0
-        if (nf == 0u) continue;
-        if (k + 1 == D) {
-          if (pass == 1) {
-            sroot[base + count] = make_uint4(nld, nrd, ncol, nf);
-            sinfo[base + count] = make_uint2((uint32_t)t, (uint32_t)D);
-          }
-          ++count;
-        } else {
-          st[k + 1] = make_uint4(nld, nrd, ncol, nf);
-          ++k;
-        }
-      }
-    }
-  }
-  if (pass == 0) {
-    if (active) nsub[t] = count;
-    uint32_t v = count;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-    if (lane == 0 && v) atomicAdd(ctr, (unsigned long long)v);
+  return lo;
+}
+
+// One source's frames: f(frame) for each, the settled count into direct.
+template <class W, class F>
+__device__ __forceinline__ void source_frames(const BatchList& l, uint32_t r, const ListArgs& a, uint32_t d, uint32_t& task,
+                                              uint32_t& in, uint32_t& direct, F&& f) {
+  const uint4 s = a.src[l.src0 + r];
+  task = l.query ? l.task0 : l.task0 + r;
+  in = a.info[task];
+  const uint32_t T = info_T(in), N = info_N(in);
+  if (T == INFO_NO_DFS || info_status(in) != TS_OK) {
+    if (info_status(in) == TS_OK) direct += info_root(in);
     return;
   }
-  const unsigned long long dv = direct << wexp;
-  if (active && per_task) per_task[t] = dv;
-  // job totals: one atomic per warp when the warp's tasks share a job
-  const uint32_t j0 = __shfl_sync(FULL, job, 0);
-  if (__all_sync(FULL, !active || job == j0)) {
-    unsigned long long v = active ? dv : 0ull;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-    if (lane == 0 && v) atomicAdd(job_totals + (j0 - job_base), v);
-  } else if (active && dv) {
-    atomicAdd(job_totals + (job - job_base), dv);
+  const W* w = (const W*)a.sched + (size_t)task * a.sw + d;
+  switch (l.D) {
+    case 0: if (s.w) f(s); break;
+    case 1: frames_at<0, 1>(s.x, s.y, s.z, s.w, w, N, T - d, direct, f); break;
+    case 2: frames_at<0, 2>(s.x, s.y, s.z, s.w, w, N, T - d, direct, f); break;
+    default: frames_at<0, 3>(s.x, s.y, s.z, s.w, w, N, T - d, direct, f); break;
   }
 }
 
-cudaError_t launch_split(int pass, int D, int64_t t0, int64_t m, const TaskArrays& ta, uint32_t* nsub, uint4* sroot,
-                         uint2* sinfo, unsigned long long* ctr, unsigned long long* per_task,
-                         unsigned long long* job_totals, uint32_t job_base, cudaStream_t st) {
-  if (m <= 0) return cudaSuccess;
-  const int B = 256;
-  const unsigned G = (unsigned)((m + B - 1) / B);
-#define NQ_SPLIT(WD, DD)                                                                                             \
-  split_kernel<WD, DD><<<G, B, 0, st>>>(pass, t0, m, ta.root, ta.info, (const typename WordT<WD>::type*)ta.sched, \
-                                        ta.sw, nsub, sroot, sinfo, ctr, per_task, job_totals, job_base)
-  if (ta.wide) {
-    if (D == 0) NQ_SPLIT(true, 0); else if (D == 1) NQ_SPLIT(true, 1); else if (D == 2) NQ_SPLIT(true, 2);
-    else NQ_SPLIT(true, 3);
-  } else {
-    if (D == 0) NQ_SPLIT(false, 0); else if (D == 1) NQ_SPLIT(false, 1); else if (D == 2) NQ_SPLIT(false, 2);
-    else NQ_SPLIT(false, 3);
+template <bool WIDE>
+__global__ void __launch_bounds__(256) list_count_kernel(const ListArgs a) {
+  using W = typename WordT<WIDE>::type;
+  const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if ((i & ~31ull) >= a.total) return;
+  const int li = find_range(a.ends, a.n, i);
+  const BatchList l = a.lists[li];
+  const uint32_t r = (uint32_t)(i - (li ? a.ends[li - 1] : 0ull));
+  const ListState st = a.state[li];
+  uint32_t n = 0, direct = 0, task, in = 0;
+  if (r < st.n) source_frames<W>(l, r, a, st.depth, task, in, direct, [&](uint4) { n++; });
+  uint32_t incl = n;
+  const unsigned lane = threadIdx.x & 31u;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t v = __shfl_up_sync(FULL, incl, o);
+    if ((int)lane >= o) incl += v;
   }
-#undef NQ_SPLIT
+  unsigned long long base = 0;
+  if (lane == 31 && incl) base = atomicAdd(&a.state[li].items, (unsigned long long)incl);
+  base = __shfl_sync(FULL, base, 31) + (incl - n);
+  a.off[i] = (uint32_t)base;
+  unsigned long long v = (unsigned long long)direct << info_wexp(in);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
+  if (lane == 0 && v) atomicAdd(&a.state[li].settled, v);
+}
+
+template <bool WIDE>
+__global__ void __launch_bounds__(256) list_write_kernel(const ListArgs a, const BatchJob* __restrict__ jobs,
+                                                         uint4* __restrict__ sroot, uint2* __restrict__ sinfo) {
+  using W = typename WordT<WIDE>::type;
+  const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.total) return;
+  const int ji = find_range(a.ends, a.n, i);
+  const BatchJob j = jobs[ji];
+  const uint32_t r = (uint32_t)(i - (ji ? a.ends[ji - 1] : 0ull));
+  const BatchList l = a.lists[j.list];
+  const ListState st = a.state[j.list];
+  if (r >= st.n) return;
+  unsigned long long at = j.base + a.off[j.off0 + r];
+  uint32_t task = 0, in, direct = 0;
+  source_frames<W>(l, r, a, st.depth, task, in, direct, [&](uint4 f) {
+    sroot[at] = f;
+    sinfo[at++] = make_uint2(task, (st.depth + l.D) | (j.job << 5));
+  });
+}
+
+cudaError_t launch_list_count(const ListArgs& a, bool wide, cudaStream_t st) {
+  if (a.total == 0) return cudaSuccess;
+  const unsigned G = (unsigned)((a.total + 255) / 256);
+  if (wide) list_count_kernel<true><<<G, 256, 0, st>>>(a); else list_count_kernel<false><<<G, 256, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_list_write(const ListArgs& a, const BatchJob* jobs, uint4* sroot, uint2* sinfo, bool wide, cudaStream_t st) {
+  if (a.total == 0) return cudaSuccess;
+  const unsigned G = (unsigned)((a.total + 255) / 256);
+  if (wide) list_write_kernel<true><<<G, 256, 0, st>>>(a, jobs, sroot, sinfo);
+  else list_write_kernel<false><<<G, 256, 0, st>>>(a, jobs, sroot, sinfo);
   return cudaGetLastError();
 }
 
@@ -391,7 +368,7 @@ __device__ __forceinline__ uint32_t cost_key(const uint4 f, uint32_t bm) {
 
 __global__ void __launch_bounds__(256) order_hist_kernel(int64_t m, const uint4* __restrict__ sroot,
                                                          const uint2* __restrict__ sinfo,
-                                                         const uint4* __restrict__ root, const uint2* __restrict__ info,
+                                                         const uint4* __restrict__ root, const uint32_t* __restrict__ info,
                                                          uint8_t* __restrict__ keys, unsigned int* hist) {
   __shared__ unsigned int h[256];
   h[threadIdx.x] = 0;
@@ -400,7 +377,7 @@ __global__ void __launch_bounds__(256) order_hist_kernel(int64_t m, const uint4*
   if (q < m) {
     const uint32_t task = sinfo ? sinfo[q].x : (uint32_t)q;
     const uint4 f = sinfo ? sroot[q] : root[q];
-    const uint32_t key = cost_key(f, (1u << info_N(info[task].x)) - 1u);
+    const uint32_t key = cost_key(f, (1u << info_N(info[task])) - 1u);
     keys[q] = (uint8_t)key;
     atomicAdd(&h[key], 1u);
   }
@@ -457,10 +434,10 @@ cudaError_t launch_order(int64_t m, const uint4* sroot, const uint2* sinfo, cons
 // ---------------------------------------------------------------------------
 struct DfsArgs {
   const uint4* root;          // task roots (when sinfo == nullptr the queue holds tasks)
-  const uint2* info;
+  const uint32_t* info;
   const void* sched;
   int sw;
-  const uint4* sroot;         // subtask frames and {task, depth} (split queue)
+  const uint4* sroot;         // subtask frames and {task, depth | job << 5} (split queue)
   const uint2* sinfo;
   int64_t m;                  // queue length, ...
   const unsigned long long* m_dev;   // ... or where it stands on the device (above qcap: the queue did not fit, no work)
@@ -652,10 +629,9 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
             const uint64_t slot = base + lane;
             const uint64_t q = a.order ? (uint64_t)a.order[slot] : slot;
             uint32_t d0 = 0;
-            if (a.sinfo) { const uint2 si = a.sinfo[q]; p_task = si.x; d0 = si.y; p_root = a.sroot[q]; }
+            if (a.sinfo) { const uint2 si = a.sinfo[q]; p_task = si.x; d0 = si.y & 31u; p_job = si.y >> 5; p_root = a.sroot[q]; }
             else { p_task = (uint32_t)q; p_root = a.root[q]; }
-            const uint2 in = a.info[p_task];
-            p_info = in.x | (d0 << 16); p_job = in.y;
+            p_info = a.info[p_task] | (d0 << 16);
           }
         }
         const unsigned give = min((unsigned)__popc(need), pool_n);
@@ -684,16 +660,8 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
             const uint32_t fr = ((1u << info_N(i_info)) - 1u) & ~r.z;
             const uint32_t R = __popc(fr);
             const W* src_w = gsched + (size_t)task * a.sw + d0;
-            uint32_t n = T - d0;                 // terminal depth
-            bool leaf = false;
-            if constexpr (WIDE) {
-              // a tall last row has one free column: its parent row is the terminal one by the compact
-              // words' rule (count the child if its row has a free square)
-              if (src_w[n].x & W_TALL) { leaf = n == 0u; n -= leaf ? 0u : 1u; }
-            }
-            if (leaf) {
-              L.cnt += __popc(r.w & fr);
-            } else if (n + 2u <= R) {            // fewer free columns than rows: no solution, no work
+            const uint32_t n = T - d0;           // terminal depth
+            if (n + 2u <= R) {                   // fewer free columns than rows: no solution, no work
               L.ld = r.x; L.rd = r.y; L.fr = fr; L.avail = r.w & fr;
               L.tf = R - n; L.sw0 = sch_sh + R * ROW; L.ram = compact_ra_mask((int)info_N(i_info));
               for (uint32_t k = 0; k <= n; k++) put_word(k, src_w[k]);

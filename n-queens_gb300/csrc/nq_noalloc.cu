@@ -29,7 +29,7 @@ constexpr int64_t kMaxRecords = 131072;
 constexpr int kMaxWords = 24;                        // schedule words per task (depths 0..23)
 constexpr size_t kCtrlBytes = 256;                   // totals, queue cursor, error word, queue length
 constexpr size_t kRootBytes = (size_t)kMaxRecords * sizeof(uint4);
-constexpr size_t kInfoBytes = (size_t)kMaxRecords * sizeof(uint2);
+constexpr size_t kInfoBytes = (size_t)kMaxRecords * sizeof(uint2);   // info words, and room to round the parts to 16 bytes
 constexpr size_t kSchedBytes = (size_t)kMaxRecords * kMaxWords * sizeof(uint32_t);
 constexpr size_t kScratchBytes = kCtrlBytes + kRootBytes + kInfoBytes + kSchedBytes;   // 15.0 MiB + 256 B
 constexpr int kMaxDevices = 64;
@@ -87,8 +87,8 @@ extern "C" int nq_exec_solutions_noalloc(int N, const nq_record* d_records, int6
   P.N = N; P.m = m; P.rec = (const uint4*)d_records; P.sw = maxt + 1; P.err = err; P.total = totals;
   P.per_task = (unsigned long long*)d_solutions; P.qn = (unsigned long long*)(c + 24);
   size_t used = kCtrlBytes;
-  P.info = (uint2*)(c + used);
-  used += ((size_t)m * sizeof(uint2) + 15) & ~(size_t)15;
+  P.info = (uint32_t*)(c + used);
+  used += ((size_t)m * sizeof(uint32_t) + 15) & ~(size_t)15;
   P.sched = (uint32_t*)(c + used);
   used += ((size_t)m * P.sw * sizeof(uint32_t) + 15) & ~(size_t)15;
   P.qcap = (kScratchBytes - used) / (sizeof(uint4) + sizeof(uint2));

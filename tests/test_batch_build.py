@@ -1,0 +1,54 @@
+"""Batches built on the device: jobs that share a board, queries of both word forms, settled jobs and a host-made list in
+one batch give each job's count alone, in one launch, from a graph and job by job."""
+import numpy as np
+import pytest
+
+from conftest import gpu_available
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not gpu_available(), reason="needs a CUDA GPU")]
+
+
+def _jobs(kind):
+    from nqueens import CompletionJob as Q, CountJob as C
+    if kind == "boards":
+        return [C(12), C(6), C(12), C(13, 6), C(12, 4), C(13, 9), C(16), C(16)]
+    if kind == "small":
+        return [C(1), C(2), C(3), C(4), C(5), Q(4, [(0, 1)]), Q(8, [(0, 0), (1, 1)]), Q(3, [(0, 0), (2, 1)]),
+                Q(4, [(2, 0), (0, 1), (3, 2), (1, 3)])]
+    if kind == "compact":
+        return [Q(14, [(3, 3)]), Q(13, []), C(13), Q(15, [(0, 7), (14, 6)]), Q(14, [(3, 3)])]
+    return [Q(14, [(4, 1), (5, 3), (6, 5), (7, 7), (8, 9)]), C(13), Q(18, [(2, 17), (9, 8), (10, 5)]), Q(5, []), C(13)]
+
+
+@pytest.mark.parametrize("split", [-1, 0, 2])
+@pytest.mark.parametrize("kind", ["boards", "small", "compact", "wide"])
+def test_batch_equals_each_job_alone(kind, split):
+    import nqueens
+    eng = nqueens.Engine(0, auto_tune=False)
+    try:
+        eng.set_config(64, 0, split)
+        jobs = _jobs(kind)
+        want = np.array([eng.count(j.N, j.preset).total if isinstance(j, nqueens.CountJob) else
+                         eng.count_completions(j.N, j.queens) for j in jobs], np.uint64)
+        b = eng.batch(jobs)
+        try:
+            assert np.array_equal(b.run(use_graph=False), want)
+            assert np.array_equal(b.run(use_graph=True), want)
+            assert np.array_equal(b.run_plain(), want)
+            assert b.device_bytes <= sum(eng.job_device_bytes(j) for j in jobs)
+        finally:
+            b.close()
+    finally:
+        eng.close()
+
+
+def test_batch_rejects_a_preset_too_deep():
+    import nqueens
+    eng = nqueens.Engine(0)
+    try:
+        for job, status in ((nqueens.CountJob(10, 3), -6), (nqueens.CompletionJob(8, [(3, 3), (3, 3)]), -1)):
+            with pytest.raises(nqueens.NQError) as e:
+                eng.batch([nqueens.CountJob(9), job])
+            assert e.value.status == status
+    finally:
+        eng.close()
