@@ -90,6 +90,7 @@ int run_records(nq_handle* h, int N, const uint4* d_rec, int64_t m, int start_mi
   unsigned char* c = (unsigned char*)h->ctrl.p;
   PrepareSplit P;
   P.N = N; P.m = m; P.m_dev = m_dev; P.rec = d_rec; P.info = (uint32_t*)h->info.p; P.sched = (uint32_t*)h->sched.p; P.sw = maxt + 1;
+  P.ra_words = !ra_in_rd(N, start_min, D);
   P.err = (unsigned int*)(c + ctl::kErr); P.tmax = (unsigned int*)(c + ctl::kTmax);
   P.per_task = d_per_task; P.qn = (unsigned long long*)(c + ctl::kSplit); P.total = (unsigned long long*)(c + ctl::kTotal);
   // Queue capacity: a bound (each level places a queen in one of at most N - 2, N - 3, ... columns) where that
@@ -106,7 +107,7 @@ int run_records(nq_handle* h, int N, const uint4* d_rec, int64_t m, int start_mi
     P.root = (uint4*)h->root.p;
   }
   DfsLaunch L;
-  L.tasks.root = (uint4*)h->root.p; L.tasks.info = P.info; L.tasks.sched = P.sched; L.tasks.sw = P.sw; L.tasks.wide = false;
+  L.tasks.root = (uint4*)h->root.p; L.tasks.info = P.info; L.tasks.sched = P.sched; L.tasks.sw = P.sw; L.tasks.wide = false; L.tasks.ra_words = P.ra_words;
   L.cursor = (unsigned long long*)(c + ctl::kCursor); L.job_totals = P.total;
   L.per_task = d_per_task; L.err = P.err; L.block = h->block; L.grid = h->grid;
   L.m = m;
@@ -190,10 +191,10 @@ int query_task(int N, int k, const int* rows, const int* cols, QueryParam* p, bo
   p->root = make_uint4(root[0], root[1], root[2], root[3]);
   p->N = (uint32_t)N; p->T = (uint32_t)(n - 2); p->target = 0;
   *wide = false;
-  for (int d = 0; d <= n - 2; d++) *wide = *wide || !compact_fits(ops[d], N);
+  for (int d = 0; d <= n - 2; d++) *wide = *wide || ops[d].ra != 0u || !compact_fits(ops[d], N);   // no RA in compact words
   p->words_wide = *wide ? 1u : 0u;
   for (int d = 0; d <= n - 2; d++)
-    p->words[d] = *wide ? make_uint2(pack_wide_x(ops[d]) ^ W_NOLOOK, ops[d].ra) : make_uint2(pack_compact(ops[d]) ^ C_NOLOOK, 0u);
+    p->words[d] = *wide ? make_uint2(device_wide_x(ops[d]), ops[d].ra) : make_uint2(device_compact(ops[d], false), 0u);
   return 1;
 }
 
@@ -201,7 +202,7 @@ int query_task(int N, int k, const int* rows, const int* cols, QueryParam* p, bo
 void widen_query(QueryParam* p) {
   for (uint32_t d = 0; d <= p->T; d++) {
     const Op o = unpack_compact(p->words[d].x ^ C_NOLOOK, (int)p->N, false);
-    p->words[d] = make_uint2(pack_wide_x(o) ^ W_NOLOOK, o.ra);
+    p->words[d] = make_uint2(device_wide_x(o), 0u);
   }
   p->words_wide = 1;
 }
@@ -764,6 +765,7 @@ struct nq_batch {
   int maxt = 1, sw = 2, grid = 0, block = 128;
   bool big = false;                        // some job's queue items may count 2^32: u64 per-lane counters
   bool wide = false;                       // 8-byte schedule words (a query with far-reaching steps); compact otherwise
+  bool ra_words = false;                   // compact words carry RA (a board too large to keep it in rd)
   std::vector<int64_t> sub_off, sub_m;     // queue range per job
   std::vector<int> job_maxt;
   std::vector<uint64_t> fixed_total;       // counts settled at build time (small tasks, full boards)
@@ -786,7 +788,7 @@ int batch_enqueue(nq_batch* b, int use_graph) {
     cudaError_t e = cudaMemsetAsync(c, 0, cb, st);
     if (e != cudaSuccess) return e;
     TaskArrays ta;
-    ta.info = (uint32_t*)b->info.p; ta.sched = b->sched.p; ta.sw = b->sw; ta.wide = b->wide;
+    ta.info = (uint32_t*)b->info.p; ta.sched = b->sched.p; ta.sw = b->sw; ta.wide = b->wide; ta.ra_words = b->ra_words;
     DfsLaunch L;
     L.tasks = ta; L.sroot = (const uint4*)b->sroot.p; L.sinfo = (const uint2*)b->sinfo.p;
     L.m = b->ms; L.cursor = (unsigned long long*)(c + (size_t)nj * 8);
@@ -890,6 +892,7 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
         if (start_constellations(J.N, bd.starts) != 0) return bad(NQ_EINVAL, "generator failed", j);
         List l;
         l.N = J.N; l.cap = board_bound(J.N, p, bd.starts); l.rows = maxt_for(J.N, p - 3);
+        b->ra_words = b->ra_words || !ra_in_rd(J.N, p - 3, 0);
         if (p > 8 || l.cap > kGenRecords) {      // more than the device generator's buffers: the host's list
           const int s = gen_constellations(J.N, p, bd.recs, 0);
           if (s != 0) return bad(s == -2 ? NQ_EPRESET : NQ_EINVAL, "generator failed", j);
@@ -998,7 +1001,7 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
     ListState* dstate = (ListState*)ds;
     unsigned int* derr = (unsigned int*)(ds + o_err);
     TaskArrays ta;
-    ta.info = (uint32_t*)b->info.p; ta.sched = b->sched.p; ta.sw = b->sw; ta.wide = b->wide;
+    ta.info = (uint32_t*)b->info.p; ta.sched = b->sched.p; ta.sw = b->sw; ta.wide = b->wide; ta.ra_words = b->ra_words;
     // ---- boards: generate (or upload) the records, prepare them into the board's tasks
     for (size_t i = 0; i < nb && e == cudaSuccess; i++) {
       const Board& bd = boards[i];
@@ -1202,7 +1205,7 @@ int nq_batch_run_plain(nq_batch* b, uint64_t* totals) {
     if (b->sub_m[j] > 0) {
       NQ_CUDA(h, cudaMemsetAsync(c, 0, 24, b->stream));
       TaskArrays ta;
-      ta.info = (uint32_t*)b->info.p; ta.sched = b->sched.p; ta.sw = b->sw; ta.wide = b->wide;
+      ta.info = (uint32_t*)b->info.p; ta.sched = b->sched.p; ta.sw = b->sw; ta.wide = b->wide; ta.ra_words = b->ra_words;
       // One job per launch over its subtask range; its tasks carry job id j, which lands in slot 0.
       DfsLaunch L;
       L.tasks = ta; L.sroot = (const uint4*)b->sroot.p + b->sub_off[j]; L.sinfo = (const uint2*)b->sinfo.p + b->sub_off[j];

@@ -326,15 +326,29 @@ NQ_HD Op unpack_compact(uint32_t w, int N, bool term) {
   o.tall = 0;
   return o;
 }
-// Device form of the words: the look-ahead flag inverted, so the DFS step folds it into the look-ahead
-// mask with one three-input op and one test ((mask | word & NOLOOK) != 0).
-constexpr uint32_t C_NOLOOK = C_FC;
-constexpr uint32_t W_NOLOOK = W_FC;
 // True when the op packs into a wide word: LA in the top s bits clear of the flags (s <= 24).
 NQ_HD bool wide_fits(const Op& o) { return o.s <= 24 && (uint64_t)o.la < (1ull << o.s); }
 NQ_HD uint32_t pack_wide_x(const Op& o) {
   return o.s | (o.fc ? W_FC : 0u) | (o.term ? W_TERM : 0u) | (o.tall ? W_TALL : 0u) |
          (o.s ? (o.la << (32 - o.s)) : 0u);
 }
+
+// Device form of the words: the look-ahead flag inverted, so the DFS step folds it into the look-ahead
+// mask with one three-input op and one test ((mask | word & NOLOOK) != 0).  Where the rows and columns left
+// fit 32 bits (ra_in_rd), RA stays out of the compact words: it is or-ed into rd at the root, above the
+// board, and shifts in by itself.  The word behind a task's last one counts: it carries the count flag, and
+// its child dies.
+constexpr uint32_t C_NOLOOK = C_FC;
+constexpr uint32_t W_NOLOOK = W_FC;
+constexpr uint32_t C_COUNT = 1u << 5;            // below RA's bits wherever RA is in the words (N >= 19)
+constexpr uint32_t W_COUNT = W_TERM;             // device words carry neither TERM nor TALL
+constexpr uint32_t kCountWord = 0xFFFFFFFFu;     // shift 31, every column of the child blocked
+// RA stands at most at bit N - 3 of a child row, at most N - 2 - start - D rows below a depth-D frame.
+NQ_HD bool ra_in_rd(int N, int start_min, int D) { return 2 * N - 5 - (start_min < 0 ? 1 : start_min) - D <= 31; }
+NQ_HD uint32_t device_compact(Op o, bool with_ra) {
+  if (!with_ra) o.ra = 0;
+  return pack_compact(o) ^ C_NOLOOK;
+}
+NQ_HD uint32_t device_wide_x(const Op& o) { return (pack_wide_x(o) & ~(W_TERM | W_TALL)) ^ W_NOLOOK; }
 
 }  // namespace nq

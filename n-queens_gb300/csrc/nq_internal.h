@@ -45,7 +45,8 @@ struct TaskArrays {
   uint32_t* info = nullptr;   // info word (T, wexp, root count, N, status)
   void* sched = nullptr;      // per-task schedule words, stride `sw` words
   int sw = 0;                 // schedule words per task (>= T+1 of every task)
-  bool wide = false;          // uint2 words (mixed batches) instead of uint32
+  bool wide = false;          // uint2 words (queries with far-reaching steps) instead of uint32
+  bool ra_words = false;      // compact words carry RA (else it is in the roots' rd)
 };
 
 struct DfsLaunch {
@@ -86,6 +87,7 @@ struct PrepareSplit {
   uint32_t* info = nullptr;
   uint32_t* sched = nullptr;
   int sw = 0;
+  bool ra_words = false;                // RA in the words; else (ra_in_rd holds) in the queue frames' rd
   unsigned int* err = nullptr;
   unsigned int* tmax = nullptr;         // optional
   unsigned long long* per_task = nullptr;    // optional; set for every task

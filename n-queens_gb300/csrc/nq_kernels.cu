@@ -61,7 +61,7 @@ template <bool WIDE> using WordT = QueryWord<WIDE>;
 // ---------------------------------------------------------------------------
 // prepare
 // ---------------------------------------------------------------------------
-// Device words of one record's task, its info word and root; returns T or -1.  emit(depth, word).
+// One record's task: info word, root, and its ops in order, emit(depth, op); returns T or -1.
 template <bool WIDE, class Emit>
 __device__ __forceinline__ int prepare_task(int N, const uint4 r, int sw, Root& rt, uint32_t& info, unsigned int* err, Emit&& emit) {
   uint32_t status = TS_OK;
@@ -79,8 +79,8 @@ __device__ __forceinline__ int prepare_task(int N, const uint4 r, int sw, Root& 
     if (status == TS_OK) {
       const int lim = sw < kMaxDepth ? sw : kMaxDepth;
       T = walk_schedule(N, h, &rt, &root_count, lim, [&](int d, const Op& o) {
-        if constexpr (WIDE) { fits = fits && wide_fits(o); emit(d, make_uint2(pack_wide_x(o) ^ W_NOLOOK, o.ra)); }
-        else { fits = fits && compact_fits(o, N); emit(d, pack_compact(o) ^ C_NOLOOK); }
+        fits = fits && (WIDE ? wide_fits(o) : compact_fits(o, N));
+        emit(d, o);
       });
       if (T == -2) status = (lim < kMaxDepth) ? TS_DEPTH : TS_NOTERM;
       else if (T >= 0 && !fits) status = TS_FORMAT;   // never seen (N=6..21, presets 4-7): fail loudly rather than miscount
@@ -100,13 +100,25 @@ __device__ __forceinline__ void max_depth_of(unsigned int* tmax, int T) {
   if ((threadIdx.x & 31u) == 0 && v) atomicMax(tmax, v);
 }
 
+// RA of a task's rows as bits of the root's rd: each stands as many places above its own as rows follow.
+struct RaInRd {
+  unsigned long long bits = 0;
+  uint32_t rows = 0;                  // below the root so far
+  __device__ __forceinline__ void add(const Op& o) { rows += o.s; bits |= (unsigned long long)o.ra << rows; }
+  __device__ __forceinline__ uint32_t at(uint32_t row, unsigned int* err) const {   // as seen from `row` below the root
+    const unsigned long long v = bits >> row;
+    if (v >> 32) atomicOr(err, DERR_FORMAT);     // not with ra_in_rd's bound: fail loudly rather than miscount
+    return (uint32_t)v;
+  }
+};
+
 template <bool WIDE>
 __global__ void __launch_bounds__(256) prepare_kernel(int N, int64_t m, const unsigned* __restrict__ m_dev,
                                                       const uint4* __restrict__ rec, uint4* __restrict__ root,
                                                       uint32_t* __restrict__ info,
-                                                      typename WordT<WIDE>::type* __restrict__ sched, int sw,
-                                                      int64_t offset, unsigned int* err, unsigned int* tmax, unsigned int* n_out) {
-  using W = typename WordT<WIDE>::type;
+                                                      typename WordT<WIDE>::type* __restrict__ sched, int sw, bool ra_words,
+                                                      int64_t offset, unsigned int* err, unsigned int* tmax,
+                                                      unsigned int* n_out) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (m_dev) m = *m_dev;
   if (i == 0) *n_out = (unsigned int)m;
@@ -115,7 +127,13 @@ __global__ void __launch_bounds__(256) prepare_kernel(int N, int64_t m, const un
     const int64_t t = offset + i;
     Root rt;
     uint32_t in;
-    T = prepare_task<WIDE>(N, rec[i], sw, rt, in, err, [&](int d, W w) { sched[t * sw + d] = w; });
+    RaInRd ra;
+    T = prepare_task<WIDE>(N, rec[i], sw, rt, in, err, [&](int d, const Op& o) {
+      if constexpr (WIDE) sched[t * sw + d] = make_uint2(device_wide_x(o), o.ra);
+      else sched[t * sw + d] = device_compact(o, ra_words);
+      ra.add(o);
+    });
+    if (!WIDE && !ra_words) rt.rd |= ra.at(0, err);
     root[t] = make_uint4(rt.ld, rt.rd, rt.col, T < 0 ? 0u : rt.avail);
     info[t] = in;
   }
@@ -128,11 +146,11 @@ cudaError_t launch_prepare(int N, int64_t m, const unsigned int* m_dev, const ui
   const int B = 256;
   const unsigned G = (unsigned)((m + B - 1) / B);
   if (out.wide)
-    prepare_kernel<true><<<G, B, 0, st>>>(N, m, m_dev, records, out.root, out.info, (uint2*)out.sched, out.sw, offset, err,
-                                          tmax, n_out);
+    prepare_kernel<true><<<G, B, 0, st>>>(N, m, m_dev, records, out.root, out.info, (uint2*)out.sched, out.sw,
+                                          out.ra_words, offset, err, tmax, n_out);
   else
-    prepare_kernel<false><<<G, B, 0, st>>>(N, m, m_dev, records, out.root, out.info, (uint32_t*)out.sched, out.sw, offset,
-                                           err, tmax, n_out);
+    prepare_kernel<false><<<G, B, 0, st>>>(N, m, m_dev, records, out.root, out.info, (uint32_t*)out.sched, out.sw,
+                                           out.ra_words, offset, err, tmax, n_out);
   return cudaGetLastError();
 }
 
@@ -190,15 +208,21 @@ __global__ void __launch_bounds__(256) prepare_split_kernel(const PrepareSplit a
   Root rt = {0, 0, 0, 0};
   uint32_t in = 0, w[D > 0 ? D : 1] = {0};
   int T = -1;
+  RaInRd ra;
+  uint32_t rows_d = 0;                           // rows from the root to depth D
   if (t < m) {
-    T = prepare_task<false>(a.N, a.rec[t], a.sw, rt, in, a.err, [&](int d, uint32_t x) {
-      a.sched[t * a.sw + d] = x;
+    T = prepare_task<false>(a.N, a.rec[t], a.sw, rt, in, a.err, [&](int d, const Op& o) {
+      a.sched[t * a.sw + d] = device_compact(o, a.ra_words);
+      Op p = o;
+      if (d < D) { rows_d += o.s; p.ra = 0; }    // above depth D the words below apply it
 #pragma unroll
       for (int k = 0; k < D; k++)
-        if (d == k) w[k] = x;
+        if (d == k) w[k] = device_compact(o, true);
+      ra.add(p);
     });
     a.info[t] = in;
     if (D == 0) {
+      if (!a.ra_words) rt.rd |= ra.at(0, a.err);
       a.root[t] = make_uint4(rt.ld, rt.rd, rt.col, T < 0 ? 0u : rt.avail);
       if (a.per_task) a.per_task[t] = 0;      // the DFS adds the task's counts
     }
@@ -219,7 +243,9 @@ __global__ void __launch_bounds__(256) prepare_split_kernel(const PrepareSplit a
     base = __shfl_sync(FULL, base, 31) + (incl - n);
     if (n && base + n <= a.qcap) {            // a queue that does not fit is sized by qn and built again
       uint32_t dummy = 0;
+      const uint32_t later = a.ra_words ? 0u : ra.at(rows_d, a.err);
       frames_at<0, D>(rt.ld, rt.rd, rt.col, rt.avail, w, (uint32_t)a.N, (uint32_t)T, dummy, [&](uint4 f) {
+        f.y |= later;
         a.sroot[base] = f;
         a.sinfo[base++] = make_uint2((uint32_t)t, (uint32_t)D);
       });
@@ -455,9 +481,9 @@ __device__ __forceinline__ void flush_job(const DfsArgs& a, unsigned job, unsign
   if (v) atomicAdd(a.job_totals + (job - a.job_base), v);
 }
 
-// Shared memory per lane: frames at depths 0..maxt above the sentinel's slot, and schedule words
-// 0..maxt with the sentinel's word behind them.
-__host__ __device__ constexpr int stack_slots(int maxt) { return maxt + 2; }
+// Shared memory per lane: the sentinel's frame, frames at depths 0..maxt and the base frame's slot, and
+// schedule words 0..maxt with the count word behind them.
+__host__ __device__ constexpr int stack_slots(int maxt) { return maxt + 3; }
 __host__ __device__ constexpr int word_slots(int maxt) { return maxt + 2; }
 
 size_t dfs_smem_bytes(bool wide, int block, int maxt) {
@@ -476,26 +502,32 @@ __device__ __forceinline__ uint2 lds_word(uint32_t a, uint2) {
   return w;
 }
 
-// The sentinel frame under a lane's stack feeds a lane that has run out of work: its word (all ones)
-// shifts by 31 and fills every column of ld, so each of its 31 candidates dies.  kStepsPerCheck <= 31
-// steps therefore never pop below it, and the step tests neither the stack's depth nor the lane's
-// activity.
+// The sentinel frame under a lane's stack feeds a lane that has run out of work: its word is the count
+// word, so each of its 31 candidates dies and is counted, and a check takes the used ones off the lane's
+// count.  kStepsPerCheck <= 31 steps therefore never pop below it, and the step tests neither the stack's
+// depth nor the lane's activity.
 constexpr uint32_t kSentinelAvail = 0xFFFFFFFEu;   // bits 1..31: ld + bit stays odd (ld = 1), so bit 31 of nld is set
-constexpr uint32_t kSentinelWord = 0xFFFFFFFFu;
 static_assert(kStepsPerCheck <= 31 && kStepsPerCheck % kStepUnroll == 0, "the sentinel holds 31 candidates");
+
+enum WordForm { kRaInRd, kRaInWords, kWideWords };   // compact words without and with RA, wide words
 
 // One lane's DFS state and its step.  Every lane runs the same predicated sequence each step: resume a
 // saved frame if the current one is exhausted, take the lowest candidate, save the frame with the rest,
-// build the child with the depth's schedule word and make it the current frame -- with no candidates if
-// the look-ahead rejects it or its row is the last (counted there), so the next step resumes the saved
-// frame.  The frame is stored whether or not candidates are left (the slot above the stack is free) and
-// only the stack pointer moves by the test: the store costs the same wavefronts either way, and no
-// select is left but the child's candidates.  Selecting between parent and child instead (four selects
-// and a predicate passed into the store) took 18.1 ALU instructions a step against 16.7: N=19 84.6 ms,
-// this form 75.1 ms; N=17 2.08 ms, 1.92 ms.  '+' and '-' replace '|' and '&~' where the bits are disjoint (a candidate is never in ld or
-// rd, and always one of the free columns), so those ops issue on the FMA pipe as well as the ALU pipe.
+// build the child with the depth's schedule word and make it the current frame, without candidates if the
+// look-ahead rejects it, so the next step resumes the saved frame.
+//  - The frame is stored whether or not candidates are left (the slot above the stack is free) and only the
+//    stack pointer moves by the test: the store costs the same wavefronts either way, and the one select
+//    left is the child's candidates.  Selecting between parent and child (four selects and a predicate
+//    passed into the store): N=19 84.6 ms, this form 75.1.
+//  - A solution is a frame in the base row: it has one column left, its word is the count word, and the
+//    step adds that word's flag.  Comparing each step's depth with the terminal one and masking the child
+//    there (3 instructions more, 1 % fewer steps): N=19 71.8 ms, this form 66.6; N=17 1.63, 1.49.
+//  - rest = avail & (avail - 1), bit = avail - rest, instead of bit = avail & -avail: 66.6 -> 65.0.
+//  - RA in rd instead of the words (one op): 65.0 -> 63.6.
+// '+' and '-' replace '|' and '&~' where the bits are disjoint (a candidate is never in ld or rd, and
+// always one of the free columns), so those ops issue on the FMA pipe as well as the ALU pipe.
 // Per-task counts are u32 (BIG: u64, where a queue item may count 2^32 solutions).
-template <bool WIDE, bool BIG>
+template <WordForm FORM, bool BIG>
 struct Lane {
   // A frame is {ld, rd, fr, avail}: fr holds the columns still free at the frame's
   // row (one fewer per level, so a frame's depth is popc(root fr) - popc(fr) and
@@ -504,12 +536,12 @@ struct Lane {
   uint32_t sp = 0;      // shared address of the next free frame of this lane's stack
   uint32_t sw0 = 0;     // shared address of the word of the depth where popc(fr) == 0 (word d sits at
                         // sw0 - popc(fr) * row, row = BLOCK words, since popc(fr) = R - d, R = popc(root fr))
-  uint32_t tf = ~0u;    // popc(fr) at the subtask's terminal depth: R - terminal depth
-  uint32_t ram = 0;     // compact words: the bits where RA << s may sit (compact_ra_mask)
+  uint32_t ram = 0;     // RA in the words: the bits where RA << s may sit (compact_ra_mask)
   typename std::conditional<BIG, unsigned long long, uint32_t>::type cnt = 0;
 
   template <int BLOCK>
   __device__ __forceinline__ void step() {
+    constexpr bool WIDE = FORM == kWideWords;
     using W = typename WordT<WIDE>::type;
     constexpr uint32_t F = BLOCK * (uint32_t)sizeof(uint4);
     constexpr uint32_t ROW = BLOCK * (uint32_t)sizeof(W);
@@ -519,8 +551,8 @@ struct Lane {
                  "@p sub.u32 %4, %4, %5;\n\t@p ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
                  : "+r"(ld), "+r"(rd), "+r"(fr), "+r"(avail), "+r"(sp) : "n"(F));
     const uint32_t pf = __popc(fr);                  // R - depth
-    const uint32_t bit = avail & (0u - avail);
-    const uint32_t rest = avail - bit;
+    const uint32_t rest = avail & (avail - 1u);
+    const uint32_t bit = avail - rest;
     const W w = lds_word(sw0 - pf * ROW, W{});
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" :: "r"(sp), "r"(ld), "r"(rd), "r"(fr), "r"(rest) : "memory");
     if (rest != 0u) sp += F;
@@ -528,23 +560,43 @@ struct Lane {
     uint32_t wx, nld, nrd, y = rd + bit;
     if constexpr (WIDE) wx = w.x; else wx = w;
     asm("shf.l.wrap.b32 %0, %1, %2, %1;" : "=r"(nld) : "r"(wx), "r"(ld + bit));
-    // compact: nrd = ((y | RA << s) >> s) = (y >> s) | RA, RA << s or-ed in from the word's bits N-1..N;
-    // wide: RA, which may sit anywhere, is or-ed after the right shift
-    if constexpr (!WIDE) asm("lop3.b32 %0, %1, %2, %3, 0xF8;" : "=r"(y) : "r"(rd + bit), "r"(wx), "r"(ram));   // a | (b & c)
+    // RA in the words: nrd = ((y | RA << s) >> s) = (y >> s) | RA, RA << s or-ed in from bits N-1..N; wide
+    // words: RA, which may sit anywhere, is or-ed after the right shift
+    if constexpr (FORM == kRaInWords) asm("lop3.b32 %0, %1, %2, %3, 0xF8;" : "=r"(y) : "r"(rd + bit), "r"(wx), "r"(ram));   // a | (b & c)
     asm("shf.r.wrap.b32 %0, %1, 0, %2;" : "=r"(nrd) : "r"(y), "r"(wx));
     if constexpr (WIDE) nrd |= w.y;
     const uint32_t free_cols = fr - bit;             // the child row's free columns
     const uint32_t nf = free_cols & ~(nld | nrd);
     const uint32_t ahead = free_cols & ~((nld + nld) | __umulhi(nrd, 0x80000000u));   // nrd >> 1
     const uint32_t keep = ahead | (wx & (WIDE ? W_NOLOOK : C_NOLOOK));
-    // terminal depth: count the child if its row has a free square (the SQd2B rule is LA bit 0 of the word);
-    // otherwise descend unless the child row or, with look-ahead, the row after is full
-    const bool term = pf == tf;
-    if (term && nf != 0u) cnt += 1u;
+    if (wx & (WIDE ? W_COUNT : C_COUNT)) cnt += 1u;
     ld = nld; rd = nrd; fr = free_cols;
-    avail = (nf != 0u && keep != 0u && !term) ? nf : 0u;
+    avail = keep != 0u ? nf : 0u;
   }
 };
+
+// Items whose schedule ends with more than one column left (no list of the generators has one): base frames
+// count once, whatever candidates they have.  One lane alone, its frames in local memory.
+template <WordForm FORM, class W>
+__device__ __noinline__ unsigned long long count_base_frames(uint4 f, uint32_t fr, uint32_t N, uint32_t n, const W* words) {
+  uint4 st[kMaxDepth];
+  unsigned long long c = 0;
+  int k = 0;
+  st[0] = make_uint4(f.x, f.y, fr, f.w & fr);
+  while (k >= 0) {
+    uint4& g = st[k];
+    if (g.w == 0u) { k--; continue; }
+    const uint32_t bit = g.w & (0u - g.w);
+    g.w ^= bit;
+    const Dec o = decode(words[k], N, (uint32_t)k, n);
+    const uint32_t nld = ((g.x | bit) << o.s) | o.la, nrd = ((g.y | bit) >> o.s) | o.ra, free_cols = g.z ^ bit;
+    const uint32_t nf = free_cols & ~(nld | nrd);
+    if (nf == 0u || (o.fc && (free_cols & ~((nld << 1) | (nrd >> 1))) == 0u)) continue;
+    if (o.term) c++;
+    else st[++k] = make_uint4(nld, nrd, free_cols, nf);
+  }
+  return c;
+}
 
 __device__ __forceinline__ void sts_frame(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
   asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" :: "r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
@@ -554,8 +606,9 @@ __device__ __forceinline__ uint4 lds_frame(uint32_t a) {
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(f.x), "=r"(f.y), "=r"(f.z), "=r"(f.w) : "r"(a) : "memory");
   return f;
 }
-template <bool WIDE, int BLOCK, bool BIG>
+template <WordForm FORM, int BLOCK, bool BIG>
 __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
+  constexpr bool WIDE = FORM == kWideWords;
   using W = typename WordT<WIDE>::type;
   extern __shared__ __align__(16) unsigned char smem[];
   W* sch = reinterpret_cast<W*>(smem + (size_t)stack_slots(a.maxt) * BLOCK * sizeof(uint4)) + threadIdx.x;  // stride BLOCK
@@ -565,8 +618,9 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
   constexpr uint32_t ROW = BLOCK * (uint32_t)sizeof(W);
   constexpr uint32_t F = BLOCK * (uint32_t)sizeof(uint4);
   auto put_word = [&](uint32_t k, W w) { sch[k * BLOCK] = w; };
-  auto sentinel_word = [] { W w; if constexpr (WIDE) w = make_uint2(kSentinelWord, 0u); else w = kSentinelWord; return w; };
-  Lane<WIDE, BIG> L;
+  auto count_word = [] { W w; if constexpr (WIDE) w = make_uint2(kCountWord, 0u); else w = kCountWord; return w; };
+  Lane<FORM, BIG> L;
+  uint32_t tf = 1;                    // popc(fr) at the terminal depth: R - terminal depth; the base frame's is one less
   const uint32_t sch_sh = (uint32_t)__cvta_generic_to_shared(sch);
   const uint32_t bottom = (uint32_t)__cvta_generic_to_shared(smem) + threadIdx.x * (uint32_t)sizeof(uint4);
   // stack pointer above the sentinel: a lane is idle when no frame but the sentinel is left.  The sentinel
@@ -574,10 +628,9 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
   uint32_t top = bottom + F;
   L.sp = top;
   L.sw0 = sch_sh;                     // a lane without work reads word 0 (the sentinel's fr is 0)
-  L.tf = 1;
-  put_word(0, sentinel_word());
-  // where popc(fr) == tf - 1 the lane's word is the sentinel's
-  auto arm = [&]() { sts_frame(top - F, 1u, 0u, (1u << (L.tf - 1u)) - 1u, kSentinelAvail); };
+  put_word(0, count_word());
+  // where popc(fr) == tf - 1 the lane's word is the count word
+  auto arm = [&]() { sts_frame(top - F, 1u, 0u, (1u << (tf - 1u)) - 1u, kSentinelAvail); };
   uint32_t wexp = 0, job = a.job_base, task = 0;
   bool have = false, exhausted = false, drained = false;   // exhausted, drained: warp-uniform, as the pool's counters
   unsigned long long m = a.m;
@@ -595,7 +648,10 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
   for (;;) {
     const bool idle = L.avail == 0u && L.sp == top;
     if (__ballot_sync(FULL, idle)) {          // some lane finished: flush, refill, maybe exit
-      if (idle) arm();                        // the steps since it finished have used some of its candidates
+      if (idle) {                             // the steps since it finished have used (and counted) some of its candidates
+        L.cnt -= 31u - (uint32_t)__popc(lds_frame(top - F).w);
+        arm();
+      }
       if (idle && have) {
         const unsigned long long v = (unsigned long long)L.cnt << wexp;
         if (a.per_task && v) atomicAdd(a.per_task + task, v);
@@ -661,11 +717,13 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
             const uint32_t R = __popc(fr);
             const W* src_w = gsched + (size_t)task * a.sw + d0;
             const uint32_t n = T - d0;           // terminal depth
-            if (n + 2u <= R) {                   // fewer free columns than rows: no solution, no work
+            if (n + 2u < R) {
+              L.cnt += count_base_frames<FORM>(r, fr, info_N(i_info), n, src_w);
+            } else if (n + 2u == R) {            // fewer free columns than rows: no solution, no work
               L.ld = r.x; L.rd = r.y; L.fr = fr; L.avail = r.w & fr;
-              L.tf = R - n; L.sw0 = sch_sh + R * ROW; L.ram = compact_ra_mask((int)info_N(i_info));
+              tf = R - n; L.sw0 = sch_sh + R * ROW; L.ram = compact_ra_mask((int)info_N(i_info));
               for (uint32_t k = 0; k <= n; k++) put_word(k, src_w[k]);
-              put_word(n + 1u, sentinel_word());
+              put_word(n + 1u, count_word());
               arm();
             }
           }
@@ -683,7 +741,7 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
           const uint32_t rest = L.avail & (L.avail - 1u);
           const uint32_t gfr = saved ? lds_frame(top).z : L.fr;
           const bool can = have && (saved ? (L.avail != 0u || L.sp != top + F) : rest != 0u) &&
-                           __popc(gfr) >= (int)L.tf + kGiveRows;
+                           __popc(gfr) >= (int)tf + kGiveRows;
           const unsigned givers = __ballot_sync(FULL, can);
           if (givers) {
             const int n = min(__popc(starved), __popc(givers));
@@ -694,13 +752,13 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
             __syncwarp();
             const int src = takes ? (int)nth_set(givers, (uint32_t)srank) : (int)lane;
             const uint32_t from = __shfl_sync(FULL, top, src), gsw0 = __shfl_sync(FULL, L.sw0, src);
-            const uint32_t gtf = __shfl_sync(FULL, L.tf, src), gram = __shfl_sync(FULL, L.ram, src);
+            const uint32_t gtf = __shfl_sync(FULL, tf, src), gram = __shfl_sync(FULL, L.ram, src);
             const uint32_t gw = __shfl_sync(FULL, wexp, src), gjob = __shfl_sync(FULL, job, src);
             const uint32_t gtask = __shfl_sync(FULL, task, src);
             if (takes) {
               const uint4 f = lds_frame(from);
               L.ld = f.x; L.rd = f.y; L.fr = f.z; L.avail = f.w;
-              L.sw0 = gsw0; L.tf = gtf; L.ram = gram; L.cnt = 0;
+              L.sw0 = gsw0; tf = gtf; L.ram = gram; L.cnt = 0;
               wexp = gw; job = gjob; task = gtask; have = true;
               top = bottom + F; L.sp = top;
               arm();
@@ -742,17 +800,17 @@ cudaError_t allow_max_dynamic_smem(K kernel) {
   return e;
 }
 
-template <bool WIDE, int BLOCK, bool BIG>
+template <WordForm FORM, int BLOCK, bool BIG>
 static cudaError_t launch_dfs_t(const DfsLaunch& L, cudaStream_t st) {
-  const size_t smem = dfs_smem_bytes(WIDE, BLOCK, L.maxt);
-  cudaError_t e = allow_max_dynamic_smem(dfs_kernel<WIDE, BLOCK, BIG>);
+  const size_t smem = dfs_smem_bytes(FORM == kWideWords, BLOCK, L.maxt);
+  cudaError_t e = allow_max_dynamic_smem(dfs_kernel<FORM, BLOCK, BIG>);
   if (e != cudaSuccess) return e;
   int grid = L.grid;
   if (grid <= 0) {
     int dev = 0, sms = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, dfs_kernel<WIDE, BLOCK, BIG>, BLOCK, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, dfs_kernel<FORM, BLOCK, BIG>, BLOCK, smem);
     if (e != cudaSuccess) return e;
     if (per <= 0) return cudaErrorInvalidConfiguration;
     grid = sms * per;
@@ -762,7 +820,7 @@ static cudaError_t launch_dfs_t(const DfsLaunch& L, cudaStream_t st) {
   a.sroot = L.sroot; a.sinfo = L.sinfo;
   a.m = L.m; a.m_dev = L.m_dev; a.qcap = L.qcap; a.order = L.order; a.cursor = L.cursor; a.job_totals = L.job_totals; a.job_base = L.job_base;
   a.per_task = L.per_task; a.err = L.err; a.maxt = L.maxt;
-  dfs_kernel<WIDE, BLOCK, BIG><<<grid, BLOCK, smem, st>>>(a);
+  dfs_kernel<FORM, BLOCK, BIG><<<grid, BLOCK, smem, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -770,9 +828,11 @@ static cudaError_t launch_dfs_t(const DfsLaunch& L, cudaStream_t st) {
 cudaError_t launch_dfs(const DfsLaunch& L, cudaStream_t st) {
   if (L.m <= 0 && !L.m_dev) return cudaSuccess;
   if (L.maxt < 1 || L.maxt > kMaxDepth) return cudaErrorInvalidValue;
-#define NQ_DFS_BLOCK(B)                                                                        \
-  if (L.tasks.wide) return L.big ? launch_dfs_t<true, B, true>(L, st) : launch_dfs_t<true, B, false>(L, st); \
-  return L.big ? launch_dfs_t<false, B, true>(L, st) : launch_dfs_t<false, B, false>(L, st);
+#define NQ_DFS_FORM(B, FORM) return L.big ? launch_dfs_t<FORM, B, true>(L, st) : launch_dfs_t<FORM, B, false>(L, st)
+#define NQ_DFS_BLOCK(B)                                   \
+  if (L.tasks.wide) NQ_DFS_FORM(B, kWideWords);           \
+  if (L.tasks.ra_words) NQ_DFS_FORM(B, kRaInWords);       \
+  NQ_DFS_FORM(B, kRaInRd);
   switch (L.block) {
     case 64: { NQ_DFS_BLOCK(64) }
     case 128: { NQ_DFS_BLOCK(128) }
@@ -780,14 +840,16 @@ cudaError_t launch_dfs(const DfsLaunch& L, cudaStream_t st) {
     default: return cudaErrorInvalidValue;
   }
 #undef NQ_DFS_BLOCK
+#undef NQ_DFS_FORM
 }
 
 template <bool WIDE, int BLOCK>
 static int occ(int maxt) {
+  constexpr WordForm FORM = WIDE ? kWideWords : kRaInWords;      // shared memory bounds it, alike for both compact forms
   const size_t smem = dfs_smem_bytes(WIDE, BLOCK, maxt);
-  if (allow_max_dynamic_smem(dfs_kernel<WIDE, BLOCK, false>) != cudaSuccess) return 0;
+  if (allow_max_dynamic_smem(dfs_kernel<FORM, BLOCK, false>) != cudaSuccess) return 0;
   int per = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, dfs_kernel<WIDE, BLOCK, false>, BLOCK, smem) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, dfs_kernel<FORM, BLOCK, false>, BLOCK, smem) != cudaSuccess)
     return 0;
   return per;
 }

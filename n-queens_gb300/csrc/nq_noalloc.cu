@@ -110,8 +110,9 @@ extern "C" int nq_exec_solutions_noalloc(int N, const nq_record* d_records, int6
       P.sinfo = (uint2*)(P.sroot + P.qcap);
       L.sroot = P.sroot; L.sinfo = P.sinfo; L.m_dev = P.qn; L.qcap = P.qcap;
     }
+    P.ra_words = !ra_in_rd(N, start_min, D);
     if (launch_prepare_split(D, m, P, st) != cudaSuccess) return NQ_ECUDA;
-    L.tasks.root = P.root; L.tasks.info = P.info; L.tasks.sched = P.sched; L.tasks.sw = P.sw; L.tasks.wide = false;
+    L.tasks.root = P.root; L.tasks.info = P.info; L.tasks.sched = P.sched; L.tasks.sw = P.sw; L.tasks.wide = false; L.tasks.ra_words = P.ra_words;
     L.cursor = cursor; L.job_totals = totals;
     L.per_task = (unsigned long long*)d_solutions; L.err = err; L.maxt = maxt - D < 1 ? 1 : maxt - D; L.block = 128; L.grid = 0;
     L.big = counts_need_u64(N, m);
