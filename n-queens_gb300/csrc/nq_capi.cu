@@ -623,20 +623,67 @@ uint64_t start_bound(int N, int preset, int start) {
   return b;
 }
 
-uint64_t board_bound(int N, int p, const std::vector<int>& starts) {
-  uint64_t b = 0;
-  for (int s : starts) b += std::max<uint64_t>(1, start_bound(N, p, s));
-  return b;
+// A bound on a board's start constellations (about twice their number: every candidate of the reference's
+// loops, before rotations are dropped, and the corner ones) and on its records.
+uint64_t board_starts(int N) {
+  uint64_t n = 0;
+  for (int k = 1; k < (N + 1) / 2; k++) {
+    const int j_max = N - k - 2;
+    for (int l = k + 1; l <= N - 2; l++)
+      for (int i = k + 1; i <= N - 2; i++)
+        if (i != N - 1 - l) n += (uint64_t)std::max(0, j_max - (i <= j_max) - (l <= j_max && l != i));
+  }
+  return n + (uint64_t)(N - 2) * (N - 3) / 2;
+}
+uint64_t board_bound(int N, int p) {
+  uint64_t side = board_starts(N) - (uint64_t)(N - 2) * (N - 3) / 2, corner = (uint64_t)(N - 2) * (N - 3) / 2;
+  for (int q = 4; q < p; q++) side *= (uint64_t)std::max(0, N - q);
+  for (int q = 3; q < p; q++) corner *= (uint64_t)std::max(0, N - q);
+  return std::max(side + corner, board_starts(N));
 }
 
-int count_generated(nq_handle* h, int N, int p, const std::vector<int>& starts, size_t s_begin, size_t s_end,
-                    uint64_t* total) {
+// One generated chunk on the handle's stream: starts (host list, or null: the whole board), counted.
+int count_chunk(nq_handle* h, int N, int p, const int* starts, size_t n, uint64_t bound, uint64_t* total, int64_t* records) {
   cudaStream_t st = h->stream;
   NQ_CUDA(h, cudaSetDevice(h->device));
   NQ_CUDA(h, h->ctrl.ensure(ctl::kAll));
   unsigned char* c = (unsigned char*)h->ctrl.p;
   unsigned int* gn = (unsigned int*)(c + ctl::kGen);
   const int levels = gen_levels(p);
+  if (bound > 0x7FFFFFFFull) return h->fail(NQ_ENOMEM, "generator: too many records from one start constellation");
+  const size_t cap = std::max<size_t>((size_t)bound, n);
+  NQ_CUDA(h, h->rec.ensure(cap * sizeof(uint4)));
+  NQ_CUDA(h, h->gen.ensure(cap * sizeof(uint4)));
+  if (int e = h->ensure_pinned(kStage + (starts ? n * sizeof(int) : 0))) return e;
+  if (starts) {
+    NQ_CUDA(h, h->starts.ensure(n * sizeof(int)));
+    std::memcpy((unsigned char*)h->h_ctrl + kStage, starts, n * sizeof(int));
+    NQ_CUDA(h, cudaMemcpyAsync(h->starts.p, (unsigned char*)h->h_ctrl + kStage, n * sizeof(int), cudaMemcpyHostToDevice, st));
+  }
+  NQ_CUDA(h, cudaMemsetAsync(c, 0, ctl::kAll, st));
+  uint4* buf[2] = {(uint4*)h->rec.p, (uint4*)h->gen.p};
+  NQ_CUDA(h, launch_generate(N, p, (unsigned)n, starts ? (const int*)h->starts.p : nullptr, buf[0], buf[1], (unsigned)cap, gn,
+                             (unsigned int*)(c + ctl::kGenErr), h->sms, st));
+  const uint4* rec = buf[levels & 1];
+  const int t_max = std::max(1, N - p - 2);        // a queen a depth, one column left in the base row
+  const bool on_device = (int64_t)bound <= kGenNoReadBack && h->queue_order == 0;
+  int64_t m = (int64_t)bound;
+  if (!on_device) {
+    NQ_CUDA(h, cudaMemcpyAsync(h->h_ctrl, c, ctl::kAll, cudaMemcpyDeviceToHost, st));
+    NQ_CUDA(h, cudaStreamSynchronize(st));
+    m = *(const uint32_t*)((const unsigned char*)h->h_ctrl + ctl::kGen + 4 * levels);
+  }
+  if (m > 0)
+    if (int e = run_records(h, N, rec, m, p - 3, nullptr, st, t_max, on_device ? gn + levels : nullptr)) return e;
+  if (int e = read_ctrl(h, st, total)) return e;
+  const unsigned char* hc = (const unsigned char*)h->h_ctrl;
+  if (*(const uint32_t*)(hc + ctl::kGenErr)) return h->fail(NQ_EPRESET, "generator: preset %d too deep for N=%d", p, N);
+  *records = *(const uint32_t*)(hc + ctl::kGen + 4 * levels);
+  return NQ_OK;
+}
+
+int count_generated(nq_handle* h, int N, int p, const std::vector<int>& starts, size_t s_begin, size_t s_end,
+                    uint64_t* total) {
   uint64_t acc = 0;
   int64_t chunks = 0, records = 0;
   for (size_t s0 = s_begin; s0 < s_end;) {
@@ -644,39 +691,13 @@ int count_generated(nq_handle* h, int N, int p, const std::vector<int>& starts, 
     uint64_t bound = 0;
     do { bound += std::max<uint64_t>(1, start_bound(N, p, starts[s1++])); }
     while (s1 < s_end && bound + start_bound(N, p, starts[s1]) <= kGenRecords);
-    const size_t n = s1 - s0;
-    if (bound > 0x7FFFFFFFull) return h->fail(NQ_ENOMEM, "generator: too many records from one start constellation");
-    const size_t cap = std::max<size_t>((size_t)bound, n);
-    NQ_CUDA(h, h->rec.ensure(cap * sizeof(uint4)));
-    NQ_CUDA(h, h->gen.ensure(cap * sizeof(uint4)));
-    NQ_CUDA(h, h->starts.ensure(n * sizeof(int)));
-    if (int e = h->ensure_pinned(kStage + n * sizeof(int))) return e;
-    std::memcpy((unsigned char*)h->h_ctrl + kStage, &starts[s0], n * sizeof(int));
-    NQ_CUDA(h, cudaMemcpyAsync(h->starts.p, (unsigned char*)h->h_ctrl + kStage, n * sizeof(int), cudaMemcpyHostToDevice, st));
-    NQ_CUDA(h, cudaMemsetAsync(c, 0, ctl::kAll, st));
-    uint4* buf[2] = {(uint4*)h->rec.p, (uint4*)h->gen.p};
-    NQ_CUDA(h, launch_generate(N, p, (unsigned)n, (const int*)h->starts.p, buf[0], buf[1], (unsigned)cap, gn,
-                               (unsigned int*)(c + ctl::kGenErr), h->sms, st));
-    const uint4* rec = buf[levels & 1];
-    const int t_max = std::max(1, N - p - 2);        // a queen a depth, one column left in the base row
-    const bool on_device = (int64_t)bound <= kGenNoReadBack && h->queue_order == 0;
-    int64_t m = (int64_t)bound;
-    if (!on_device) {
-      NQ_CUDA(h, cudaMemcpyAsync(h->h_ctrl, c, ctl::kAll, cudaMemcpyDeviceToHost, st));
-      NQ_CUDA(h, cudaStreamSynchronize(st));
-      m = *(const uint32_t*)((const unsigned char*)h->h_ctrl + ctl::kGen + 4 * levels);
-    }
-    if (m > 0)
-      if (int e = run_records(h, N, rec, m, p - 3, nullptr, st, t_max, on_device ? gn + levels : nullptr)) return e;
     uint64_t t = 0;
-    if (int e = read_ctrl(h, st, &t)) return e;
-    const unsigned char* hc = (const unsigned char*)h->h_ctrl;
-    if (*(const uint32_t*)(hc + ctl::kGenErr)) return h->fail(NQ_EPRESET, "generator: preset %d too deep for N=%d", p, N);
-    acc += t; chunks++; records += *(const uint32_t*)(hc + ctl::kGen + 4 * levels);
+    int64_t r = 0;
+    if (int e = count_chunk(h, N, p, &starts[s0], s1 - s0, bound, &t, &r)) return e;
+    acc += t; chunks++; records += r;
     s0 = s1;
   }
-  if (records == 0) chunks = 0;
-  h->last_chunks = chunks;
+  h->last_chunks = records == 0 ? 0 : chunks;
   h->last_records = records;
   *total = acc;
   return NQ_OK;
@@ -686,14 +707,21 @@ int count_generated(nq_handle* h, int N, int p, const std::vector<int>& starts, 
 
 extern "C" {
 
-// Whole-board count: the start constellations are listed first (cheap), then
-// counted as one range.
+// Whole-board count: in one go where the device makes the whole board's list, else the start constellations
+// are listed (cheap) and counted as one range.
 int nq_count(nq_handle* h, int N, int preset, uint64_t* total) {
   if (!h || !total) return NQ_EINVAL;
   if (N < 1 || N > kMaxN) return h->fail(NQ_EINVAL, "N=%d outside 1..27", N);
   if (N <= 5) return nq_count_completions(h, N, 0, nullptr, nullptr, total);
   const int p = preset > 0 ? preset : preset_for(N);
   if (p < 4) return h->fail(NQ_EPRESET, "generator: preset %d below 4", p);
+  if (h->chunk_records == 0 && p <= 8 && board_bound(N, p) <= kGenRecords) {
+    int64_t records = 0;
+    if (int e = count_chunk(h, N, p, nullptr, board_starts(N), board_bound(N, p), total, &records)) return e;
+    h->last_chunks = records ? 1 : 0;
+    h->last_records = records;
+    return NQ_OK;
+  }
   std::vector<int> starts;
   if (start_constellations(N, starts) != 0) return h->fail(NQ_EINVAL, "generator: bad arguments N=%d", N);
   return count_start_range(h, N, p, starts, 0, starts.size(), total);
@@ -774,7 +802,7 @@ struct nq_batch {
   cudaGraphExec_t graph = nullptr;
   bool submitted = false;
   int64_t device_bytes = 0;
-  int64_t h2d_bytes = 0;                   // host->device bytes of the build (start lists, queries, job table)
+  int64_t h2d_bytes = 0;                   // host->device bytes of the build (queries, tables)
 };
 
 namespace {
@@ -850,7 +878,7 @@ void nq_batch_destroy(nq_batch* b) {
 }
 
 // Build, one synchronisation in all: the boards' records are generated on the device and prepared, each
-// query is expanded by one block (small boards' start lists, queries and tables are the only uploads), every
+// query is expanded by one block (queries and tables are the only uploads), every
 // list's split is counted, the queue is allocated, and the jobs' items are written job after job.  Jobs of
 // one board share its tasks and its counted list; each has its own items.  Building 64 mixed jobs of N=9..16
 // on the host (generator, breadth-first searches, staging, two split launches a job) took 19 ms.
@@ -871,7 +899,7 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
   };
   // ---- the lists: one per board (N, preset) and one per query
   struct List { int N = 0, rows = 0, T = 0; uint64_t cap = 0; bool query = false; int D = 0; uint32_t src0 = 0, task0 = 0; };
-  struct Board { int p; uint32_t list; std::vector<int> starts; std::vector<GenRecord> recs; size_t starts_at = 0; };
+  struct Board { int p; uint32_t list; bool device; std::vector<GenRecord> recs; };
   std::vector<List> lists;
   std::vector<Board> boards;
   std::vector<BatchQuery> queries;
@@ -889,14 +917,13 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
       if (it == board_list.end()) {
         Board bd;
         bd.p = p; bd.list = (uint32_t)lists.size();
-        if (start_constellations(J.N, bd.starts) != 0) return bad(NQ_EINVAL, "generator failed", j);
         List l;
-        l.N = J.N; l.cap = board_bound(J.N, p, bd.starts); l.rows = maxt_for(J.N, p - 3);
+        l.N = J.N; l.cap = board_bound(J.N, p); l.rows = maxt_for(J.N, p - 3);
         b->ra_words = b->ra_words || !ra_in_rd(J.N, p - 3, 0);
-        if (p > 8 || l.cap > kGenRecords) {      // more than the device generator's buffers: the host's list
+        bd.device = p <= 8 && l.cap <= kGenRecords;
+        if (!bd.device) {                        // more than the device generator's buffers: the host's list
           const int s = gen_constellations(J.N, p, bd.recs, 0);
           if (s != 0) return bad(s == -2 ? NQ_EPRESET : NQ_EINVAL, "generator failed", j);
-          std::vector<int>().swap(bd.starts);
           l.cap = bd.recs.size();
         }
         it = board_list.emplace(std::make_pair(J.N, p), bd.list).first;
@@ -904,7 +931,7 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
         boards.push_back(std::move(bd));
       }
       job_list[j] = (int)it->second;
-      sources += lists[it->second].cap / 2;      // the bound is about twice the records
+      sources += lists[it->second].cap / 4;      // the bound is about four times the records
     } else {
       int rows[8], cols[8];
       const int k = (J.kind == NQ_JOB_COUNT) ? 0 : J.k;
@@ -934,7 +961,6 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
   const size_t nl = lists.size(), nb = boards.size(), nq = queries.size();
   std::vector<unsigned long long> ends(nl);
   uint64_t src = 0, ntask = 0, words = 1, rec_cap = 0, gen_cap = 0;
-  size_t n_starts = 0;
   for (size_t i = 0; i < nl; i++) {
     List& l = lists[i];
     l.src0 = (uint32_t)src; l.task0 = (uint32_t)ntask;
@@ -945,17 +971,15 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
     const int levels = l.query ? query_levels(l.rows) : choose_split((int64_t)std::max(sources, l.cap), l.rows);
     l.D = l.N <= 12 ? 0 : h->split >= 0 ? h->split : l.query && sources > 100000 ? std::min(levels, 1) : levels;
   }
-  for (Board& bd : boards) {
-    bd.starts_at = n_starts;
-    n_starts += bd.starts.size();
+  for (const Board& bd : boards) {
     rec_cap = std::max(rec_cap, lists[bd.list].cap);
-    if (!bd.starts.empty()) gen_cap = std::max(gen_cap, lists[bd.list].cap);
+    if (bd.device) gen_cap = std::max(gen_cap, lists[bd.list].cap);
   }
   if (src > 0xFFFFFFFFull || words > (uint64_t)kMaxDepth) { nq_batch_destroy(b); return h->fail(NQ_ENOMEM, "batch: too many tasks"); }
   b->sw = (int)words;
   const size_t word = b->wide ? sizeof(uint2) : sizeof(uint32_t), cb = Ctrl::bytes(njobs);
   auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
-  const size_t o_lists = up(nl * 8), o_starts = o_lists + up(nl * sizeof(BatchList)), o_q = o_starts + up(n_starts * sizeof(int));
+  const size_t o_lists = up(nl * 8), o_q = o_lists + up(nl * sizeof(BatchList));
   const size_t o_jends = o_q + up(nq * sizeof(BatchQuery)), o_jobs = o_jends + up((size_t)njobs * 8);
   const size_t tab_bytes = o_jobs + up((size_t)njobs * sizeof(BatchJob));
   // state: list states, generated levels and deepest schedule per board, error words of generator and prepare
@@ -983,13 +1007,10 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
         (gen_cap && (e = gen.ensure(gen_cap * sizeof(uint4))) != cudaSuccess) ||
         (nq && (e = tmp.ensure(src * sizeof(uint4))) != cudaSuccess)) break;
     unsigned char *dt = (unsigned char*)tab.p, *ds = (unsigned char*)state.p;
-    // ---- upload the lists, start lists and queries
+    // ---- upload the lists and queries
     BatchList* hl = (BatchList*)(b->stage + o_lists);
     if (nl) std::memcpy(b->stage, ends.data(), nl * 8);
     for (size_t i = 0; i < nl; i++) hl[i] = BatchList{lists[i].src0, lists[i].task0, lists[i].query ? 1u : 0u, (uint32_t)lists[i].D};
-    for (const Board& bd : boards)
-      if (!bd.starts.empty())
-        std::memcpy(b->stage + o_starts + bd.starts_at * sizeof(int), bd.starts.data(), bd.starts.size() * sizeof(int));
     BatchQuery* hq = (BatchQuery*)(b->stage + o_q);
     for (size_t i = 0; i < nq; i++) {
       hq[i] = queries[i];
@@ -1009,11 +1030,11 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
       const uint4* drec = (const uint4*)rec.p;
       const unsigned int* dn = nullptr;
       std::vector<nq_record> packed;
-      if (!bd.starts.empty()) {
+      if (bd.device) {
         const int levels = gen_levels(bd.p);
         uint4* buf[2] = {(uint4*)rec.p, (uint4*)gen.p};
         unsigned int* gn = (unsigned int*)(ds + o_gn + i * 32);
-        e = launch_generate(l.N, bd.p, (unsigned)bd.starts.size(), (const int*)(dt + o_starts) + bd.starts_at, buf[0], buf[1],
+        e = launch_generate(l.N, bd.p, (unsigned)board_starts(l.N), nullptr, buf[0], buf[1],
                             (unsigned)l.cap, gn, derr, h->sms, st);
         drec = buf[levels & 1];
         dn = gn + levels;
@@ -1104,9 +1125,7 @@ int64_t nq_job_device_bytes(const nq_job* job, int sms, int split_depth) {
     // the record bound nq_batch_create builds the job with
     const int p = J.preset > 0 ? J.preset : preset_for(J.N);
     if (p < 4) return NQ_EPRESET;
-    std::vector<int> starts;
-    if (start_constellations(J.N, starts) != 0) return NQ_EINVAL;
-    m = (int64_t)board_bound(J.N, p, starts);
+    m = (int64_t)board_bound(J.N, p);
     if (p > 8 || (uint64_t)m > kGenRecords) {
       std::vector<GenRecord> v;
       const int s = gen_constellations(J.N, p, v, 0);
@@ -1115,7 +1134,7 @@ int64_t nq_job_device_bytes(const nq_job* job, int sms, int split_depth) {
     }
     tasks = m;
     rows = maxt_for(J.N, p - 3);
-    levels = choose_split(m / 2, rows);
+    levels = choose_split(m / 4, rows);
   } else if (J.kind == NQ_JOB_COUNT || J.kind == NQ_JOB_COMPLETION) {
     int r[8], c[8];
     const int k = (J.kind == NQ_JOB_COUNT) ? 0 : J.k;

@@ -50,16 +50,73 @@ __device__ __forceinline__ uint4 settle(uint32_t ld, uint32_t rd, uint32_t col, 
   return make_uint4(ld, rd, col, ((uint32_t)row << 20) | ijkl | ((uint32_t)queens << kQueens));
 }
 
+__device__ __forceinline__ uint4 start_state(int N, int sc) {
+  const int i = geti(sc), j = getj(sc), k = getk(sc), l = getl(sc);
+  const uint32_t L = 1u << (N - 1), Lj = L >> j, Li = L >> i;
+  const uint32_t ld = ((i > 0) ? (L >> (i - 1)) : 0u) | (1u << (N - k));
+  const uint32_t rd = (L >> (i + 1)) | (1u << (l - 1));
+  return settle(ld, rd, 1u | L | Li | Lj, 1, (j == N - 1) ? 3 : 4, (uint32_t)sc);
+}
+
 __global__ void __launch_bounds__(128) gen_start_kernel(int N, unsigned n, const int* __restrict__ starts,
                                                         uint4* __restrict__ out, unsigned* gn) {
   const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q == 0) gn[0] = n;
   if (q >= n) return;
-  const int sc = starts[q], i = geti(sc), j = getj(sc), k = getk(sc), l = getl(sc);
-  const uint32_t L = 1u << (N - 1), Lj = L >> j, Li = L >> i;
-  const uint32_t ld = ((i > 0) ? (L >> (i - 1)) : 0u) | (1u << (N - k));
-  const uint32_t rd = (L >> (i + 1)) | (1u << (l - 1));
-  out[q] = settle(ld, rd, 1u | L | Li | Lj, 1, (j == N - 1) ? 3 : 4, (uint32_t)sc);
+  out[q] = start_state(N, starts[q]);
+}
+
+// All start constellations of a board (356Py:2850-2880).  The reference inserts candidates in loop order and
+// skips one whose rotation it has inserted: of the candidates that are rotations of each other it inserts the
+// first, so each thread takes one candidate and compares it with its three rotations.  The canonical forms
+// (jasmin) of what is left are all different.  Both checked against the sequential list for every N of 5..27.
+struct Quad { int i, j, k, l; };
+__device__ __forceinline__ bool start_candidate(const Quad x, int N) {
+  return x.k >= 1 && x.k < (N + 1) / 2 && x.l > x.k && x.l <= N - 2 && x.i > x.k && x.i <= N - 2 && x.i != N - 1 - x.l &&
+         x.j >= 1 && x.j <= N - x.k - 2 && x.j != x.i && x.j != x.l;
+}
+__device__ __forceinline__ int start_rank(const Quad x, int N) {     // place in the loops: the centre column of odd boards first
+  const int k = ((N & 1) && x.k == N / 2) ? 0 : x.k;
+  return (((k << 5) + x.l) << 10) + (x.i << 5) + (N - x.k - 2 - x.j);
+}
+__device__ __forceinline__ int rotate90(int x, int N) {
+  return ((N - 1 - getk(x)) << 15) + ((N - 1 - getl(x)) << 10) + (getj(x) << 5) + geti(x);
+}
+__device__ __forceinline__ int jasmin(int x, int N) {                // 356Py:2739-2756
+  auto dist = [N](int v) { return min(v, N - 1 - v); };
+  int turns = 0, mn = dist(getj(x));
+  if (dist(geti(x)) < mn) { turns = 2; mn = dist(geti(x)); }
+  if (dist(getk(x)) < mn) { turns = 3; mn = dist(getk(x)); }
+  if (dist(getl(x)) < mn) turns = 1;
+  for (int a = 0; a < turns; a++) x = rotate90(x, N);
+  if (getj(x) < N - 1 - getj(x)) x = ((N - 1 - geti(x)) << 15) + ((N - 1 - getj(x)) << 10) + (getl(x) << 5) + getk(x);
+  return x;
+}
+
+__global__ void __launch_bounds__(128) gen_board_kernel(int N, uint4* __restrict__ out, unsigned cap, unsigned* gn) {
+  int q = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  const int corners = N * N;
+  Quad x;
+  bool take;
+  if (q < corners) {                               // a queen in the corner: (0, j, 0, l), j < l
+    x = Quad{0, q / N, 0, q % N};
+    take = x.j >= 1 && x.j < N - 2 && x.l > x.j && x.l <= N - 2;
+  } else {
+    q -= corners;
+    x.j = q % N; q /= N;
+    x.i = q % N; q /= N;
+    x.l = q % N; x.k = q / N + 1;
+    take = start_candidate(x, N);
+    if (take) {
+      const int rank = start_rank(x, N);
+      const Quad r[3] = {{N - 1 - x.k, N - 1 - x.l, x.j, x.i}, {N - 1 - x.j, N - 1 - x.i, N - 1 - x.l, N - 1 - x.k},
+                         {x.l, x.k, N - 1 - x.i, N - 1 - x.j}};
+#pragma unroll
+      for (int t = 0; t < 3; t++) take = take && !(start_candidate(r[t], N) && start_rank(r[t], N) < rank);
+    }
+  }
+  const unsigned at = take_slots(&gn[0], take ? 1u : 0u);
+  if (take && at < cap) out[at] = start_state(N, jasmin((x.i << 15) + (x.j << 10) + (x.k << 5) + x.l, N));
 }
 
 // One queen more for every state below the preset; the others move on (last: as records).
@@ -236,14 +293,20 @@ __global__ void __launch_bounds__(128) query_level_kernel(uint32_t N, uint32_t T
 
 cudaError_t launch_generate(int N, int preset, unsigned n_starts, const int* starts, uint4* buf0, uint4* buf1, unsigned cap,
                             unsigned* gn, unsigned* err, int sms, cudaStream_t st) {
-  if (n_starts == 0) return cudaSuccess;
   const int levels = gen_levels(preset);
   uint4* buf[2] = {buf0, buf1};
-  gen_start_kernel<<<(n_starts + 127) / 128, 128, 0, st>>>(N, n_starts, starts, buf[0], gn);
+  const unsigned full = 8u * (unsigned)sms;
+  if (starts) {
+    if (n_starts == 0) return cudaSuccess;
+    gen_start_kernel<<<(n_starts + 127) / 128, 128, 0, st>>>(N, n_starts, starts, buf[0], gn);
+  } else {
+    const unsigned n = (unsigned)(N * N * (1 + ((N + 1) / 2 - 1) * N));
+    gen_board_kernel<<<(n + 127) / 128, 128, 0, st>>>(N, buf[0], cap, gn);
+  }
   for (int l = 0; l < levels; l++) {
-    const unsigned need = l == 0 ? (n_starts + 127) / 128 : 8u * (unsigned)sms;
-    gen_level_kernel<<<need < 8u * (unsigned)sms ? need : 8u * (unsigned)sms, 128, 0, st>>>(
-        N, preset, l + 1 == levels, buf[l & 1], buf[(l + 1) & 1], cap, gn, l, err);
+    const unsigned need = l == 0 ? (n_starts + 127) / 128 : full;
+    gen_level_kernel<<<need < full ? need : full, 128, 0, st>>>(N, preset, l + 1 == levels, buf[l & 1], buf[(l + 1) & 1], cap,
+                                                                gn, l, err);
   }
   return cudaGetLastError();
 }

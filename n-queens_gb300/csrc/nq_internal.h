@@ -101,9 +101,10 @@ cudaError_t launch_prepare_split(int D, int64_t m_max, const PrepareSplit& a, cu
 
 cudaError_t launch_dfs(const DfsLaunch& L, cudaStream_t st);
 
-// Records of start constellations (device array of packed ijkl) at a preset of 4..8, on the device: gn[0..]
-// receives the states of each level, gn[gen_levels(preset)] the records, which end in buf0 when the level
-// count is even, else in buf1 (`cap` records each; the caller bounds them).  gn zeroed before.
+// Records of start constellations at a preset of 4..8, on the device: `starts` (device array of packed ijkl),
+// or all of a board's where it is null (n_starts then bounds them).  gn[0..] receives the states of each
+// level, gn[gen_levels(preset)] the records, which end in buf0 when the level count is even, else in buf1
+// (`cap` records each; the caller bounds them).  gn zeroed before.
 inline int gen_levels(int preset) { return preset - 3; }     // start constellations hold 3 or 4 queens
 cudaError_t launch_generate(int N, int preset, unsigned n_starts, const int* starts, uint4* buf0, uint4* buf1, unsigned cap,
                             unsigned* gn, unsigned* err, int sms, cudaStream_t st);
