@@ -119,7 +119,7 @@ int run_records(nq_handle* h, int N, const uint4* d_rec, int64_t m, int start_mi
     NQ_CUDA(h, launch_prepare_split(D, m, P, st));
     if (D > 0) { L.sroot = P.sroot; L.sinfo = P.sinfo; }
     if (!read_back) {
-      if (D > 0 || m_dev) { L.m_dev = P.qn; L.qcap = D > 0 ? P.qcap : ~0ull; }
+      if (D > 0 || m_dev) { L.m_dev = P.qn; L.qcap = D > 0 ? P.qcap : ~0ull; L.m_bound = (int64_t)std::min<uint64_t>(bound, 1ull << 40); }
       L.maxt = std::max(1, std::min(maxt, t_max) - D);
       break;
     }

@@ -56,6 +56,7 @@ struct DfsLaunch {
   int64_t m = 0;                        // queue length ...
   const unsigned long long* m_dev = nullptr;   // ... or where it stands on the device; above qcap the DFS does nothing
   unsigned long long qcap = 0;
+  int64_t m_bound = 0;                  // bound of a length on the device, 0: none
   const uint32_t* order = nullptr;      // optional queue order (task index per slot)
   unsigned long long* cursor = nullptr; // queue cursor (device, zeroed before launch; 64-bit, so it never wraps)
   unsigned long long* job_totals = nullptr;  // weighted totals, slot (job id - job_base) (device)

@@ -55,6 +55,9 @@ constexpr unsigned kMinChunk = 8;
 // A frame is given to a lane without work when it is at least this many levels above the terminal depth
 // (fewer: not worth the exchange; 3 and 7 measured the same from N=16 on, 7 is 25 % slower at N=14).
 constexpr int kGiveRows = 5;
+// What a pool entry needs besides its frame, ready when it is loaded: terminal depth (5 bits), weight (2),
+// root count (1), N (5), depth of its first word (5) and what to do with it.
+constexpr uint32_t kItemWork = 1u << 18, kItemSpare = 1u << 19;   // search it; more columns than rows are left
 
 template <bool WIDE> using WordT = QueryWord<WIDE>;
 
@@ -620,17 +623,17 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
   auto put_word = [&](uint32_t k, W w) { sch[k * BLOCK] = w; };
   auto count_word = [] { W w; if constexpr (WIDE) w = make_uint2(kCountWord, 0u); else w = kCountWord; return w; };
   Lane<FORM, BIG> L;
-  uint32_t tf = 1;                    // popc(fr) at the terminal depth: R - terminal depth; the base frame's is one less
   const uint32_t sch_sh = (uint32_t)__cvta_generic_to_shared(sch);
   const uint32_t bottom = (uint32_t)__cvta_generic_to_shared(smem) + threadIdx.x * (uint32_t)sizeof(uint4);
   // stack pointer above the sentinel: a lane is idle when no frame but the sentinel is left.  The sentinel
   // is the lane's first slot until a frame above it is given away (below).
   uint32_t top = bottom + F;
   L.sp = top;
-  L.sw0 = sch_sh;                     // a lane without work reads word 0 (the sentinel's fr is 0)
+  // a base frame has one column (a terminal one two), and where popc(fr) == 1 the word is the count word,
+  // for the sentinel too; a lane that never had work reads word 0
+  L.sw0 = sch_sh + ROW;
   put_word(0, count_word());
-  // where popc(fr) == tf - 1 the lane's word is the count word
-  auto arm = [&]() { sts_frame(top - F, 1u, 0u, (1u << (tf - 1u)) - 1u, kSentinelAvail); };
+  auto arm = [&]() { sts_frame(top - F, 1u, 0u, 1u, kSentinelAvail); };
   uint32_t wexp = 0, job = a.job_base, task = 0;
   bool have = false, exhausted = false, drained = false;   // exhausted, drained: warp-uniform, as the pool's counters
   unsigned long long m = a.m;
@@ -641,7 +644,7 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
   const float share = 1.0f / (kChunkShare * (float)warps);
   unsigned chunk = chunk0, pool_n = 0, pool_at = 0;
   uint4 p_root = make_uint4(0, 0, 0, 0);
-  uint32_t p_task = 0, p_info = 0, p_job = 0;
+  uint32_t p_task = 0, p_meta = 0, p_job = 0;
   unsigned long long acc = 0;
   uint32_t acc_job = a.job_base;
 
@@ -659,9 +662,10 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
         acc += v;
         have = false;
       }
-      // Refill from the warp's pool of queue items: lane i holds item i of the last chunk taken, loaded by
-      // the whole warp at once, so a lane that needs work costs seven shuffles, not an atomic and two
-      // dependent rounds of loads.
+      // Refill from the warp's pool of queue items: lane i holds item i of the last chunk taken, loaded and
+      // decoded by the whole warp at once, so a lane that needs work costs seven shuffles and its words, not
+      // an atomic and two dependent rounds of loads.  (Decoding here, a lane at a time: N=16 307 us, 296 so;
+      // serving lanes only by twos or more: N=17 1.380 ms against 1.393, N=19 64.2 against 63.8.)
       bool want = idle && !exhausted;
       for (unsigned need = __ballot_sync(FULL, want); need; need = __ballot_sync(FULL, want)) {
         if (pool_n == 0u) {
@@ -687,7 +691,18 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
             uint32_t d0 = 0;
             if (a.sinfo) { const uint2 si = a.sinfo[q]; p_task = si.x; d0 = si.y & 31u; p_job = si.y >> 5; p_root = a.sroot[q]; }
             else { p_task = (uint32_t)q; p_root = a.root[q]; }
-            p_info = a.info[p_task] | (d0 << 16);
+            // free columns for used ones, R of them; depth d has R - d (one queen per depth), so word d is
+            // found from popc(fr) alone
+            const uint32_t in = a.info[p_task], T = info_T(in), N = info_N(in), n = T - d0;   // n: terminal depth
+            p_root.z = ((1u << N) - 1u) & ~p_root.z;
+            p_root.w &= p_root.z;
+            const uint32_t R = __popc(p_root.z);
+            p_meta = (info_wexp(in) << 5) | (d0 == 0u ? info_root(in) << 7 : 0u) | (N << 8) | (d0 << 13);
+            if (T != INFO_NO_DFS && info_status(in) == TS_OK && T >= d0) {
+              if ((int)n > a.maxt) atomicOr(a.err, DERR_DEPTH);    // frames at depths 0..n, words 0..n
+              else if (n + 2u == R) p_meta |= n | kItemWork;       // fewer free columns than rows: no solution
+              else if (n + 2u < R) p_meta |= n | kItemSpare;
+            }
           }
         }
         const unsigned give = min((unsigned)__popc(need), pool_n);
@@ -696,37 +711,33 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
         uint4 r;
         r.x = __shfl_sync(FULL, p_root.x, src); r.y = __shfl_sync(FULL, p_root.y, src);
         r.z = __shfl_sync(FULL, p_root.z, src); r.w = __shfl_sync(FULL, p_root.w, src);
-        const uint32_t i_task = __shfl_sync(FULL, p_task, src), i_info = __shfl_sync(FULL, p_info, src);
+        const uint32_t i_task = __shfl_sync(FULL, p_task, src), meta = __shfl_sync(FULL, p_meta, src);
         const uint32_t i_job = __shfl_sync(FULL, p_job, src);
         pool_at += give; pool_n -= give;
         if (want && rank < give) {
           want = false;
-          const uint32_t d0 = i_info >> 16, T = info_T(i_info);
-          task = i_task; job = i_job;
           have = true;
-          L.cnt = (d0 == 0) ? info_root(i_info) : 0u;
-          wexp = info_wexp(i_info);
-          if (T == INFO_NO_DFS || info_status(i_info) != TS_OK || T < d0) {
-            // no DFS work: the lane stays on its sentinel
-          } else if ((int)(T - d0) > a.maxt) {    // frames at depths 0..T', words 0..T'
-            atomicOr(a.err, DERR_DEPTH);
-          } else {
-            // root: the free columns of the board, R of them; depth d has R - d (one queen per depth,
-            // T' + 1 <= R of them), so word d is found from popc(fr) alone
-            const uint32_t fr = ((1u << info_N(i_info)) - 1u) & ~r.z;
-            const uint32_t R = __popc(fr);
-            const W* src_w = gsched + (size_t)task * a.sw + d0;
-            const uint32_t n = T - d0;           // terminal depth
-            if (n + 2u < R) {
-              L.cnt += count_base_frames<FORM>(r, fr, info_N(i_info), n, src_w);
-            } else if (n + 2u == R) {            // fewer free columns than rows: no solution, no work
-              L.ld = r.x; L.rd = r.y; L.fr = fr; L.avail = r.w & fr;
-              tf = R - n; L.sw0 = sch_sh + R * ROW; L.ram = compact_ra_mask((int)info_N(i_info));
-              for (uint32_t k = 0; k <= n; k++) put_word(k, src_w[k]);
-              put_word(n + 1u, count_word());
-              arm();
+          task = i_task; job = i_job;
+          wexp = (meta >> 5) & 3u;
+          L.cnt = (meta >> 7) & 1u;
+          const uint32_t n = meta & 31u, N = (meta >> 8) & 31u;
+          const W* w = gsched + (size_t)task * a.sw + ((meta >> 13) & 31u);
+          if (meta & kItemWork) {
+            L.ld = r.x; L.rd = r.y; L.fr = r.z; L.avail = r.w;
+            L.sw0 = sch_sh + (n + 2u) * ROW;
+            if constexpr (FORM == kRaInWords) L.ram = compact_ra_mask((int)N);
+            uint32_t k = 0;
+#pragma unroll 1
+            for (; k + 3u <= n; k += 4) {
+              const W w0 = w[k], w1 = w[k + 1], w2 = w[k + 2], w3 = w[k + 3];
+              put_word(k, w0); put_word(k + 1, w1); put_word(k + 2, w2); put_word(k + 3, w3);
             }
-          }
+            for (; k <= n; k++) put_word(k, w[k]);
+            put_word(k, count_word());
+            arm();
+          } else if (meta & kItemSpare) {
+            L.cnt += count_base_frames<FORM>(r, r.z, N, n, w);
+          }                                    // else no work: the lane stays on its sentinel
         }
       }
       if (exhausted) {
@@ -741,7 +752,7 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
           const uint32_t rest = L.avail & (L.avail - 1u);
           const uint32_t gfr = saved ? lds_frame(top).z : L.fr;
           const bool can = have && (saved ? (L.avail != 0u || L.sp != top + F) : rest != 0u) &&
-                           __popc(gfr) >= (int)tf + kGiveRows;
+                           __popc(gfr) >= 2 + kGiveRows;
           const unsigned givers = __ballot_sync(FULL, can);
           if (givers) {
             const int n = min(__popc(starved), __popc(givers));
@@ -752,13 +763,13 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
             __syncwarp();
             const int src = takes ? (int)nth_set(givers, (uint32_t)srank) : (int)lane;
             const uint32_t from = __shfl_sync(FULL, top, src), gsw0 = __shfl_sync(FULL, L.sw0, src);
-            const uint32_t gtf = __shfl_sync(FULL, tf, src), gram = __shfl_sync(FULL, L.ram, src);
+            const uint32_t gram = FORM == kRaInWords ? __shfl_sync(FULL, L.ram, src) : 0u;
             const uint32_t gw = __shfl_sync(FULL, wexp, src), gjob = __shfl_sync(FULL, job, src);
             const uint32_t gtask = __shfl_sync(FULL, task, src);
             if (takes) {
               const uint4 f = lds_frame(from);
               L.ld = f.x; L.rd = f.y; L.fr = f.z; L.avail = f.w;
-              L.sw0 = gsw0; tf = gtf; L.ram = gram; L.cnt = 0;
+              L.sw0 = gsw0; L.ram = gram; L.cnt = 0;
               wexp = gw; job = gjob; task = gtask; have = true;
               top = bottom + F; L.sp = top;
               arm();
@@ -814,6 +825,9 @@ static cudaError_t launch_dfs_t(const DfsLaunch& L, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     if (per <= 0) return cudaErrorInvalidConfiguration;
     grid = sms * per;
+    // a short queue takes a warp an item: more blocks than that only start and end
+    const int64_t most = L.m_dev ? L.m_bound : L.m;
+    if (most > 0) grid = (int)std::min<int64_t>(grid, (most + BLOCK / 32 - 1) / (BLOCK / 32));
   }
   DfsArgs a;
   a.root = L.tasks.root; a.info = L.tasks.info; a.sched = L.tasks.sched; a.sw = L.tasks.sw;
