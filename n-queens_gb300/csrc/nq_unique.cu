@@ -17,9 +17,8 @@
 // row per launch, into the task queue (unique_init_kernel,
 // unique_expand_kernel).  unique_kernel is persistent, queue-fed and
 // explicit-stack like the constellation DFS (one candidate per lane per step,
-// predicated pop/push, the row carried in `down`'s high bits, work shared in a
-// warp at the end of the queue), keeping each lane's board (one bit per row)
-// in shared memory for the leaf classification.
+// work shared in a warp at the end of the queue), keeping each lane's board
+// (one bit per row) in shared memory for the leaf classification.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -34,14 +33,20 @@ namespace {
 
 constexpr unsigned FULLM = 0xFFFFFFFFu;
 constexpr int kBoardRows = 8;    // rows of the board prefix carried by a task
-constexpr int kUniqueSteps = 16;   // steps per lane between checks for finished lanes
-constexpr int kReadBackN = 14;     // boards from here on size the stacks to the tasks' rows
-constexpr uint32_t kGiveRows = 5;   // rows below a frame worth giving away
+// Steps per lane between checks for finished lanes, a multiple of the steps unrolled.  Unrolled further the loop
+// and the classification in it outgrow the instruction cache (us of a whole count at N=18, unrolled by 1 / 2 / 5 /
+// 10 / 15 / 30 with every board classified by the warp: 24.5 / 23.4 / 23.4 / 23.3 / 24.0 / 28.9 ms; as it is now,
+// by 5 and by 10 19.6 ms), and 16 or 20 steps a check gave 21.7 ms where 30 gave 21.5.
+constexpr int kUniqueSteps = 30, kUniqueUnroll = 5;
+// Boards from here on size the stacks to the tasks' rows (N=14 96 us without the read-back, 111 with; N=15 187
+// against 190, and the search grows sixfold a size from there).
+constexpr int kReadBackN = 15;
+constexpr int kGiveRows = 6;         // rows left in a frame worth giving away
 
 // One start configuration (symmetry part and its bounds).
 struct UConf {
   uint32_t part;       // 1 corner, 2 no corner
-  uint32_t bound1, bound2, endbit, lastmask, sidemask, topbit;
+  uint32_t bound1, bound2, lastmask, sidemask;
 };
 
 // A task: the search state at `row` plus the board rows above it (one byte each, the queen's column), 32 bytes.
@@ -58,44 +63,31 @@ __device__ __forceinline__ void board_set(UTask& t, uint32_t r, uint32_t bit) {
   if (r < 4u) t.board[0] |= v; else t.board[1] |= v;
 }
 
-// symmetryops (07Py_bit_symmetry.py:65-125): 2, 4 or 8 for a canonical
-// solution, 0 for a rotated copy.  `b(k)` reads board row k.
-template <typename B>
-__device__ __forceinline__ uint32_t classify(const B& b, int size, const UConf& c) {
-  int own, you;
-  uint32_t bit, ptn;
-  if (b(c.bound2) == 1u) {                        // 90 degrees
-    own = 1; ptn = 2;
-    while (own <= size - 1) {
-      bit = 1; you = size - 1;
-      while (b(you) != ptn && b(own) >= bit) { bit <<= 1; you--; }
-      if (b(own) > bit) return 0;
-      if (b(own) < bit) break;
-      own++; ptn <<= 1;
-    }
-    if (own > size - 1) return 2;
-  }
-  if (b(size - 1) == c.endbit) {                  // 180 degrees
-    own = 1; you = size - 2;
-    while (own <= size - 1) {
-      bit = 1; ptn = c.topbit;
-      while (b(you) != ptn && b(own) >= bit) { bit <<= 1; ptn >>= 1; }
-      if (b(own) > bit) return 0;
-      if (b(own) < bit) break;
-      own++; you--;
-    }
-    if (own > size - 1) return 4;
-  }
-  if (b(c.bound1) == c.topbit) {                  // 270 degrees
-    own = 1; ptn = c.topbit >> 1;
-    while (own <= size - 1) {
-      bit = 1; you = 0;
-      while (b(you) != ptn && b(own) >= bit) { bit <<= 1; you++; }
-      if (b(own) > bit) return 0;
-      if (b(own) < bit) break;
-      own++; ptn >>= 1;
-    }
-  }
+// symmetryops (07Py_bit_symmetry.py:65-125) on one board, by the warp: 2, 4 or 8 for a canonical solution, 0 for
+// a rotated copy.  Lane r holds row r's column `c` (lanes from N on hold nothing).  Row r of the board turned by
+// 90, 180 and 270 degrees comes from the row of column r, row N-1-r, and the row of column N-1-r; a rotation
+// whose row 0 differs is left out, otherwise the first row that differs decides.  `inv` is 32 words of the warp's
+// shared memory for the rows by column.
+// Bound by issue: about 60 instructions of the warp a board, on the quarter of the boards that have a rotation
+// with their own row 0 (the others count x8 after three loads of their own lane).  One step in 125 ends in such a
+// board's last row (N=16), so a warp's step has one with odds of 1 in 4: at N=18 a count took 15.0 ms without
+// any classification, 21.0 with a lane searching its own board for each column, 23.4 with every board here, and
+// takes 19.6 with the check before.
+__device__ __forceinline__ uint32_t classify(uint32_t c, uint32_t lane, uint32_t N, uint32_t* inv) {
+  const bool in = lane < N;
+  const uint32_t other = in ? N - 1u - lane : lane;
+  if (in) inv[c] = lane;
+  const uint32_t c180 = N - 1u - __shfl_sync(FULLM, c, (int)other);
+  __syncwarp();
+  const uint32_t c90 = N - 1u - inv[lane], c270 = inv[other];
+  const uint32_t ne90 = __ballot_sync(FULLM, in && c != c90), gt90 = __ballot_sync(FULLM, c > c90);
+  const uint32_t ne180 = __ballot_sync(FULLM, in && c != c180), gt180 = __ballot_sync(FULLM, c > c180);
+  const uint32_t ne270 = __ballot_sync(FULLM, in && c != c270), gt270 = __ballot_sync(FULLM, c > c270);
+  if (ne90 == 0u) return 2;
+  if (!(ne90 & 1u) && (gt90 & ne90 & (0u - ne90))) return 0;
+  if (ne180 == 0u) return 4;
+  if (!(ne180 & 1u) && (gt180 & ne180 & (0u - ne180))) return 0;
+  if (!(ne270 & 1u) && (gt270 & ne270 & (0u - ne270))) return 0;
   return 8;
 }
 
@@ -131,22 +123,19 @@ struct UArgs {
   const UTask* tasks[2];
   const UConf* confs;
   int N;
-  int maxf;                     // stack frames per lane: N - 2 - (smallest task row)
+  int nconf;
+  int maxf;                     // stack frames per lane: the sentinel's and one per row from the smallest task row
   unsigned cap;                 // tasks a buffer holds
   UCtl* ctl;
 };
 
-// Predicated shared-memory stores (32-bit shared-window addresses), so the push is
-// a single predicated instruction, not a branch.
-__device__ __forceinline__ void sts_frame_if(uint32_t p, uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
-  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q st.shared.v4.u32 [%1], {%2, %3, %4, %5};\n\t}"
-               :: "r"(p), "r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+// Shared-memory accesses at 32-bit shared-window addresses.
+__device__ __forceinline__ void sts_frame_u(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" :: "r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
-__device__ __forceinline__ void sts_word_if(uint32_t p, uint32_t a, uint32_t x) {
-  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %0, 0;\n\t@q st.shared.u32 [%1], %2;\n\t}"
-               :: "r"(p), "r"(a), "r"(x) : "memory");
+__device__ __forceinline__ void sts_word_u(uint32_t a, uint32_t x) {
+  asm volatile("st.shared.u32 [%0], %1;" :: "r"(a), "r"(x) : "memory");
 }
-
 __device__ __forceinline__ uint32_t lds_word_u(uint32_t a) {
   uint32_t w;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"(a) : "memory");
@@ -156,49 +145,86 @@ __device__ __forceinline__ void lds_frame_u(uint32_t a, uint32_t& x, uint32_t& y
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(x), "=r"(y), "=r"(z), "=r"(w) : "r"(a) : "memory");
 }
 
-// One lane per task, one candidate per step, all lanes on the same predicated
-// sequence: resume a saved frame, take the lowest candidate, record it in the
-// board, build the next row with the part's row rules, then count (last row)
-// or descend.  The row of a frame rides in `down` bits 27-31 (columns use bits
-// 0..N-1, N <= 27), so a saved frame is exactly {left, down, right, avail}.
+// The rules of a configuration's rows as words, read by the columns left (popc(fr)) of a frame: the columns
+// its child's row may use, what a frame in the last row counts, and whether the child must have both side
+// columns behind it.
+constexpr uint32_t U_COUNT = 1u << 27;      // part 1, last row: a solution, x8
+constexpr uint32_t U_CLASSIFY = 1u << 28;   // part 2, last row: a board to classify
+constexpr uint32_t U_SIDES = 1u << 31;      // part 2, row bound2 + 1: dead while a side column is free
+__device__ __forceinline__ uint32_t row_word(const UConf& c, int N, int left) {
+  if (left == 0) return 0u;                 // the sentinel: every child dies
+  if (left == 1) return c.part == 1 ? U_COUNT : U_CLASSIFY;
+  const uint32_t child = (uint32_t)(N - left + 1);
+  uint32_t w = (1u << N) - 1u;
+  if (child < c.bound1) w &= c.part == 1 ? ~2u : ~c.sidemask;
+  if (c.part != 1) {
+    if (child == (uint32_t)N - 1u) w &= ~c.lastmask;
+    // Row bound2 must take the last free side column (backTrack2, :126-151): after it both are behind.  Its
+    // own candidates go unfiltered and die one step on: 5 % more steps (N=15 39.7 10^6 against 37.6, N=16 259
+    // against 246), each about four instructions of 32 shorter.
+    if (child == c.bound2 + 1u) w |= U_SIDES;
+  }
+  return w;
+}
+
+// One lane per task, one candidate per step, all lanes on the same predicated sequence, as in the
+// constellation DFS (nq_kernels.cu): the child always becomes the current frame, the frame is saved with the
+// rest of its candidates whether or not there are any, a solution is a frame in the last row, and a sentinel
+// frame whose 31 candidates die feeds a lane without work.  Each step also records its queen in the lane's
+// board.  A frame is {left, right, free columns, candidates}; its row is N - popc(free columns).
+// Bound by issue and by shared memory together: a step writes 16 bytes and mostly reads 16, writes 4 for the
+// board, and reads the row's word from a table that the lanes of a configuration share.  With the row in `down`'s
+// high bits, the rules computed at each step and predicated pushes a count took 27.3 ms at N=18 and 4.2 ms at
+// N=17; with the same steps as here 21.5 and 3.4, with boards classified by the warp 19.6 and 3.08.
+constexpr uint32_t kUSentinel = 0xFFFFFFFEu;
+static_assert(kUniqueSteps <= 30, "the sentinel holds 31 candidates, and one has to be left at a check");
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) unique_kernel(const UArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int N = a.N;
   constexpr uint32_t F = BLOCK * (uint32_t)sizeof(uint4);          // frame stride of one lane's stack
-  constexpr uint32_t RB = BLOCK * (uint32_t)sizeof(uint32_t);      // board row stride
-  // a lane pushes at most one frame per row from its task's row to N - 3
-  uint4* stk = reinterpret_cast<uint4*>(smem) + threadIdx.x;                            // maxf frames, stride BLOCK
-  uint32_t* brd = reinterpret_cast<uint32_t*>(smem + (size_t)a.maxf * BLOCK * sizeof(uint4)) + threadIdx.x;  // N rows
-  const uint32_t bottom = (uint32_t)__cvta_generic_to_shared(stk);
-  uint32_t sbase = bottom;            // moves up when the lane gives its bottom frame away
-  const uint32_t bbase = (uint32_t)__cvta_generic_to_shared(brd);
+  constexpr uint32_t RB = (BLOCK + 1) * (uint32_t)sizeof(uint32_t);   // board row stride: a lane's rows lie in different banks
+  // maxf frames (the sentinel's, one per row), N + 1 board rows (the last one is the sentinel's), 32 words a
+  // warp for classify, the rows' words
+  uint32_t* inv = reinterpret_cast<uint32_t*>(smem + (size_t)a.maxf * F + (size_t)(N + 1) * RB) + (threadIdx.x & ~31u);
+  uint32_t* table = reinterpret_cast<uint32_t*>(smem + (size_t)a.maxf * F + (size_t)(N + 1) * RB) + BLOCK;
+  const uint32_t bottom = (uint32_t)__cvta_generic_to_shared(smem) + threadIdx.x * (uint32_t)sizeof(uint4);
+  const uint32_t brd = (uint32_t)__cvta_generic_to_shared(smem) + (uint32_t)a.maxf * F + threadIdx.x * 4u;   // row 0
+  const uint32_t tab = (uint32_t)__cvta_generic_to_shared(table);
+  for (int q = threadIdx.x; q < a.nconf * (N + 1); q += BLOCK) table[q] = row_word(a.confs[q / (N + 1)], N, q % (N + 1));
+  __syncthreads();
   const unsigned lane = threadIdx.x & 31u;
-  const uint32_t mask = (1u << N) - 1u;
-  const uint32_t last_row = (uint32_t)N - 1u;
-  uint32_t left = 0, down = 0, right = 0, avail = 0, sp = sbase;
-  UConf cf = {0, 0, 0, 0, 0, 0, 0};
-  uint32_t lowmask = ~0u, b2 = ~0u;      // row rules of the task's part
-  // part 1: rows above bound1 avoid column 1; part 2: they avoid the side
-  // columns, and row bound2 is gated on the side columns used so far
-  auto load_conf = [&](const UConf& c) {
-    cf = c;
-    lowmask = (cf.part == 1) ? ~2u : ~cf.sidemask;
-    b2 = (cf.part == 1) ? ~0u : cf.bound2;
+  const uint32_t mask = (1u << N) - 1u, side = (1u << (N - 1)) | 1u;
+  const uint32_t brd_end = brd + (uint32_t)N * RB;
+  uint32_t left = 0, right = 0, fr = 0, avail = 0;
+  uint32_t top = bottom + F;            // above the sentinel; moves up when the lane gives its bottom frame away
+  uint32_t sp = top, conf = 0, words = tab;
+  uint32_t brd1 = brd, brd2 = brd, last_col = 0;   // part 2: rows bound1 and bound2 of the board, 1 << bound2
+  const uint32_t topbit = 1u << (N - 1);
+  auto set_conf = [&](uint32_t k) {
+    const uint32_t b1 = a.confs[k].bound1, b2 = a.confs[k].bound2;
+    conf = k;
+    words = tab + k * (uint32_t)(N + 1) * 4u;
+    brd1 = brd + b1 * RB; brd2 = brd + b2 * RB; last_col = 1u << b2;
   };
-  unsigned long long c2 = 0, c4 = 0, c8 = 0;
+  uint32_t cnt = 0;
+  unsigned long long c8 = 0;
+  unsigned long long w2 = 0, w4 = 0, w8 = 0;   // the warp's classified boards, the same in its lanes
   bool exhausted = false;
+  auto arm = [&]() { sts_frame_u(top - F, 0u, 0u, 0u, kUSentinel); };
+  arm();
   const int level = queue_level(a.ctl, a.cap);
   const UTask* __restrict__ tasks = a.tasks[level & 1];
   const unsigned m = a.ctl->n[level];
   // where the queue is smaller than the lanes, each warp takes its share and shares it among its lanes
   const unsigned warps = gridDim.x * (BLOCK / 32);
   const unsigned take = min(32u, (m + warps - 1u) / warps);
-  uint32_t conf_ix = 0;
   for (;;) {
-    const bool idle = (avail | (sp - sbase)) == 0u;
+    c8 += cnt;
+    cnt = 0;
+    bool idle = avail == 0u && sp == top;
     if (__ballot_sync(FULLM, idle)) {
-      if (idle) sbase = sp = bottom;
+      if (idle) { top = bottom + F; sp = top; arm(); }
       const bool want = idle && !exhausted;
       const unsigned need = __ballot_sync(FULLM, want);
       if (need) {
@@ -209,98 +235,93 @@ __global__ void __launch_bounds__(BLOCK) unique_kernel(const UArgs a) {
         const unsigned rank = __popc(need & ((1u << lane) - 1u));
         if (want && rank < n_take && base + rank < m) {
           const UTask t = tasks[base + rank];
-          conf_ix = t.conf;
-          load_conf(a.confs[conf_ix]);
-          left = t.left; down = (t.down & mask) | (t.row << 27); right = t.right; avail = t.avail;
-          for (uint32_t r = 0; r < t.row && r < (uint32_t)kBoardRows; r++) brd[r * BLOCK] = board_bit(t, r);
+          set_conf(t.conf);
+          left = t.left; right = t.right; fr = mask & ~t.down; avail = t.avail;
+          for (uint32_t r = 0; r < t.row && r < (uint32_t)kBoardRows; r++) sts_word_u(brd + r * RB, board_bit(t, r));
+          idle = false;
         }
         exhausted = take < 32u || base + n_take >= m;   // warp-uniform
       }
       if (exhausted) {
         // The queue is empty: a lane without work takes the bottom saved frame of a busy lane of its warp,
         // or all but one candidate of its current frame, with the rows of the board above it.
-        const bool busy = avail != 0u || sp != sbase;
-        const unsigned starved = __ballot_sync(FULLM, !busy);
-        const bool saved = sp != sbase;
+        const unsigned starved = __ballot_sync(FULLM, idle);
+        const bool saved = sp != top;
         const uint32_t rest = avail & (avail - 1u);
-        const uint32_t gdown = saved ? lds_word_u(sbase + 4u) : down;
-        const bool can = busy && (saved ? (avail != 0u || sp != sbase + F) : rest != 0u) &&
-                         (gdown >> 27) + kGiveRows <= last_row;
+        const uint32_t gfr = saved ? lds_word_u(top + 8u) : fr;
+        const bool can = !idle && (saved ? (avail != 0u || sp != top + F) : rest != 0u) && __popc(gfr) >= kGiveRows;
         const unsigned givers = starved ? __ballot_sync(FULLM, can) : 0u;
         if (givers) {
           const unsigned lt = (1u << lane) - 1u;
           const int n = min(__popc(starved), __popc(givers));
           const bool gives = can && __popc(givers & lt) < n;
           const int srank = __popc(starved & lt);
-          const bool takes = !busy && srank < n;
-          if (gives && !saved) { sts_frame_if(1u, sbase, left, down, right, rest); avail ^= rest; }
+          const bool takes = idle && srank < n;
+          if (gives && !saved) { sts_frame_u(top, left, right, fr, rest); avail ^= rest; }
           __syncwarp();
           const int src = takes ? (int)nth_set(givers, (uint32_t)srank) : (int)lane;
-          const uint32_t from = __shfl_sync(FULLM, sbase, src), fconf = __shfl_sync(FULLM, conf_ix, src);
-          const uint32_t fbrd = __shfl_sync(FULLM, bbase, src);
+          const uint32_t from = __shfl_sync(FULLM, top, src), fconf = __shfl_sync(FULLM, conf, src);
+          const uint32_t fbrd = __shfl_sync(FULLM, brd, src);
           if (takes) {
-            lds_frame_u(from, left, down, right, avail);
-            conf_ix = fconf;
-            load_conf(a.confs[conf_ix]);
-            const uint32_t rows = down >> 27;
-            for (uint32_t r = 0; r < rows; r++) brd[r * BLOCK] = lds_word_u(fbrd + r * RB);
+            lds_frame_u(from, left, right, fr, avail);
+            set_conf(fconf);
+            const uint32_t rows = (uint32_t)(N - __popc(fr));
+            for (uint32_t r = 0; r < rows; r++) sts_word_u(brd + r * RB, lds_word_u(fbrd + r * RB));
+            idle = false;
           }
           __syncwarp();
-          if (gives && saved) sbase += F;
+          if (gives && saved) { top += F; arm(); }
         }
       }
-      if (__all_sync(FULLM, exhausted && (avail | (sp - sbase)) == 0u)) break;
-      asm volatile("" ::: "memory");   // board stores of the refill before the steps' accesses
+      if (__all_sync(FULLM, exhausted && idle)) break;
     }
     // kUniqueSteps steps between two checks for finished lanes (two ballots each)
-#pragma unroll 1
+#pragma unroll kUniqueUnroll
     for (int s = 0; s < kUniqueSteps; ++s) {
-      // pop with its condition formed in a predicate register inside the block (no 0/1 value for it)
-      asm volatile("{\n\t.reg .pred q;\n\tsetp.eq.u32 q, %3, 0;\n\tsetp.ne.and.u32 q, %4, %5, q;\n\t"
-                   "@q sub.u32 %4, %4, %6;\n\t@q ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
-                   : "+r"(left), "+r"(down), "+r"(right), "+r"(avail), "+r"(sp) : "r"(sbase), "n"(F));
-      const uint32_t row = __umulhi(down, 32u);                 // down >> 27
-      const bool act = avail != 0u;
-      const uint32_t bit = avail & (0u - avail);
-      avail -= bit;
-      sts_word_if(act ? 1u : 0u, bbase + row * RB, bit);        // board row `row` = the queen taken
+      asm volatile("{\n\t.reg .pred q;\n\tsetp.eq.u32 q, %3, 0;\n\t"
+                   "@q sub.u32 %4, %4, %5;\n\t@q ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+                   : "+r"(left), "+r"(right), "+r"(fr), "+r"(avail), "+r"(sp) : "n"(F));
+      const uint32_t pf = __popc(fr);                           // columns, and rows, left
+      const uint32_t w = lds_word_u(words + pf * 4u);
+      const uint32_t rest = avail & (avail - 1u);
+      const uint32_t bit = avail - rest;
+      sts_frame_u(sp, left, right, fr, rest);
+      if (rest != 0u) sp += F;
+      sts_word_u(brd_end - pf * RB, bit);                       // the row's queen
       const uint32_t nl = (left + bit) * 2u;
-      const uint32_t nd = down + bit;
       const uint32_t nr = __umulhi(right + bit, 0x80000000u);   // (right | bit) >> 1
-      const uint32_t nrow = row + 1u;
-      const uint32_t nb = mask & ~(nl | nd | nr);
-      const bool last = nrow == last_row;
-      // row rules of backTrack1/backTrack2 (row_filter) as selects
-      uint32_t nbf = nb & ((nrow < cf.bound1) ? lowmask : ~0u);
-      const uint32_t ds = nd & cf.sidemask;
-      const uint32_t at_b2 = (ds == 0u) ? 0u : ((ds != cf.sidemask) ? (nbf & cf.sidemask) : nbf);
-      nbf = (nrow == b2) ? at_b2 : nbf;
-      // last row: a solution (part 1: x8) or a board to classify (part 2)
-      if (act && last && nb != 0u) {
-        if (cf.part == 1) {
-          c8++;
-        } else if ((nb & cf.lastmask) == 0u) {
-          brd[nrow * BLOCK] = nb;
-          const uint32_t k = classify([&](int r) { return brd[r * BLOCK]; }, N, cf);
-          c2 += (k == 2); c4 += (k == 4); c8 += (k == 8);
+      const uint32_t free_cols = fr - bit;
+      const uint32_t nb = free_cols & ~(nl | nr) & w;
+      const bool dead = (free_cols & side & (uint32_t)((int32_t)w >> 31)) != 0u;
+      if (w & U_COUNT) cnt += 1u;
+      if (__any_sync(FULLM, (w & U_CLASSIFY) != 0u)) {
+        bool turns = false;               // a rotation has the board's own row 0
+        if (w & U_CLASSIFY) {
+          turns = lds_word_u(brd2) == 1u || lds_word_u(brd1) == topbit || bit == last_col;
+          if (!turns) cnt += 1u;
+        }
+        unsigned boards = __ballot_sync(FULLM, turns);
+        __syncwarp();
+        while (boards) {
+          const int src = __ffs((int)boards) - 1;
+          boards &= boards - 1u;
+          const uint32_t from = __shfl_sync(FULLM, brd, src);
+          const uint32_t row = lane < (uint32_t)N ? lds_word_u(from + lane * RB) : 1u;
+          const uint32_t k = classify((31u - (uint32_t)__clz((int)row)) & 31u, lane, (uint32_t)N, inv);
+          w2 += (k == 2); w4 += (k == 4); w8 += (k == 8);
+          __syncwarp();
         }
       }
-      const bool desc = act && !last && nbf != 0u;
-      const uint32_t push = (desc && avail != 0u) ? 1u : 0u;
-      sts_frame_if(push, sp, left, down, right, avail);
-      sp += push ? F : 0u;
-      if (desc) { left = nl; down = nd + (1u << 27); right = nr; avail = nbf; }
+      left = nl; right = nr; fr = free_cols;
+      avail = dead ? 0u : nb;
     }
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    c2 += __shfl_xor_sync(FULLM, c2, o);
-    c4 += __shfl_xor_sync(FULLM, c4, o);
-    c8 += __shfl_xor_sync(FULLM, c8, o);
-  }
+  for (int o = 16; o > 0; o >>= 1) c8 += __shfl_xor_sync(FULLM, c8, o);
+  c8 += w8;
   if (lane == 0) {
-    if (c2) atomicAdd(&a.ctl->c2, c2);
-    if (c4) atomicAdd(&a.ctl->c4, c4);
+    if (w2) atomicAdd(&a.ctl->c2, w2);
+    if (w4) atomicAdd(&a.ctl->c4, w4);
     if (c8) atomicAdd(&a.ctl->c8, c8);
   }
 }
@@ -316,12 +337,12 @@ __global__ void __launch_bounds__(BLOCK) unique_kernel(const UArgs a) {
 __device__ __forceinline__ UConf make_conf(int N, int i) {
   const uint32_t topbit = 1u << (N - 1);
   const int n1 = N - 3;                                 // part 1: bound1 = 2..N-2
-  if (i < n1) return UConf{1, (uint32_t)(i + 2), 0, 0, 0, 0, topbit};
+  if (i < n1) return UConf{1, (uint32_t)(i + 2), 0, 0, 0};
   const int k = i - n1;                                 // part 2: bound1 = 1.., bound2 = N-1-bound1
   const uint32_t sidemask = topbit | 1u;
   uint32_t lastmask = sidemask;
   for (int q = 0; q < k; q++) lastmask = (lastmask << 1) | lastmask | (lastmask >> 1);
-  return UConf{2, (uint32_t)(k + 1), (uint32_t)(N - 2 - k), topbit >> (k + 1), lastmask, sidemask, topbit};
+  return UConf{2, (uint32_t)(k + 1), (uint32_t)(N - 2 - k), lastmask, sidemask};
 }
 
 __device__ __forceinline__ uint32_t candidates(const UTask& t, uint32_t mask, const UConf& c) {
@@ -416,9 +437,9 @@ extern "C" int nq_count_unique(nq_handle* h, int N, uint64_t* unique, uint64_t* 
   const int nconf = (N - 3) + (N - 2) / 2;      // part 1: bound1 2..N-2; part 2: bound1 < N - 1 - bound1
   // Rows are expanded until the queue holds `target` tasks, unless the next row does not fit the buffer.
   // Lanes share work within a warp only, so the warps' sums have to even out: us of a whole count on GB300
-  // with a target of 512 / 1024 / 4096 tasks per SM, N=15 303 / 303 / 227, N=16 921 / 936 / 736, N=17 11323 /
-  // 4154 / 4204, N=18 56174 / 59898 / 27268 (5 10^5 tasks against 4.9 10^6).
-  const unsigned target = (unsigned)sms * (N <= 15 ? 1024u : N <= 17 ? 4096u : 13824u);
+  // with a target of 512 / 1024 / 4096 / 13824 tasks per SM, N=15 235 / 235 / 186 / 187, N=16 620 / 626 / 575 /
+  // 582, N=17 7770 / 3088 / 3090 / 3077, N=18 37772 / 37105 / 21139 / 19606.
+  const unsigned target = (unsigned)sms * (N <= 17 ? 4096u : 13824u);
   const size_t cap = (size_t)target * 5;
   NQ_CUDA(h, h->utasks.ensure(2 * cap * sizeof(UTask)));
   NQ_CUDA(h, h->uconfs.ensure((size_t)nconf * sizeof(UConf)));
@@ -441,9 +462,10 @@ extern "C" int nq_count_unique(nq_handle* h, int N, uint64_t* unique, uint64_t* 
     NQ_CUDA(h, cudaStreamSynchronize(st));
     row = 1 + queue_level((const UCtl*)h->h_ctrl, (unsigned)cap);
   }
-  const int maxf = std::max(1, N - 2 - row);
-  constexpr int B = 128;
-  const size_t smem = (size_t)B * ((size_t)maxf * sizeof(uint4) + (size_t)N * sizeof(uint32_t));
+  const int maxf = N - row + 1;
+  constexpr int B = 128;   // N=18: 64 / 128 / 256 threads 20.3 / 19.6 / 19.9 ms
+  const size_t smem = (size_t)B * maxf * sizeof(uint4) + (size_t)(N + 1) * (B + 1) * sizeof(uint32_t) +
+                      (size_t)B * sizeof(uint32_t) + (size_t)nconf * (N + 1) * sizeof(uint32_t);
   int optin = 0;   // the cap is process-wide: set it to the device maximum, never to one launch's size
   NQ_CUDA(h, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   NQ_CUDA(h, cudaFuncSetAttribute(unique_kernel<B>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
@@ -451,7 +473,7 @@ extern "C" int nq_count_unique(nq_handle* h, int N, uint64_t* unique, uint64_t* 
   NQ_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, unique_kernel<B>, B, smem));
   if (per <= 0) return h->fail(NQ_ECUDA, "count_unique: N=%d does not fit on an SM", N);
   UArgs a;
-  a.tasks[0] = buf[0]; a.tasks[1] = buf[1]; a.confs = confs; a.N = N; a.maxf = maxf; a.cap = (unsigned)cap; a.ctl = ctl;
+  a.tasks[0] = buf[0]; a.tasks[1] = buf[1]; a.confs = confs; a.nconf = nconf; a.N = N; a.maxf = maxf; a.cap = (unsigned)cap; a.ctl = ctl;
   unique_kernel<B><<<sms * per, B, smem, st>>>(a);
   NQ_CUDA(h, cudaGetLastError());
   NQ_CUDA(h, cudaMemcpyAsync(h->h_ctrl, ctl, sizeof(UCtl), cudaMemcpyDeviceToHost, st));
