@@ -103,7 +103,9 @@ int nq_exec_solutions_device(nq_handle *h, int N, const nq_record *d_records, in
  * handle's own stream. */
 int nq_sync(nq_handle *h);
 /* Device time of the last exec_solutions call's prepare and DFS kernels
- * (CUDA events recorded on the launching stream); waits for them. */
+ * (CUDA events recorded on the launching stream, or the device's clock read
+ * by the kernels where a short list's launches follow each other without a
+ * read-back); waits for them. */
 int nq_last_kernel_ms(nq_handle *h, float *prepare_ms, float *dfs_ms);
 /* Split depth used by the last exec_solutions call and the length of the
  * DFS queue it built (records, or subtasks when split). */

@@ -61,6 +61,8 @@ __device__ __forceinline__ uint4 start_state(int N, int sc) {
 __global__ void __launch_bounds__(128) gen_start_kernel(int N, unsigned n, const int* __restrict__ starts,
                                                         uint4* __restrict__ out, unsigned* gn) {
   const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
+  chain_next();
+  chain_wait();
   if (q == 0) gn[0] = n;
   if (q >= n) return;
   out[q] = start_state(N, starts[q]);
@@ -94,6 +96,8 @@ __device__ __forceinline__ int jasmin(int x, int N) {                // 356Py:27
 }
 
 __global__ void __launch_bounds__(128) gen_board_kernel(int N, uint4* __restrict__ out, unsigned cap, unsigned* gn) {
+  chain_next();
+  chain_wait();
   int q = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   const int corners = N * N;
   Quad x;
@@ -123,6 +127,8 @@ __global__ void __launch_bounds__(128) gen_board_kernel(int N, uint4* __restrict
 __global__ void __launch_bounds__(128) gen_level_kernel(int N, int preset, bool last, const uint4* __restrict__ in,
                                                         uint4* __restrict__ out, unsigned cap, unsigned* gn, int level,
                                                         unsigned* err) {
+  chain_next();
+  chain_wait();
   const unsigned n = gn[level];
   for (unsigned q0 = blockIdx.x * blockDim.x; q0 < n; q0 += gridDim.x * blockDim.x) {
     const unsigned q = q0 + threadIdx.x;
@@ -227,6 +233,7 @@ template <bool WIDE>
 __global__ void __launch_bounds__(1024) query_kernel(const __grid_constant__ QueryParam p, QueryBuffers b) {
   using W = typename QueryWord<WIDE>::type;
   __shared__ W words[kMaxDepth];
+  chain_next();
   if (threadIdx.x <= p.T) {
     const uint2 w = p.words[threadIdx.x];
     if constexpr (WIDE) words[threadIdx.x] = w; else words[threadIdx.x] = w.x;
@@ -247,6 +254,8 @@ __global__ void __launch_bounds__(512) batch_query_kernel(const BatchQuery* __re
                                                           ListState* state, uint32_t* info, void* sched, int sw) {
   using W = typename QueryWord<WIDE>::type;
   __shared__ W words[kMaxDepth];
+  chain_next();
+  chain_wait();
   const BatchQuery& q = qs[blockIdx.x];
   if (threadIdx.x <= q.p.T) {
     const uint2 w = q.p.words[threadIdx.x];
@@ -267,6 +276,8 @@ __global__ void __launch_bounds__(512) batch_query_kernel(const BatchQuery* __re
 template <bool WIDE>
 __global__ void __launch_bounds__(128) query_level_kernel(uint32_t N, uint32_t T, QueryBuffers b, int level) {
   using W = typename QueryWord<WIDE>::type;
+  chain_next();
+  chain_wait();
   const unsigned n = b.ctl[QueryCtl::kQueue + level];
   const unsigned cap = b.cap[level + 1];
   const uint4* __restrict__ in = b.sroot[level];
@@ -298,15 +309,18 @@ cudaError_t launch_generate(int N, int preset, unsigned n_starts, const int* sta
   const unsigned full = 8u * (unsigned)sms;
   if (starts) {
     if (n_starts == 0) return cudaSuccess;
-    gen_start_kernel<<<(n_starts + 127) / 128, 128, 0, st>>>(N, n_starts, starts, buf[0], gn);
+    const cudaError_t e = launch_after(gen_start_kernel, (n_starts + 127) / 128, 128, 0, st, N, n_starts, starts, buf[0], gn);
+    if (e != cudaSuccess) return e;
   } else {
     const unsigned n = (unsigned)(N * N * (1 + ((N + 1) / 2 - 1) * N));
-    gen_board_kernel<<<(n + 127) / 128, 128, 0, st>>>(N, buf[0], cap, gn);
+    const cudaError_t e = launch_after(gen_board_kernel, (n + 127) / 128, 128, 0, st, N, buf[0], cap, gn);
+    if (e != cudaSuccess) return e;
   }
   for (int l = 0; l < levels; l++) {
     const unsigned need = l == 0 ? (n_starts + 127) / 128 : full;
-    gen_level_kernel<<<need < full ? need : full, 128, 0, st>>>(N, preset, l + 1 == levels, buf[l & 1], buf[(l + 1) & 1], cap,
-                                                                gn, l, err);
+    const cudaError_t e = launch_after(gen_level_kernel, need < full ? need : full, 128, 0, st, N, preset, l + 1 == levels, buf[l & 1],
+                                       buf[(l + 1) & 1], cap, gn, l, err);
+    if (e != cudaSuccess) return e;
   }
   return cudaGetLastError();
 }
@@ -315,8 +329,9 @@ cudaError_t launch_query(const QueryParam& p, const QueryBuffers& b, bool wide, 
   if (wide) query_kernel<true><<<1, 1024, 0, st>>>(p, b);
   else query_kernel<false><<<1, 1024, 0, st>>>(p, b);
   for (int l = 0; l < levels; l++) {
-    if (wide) query_level_kernel<true><<<4 * sms, 128, 0, st>>>(p.N, p.T, b, l);
-    else query_level_kernel<false><<<4 * sms, 128, 0, st>>>(p.N, p.T, b, l);
+    const cudaError_t e = wide ? launch_after(query_level_kernel<true>, 4 * sms, 128, 0, st, p.N, p.T, b, l)
+                               : launch_after(query_level_kernel<false>, 4 * sms, 128, 0, st, p.N, p.T, b, l);
+    if (e != cudaSuccess) return e;
   }
   return cudaGetLastError();
 }
@@ -324,9 +339,8 @@ cudaError_t launch_query(const QueryParam& p, const QueryBuffers& b, bool wide, 
 cudaError_t launch_batch_queries(int n, const BatchQuery* q, uint4* src, uint4* tmp, ListState* state, const TaskArrays& ta,
                                  cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  if (ta.wide) batch_query_kernel<true><<<n, 512, 0, st>>>(q, src, tmp, state, ta.info, ta.sched, ta.sw);
-  else batch_query_kernel<false><<<n, 512, 0, st>>>(q, src, tmp, state, ta.info, ta.sched, ta.sw);
-  return cudaGetLastError();
+  if (ta.wide) return launch_after(batch_query_kernel<true>, n, 512, 0, st, q, src, tmp, state, ta.info, ta.sched, ta.sw);
+  return launch_after(batch_query_kernel<false>, n, 512, 0, st, q, src, tmp, state, ta.info, ta.sched, ta.sw);
 }
 
 }  // namespace nq

@@ -45,11 +45,12 @@ struct Ctrl {
 
 // Control block of a single-N run (device, zeroed before each run):
 //   job total (u64), queue cursor (u64), error word (u32), deepest schedule (u32),
-//   split counters (u64 queue length, u64 unused); behind them, zeroed when a list is
+//   split queue length (u64), blocks of the DFS that have ended (u32), pad, device clock (ns, u64 x 3) at the start
+//   of prepare, the start of the DFS and its end; behind them, zeroed when a list is
 //   generated on the device: the states of each level (u32 x 7) and its error word (u32).
 namespace ctl {
-constexpr size_t kTotal = 0, kCursor = 8, kErr = 16, kTmax = 20, kSplit = 24, kBytes = 40;
-constexpr size_t kGen = 40, kGenErr = 68, kAll = 72;
+constexpr size_t kTotal = 0, kCursor = 8, kErr = 16, kTmax = 20, kSplit = 24, kDone = 32, kStamp = 40, kBytes = 64;
+constexpr size_t kGen = 64, kGenErr = 92, kAll = 96;
 }
 
 }  // namespace nq
@@ -75,6 +76,9 @@ struct nq_handle {
   cudaEvent_t done = nullptr;            // recorded after the last asynchronous count (nq_sync waits on it)
   uint64_t* h_ctrl = nullptr;   // pinned read-back of the control block
   size_t h_ctrl_cap = 0;
+  uint32_t* h_result = nullptr; // pinned, the control block as the last run's DFS left it, ...
+  bool result_written = false;  // ... if that run launched one
+  bool stamped = false;         // the last run's times stand in h_result, not in ev
   // pinned read-back blocks for batches, reused (freeing pinned memory can
   // synchronise the device, which would stall other batches in flight)
   std::mutex pin_mu;

@@ -67,6 +67,14 @@ struct DfsLaunch {
   bool big = false;                     // u64 per-task counters (some task has N >= 24)
   int block = 128;
   int grid = 0;                         // 0: one wave of resident blocks
+  // Optional: the last block to end copies ctl_words u32 of the control block to pinned host memory (blocks_done:
+  // zeroed before), so the caller only waits for the stream.
+  const uint32_t* ctl = nullptr;
+  unsigned ctl_words = 0;
+  unsigned int* blocks_done = nullptr;
+  uint32_t* host_ctl = nullptr;
+  unsigned long long* stamp = nullptr;  // optional: the device clock at its start and (with host_ctl) at its end
+  bool chained = false;                 // the kernel before it in the stream calls chain_next
 };
 
 // Prepare: records {ld, rd, col, startijkl} (the reference's 16-byte task
@@ -97,6 +105,7 @@ struct PrepareSplit {
   unsigned long long qcap = 0;
   unsigned long long* qn = nullptr;     // zeroed before
   unsigned long long* total = nullptr;
+  unsigned long long* stamp = nullptr;  // optional: the device clock at its start
 };
 cudaError_t launch_prepare_split(int D, int64_t m_max, const PrepareSplit& a, cudaStream_t st);
 
@@ -118,7 +127,8 @@ struct QueryParam {
   uint32_t words_wide;          // the words' form
   uint2 words[28];
 };
-// Its control block (u64 words): total, queue cursor, error word, queue length after each level.
+// Its control block (u64 words): total, queue cursor, error word and DFS blocks that have ended, queue length
+// after each level.
 struct QueryCtl {
   static constexpr unsigned kTotal = 0, kCursor = 1, kErr = 2, kQueue = 3, kWords = 6;
 };
@@ -181,6 +191,53 @@ cudaError_t int_peak(int kind, int iters, int grid, uint32_t* out, cudaStream_t 
 size_t dfs_smem_bytes(bool wide, int block, int maxt);
 
 #ifdef __CUDACC__
+// Chains of short kernels: launch_after lets a kernel's blocks be placed while the kernel before it in the stream
+// still runs.  They wait at chain_wait, which every such kernel calls before it touches memory (in a plain launch
+// it returns at once), until that kernel has ended and its writes are visible.  chain_next, at the top of a
+// kernel, lets the launch behind it be placed once all of its own blocks have been.  A boundary between two
+// kernels costs 1 to 2.5 us less so: a completion query of N=10 / N=17 31.7 / 106 us, 29.5 / 99 chained; a
+// unique count of N=12 79 us, 57.
+template <class... P, class... A>
+cudaError_t launch_after(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid); c.blockDim = dim3(block); c.dynamicSmemBytes = smem; c.stream = st;
+  c.attrs = &at; c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+__device__ __forceinline__ void chain_wait() { cudaGridDependencySynchronize(); }
+__device__ __forceinline__ void chain_next() { cudaTriggerProgrammaticLaunchCompletion(); }
+
+// The device's clock in ns.
+__device__ __forceinline__ unsigned long long device_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
+// Called by all threads of all blocks as their last step: the last block to end copies `words` u32 of the control
+// block `ctl` to pinned host memory (`done`: zeroed before).  A copy queued behind the kernel instead takes the
+// copy engine's start and end: completion query of N=10 / N=17 36 / 129 us with one, 31.7 / 106 so.  `end`:
+// optional, a word pair of ctl that receives the device's clock.
+__device__ __forceinline__ void hand_over(const uint32_t* ctl, unsigned words, unsigned* done, uint32_t* host,
+                                          unsigned long long* end = nullptr) {
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x >= 32u) return;
+  unsigned n = 0;
+  if (threadIdx.x == 0u) {
+    n = atomicAdd(done, 1u);
+    if (n == gridDim.x - 1u && end) *(volatile unsigned long long*)end = device_ns();
+    __threadfence();
+  }
+  if (__shfl_sync(0xFFFFFFFFu, n, 0) != gridDim.x - 1u) return;
+  __syncwarp();
+  for (unsigned w = threadIdx.x; w < words; w += 32u)
+    ((volatile uint32_t*)host)[w] = ((const volatile uint32_t*)ctl)[w];
+}
+
 // position of the r-th set bit of m (r < popc(m))
 __device__ __forceinline__ uint32_t nth_set(uint32_t m, uint32_t r) {
   uint32_t pos = 0;

@@ -123,6 +123,8 @@ __global__ void __launch_bounds__(256) prepare_kernel(int N, int64_t m, const un
                                                       int64_t offset, unsigned int* err, unsigned int* tmax,
                                                       unsigned int* n_out) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  chain_next();
+  chain_wait();
   if (m_dev) m = *m_dev;
   if (i == 0) *n_out = (unsigned int)m;
   int T = -1;
@@ -149,12 +151,10 @@ cudaError_t launch_prepare(int N, int64_t m, const unsigned int* m_dev, const ui
   const int B = 256;
   const unsigned G = (unsigned)((m + B - 1) / B);
   if (out.wide)
-    prepare_kernel<true><<<G, B, 0, st>>>(N, m, m_dev, records, out.root, out.info, (uint2*)out.sched, out.sw,
-                                          out.ra_words, offset, err, tmax, n_out);
-  else
-    prepare_kernel<false><<<G, B, 0, st>>>(N, m, m_dev, records, out.root, out.info, (uint32_t*)out.sched, out.sw,
-                                           out.ra_words, offset, err, tmax, n_out);
-  return cudaGetLastError();
+    return launch_after(prepare_kernel<true>, G, B, 0, st, N, m, m_dev, records, out.root, out.info, (uint2*)out.sched, out.sw,
+                        out.ra_words, offset, err, tmax, n_out);
+  return launch_after(prepare_kernel<false>, G, B, 0, st, N, m, m_dev, records, out.root, out.info, (uint32_t*)out.sched, out.sw,
+                      out.ra_words, offset, err, tmax, n_out);
 }
 
 // ---------------------------------------------------------------------------
@@ -203,6 +203,9 @@ __device__ __forceinline__ void frames_at(uint32_t ld, uint32_t rd, uint32_t col
 
 template <int D>
 __global__ void __launch_bounds__(256) prepare_split_kernel(const PrepareSplit a) {
+  chain_next();
+  chain_wait();
+  if (a.stamp && blockIdx.x == 0 && threadIdx.x == 0) *a.stamp = device_ns();
   const int64_t m = a.m_dev ? (int64_t)*a.m_dev : a.m;
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (D == 0 && t == 0) *a.qn = (unsigned long long)m;
@@ -266,10 +269,10 @@ cudaError_t launch_prepare_split(int D, int64_t m_max, const PrepareSplit& a, cu
   if (m_max <= 0) return cudaSuccess;
   const unsigned B = 256, G = (unsigned)((m_max + B - 1) / B);
   switch (D) {
-    case 0: prepare_split_kernel<0><<<G, B, 0, st>>>(a); break;
-    case 1: prepare_split_kernel<1><<<G, B, 0, st>>>(a); break;
-    case 2: prepare_split_kernel<2><<<G, B, 0, st>>>(a); break;
-    case 3: prepare_split_kernel<3><<<G, B, 0, st>>>(a); break;
+    case 0: return launch_after(prepare_split_kernel<0>, G, B, 0, st, a);
+    case 1: return launch_after(prepare_split_kernel<1>, G, B, 0, st, a);
+    case 2: return launch_after(prepare_split_kernel<2>, G, B, 0, st, a);
+    case 3: return launch_after(prepare_split_kernel<3>, G, B, 0, st, a);
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
@@ -317,6 +320,8 @@ template <bool WIDE>
 __global__ void __launch_bounds__(256) list_count_kernel(const ListArgs a) {
   using W = typename WordT<WIDE>::type;
   const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+  chain_next();
+  chain_wait();
   if ((i & ~31ull) >= a.total) return;
   const int li = find_range(a.ends, a.n, i);
   const BatchList l = a.lists[li];
@@ -364,8 +369,7 @@ __global__ void __launch_bounds__(256) list_write_kernel(const ListArgs a, const
 cudaError_t launch_list_count(const ListArgs& a, bool wide, cudaStream_t st) {
   if (a.total == 0) return cudaSuccess;
   const unsigned G = (unsigned)((a.total + 255) / 256);
-  if (wide) list_count_kernel<true><<<G, 256, 0, st>>>(a); else list_count_kernel<false><<<G, 256, 0, st>>>(a);
-  return cudaGetLastError();
+  return wide ? launch_after(list_count_kernel<true>, G, 256, 0, st, a) : launch_after(list_count_kernel<false>, G, 256, 0, st, a);
 }
 
 cudaError_t launch_list_write(const ListArgs& a, const BatchJob* jobs, uint4* sroot, uint2* sinfo, bool wide, cudaStream_t st) {
@@ -478,6 +482,11 @@ struct DfsArgs {
   unsigned long long* per_task;
   unsigned int* err;
   int maxt;
+  const uint32_t* ctl;        // copied to host_ctl by the last block to end, where that is set
+  unsigned ctl_words;
+  unsigned int* blocks_done;
+  uint32_t* host_ctl;
+  unsigned long long* stamp;
 };
 
 __device__ __forceinline__ void flush_job(const DfsArgs& a, unsigned job, unsigned long long v) {
@@ -636,6 +645,8 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
   auto arm = [&]() { sts_frame(top - F, 1u, 0u, 1u, kSentinelAvail); };
   uint32_t wexp = 0, job = a.job_base, task = 0;
   bool have = false, exhausted = false, drained = false;   // exhausted, drained: warp-uniform, as the pool's counters
+  chain_wait();
+  if (a.stamp && blockIdx.x == 0 && threadIdx.x == 0) *a.stamp = device_ns();
   unsigned long long m = a.m;
   if (a.m_dev) { m = *a.m_dev; if (m > a.qcap) m = 0; }
   // queue items a warp takes first: 32, or its share of a queue smaller than the grid
@@ -796,6 +807,7 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
   } else {
     flush_job(a, acc_job, acc);
   }
+  if (a.host_ctl) hand_over(a.ctl, a.ctl_words, a.blocks_done, a.host_ctl, a.stamp ? a.stamp + 1 : nullptr);
 }
 
 // The dynamic shared-memory cap of a kernel is one process-wide attribute.
@@ -834,6 +846,8 @@ static cudaError_t launch_dfs_t(const DfsLaunch& L, cudaStream_t st) {
   a.sroot = L.sroot; a.sinfo = L.sinfo;
   a.m = L.m; a.m_dev = L.m_dev; a.qcap = L.qcap; a.order = L.order; a.cursor = L.cursor; a.job_totals = L.job_totals; a.job_base = L.job_base;
   a.per_task = L.per_task; a.err = L.err; a.maxt = L.maxt;
+  a.ctl = L.ctl; a.ctl_words = L.ctl_words; a.blocks_done = L.blocks_done; a.host_ctl = L.host_ctl; a.stamp = L.stamp;
+  if (L.chained) return launch_after(dfs_kernel<FORM, BLOCK, BIG>, (unsigned)grid, BLOCK, smem, st, a);
   dfs_kernel<FORM, BLOCK, BIG><<<grid, BLOCK, smem, st>>>(a);
   return cudaGetLastError();
 }

@@ -107,7 +107,7 @@ __host__ __device__ __forceinline__ uint32_t row_filter(uint32_t bitmap, uint32_
 constexpr int kLevels = kBoardRows - 2;   // expanded rows at most: from row 1, and a task carries the rows above its own
 struct UCtl {
   unsigned long long c2, c4, c8;
-  unsigned int cursor, pad;
+  unsigned int cursor, done;    // done: blocks of unique_kernel that have ended
   unsigned int n[kLevels + 1];
 };
 // The queue is the last level with states in it that its buffer holds (levels alternate between two
@@ -127,6 +127,7 @@ struct UArgs {
   int maxf;                     // stack frames per lane: the sentinel's and one per row from the smallest task row
   unsigned cap;                 // tasks a buffer holds
   UCtl* ctl;
+  uint32_t* host;               // pinned: receives the control block
 };
 
 // Shared-memory accesses at 32-bit shared-window addresses.
@@ -191,6 +192,7 @@ __global__ void __launch_bounds__(BLOCK) unique_kernel(const UArgs a) {
   const uint32_t bottom = (uint32_t)__cvta_generic_to_shared(smem) + threadIdx.x * (uint32_t)sizeof(uint4);
   const uint32_t brd = (uint32_t)__cvta_generic_to_shared(smem) + (uint32_t)a.maxf * F + threadIdx.x * 4u;   // row 0
   const uint32_t tab = (uint32_t)__cvta_generic_to_shared(table);
+  chain_wait();
   for (int q = threadIdx.x; q < a.nconf * (N + 1); q += BLOCK) table[q] = row_word(a.confs[q / (N + 1)], N, q % (N + 1));
   __syncthreads();
   const unsigned lane = threadIdx.x & 31u;
@@ -324,6 +326,7 @@ __global__ void __launch_bounds__(BLOCK) unique_kernel(const UArgs a) {
     if (w4) atomicAdd(&a.ctl->c4, w4);
     if (c8) atomicAdd(&a.ctl->c8, c8);
   }
+  hand_over((const uint32_t*)a.ctl, sizeof(UCtl) / 4, &a.ctl->done, a.host);
 }
 
 // ---------------------------------------------------------------------------
@@ -351,6 +354,7 @@ __device__ __forceinline__ uint32_t candidates(const UTask& t, uint32_t mask, co
 
 __global__ void __launch_bounds__(64) unique_init_kernel(int N, int nconf, UConf* confs, UTask* tasks, UCtl* ctl) {
   const int i = threadIdx.x;
+  chain_next();
   if (i < (int)(sizeof(UCtl) / 4)) reinterpret_cast<unsigned int*>(ctl)[i] = 0;
   __syncthreads();
   if (i >= nconf) return;
@@ -376,6 +380,8 @@ __global__ void __launch_bounds__(64) unique_init_kernel(int N, int nconf, UConf
 __global__ void __launch_bounds__(128) unique_expand_kernel(int N, int level, unsigned target, unsigned cap, const UConf* __restrict__ confs,
                                                             const UTask* __restrict__ in, UTask* __restrict__ out,
                                                             UCtl* ctl) {
+  chain_next();
+  chain_wait();
   const unsigned n = ctl->n[level];
   if (n >= target) return;
   const uint32_t mask = (1u << N) - 1u;
@@ -450,8 +456,8 @@ extern "C" int nq_count_unique(nq_handle* h, int N, uint64_t* unique, uint64_t* 
   unique_init_kernel<<<1, 64, 0, st>>>(N, nconf, confs, buf[0], ctl);
   const int levels = N <= 9 ? 1 : std::min(kLevels, N - 3);   // N <= 9: a launch costs more than it balances
   for (int l = 0; l < levels; l++)
-    unique_expand_kernel<<<l < 2 ? 1 : l == 2 ? sms : 4 * sms, 128, 0, st>>>(N, l, target, (unsigned)cap, confs, buf[l & 1],
-                                                                            buf[(l + 1) & 1], ctl);
+    NQ_CUDA(h, launch_after(unique_expand_kernel, l < 2 ? 1 : l == 2 ? sms : 4 * sms, 128, 0, st, N, l, target, (unsigned)cap, confs,
+                            buf[l & 1], buf[(l + 1) & 1], ctl));
   NQ_CUDA(h, cudaGetLastError());
   if (int s = h->ensure_pinned(sizeof(UCtl))) return s;
   // Stacks sized to the tasks' rows need the level reached (one read-back); boards whose search takes less
@@ -474,9 +480,8 @@ extern "C" int nq_count_unique(nq_handle* h, int N, uint64_t* unique, uint64_t* 
   if (per <= 0) return h->fail(NQ_ECUDA, "count_unique: N=%d does not fit on an SM", N);
   UArgs a;
   a.tasks[0] = buf[0]; a.tasks[1] = buf[1]; a.confs = confs; a.nconf = nconf; a.N = N; a.maxf = maxf; a.cap = (unsigned)cap; a.ctl = ctl;
-  unique_kernel<B><<<sms * per, B, smem, st>>>(a);
-  NQ_CUDA(h, cudaGetLastError());
-  NQ_CUDA(h, cudaMemcpyAsync(h->h_ctrl, ctl, sizeof(UCtl), cudaMemcpyDeviceToHost, st));
+  a.host = (uint32_t*)h->h_ctrl;
+  NQ_CUDA(h, launch_after(unique_kernel<B>, sms * per, B, smem, st, a));
   NQ_CUDA(h, cudaStreamSynchronize(st));
   const UCtl* hc = (const UCtl*)h->h_ctrl;
   *unique = hc->c2 + hc->c4 + hc->c8;

@@ -359,7 +359,8 @@ class Engine:
         return d.value, q.value
 
     def last_kernel_ms(self) -> Tuple[float, float]:
-        """(prepare_ms, dfs_ms) of the last exec call, from CUDA events on its stream."""
+        """(prepare_ms, dfs_ms) of the last exec call, from CUDA events on its stream
+        or, for short lists, the device's clock."""
         a, b = ctypes.c_float(), ctypes.c_float()
         _check(lib().nq_last_kernel_ms(self._h, ctypes.byref(a), ctypes.byref(b)), self._h, "last_kernel_ms")
         return a.value, b.value
