@@ -71,8 +71,10 @@ namespace {
 
 // Lists up to this length run without a read-back between the launches: the DFS takes the queue's length
 // from the device and stacks for the deepest task the start rows allow.  Longer ones read the queue's length
-// and the deepest schedule first (about 15 us), which buys a tighter stack (more resident warps).
-constexpr int64_t kNoReadBack = 16384;
+// and the deepest schedule first (18 us with the events), which buys a tighter stack (more resident warps).
+// us without / with, records of N=15 16385 95 / 112, 21270 107 / 125, N=16 20000 216 / 234, 33046 305 / 314 (rows
+// left up to 12); N=17 16385 583 / 585, 30000 952 / 930, 49207 1468 / 1412, N=19 20000 1858 / 1787.
+int64_t no_read_back(int rows) { return rows <= 12 ? 65536 : 16384; }
 constexpr int64_t kQueueBytes = 256 << 20;   // queue buffer a short list may bound its queue by
 
 // records (device) -> counts on st; totals land in ctrl[0].  One launch prepares and splits, one counts.
@@ -99,11 +101,10 @@ int run_records(nq_handle* h, int N, const uint4* d_rec, int64_t m, int start_mi
   // is small, else 8 a level (measured: 6.2 to 8), built again if it was too small.
   uint64_t bound = (uint64_t)m, guess = (uint64_t)m + 1024;
   for (int d = 0; d < D; d++) { bound *= (uint64_t)(N - 2 - d); guess *= 8; }
-  const bool read_back = (m > kNoReadBack && !m_dev) || h->queue_order == 1 || (D > 0 && bound * 24 > (uint64_t)kQueueBytes);
+  const bool read_back = (m > no_read_back(maxt) && !m_dev) || h->queue_order == 1 || (D > 0 && bound * sizeof(uint4) > (uint64_t)kQueueBytes);
   if (D > 0) {
     const uint64_t q = std::max(read_back ? std::min(bound, guess) : bound, (uint64_t)(h->sroot.cap / sizeof(uint4)));
     NQ_CUDA(h, h->sroot.ensure((size_t)q * sizeof(uint4)));
-    NQ_CUDA(h, h->sinfo.ensure((size_t)q * sizeof(uint2)));
   } else {
     NQ_CUDA(h, h->root.ensure((size_t)m * sizeof(uint4)));
     P.root = (uint4*)h->root.p;
@@ -120,11 +121,11 @@ int run_records(nq_handle* h, int N, const uint4* d_rec, int64_t m, int start_mi
   if (read_back) NQ_CUDA(h, cudaEventRecord(h->ev[0], st));
   else P.stamp = (unsigned long long*)(c + ctl::kStamp);
   for (bool zeroed = m_dev != nullptr;; zeroed = false) {   // with m_dev, by the list's generator
-    P.sroot = (uint4*)h->sroot.p; P.sinfo = (uint2*)h->sinfo.p;
-    P.qcap = std::min(h->sroot.cap / sizeof(uint4), h->sinfo.cap / sizeof(uint2));
+    P.sroot = (uint4*)h->sroot.p;
+    P.qcap = h->sroot.cap / sizeof(uint4);
     if (!zeroed) NQ_CUDA(h, cudaMemsetAsync(c, 0, ctl::kBytes, st));
     NQ_CUDA(h, launch_prepare_split(D, m, P, st));
-    if (D > 0) { L.sroot = P.sroot; L.sinfo = P.sinfo; }
+    if (D > 0) { L.sroot = P.sroot; L.depth = (uint32_t)D; }
     if (!read_back) {
       if (D > 0 || m_dev) { L.m_dev = P.qn; L.qcap = D > 0 ? P.qcap : ~0ull; L.m_bound = (int64_t)std::min<uint64_t>(bound, 1ull << 40); }
       L.maxt = std::max(1, std::min(maxt, t_max) - D);
@@ -142,14 +143,13 @@ int run_records(nq_handle* h, int N, const uint4* d_rec, int64_t m, int start_mi
     L.m = (int64_t)ns;
     if (ns <= P.qcap) break;
     NQ_CUDA(h, h->sroot.ensure((size_t)ns * sizeof(uint4)));
-    NQ_CUDA(h, h->sinfo.ensure((size_t)ns * sizeof(uint2)));
   }
   L.big = counts_need_u64(N, D > 0 && !read_back ? m : L.m);
   if (h->queue_order == 1) {
     NQ_CUDA(h, h->okeys.ensure((size_t)std::max<int64_t>(L.m, 1)));
     NQ_CUDA(h, h->oorder.ensure((size_t)std::max<int64_t>(L.m, 1) * sizeof(uint32_t)));
     NQ_CUDA(h, h->ohist.ensure(512 * sizeof(unsigned int)));
-    NQ_CUDA(h, launch_order(L.m, L.sroot, L.sinfo, L.tasks, (uint8_t*)h->okeys.p, (unsigned int*)h->ohist.p,
+    NQ_CUDA(h, launch_order(L.m, L.sroot, L.tasks, (uint8_t*)h->okeys.p, (unsigned int*)h->ohist.p,
                             (uint32_t*)h->oorder.p, st));
     L.order = (const uint32_t*)h->oorder.p;
   }
@@ -264,7 +264,7 @@ void nq_destroy(nq_handle* h) {
   cudaSetDevice(h->device);
   if (h->stream) cudaStreamSynchronize(h->stream);
   h->rec.release(); h->root.release(); h->info.release(); h->sched.release(); h->per_task.release(); h->ctrl.release();
-  h->sroot.release(); h->sinfo.release(); h->gen.release(); h->starts.release();
+  h->sroot.release(); h->gen.release(); h->starts.release();
   h->okeys.release(); h->oorder.release(); h->ohist.release();
   h->utasks.release(); h->uconfs.release(); h->uctl.release();
   if (h->h_ctrl) cudaFreeHost(h->h_ctrl);

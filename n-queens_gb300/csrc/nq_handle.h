@@ -61,7 +61,7 @@ struct nq_handle {
   cudaStream_t stream = nullptr;
   int block = 64, grid = 0, split = -1;    // split: -1 automatic, 0..3 fixed depth
   std::string err;
-  nq::DevBuf rec, root, info, sched, per_task, ctrl, sroot, sinfo;
+  nq::DevBuf rec, root, info, sched, per_task, ctrl, sroot;
   nq::DevBuf gen, starts;                // device generator: the other state buffer, the start list
   nq::DevBuf utasks, uconfs, uctl;       // unique counter (nq_count_unique)
   // completion queries: a stream and buffers of their own, so a query may run beside an asynchronous count

@@ -52,7 +52,8 @@ struct TaskArrays {
 struct DfsLaunch {
   TaskArrays tasks;
   const uint4* sroot = nullptr;         // split queue: subtask frames ...
-  const uint2* sinfo = nullptr;         // ... and {task, depth | job << 5}; nullptr: the queue holds tasks (job 0)
+  const uint2* sinfo = nullptr;         // ... and {task, depth | job << 5}; nullptr: the task stands in the frames' w
+  uint32_t depth = 0;                   // and all are at this depth (job 0); no sroot either: the queue holds the tasks
   int64_t m = 0;                        // queue length ...
   const unsigned long long* m_dev = nullptr;   // ... or where it stands on the device; above qcap the DFS does nothing
   unsigned long long qcap = 0;
@@ -85,7 +86,7 @@ cudaError_t launch_prepare(int N, int64_t m, const unsigned int* m_dev, const ui
                            int64_t offset, unsigned int* err, cudaStream_t st, unsigned int* tmax, unsigned int* n_out);
 
 // Prepare and split a single-N list (compact words) in one launch: tasks, and for D = 1..3 the queue of their
-// depth-D frames (qn counts them, also past qcap, where nothing is written any more) and the counts settled
+// depth-D frames {ld, rd, col, task} (qn counts them, also past qcap, where nothing is written any more) and the counts settled
 // above depth D.  D = 0 writes the tasks' roots instead, which are the queue.
 struct PrepareSplit {
   int N = 0;
@@ -101,7 +102,6 @@ struct PrepareSplit {
   unsigned int* tmax = nullptr;         // optional
   unsigned long long* per_task = nullptr;    // optional; set for every task
   uint4* sroot = nullptr;               // D > 0
-  uint2* sinfo = nullptr;
   unsigned long long qcap = 0;
   unsigned long long* qn = nullptr;     // zeroed before
   unsigned long long* total = nullptr;
@@ -177,9 +177,9 @@ cudaError_t launch_batch_queries(int n, const BatchQuery* q, uint4* src, uint4* 
                                  cudaStream_t st);
 
 // Queue order, largest estimated subtree first: order[0..m) receives the queue
-// indices (subtasks when sinfo is set, else tasks); keys: m bytes of scratch,
+// indices (subtasks when sroot is set, else tasks); keys: m bytes of scratch,
 // hist_offs: 512 u32 of scratch.
-cudaError_t launch_order(int64_t m, const uint4* sroot, const uint2* sinfo, const TaskArrays& ta, uint8_t* keys,
+cudaError_t launch_order(int64_t m, const uint4* sroot, const TaskArrays& ta, uint8_t* keys,
                          unsigned int* hist_offs, uint32_t* order, cudaStream_t st);
 
 // Largest block count per SM for a given stack depth (occupancy query).

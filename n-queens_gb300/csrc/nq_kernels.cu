@@ -251,9 +251,7 @@ __global__ void __launch_bounds__(256) prepare_split_kernel(const PrepareSplit a
       uint32_t dummy = 0;
       const uint32_t later = a.ra_words ? 0u : ra.at(rows_d, a.err);
       frames_at<0, D>(rt.ld, rt.rd, rt.col, rt.avail, w, (uint32_t)a.N, (uint32_t)T, dummy, [&](uint4 f) {
-        f.y |= later;
-        a.sroot[base] = f;
-        a.sinfo[base++] = make_uint2((uint32_t)t, (uint32_t)D);
+        a.sroot[base++] = make_uint4(f.x, f.y | later, f.z, (uint32_t)t);
       });
     }
     const unsigned long long dv = (unsigned long long)direct << info_wexp(in);
@@ -400,7 +398,6 @@ __device__ __forceinline__ uint32_t cost_key(const uint4 f, uint32_t bm) {
 }
 
 __global__ void __launch_bounds__(256) order_hist_kernel(int64_t m, const uint4* __restrict__ sroot,
-                                                         const uint2* __restrict__ sinfo,
                                                          const uint4* __restrict__ root, const uint32_t* __restrict__ info,
                                                          uint8_t* __restrict__ keys, unsigned int* hist) {
   __shared__ unsigned int h[256];
@@ -408,9 +405,10 @@ __global__ void __launch_bounds__(256) order_hist_kernel(int64_t m, const uint4*
   __syncthreads();
   const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (q < m) {
-    const uint32_t task = sinfo ? sinfo[q].x : (uint32_t)q;
-    const uint4 f = sinfo ? sroot[q] : root[q];
-    const uint32_t key = cost_key(f, (1u << info_N(info[task])) - 1u);
+    uint4 f = sroot ? sroot[q] : root[q];
+    const uint32_t bm = (1u << info_N(info[sroot ? f.w : (uint32_t)q])) - 1u;
+    if (sroot) f.w = bm & ~(f.x | f.y | f.z);
+    const uint32_t key = cost_key(f, bm);
     keys[q] = (uint8_t)key;
     atomicAdd(&h[key], 1u);
   }
@@ -450,13 +448,13 @@ __global__ void __launch_bounds__(256) order_scatter_kernel(int64_t m, const uin
   order[base + __popc(same & ((1u << lane) - 1u))] = (uint32_t)q;
 }
 
-cudaError_t launch_order(int64_t m, const uint4* sroot, const uint2* sinfo, const TaskArrays& ta, uint8_t* keys,
+cudaError_t launch_order(int64_t m, const uint4* sroot, const TaskArrays& ta, uint8_t* keys,
                          unsigned int* hist_offs, uint32_t* order, cudaStream_t st) {
   if (m <= 0) return cudaSuccess;
   const unsigned G = (unsigned)((m + 255) / 256);
   cudaError_t e = cudaMemsetAsync(hist_offs, 0, 256 * sizeof(unsigned int), st);
   if (e != cudaSuccess) return e;
-  order_hist_kernel<<<G, 256, 0, st>>>(m, sroot, sinfo, ta.root, ta.info, keys, hist_offs);
+  order_hist_kernel<<<G, 256, 0, st>>>(m, sroot, ta.root, ta.info, keys, hist_offs);
   order_scan_kernel<<<1, 256, 0, st>>>(hist_offs, hist_offs + 256);
   order_scatter_kernel<<<G, 256, 0, st>>>(m, keys, hist_offs + 256, order);
   return cudaGetLastError();
@@ -466,12 +464,13 @@ cudaError_t launch_order(int64_t m, const uint4* sroot, const uint2* sinfo, cons
 // DFS
 // ---------------------------------------------------------------------------
 struct DfsArgs {
-  const uint4* root;          // task roots (when sinfo == nullptr the queue holds tasks)
+  const uint4* root;          // task roots (when sroot == nullptr the queue holds tasks)
   const uint32_t* info;
   const void* sched;
   int sw;
-  const uint4* sroot;         // subtask frames and {task, depth | job << 5} (split queue)
-  const uint2* sinfo;
+  const uint4* sroot;         // split queue: subtask frames, and ...
+  const uint2* sinfo;         // ... {task, depth | job << 5}; or, where this is null, the task in the frames' w and ...
+  uint32_t depth;             // ... all of them at this depth (their candidates follow from ld, rd and col)
   int64_t m;                  // queue length, ...
   const unsigned long long* m_dev;   // ... or where it stands on the device (above qcap: the queue did not fit, no work)
   unsigned long long qcap;
@@ -701,6 +700,7 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
             const uint64_t q = a.order ? (uint64_t)a.order[slot] : slot;
             uint32_t d0 = 0;
             if (a.sinfo) { const uint2 si = a.sinfo[q]; p_task = si.x; d0 = si.y & 31u; p_job = si.y >> 5; p_root = a.sroot[q]; }
+            else if (a.sroot) { p_root = a.sroot[q]; p_task = p_root.w; d0 = a.depth; p_root.w = ~(p_root.x | p_root.y); }
             else { p_task = (uint32_t)q; p_root = a.root[q]; }
             // free columns for used ones, R of them; depth d has R - d (one queen per depth), so word d is
             // found from popc(fr) alone
@@ -843,7 +843,7 @@ static cudaError_t launch_dfs_t(const DfsLaunch& L, cudaStream_t st) {
   }
   DfsArgs a;
   a.root = L.tasks.root; a.info = L.tasks.info; a.sched = L.tasks.sched; a.sw = L.tasks.sw;
-  a.sroot = L.sroot; a.sinfo = L.sinfo;
+  a.sroot = L.sroot; a.sinfo = L.sinfo; a.depth = L.depth;
   a.m = L.m; a.m_dev = L.m_dev; a.qcap = L.qcap; a.order = L.order; a.cursor = L.cursor; a.job_totals = L.job_totals; a.job_base = L.job_base;
   a.per_task = L.per_task; a.err = L.err; a.maxt = L.maxt;
   a.ctl = L.ctl; a.ctl_words = L.ctl_words; a.blocks_done = L.blocks_done; a.host_ctl = L.host_ctl; a.stamp = L.stamp;

@@ -17,6 +17,7 @@
 // threads at the same time) race: the caller must serialise them.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "../../include/nqueens_gb300.h"
@@ -91,14 +92,19 @@ extern "C" int nq_exec_solutions_noalloc(int N, const nq_record* d_records, int6
   used += ((size_t)m * sizeof(uint32_t) + 15) & ~(size_t)15;
   P.sched = (uint32_t*)(c + used);
   used += ((size_t)m * P.sw * sizeof(uint32_t) + 15) & ~(size_t)15;
-  P.qcap = (kScratchBytes - used) / (sizeof(uint4) + sizeof(uint2));
-  // Split as deep as the usual rule says while the queue should fit (8 items a level); one that does not
-  // after all leaves the DFS without work, and the call runs again unsplit (the scratch always holds that).
-  // 20,011 records of N=16: unsplit 417 us, one level 324 us.
+  P.qcap = (kScratchBytes - used) / sizeof(uint4);
+  // Split as deep as the usual rule says while the queue should fit: its items a task, from the generated lists
+  // (one level makes 4.5 / 5.4 / 6.2 / 7.1 at 10 / 11 / 12 / 13 rows, two make 3.9 / 4.7 / 5.5 / 6.3 each).  A
+  // queue that does not fit after all leaves the DFS without work, and the call runs again with a level less
+  // (the scratch always holds the tasks).  us with no, one and two levels: 20,011 records of N=16 354 / 288 /
+  // 219, of N=17 1640 / 972 / 665.
   int D = choose_split(m, maxt);
-  while (D > 0 && ((uint64_t)m << (3 * D)) > P.qcap) D--;
+  for (; D > 0; D--) {
+    const double first = std::max(1.0, 0.8 * maxt - 3.2), next = std::max(1.0, 0.8 * maxt - 4.0);
+    if ((double)m * (D == 1 ? first : D == 2 ? next * next : next * next * next) <= (double)P.qcap) break;
+  }
   uint64_t hc[4];
-  for (;; D = 0) {
+  for (;; D--) {
     // the array keeps the previous call's contents: clear what must start at zero
     if (cudaMemsetAsync(c, 0, 32, st) != cudaSuccess) return NQ_ECUDA;
     DfsLaunch L;
@@ -107,14 +113,14 @@ extern "C" int nq_exec_solutions_noalloc(int N, const nq_record* d_records, int6
       L.m = m;
     } else {
       P.sroot = (uint4*)(c + used);
-      P.sinfo = (uint2*)(P.sroot + P.qcap);
-      L.sroot = P.sroot; L.sinfo = P.sinfo; L.m_dev = P.qn; L.qcap = P.qcap;
+      L.sroot = P.sroot; L.depth = (uint32_t)D; L.m_dev = P.qn; L.qcap = P.qcap;
     }
     P.ra_words = !ra_in_rd(N, start_min, D);
     if (launch_prepare_split(D, m, P, st) != cudaSuccess) return NQ_ECUDA;
     L.tasks.root = P.root; L.tasks.info = P.info; L.tasks.sched = P.sched; L.tasks.sw = P.sw; L.tasks.wide = false; L.tasks.ra_words = P.ra_words;
     L.cursor = cursor; L.job_totals = totals;
     L.per_task = (unsigned long long*)d_solutions; L.err = err; L.maxt = maxt - D < 1 ? 1 : maxt - D; L.block = 128; L.grid = 0;
+    L.chained = true;
     L.big = counts_need_u64(N, m);
     if (launch_dfs(L, st) != cudaSuccess) return NQ_ECUDA;
     if (cudaMemcpyAsync(d_total, totals, 8, cudaMemcpyDeviceToDevice, st) != cudaSuccess) return NQ_ECUDA;

@@ -8,7 +8,7 @@ from conftest import gpu_available
 pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not gpu_available(), reason="needs a CUDA GPU")]
 
 
-@pytest.mark.parametrize("N,m", [(6, 5), (8, 1), (10, 1007), (13, 7731), (16, 16384), (16, 16385)])
+@pytest.mark.parametrize("N,m", [(6, 5), (8, 1), (10, 1007), (13, 7731), (16, 16384), (16, 33046), (17, 16384), (17, 16385)])
 def test_same_counts_with_and_without_read_back(N, m):
     import nqueens
     r = np.ascontiguousarray(nqueens.gen_records(N)[:m])

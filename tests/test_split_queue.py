@@ -43,11 +43,24 @@ def test_every_depth_gives_the_same_counts(eng, N, m):
 
 @pytest.mark.parametrize("N,m", [(14, 1), (16, 20011), (17, 49207), (22, 30001), (22, 57000)])
 def test_noalloc_queue_in_the_fixed_scratch(eng, N, m):
-    """The no-allocation call splits as far as its scratch holds the queue (N=22, 57,000 records: 8 items a task
-    would fit, the list has more, so it is counted unsplit): per record the regular call's counts."""
+    """The no-allocation call splits as far as its scratch holds the queue: per record the regular call's counts."""
+    _check_noalloc(eng, N, _sample(N, m))
+
+
+@pytest.mark.parametrize("m", [20000, 21700, 24000])
+def test_noalloc_queue_longer_than_expected(eng, m):
+    """The eighth of N=17's list with the most frames a task, over and over: two levels make 42 items a task where
+    41 are expected.  The queue fits (20,000), does not though it should (21,700: built again), or should not."""
+    import nqueens
+    recs = nqueens.gen_records(17)
+    recs = np.ascontiguousarray(np.resize(recs[:len(recs) // 8], m))
+    _check_noalloc(eng, 17, recs)
+
+
+def _check_noalloc(eng, N, recs):
     torch = pytest.importorskip("torch")
     import nqueens
-    recs = _sample(N, m)
+    m = len(recs)
     want_total, want = eng.exec_records(N, recs, want_solutions=True)
     d_rec = torch.from_numpy(recs.view(np.uint8).copy()).cuda()
     d_total = torch.full((1,), -1, dtype=torch.int64, device="cuda")
