@@ -33,10 +33,10 @@ namespace {
 
 constexpr unsigned FULLM = 0xFFFFFFFFu;
 constexpr int kBoardRows = 8;    // rows of the board prefix carried by a task
-// Steps per lane between checks for finished lanes, a multiple of the steps unrolled.  Unrolled further the loop
-// and the classification in it outgrow the instruction cache (us of a whole count at N=18, unrolled by 1 / 2 / 5 /
-// 10 / 15 / 30 with every board classified by the warp: 24.5 / 23.4 / 23.4 / 23.3 / 24.0 / 28.9 ms; as it is now,
-// by 5 and by 10 19.6 ms), and 16 or 20 steps a check gave 21.7 ms where 30 gave 21.5.
+// Steps per lane between checks for finished lanes, a multiple of the steps unrolled.  Unrolled far the loop and
+// the classification in it outgrow the instruction cache (a whole count at N=18, unrolled by 1 / 2 / 5 / 10 / 15 /
+// 30 with every board classified by the warp: 24.5 / 23.4 / 23.4 / 23.3 / 24.0 / 28.9 ms; as it is now, by 2 / 5 /
+// 10: 18.7 / 18.2 / 18.1), and 20 steps a check gave 21.7 ms where 30 gave 21.5.
 constexpr int kUniqueSteps = 30, kUniqueUnroll = 5;
 // Boards from here on size the stacks to the tasks' rows (N=14 96 us without the read-back, 111 with; N=15 187
 // against 190, and the search grows sixfold a size from there).
@@ -69,10 +69,10 @@ __device__ __forceinline__ void board_set(UTask& t, uint32_t r, uint32_t bit) {
 // whose row 0 differs is left out, otherwise the first row that differs decides.  `inv` is 32 words of the warp's
 // shared memory for the rows by column.
 // Bound by issue: about 60 instructions of the warp a board, on the quarter of the boards that have a rotation
-// with their own row 0 (the others count x8 after three loads of their own lane).  One step in 125 ends in such a
-// board's last row (N=16), so a warp's step has one with odds of 1 in 4: at N=18 a count took 15.0 ms without
-// any classification, 21.0 with a lane searching its own board for each column, 23.4 with every board here, and
-// takes 19.6 with the check before.
+// with their own row 0 (the others count x8 after two loads of their own lane).  One step in 104 stands on such a
+// part's last row (N=16), so one warp step in 4 has one: at N=18 a count took 15.0 ms without any
+// classification, 21.0 with a lane searching its own board for each column, 23.4 with every board here, and
+// 19.6 with the check before.
 __device__ __forceinline__ uint32_t classify(uint32_t c, uint32_t lane, uint32_t N, uint32_t* inv) {
   const bool in = lane < N;
   const uint32_t other = in ? N - 1u - lane : lane;
@@ -151,18 +151,20 @@ __device__ __forceinline__ void lds_frame_u(uint32_t a, uint32_t& x, uint32_t& y
 // columns behind it.
 constexpr uint32_t U_COUNT = 1u << 27;      // part 1, last row: a solution, x8
 constexpr uint32_t U_CLASSIFY = 1u << 28;   // part 2, last row: a board to classify
+constexpr uint32_t U_NOLOOK = 1u << 29;     // the child's row is the last one: there is none behind it
 constexpr uint32_t U_SIDES = 1u << 31;      // part 2, row bound2 + 1: dead while a side column is free
 __device__ __forceinline__ uint32_t row_word(const UConf& c, int N, int left) {
   if (left == 0) return 0u;                 // the sentinel: every child dies
   if (left == 1) return c.part == 1 ? U_COUNT : U_CLASSIFY;
   const uint32_t child = (uint32_t)(N - left + 1);
   uint32_t w = (1u << N) - 1u;
+  if (left == 2) w |= U_NOLOOK;
   if (child < c.bound1) w &= c.part == 1 ? ~2u : ~c.sidemask;
   if (c.part != 1) {
     if (child == (uint32_t)N - 1u) w &= ~c.lastmask;
     // Row bound2 must take the last free side column (backTrack2, :126-151): after it both are behind.  Its
     // own candidates go unfiltered and die one step on: 5 % more steps (N=15 39.7 10^6 against 37.6, N=16 259
-    // against 246), each about four instructions of 32 shorter.
+    // against 246, before the look-ahead), each about four instructions shorter.
     if (child == c.bound2 + 1u) w |= U_SIDES;
   }
   return w;
@@ -173,10 +175,12 @@ __device__ __forceinline__ uint32_t row_word(const UConf& c, int N, int left) {
 // rest of its candidates whether or not there are any, a solution is a frame in the last row, and a sentinel
 // frame whose 31 candidates die feeds a lane without work.  Each step also records its queen in the lane's
 // board.  A frame is {left, right, free columns, candidates}; its row is N - popc(free columns).
-// Bound by issue and by shared memory together: a step writes 16 bytes and mostly reads 16, writes 4 for the
-// board, and reads the row's word from a table that the lanes of a configuration share.  With the row in `down`'s
-// high bits, the rules computed at each step and predicated pushes a count took 27.3 ms at N=18 and 4.2 ms at
-// N=17; with the same steps as here 21.5 and 3.4, with boards classified by the warp 19.6 and 3.08.
+// Bound by issue and latency (N=17: 46 warp instructions a step, a quarter of them the last rows' boards; issue 70 %,
+// shared memory 74 % of its wavefronts, ALU 56 %, 24 warps an SM by shared memory).  With the row in `down`'s high
+// bits, the rules computed at each step and predicated pushes a count took 27.3 ms at N=18 and 4.2 at N=17; with
+// the step as here 21.5 and 3.4; boards classified by the warp 19.6 and 3.08; look-ahead over the row after the
+// child (17 % fewer steps for 4 instructions) 18.5 and 2.94; board rows BLOCK words apart, so a step's stores
+// meet no bank twice (one word more made the warp's reads of a board meet none instead) 18.2 and 2.90.
 constexpr uint32_t kUSentinel = 0xFFFFFFFEu;
 static_assert(kUniqueSteps <= 30, "the sentinel holds 31 candidates, and one has to be left at a check");
 template <int BLOCK>
@@ -184,7 +188,7 @@ __global__ void __launch_bounds__(BLOCK) unique_kernel(const UArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int N = a.N;
   constexpr uint32_t F = BLOCK * (uint32_t)sizeof(uint4);          // frame stride of one lane's stack
-  constexpr uint32_t RB = (BLOCK + 1) * (uint32_t)sizeof(uint32_t);   // board row stride: a lane's rows lie in different banks
+  constexpr uint32_t RB = BLOCK * (uint32_t)sizeof(uint32_t);      // board row stride
   // maxf frames (the sentinel's, one per row), N + 1 board rows (the last one is the sentinel's), 32 words a
   // warp for classify, the rows' words
   uint32_t* inv = reinterpret_cast<uint32_t*>(smem + (size_t)a.maxf * F + (size_t)(N + 1) * RB) + (threadIdx.x & ~31u);
@@ -294,6 +298,7 @@ __global__ void __launch_bounds__(BLOCK) unique_kernel(const UArgs a) {
       const uint32_t nr = __umulhi(right + bit, 0x80000000u);   // (right | bit) >> 1
       const uint32_t free_cols = fr - bit;
       const uint32_t nb = free_cols & ~(nl | nr) & w;
+      const uint32_t keep = (free_cols & ~((nl + nl) | __umulhi(nr, 0x80000000u))) | (w & U_NOLOOK);   // look-ahead
       const bool dead = (free_cols & side & (uint32_t)((int32_t)w >> 31)) != 0u;
       if (w & U_COUNT) cnt += 1u;
       if (__any_sync(FULLM, (w & U_CLASSIFY) != 0u)) {
@@ -315,7 +320,7 @@ __global__ void __launch_bounds__(BLOCK) unique_kernel(const UArgs a) {
         }
       }
       left = nl; right = nr; fr = free_cols;
-      avail = dead ? 0u : nb;
+      avail = dead || keep == 0u ? 0u : nb;
     }
   }
 #pragma unroll
@@ -444,7 +449,7 @@ extern "C" int nq_count_unique(nq_handle* h, int N, uint64_t* unique, uint64_t* 
   // Rows are expanded until the queue holds `target` tasks, unless the next row does not fit the buffer.
   // Lanes share work within a warp only, so the warps' sums have to even out: us of a whole count on GB300
   // with a target of 512 / 1024 / 4096 / 13824 tasks per SM, N=15 235 / 235 / 186 / 187, N=16 620 / 626 / 575 /
-  // 582, N=17 7770 / 3088 / 3090 / 3077, N=18 37772 / 37105 / 21139 / 19606.
+  // 582, N=17 7770 / 3088 / 3090 / 3077, N=18 37772 / 37105 / 21139 / 19606 (now 170, 540, 2900 and 18208).
   const unsigned target = (unsigned)sms * (N <= 17 ? 4096u : 13824u);
   const size_t cap = (size_t)target * 5;
   NQ_CUDA(h, h->utasks.ensure(2 * cap * sizeof(UTask)));
@@ -470,7 +475,7 @@ extern "C" int nq_count_unique(nq_handle* h, int N, uint64_t* unique, uint64_t* 
   }
   const int maxf = N - row + 1;
   constexpr int B = 128;   // N=18: 64 / 128 / 256 threads 20.3 / 19.6 / 19.9 ms
-  const size_t smem = (size_t)B * maxf * sizeof(uint4) + (size_t)(N + 1) * (B + 1) * sizeof(uint32_t) +
+  const size_t smem = (size_t)B * maxf * sizeof(uint4) + (size_t)(N + 1) * B * sizeof(uint32_t) +
                       (size_t)B * sizeof(uint32_t) + (size_t)nconf * (N + 1) * sizeof(uint32_t);
   int optin = 0;   // the cap is process-wide: set it to the device maximum, never to one launch's size
   NQ_CUDA(h, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
