@@ -177,13 +177,18 @@ int read_ctrl(nq_handle* h, cudaStream_t st, uint64_t* total) {
 }
 
 // Queue of a completion query: one block expands it to kQueryTarget frames and more, then the whole GPU by
-// another level or two where the rows left make the frames large.  us of a query, 0 / 1 / 2 levels over the
-// GPU: N=14 one queen 84 / 71 / 71, N=17 two queens 169 / 139 / 139, N=18 two queens 612 / 530 / 397, N=20
-// three queens 2574 / 1888 / 1285; with a target of 8192: N=15 two queens 72 us against 60.
+// another one to three levels where the rows left make the frames large.  us of a query (mean of six), levels
+// over the GPU: 10 rows (N=12, two queens) 0 / 1 level 36 / 42; 13 rows (N=14, one) 1 / 2 60 / 53; 14 rows (N=15,
+// one) 1 / 2 / 3 88 / 80 / 98; 15 rows (N=17, two) 143 / 122 / 129; 16 and more, 2 / 3: N=19 two queens 2118 / 1630,
+// N=20 three 1110 / 965.  A target of 1024 / 2048 / 4096 frames: N=19 three queens 366 / 256 / 257, N=13 one 44 /
+// 45 / 52.
 constexpr unsigned kQueryCap = 65536;
 constexpr unsigned kQueryTarget = 2048;
 constexpr unsigned kQueryCap2 = 4 << 20;     // queue after two levels (never reached: 7 children a frame on average)
-int query_levels(int rows) { return rows >= 15 ? 2 : rows >= 12 ? 1 : 0; }
+constexpr unsigned kQueryCap3 = 5 << 20;     // ... after three (0.5 to 4.5 10^6 measured for N=18..25; some of N=27 are longer)
+int query_levels(int rows) { return rows >= 16 ? 3 : rows >= 13 ? 2 : rows >= 11 ? 1 : 0; }
+// A batch's queries share the lanes with its other jobs, so the same need not be cut as fine.
+int batch_query_levels(int rows) { return rows >= 15 ? 2 : rows >= 12 ? 1 : 0; }
 
 // The query as a device task.  Returns 1, 0 when the count is settled here (*fixed), or -1 on bad arguments.
 // The last free row holds one column for every board, so its parent row is the task's terminal depth (count
@@ -991,7 +996,7 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
     ends[i] = src;
     ntask += l.query ? 1 : l.cap;
     words = std::max<uint64_t>(words, l.query ? l.T + 1 : l.rows + 1);
-    const int levels = l.query ? query_levels(l.rows) : choose_split((int64_t)std::max(sources, l.cap), l.rows);
+    const int levels = l.query ? batch_query_levels(l.rows) : choose_split((int64_t)std::max(sources, l.cap), l.rows);
     l.D = l.N <= 12 ? 0 : h->split >= 0 ? h->split : l.query && sources > 100000 ? std::min(levels, 1) : levels;
   }
   for (const Board& bd : boards) {
@@ -1170,7 +1175,7 @@ int64_t nq_job_device_bytes(const nq_job* job, int sms, int split_depth) {
     if (s > 0) {
       m = (int64_t)std::min(kQueryTarget, kQueryCap / (unsigned)J.N) * J.N;
       rows = (int)p.T + 2;
-      levels = query_levels(rows);
+      levels = batch_query_levels(rows);
     }
   } else {
     return NQ_EINVAL;
@@ -1286,9 +1291,9 @@ int nq_count_completions(nq_handle* h, int N, int k, const int* rows, const int*
   if (!h->h_query) NQ_CUDA(h, cudaMallocHost((void**)&h->h_query, QueryCtl::kWords * 8));
   cudaStream_t st = h->q_stream;
   p.target = std::min(kQueryTarget, kQueryCap / (unsigned)N);
-  for (int levels = query_levels((int)p.T + 2);; levels = 1) {
+  for (int levels = query_levels((int)p.T + 2);; levels--) {      // a level less where the queue did not fit
     QueryBuffers b{};
-    b.cap[0] = kQueryCap; b.cap[1] = kQueryCap * (unsigned)N; b.cap[2] = kQueryCap2;
+    b.cap[0] = kQueryCap; b.cap[1] = kQueryCap * (unsigned)N; b.cap[2] = kQueryCap2; b.cap[3] = kQueryCap3;
     size_t items = 0;
     for (int l = 0; l <= levels; l++) items += b.cap[l];
     NQ_CUDA(h, h->qbuf.ensure(1024 + (kQueryCap + items) * sizeof(uint4) + items * sizeof(uint2)));
@@ -1314,7 +1319,7 @@ int nq_count_completions(nq_handle* h, int N, int k, const int* rows, const int*
     L.chained = true;
     NQ_CUDA(h, launch_dfs(L, st));
     NQ_CUDA(h, cudaStreamSynchronize(st));
-    if (levels < 2 || h->h_query[QueryCtl::kQueue + 2] <= b.cap[2]) break;
+    if (levels < 2 || (h->h_query[QueryCtl::kQueue + 2] <= b.cap[2] && (levels < 3 || h->h_query[QueryCtl::kQueue + 3] <= b.cap[3]))) break;
   }
   const uint32_t e = (uint32_t)h->h_query[QueryCtl::kErr];
   if (e) return h->fail(derr_to_status(e), "device: %s", derr_text(e));

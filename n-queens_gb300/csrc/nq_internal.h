@@ -130,18 +130,18 @@ struct QueryParam {
 // Its control block (u64 words): total, queue cursor, error word and DFS blocks that have ended, queue length
 // after each level.
 struct QueryCtl {
-  static constexpr unsigned kTotal = 0, kCursor = 1, kErr = 2, kQueue = 3, kWords = 6;
+  static constexpr unsigned kTotal = 0, kCursor = 1, kErr = 2, kQueue = 3, kWords = 7;
 };
 struct QueryBuffers {
   unsigned long long* ctl;
   uint32_t* info;               // one task
   void* sched;
   uint4* tmp;                   // cap[0] frames
-  uint4* sroot[3];              // the queue from one block, and after one and two levels over the whole GPU
-  uint2* sinfo[3];
-  unsigned cap[3];              // items each holds; cap[1] = cap[0] * N, so only the last can be too small
+  uint4* sroot[4];              // the queue from one block, and after one to three levels over the whole GPU
+  uint2* sinfo[4];
+  unsigned cap[4];              // items each holds; cap[1] = cap[0] * N, so only the later ones can be too small
 };
-// Writes the task, its queue and the control block, the queue expanded by `levels` (0..2) more levels.  A
+// Writes the task, its queue and the control block, the queue expanded by `levels` (0..3) more levels.  A
 // queue longer than its buffer leaves ctl[kQueue + levels] above cap[levels]: the DFS does nothing.
 cudaError_t launch_query(const QueryParam& p, const QueryBuffers& b, bool wide, int levels, int sms, cudaStream_t st);
 

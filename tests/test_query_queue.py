@@ -30,6 +30,22 @@ def test_neighbouring_rows(eng, oracle_mod, N, queens):
     assert eng.count_completions(N, queens) == want
 
 
+@pytest.mark.parametrize("N,queens", [
+    (17, [(3, 4), (9, 11)]), (18, [(2, 2), (10, 7), (13, 16)]), (19, [(0, 3), (8, 12), (15, 5)]),   # attacked: none
+    (19, [(0, 3), (8, 12), (15, 6)]),
+    (27, [(26, 5), (18, 22), (12, 2), (13, 12), (19, 24), (14, 20), (23, 9), (16, 8)])])
+def test_levels_over_the_gpu(eng, N, queens):
+    """Two and three levels over the whole GPU, and a board whose top rows are free, where three do not fit the queue
+    and two are counted: the counts of the same queries built as a batch."""
+    from nqueens import CompletionJob
+    b = eng.batch([CompletionJob(N, queens)])
+    try:
+        want = b.run()[0]
+    finally:
+        b.close()
+    assert eng.count_completions(N, queens) == int(want)
+
+
 def test_queries_beside_an_asynchronous_count(eng, oracle_mod):
     """A query has its own stream and buffers: one issued while an asynchronous count is outstanding leaves that
     count's result and status alone."""
