@@ -156,7 +156,7 @@ int run_records(nq_handle* h, int N, const uint4* d_rec, int64_t m, int start_mi
   h->last_split = D; h->last_queue = L.m; h->queue_on_device = L.m_dev != nullptr;
   if (read_back) NQ_CUDA(h, cudaEventRecord(h->ev[1], st));
   else { L.chained = true; L.stamp = P.stamp + 1; }
-  L.ctl = (const uint32_t*)c; L.ctl_words = ctl::kAll / 4; L.blocks_done = (unsigned int*)(c + ctl::kDone); L.host_ctl = h->h_result;
+  L.ctl = (const uint32_t*)c; L.ctl_words = ctl::kAll / 8; L.blocks_done = (unsigned int*)(c + ctl::kDone); L.host_ctl = h->h_result;
   NQ_CUDA(h, launch_dfs(L, st));
   h->result_written = L.m > 0 || L.m_dev;
   if (read_back) NQ_CUDA(h, cudaEventRecord(h->ev[2], st));
@@ -835,6 +835,10 @@ struct nq_batch {
 
 namespace {
 
+// Jobs up to which the search's last block hands the totals over (one warp, 256 of them at a time); above, a copy.
+// us of a replay, so / by a copy: 4 jobs of N=6..8 19.3 / 27.5, 256 24.0 / 28.9, 1024 25.5 / 28.0.
+constexpr int kHandOver = 2048;
+
 int batch_enqueue(nq_batch* b, int use_graph) {
   nq_handle* h = b->h;
   const int nj = (int)b->jobs.size();
@@ -850,8 +854,13 @@ int batch_enqueue(nq_batch* b, int use_graph) {
     L.m = b->ms; L.cursor = (unsigned long long*)(c + (size_t)nj * 8);
     L.job_totals = (unsigned long long*)c; L.err = (unsigned int*)(c + (size_t)nj * 8 + 8);
     L.maxt = b->maxt; L.block = b->block; L.grid = b->grid; L.big = b->big;
+    const bool hand = b->ms > 0 && nj <= kHandOver;
+    if (hand) {
+      L.ctl = (const uint32_t*)c; L.ctl_words = (unsigned)(cb / 8); L.host_ctl = (uint32_t*)b->h_out;
+      L.blocks_done = L.err + 1;
+    }
     e = launch_dfs(L, st);
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess || hand) return e;
     return cudaMemcpyAsync(b->h_out, c, cb, cudaMemcpyDeviceToHost, st);
   };
   NQ_CUDA(h, cudaSetDevice(h->device));
@@ -1314,7 +1323,7 @@ int nq_count_completions(nq_handle* h, int N, int k, const int* rows, const int*
     for (uint64_t f = 1; f < p.target; f *= (uint64_t)N) depth++;
     L.maxt = std::max(1, (int)p.T - depth); L.block = h->block; L.grid = h->grid;
     L.big = counts_need_u64(N, p.target);      // a queue below the target stands at its terminal depth
-    L.ctl = (const uint32_t*)b.ctl; L.ctl_words = QueryCtl::kWords * 2; L.host_ctl = (uint32_t*)h->h_query;
+    L.ctl = (const uint32_t*)b.ctl; L.ctl_words = QueryCtl::kWords; L.host_ctl = (uint32_t*)h->h_query;
     L.blocks_done = (unsigned int*)(b.ctl + QueryCtl::kErr) + 1;
     L.chained = true;
     NQ_CUDA(h, launch_dfs(L, st));

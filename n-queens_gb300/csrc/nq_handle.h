@@ -38,7 +38,8 @@ struct DevBuf {
 };
 
 // Control block of a batch run: totals (u64 per job), then the queue cursor
-// (u64) and the error word (u32) at totals_bytes + 0 / + 8.
+// (u64), the error word (u32) and the blocks that have ended (u32) at
+// totals_bytes + 0 / + 8 / + 12.
 struct Ctrl {
   static size_t bytes(int njobs) { return (size_t)njobs * 8 + 16; }
 };

@@ -68,7 +68,7 @@ struct DfsLaunch {
   bool big = false;                     // u64 per-task counters (some task has N >= 24)
   int block = 128;
   int grid = 0;                         // 0: one wave of resident blocks
-  // Optional: the last block to end copies ctl_words u32 of the control block to pinned host memory (blocks_done:
+  // Optional: the last block to end copies ctl_words u64 of the control block to pinned host memory (blocks_done:
   // zeroed before), so the caller only waits for the stream.
   const uint32_t* ctl = nullptr;
   unsigned ctl_words = 0;
@@ -217,10 +217,10 @@ __device__ __forceinline__ unsigned long long device_ns() {
   return t;
 }
 
-// Called by all threads of all blocks as their last step: the last block to end copies `words` u32 of the control
+// Called by all threads of all blocks as their last step: the last block to end copies `words` u64 of the control
 // block `ctl` to pinned host memory (`done`: zeroed before).  A copy queued behind the kernel instead takes the
 // copy engine's start and end: completion query of N=10 / N=17 36 / 129 us with one, 31.7 / 106 so.  `end`:
-// optional, a word pair of ctl that receives the device's clock.
+// optional, a word of ctl that receives the device's clock.
 __device__ __forceinline__ void hand_over(const uint32_t* ctl, unsigned words, unsigned* done, uint32_t* host,
                                           unsigned long long* end = nullptr) {
   __threadfence();
@@ -234,8 +234,17 @@ __device__ __forceinline__ void hand_over(const uint32_t* ctl, unsigned words, u
   }
   if (__shfl_sync(0xFFFFFFFFu, n, 0) != gridDim.x - 1u) return;
   __syncwarp();
-  for (unsigned w = threadIdx.x; w < words; w += 32u)
-    ((volatile uint32_t*)host)[w] = ((const volatile uint32_t*)ctl)[w];
+  const volatile unsigned long long* from = (const volatile unsigned long long*)ctl;
+  volatile unsigned long long* to = (volatile unsigned long long*)host;
+  constexpr unsigned kAtOnce = 8;         // loads in flight a lane: a batch's block (258 of them) copied one by one took 15 us
+  for (unsigned w0 = threadIdx.x; w0 < words; w0 += 32u * kAtOnce) {
+    unsigned long long v[kAtOnce];
+#pragma unroll
+    for (unsigned k = 0; k < kAtOnce; k++) v[k] = w0 + 32u * k < words ? from[w0 + 32u * k] : 0ull;
+#pragma unroll
+    for (unsigned k = 0; k < kAtOnce; k++)
+      if (w0 + 32u * k < words) to[w0 + 32u * k] = v[k];
+  }
 }
 
 // position of the r-th set bit of m (r < popc(m))

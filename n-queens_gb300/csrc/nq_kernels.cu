@@ -40,11 +40,15 @@ constexpr unsigned FULL = 0xFFFFFFFFu;
 // DFS steps each lane takes between two checks for finished lanes (flush +
 // refill), unrolled.  A lane that runs dry mid-round idles for the rest of the
 // round; a check costs two ballots, so checking less often wins until that
-// idle time dominates.  At most 31: the sentinel frame holds 31 candidates.
+// idle time dominates.  At most 30: the sentinel frame holds 31 candidates.
 // N=19 / N=17, ms: 30 steps unrolled 30 75.1 / 1.92, 15 76.1 / 1.93, 10 76.5 /
 // 1.91, 6 77.4 / 1.97; 20 steps 76.7 / 2.01; 15 steps 75.6 / 1.99.
 constexpr int kStepsPerCheck = 30;
-constexpr int kStepUnroll = kStepsPerCheck;
+// Searches of at most kShortDepth rows (2 to 40 steps an item) check twice as often, so lanes wait less for their
+// next item: us of 256 jobs of N=10..13 replayed 262 -> 258, of the counts N=6..13 300 -> 292.  At 7 rows 64 jobs of
+// N=12..15 took 1241 us for 1213; 10 steps a check 1270, 6 steps 1311.  A kernel of its own: a branch between the
+// two loops in one kernel took N=19 from 63.4 to 63.9 ms.
+constexpr int kShortDepth = 6, kShortSteps = 15;
 
 // A warp takes 32 queue items at a time (one atomic and one coalesced load round for the 32), less towards
 // the end of the queue: 1/8 of its even share of what is left, at least 8, so the warps end together.
@@ -515,10 +519,10 @@ __device__ __forceinline__ uint2 lds_word(uint32_t a, uint2) {
 
 // The sentinel frame under a lane's stack feeds a lane that has run out of work: its word is the count
 // word, so each of its 31 candidates dies and is counted, and a check takes the used ones off the lane's
-// count.  kStepsPerCheck <= 31 steps therefore never pop below it, and the step tests neither the stack's
+// count.  kStepsPerCheck <= 30 steps therefore never pop below it, and the step tests neither the stack's
 // depth nor the lane's activity.
 constexpr uint32_t kSentinelAvail = 0xFFFFFFFEu;   // bits 1..31: ld + bit stays odd (ld = 1), so bit 31 of nld is set
-static_assert(kStepsPerCheck <= 31 && kStepsPerCheck % kStepUnroll == 0, "the sentinel holds 31 candidates");
+static_assert(kStepsPerCheck <= 30, "the sentinel holds 31 candidates, and one has to be left at a check");
 
 enum WordForm { kRaInRd, kRaInWords, kWideWords };   // compact words without and with RA, wide words
 
@@ -617,7 +621,7 @@ __device__ __forceinline__ uint4 lds_frame(uint32_t a) {
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(f.x), "=r"(f.y), "=r"(f.z), "=r"(f.w) : "r"(a) : "memory");
   return f;
 }
-template <WordForm FORM, int BLOCK, bool BIG>
+template <WordForm FORM, int BLOCK, bool BIG, int STEPS>
 __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
   constexpr bool WIDE = FORM == kWideWords;
   using W = typename WordT<WIDE>::type;
@@ -793,8 +797,8 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
       if (__all_sync(FULL, exhausted && !have)) break;
       asm volatile("" ::: "memory");   // refill stores to the schedule before the steps' loads
     }
-#pragma unroll kStepUnroll
-    for (int s = 0; s < kStepsPerCheck; ++s) L.template step<BLOCK>();
+#pragma unroll
+    for (int s = 0; s < STEPS; ++s) L.template step<BLOCK>();
   }
 
   const uint32_t j0 = __shfl_sync(FULL, acc_job, 0);
@@ -823,17 +827,17 @@ cudaError_t allow_max_dynamic_smem(K kernel) {
   return e;
 }
 
-template <WordForm FORM, int BLOCK, bool BIG>
+template <WordForm FORM, int BLOCK, bool BIG, int STEPS = kStepsPerCheck>
 static cudaError_t launch_dfs_t(const DfsLaunch& L, cudaStream_t st) {
   const size_t smem = dfs_smem_bytes(FORM == kWideWords, BLOCK, L.maxt);
-  cudaError_t e = allow_max_dynamic_smem(dfs_kernel<FORM, BLOCK, BIG>);
+  cudaError_t e = allow_max_dynamic_smem(dfs_kernel<FORM, BLOCK, BIG, STEPS>);
   if (e != cudaSuccess) return e;
   int grid = L.grid;
   if (grid <= 0) {
     int dev = 0, sms = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, dfs_kernel<FORM, BLOCK, BIG>, BLOCK, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, dfs_kernel<FORM, BLOCK, BIG, STEPS>, BLOCK, smem);
     if (e != cudaSuccess) return e;
     if (per <= 0) return cudaErrorInvalidConfiguration;
     grid = sms * per;
@@ -847,8 +851,8 @@ static cudaError_t launch_dfs_t(const DfsLaunch& L, cudaStream_t st) {
   a.m = L.m; a.m_dev = L.m_dev; a.qcap = L.qcap; a.order = L.order; a.cursor = L.cursor; a.job_totals = L.job_totals; a.job_base = L.job_base;
   a.per_task = L.per_task; a.err = L.err; a.maxt = L.maxt;
   a.ctl = L.ctl; a.ctl_words = L.ctl_words; a.blocks_done = L.blocks_done; a.host_ctl = L.host_ctl; a.stamp = L.stamp;
-  if (L.chained) return launch_after(dfs_kernel<FORM, BLOCK, BIG>, (unsigned)grid, BLOCK, smem, st, a);
-  dfs_kernel<FORM, BLOCK, BIG><<<grid, BLOCK, smem, st>>>(a);
+  if (L.chained) return launch_after(dfs_kernel<FORM, BLOCK, BIG, STEPS>, (unsigned)grid, BLOCK, smem, st, a);
+  dfs_kernel<FORM, BLOCK, BIG, STEPS><<<grid, BLOCK, smem, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -856,7 +860,9 @@ static cudaError_t launch_dfs_t(const DfsLaunch& L, cudaStream_t st) {
 cudaError_t launch_dfs(const DfsLaunch& L, cudaStream_t st) {
   if (L.m <= 0 && !L.m_dev) return cudaSuccess;
   if (L.maxt < 1 || L.maxt > kMaxDepth) return cudaErrorInvalidValue;
-#define NQ_DFS_FORM(B, FORM) return L.big ? launch_dfs_t<FORM, B, true>(L, st) : launch_dfs_t<FORM, B, false>(L, st)
+#define NQ_DFS_FORM(B, FORM)                                                                \
+  return L.big ? launch_dfs_t<FORM, B, true>(L, st)                                         \
+       : L.maxt <= kShortDepth ? launch_dfs_t<FORM, B, false, kShortSteps>(L, st) : launch_dfs_t<FORM, B, false>(L, st)
 #define NQ_DFS_BLOCK(B)                                   \
   if (L.tasks.wide) NQ_DFS_FORM(B, kWideWords);           \
   if (L.tasks.ra_words) NQ_DFS_FORM(B, kRaInWords);       \
@@ -875,9 +881,9 @@ template <bool WIDE, int BLOCK>
 static int occ(int maxt) {
   constexpr WordForm FORM = WIDE ? kWideWords : kRaInWords;      // shared memory bounds it, alike for both compact forms
   const size_t smem = dfs_smem_bytes(WIDE, BLOCK, maxt);
-  if (allow_max_dynamic_smem(dfs_kernel<FORM, BLOCK, false>) != cudaSuccess) return 0;
+  if (allow_max_dynamic_smem(dfs_kernel<FORM, BLOCK, false, kStepsPerCheck>) != cudaSuccess) return 0;
   int per = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, dfs_kernel<FORM, BLOCK, false>, BLOCK, smem) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, dfs_kernel<FORM, BLOCK, false, kStepsPerCheck>, BLOCK, smem) != cudaSuccess)
     return 0;
   return per;
 }

@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(BLOCK) unique_kernel(const UArgs a) {
     if (w4) atomicAdd(&a.ctl->c4, w4);
     if (c8) atomicAdd(&a.ctl->c8, c8);
   }
-  hand_over((const uint32_t*)a.ctl, sizeof(UCtl) / 4, &a.ctl->done, a.host);
+  hand_over((const uint32_t*)a.ctl, sizeof(UCtl) / 8, &a.ctl->done, a.host);
 }
 
 // ---------------------------------------------------------------------------

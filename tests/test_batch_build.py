@@ -52,3 +52,20 @@ def test_batch_rejects_a_preset_too_deep():
             assert e.value.status == status
     finally:
         eng.close()
+
+
+@pytest.mark.parametrize("n", [1, 15, 254, 255, 2048, 2049])
+def test_totals_of_many_jobs(oracle_mod, n):
+    """Numbers of jobs on both sides of the read-back's rules: every total, run after run."""
+    import nqueens
+    eng = nqueens.Engine(0, auto_tune=False)
+    sizes = [6 + (i * 7 + i // 5) % 4 for i in range(n)]
+    try:
+        b = eng.batch([nqueens.CountJob(N) for N in sizes])
+        try:
+            for use_graph in (False, True, True):
+                assert list(b.run(use_graph=use_graph)) == [oracle_mod.EXPECTED_TOTAL[N] for N in sizes]
+        finally:
+            b.close()
+    finally:
+        eng.close()
