@@ -278,6 +278,7 @@ void nq_destroy(nq_handle* h) {
   for (auto& e : h->ev) if (e) cudaEventDestroy(e);
   if (h->done) cudaEventDestroy(h->done);
   h->qbuf.release();
+  if (h->pool) cudaMemPoolDestroy(h->pool);
   if (h->h_query) cudaFreeHost(h->h_query);
   if (h->q_stream) cudaStreamDestroy(h->q_stream);
   if (h->stream) cudaStreamDestroy(h->stream);
@@ -1027,11 +1028,13 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
   DevBuf tab, state, rec, gen, frames, tmp, off;
   int status = NQ_OK;
   do {
-    if ((e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking)) != cudaSuccess ||
+    if ((e = h->ensure_pool()) != cudaSuccess ||
+        (e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming)) != cudaSuccess) break;
     st = b->stream;
-    for (DevBuf* d : {&b->info, &b->sched, &b->ctrl, &b->sroot, &b->sinfo, &tab, &state, &rec, &gen, &frames, &tmp, &off})
-      d->ordered = st;
+    for (DevBuf* d : {&b->info, &b->sched, &b->ctrl, &b->sroot, &b->sinfo, &tab, &state, &rec, &gen, &frames, &tmp, &off}) {
+      d->ordered = st; d->pool = h->pool;
+    }
     b->h_out = (uint64_t*)h->pin_get(std::max(cb, state_bytes));
     b->stage = (unsigned char*)h->pin_get(tab_bytes);
     if (!b->h_out || !b->stage) { e = cudaErrorMemoryAllocation; break; }

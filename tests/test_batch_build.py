@@ -69,3 +69,38 @@ def test_totals_of_many_jobs(oracle_mod, n):
             b.close()
     finally:
         eng.close()
+
+
+def test_batches_from_two_threads_give_their_memory_back(oracle_mod):
+    """Batches of all sizes built, run and released by two threads at once on one handle, one of them larger than what
+    the handle keeps between batches: right counts, and the device's memory is free again after the handle."""
+    import threading
+    import nqueens
+    torch = pytest.importorskip("torch")
+    wrong = []
+
+    def work(eng, sizes):
+        for N, n in sizes:
+            b = eng.batch([nqueens.CountJob(N)] * n)
+            try:
+                if list(b.run(use_graph=False)) != [oracle_mod.EXPECTED_TOTAL[N]] * n:
+                    wrong.append((N, n))
+            finally:
+                b.close()
+
+    def cycle():
+        eng = nqueens.Engine(0, auto_tune=False)
+        try:
+            threads = [threading.Thread(target=work, args=(eng, s))
+                       for s in ([(8, 3), (13, 40), (15, 24), (9, 100)], [(12, 64), (10, 2), (14, 20), (11, 9)])]
+            for t in threads:
+                t.start()
+            for t in threads:
+                t.join()
+        finally:
+            eng.close()
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    first = cycle()
+    assert cycle() >= first - (8 << 20) and not wrong
