@@ -336,7 +336,7 @@ def ours_arm(args):
     at_profile = N == 19                     # the committed ncu capture is of the N=19 launch
     traffic = read_traffic() if at_profile else None
     # Executed instructions against the issue limit (one warp instruction per clock per SM sub-partition):
-    # the step is issue/math-pipe bound, so this is the fraction that measures the kernel.
+    # the rest of the issue slots wait on shared memory, whose data pipe bounds the step (shared_pipe_pct_of_peak_ncu).
     warp_instr = read_profile_figure("warp_instructions_per_launch") if at_profile else None
     sm_count = torch.cuda.get_device_properties(dev).multi_processor_count
     issue = None
@@ -366,10 +366,11 @@ def ours_arm(args):
                      "ops_per_node": OPS_PER_NODE, "issue": issue,
                      "alu_pipe_pct_of_peak_ncu": read_profile_figure("alu_pipe_pct_of_peak") if at_profile else None,
                      "issue_active_pct_ncu": read_profile_figure("issue_active_pct") if at_profile else None,
+                     "shared_pipe_pct_of_peak_ncu": read_profile_figure("shared_pipe_pct_of_peak") if at_profile else None,
                      "hbm_frac": (m * 16 + m * 16 + m * 8 + m * 4 * 15) / (dfs_avg * 1e-3) / (
                          (peaks or {}).get("hbm_gbs", 6800.0) * 1e9)},
         "clocks": clk,
-        "gpu_launches": (4 if split_depth > 0 else 2) * args.steps,
+        "gpu_launches": 2 * args.steps,          # prepare + split, and the DFS
     }
     if rank == 0 and not args.no_cpu:
         cb = run_cpu(N, args.cpu_seconds)

@@ -90,11 +90,12 @@ int nq_exec_solutions(nq_handle *h, int N, const nq_record *records, int64_t m, 
 
 /* Same on device-resident buffers on `stream` (NULL: the handle's stream).
  * `start_min` is the smallest start row (startijkl >> 20) over the records,
- * or -1 to use the bound 1.  d_total (device, 1 x u64) is overwritten.  The
- * call waits once for a 40-byte read-back (the subtask count and the deepest
- * schedule, which size the DFS queue and stacks) before launching the DFS,
- * then returns.  Call nq_sync() to wait for the result and collect the
- * status. */
+ * or -1 to use the bound 1.  d_total (device, 1 x u64) is overwritten.  Long
+ * lists (from 16,385 records, 65,537 where at most 12 rows follow start_min)
+ * wait once for a 64-byte read-back (the subtask count and the deepest
+ * schedule, which size the DFS queue and stacks) before launching the DFS;
+ * shorter ones are only queued.  Call nq_sync() to wait for the result and
+ * collect the status. */
 int nq_exec_solutions_device(nq_handle *h, int N, const nq_record *d_records, int64_t m, int start_min,
                              uint64_t *d_solutions, uint64_t *d_total, void *stream);
 /* Waits for the handle's last nq_exec_solutions_device call (an event
@@ -147,11 +148,11 @@ int nq_tune(nq_handle *h, int N, int repeats, int *best_block, int *best_split, 
 /* Whole-board total for N, the loop body of the reference's main()
  * (356Py_savesp_narrow.py:6036-6046): brute force on the GPU for N <= 5
  * (the reference's _bit_total, :5755-5767), the constellation path above.
- * preset <= 0 selects nq_preset_for(N).  The records are generated and
- * counted in chunks (the reference's streamed generation,
- * gen_constellations_stream_to_bin, :2988-3084), so host memory stays bounded
- * at the largest boards: the next chunk is generated while the previous one
- * counts on the GPU. */
+ * preset <= 0 selects nq_preset_for(N).  The records are generated on the
+ * device (presets 4..8; deeper ones on the host while the previous chunk
+ * counts) and counted in chunks (the reference's streamed generation,
+ * gen_constellations_stream_to_bin, :2988-3084), so memory stays bounded at
+ * the largest boards. */
 int nq_count(nq_handle *h, int N, int preset, uint64_t *total);
 /* The canonical start constellations of N (6 <= N <= 27; packed
  * i<<15 | j<<10 | k<<5 | l, ascending), the first stage of
@@ -176,8 +177,8 @@ int64_t nq_gen_constellations_starts(int N, int preset, int64_t first, int64_t c
  * 356Py_savesp_narrow.py:2418-2435, with a progress TSV, :3330-3338).  A range
  * outside the list is NQ_EINVAL; an empty range counts 0. */
 int nq_count_starts(nq_handle *h, int N, int preset, int64_t first, int64_t count, uint64_t *total);
-/* Records per chunk of nq_count (0: the default, 8 Mi records, about 32 MB of
- * host records per chunk; one chunk up to N=21). */
+/* Records per chunk of nq_count, generated on the host chunk by chunk (0: the
+ * default, chunks of at most 8 Mi records generated on the device). */
 int nq_set_chunk_records(nq_handle *h, int64_t records);
 /* Chunks and records of the handle's last nq_count. */
 int nq_last_count_info(const nq_handle *h, int64_t *chunks, int64_t *records);
@@ -246,8 +247,8 @@ int nq_batch_resident_blocks(const nq_batch *b, int *blocks);
  * before building it.  No counterpart in the reference (it runs one N per
  * process).  Returns the bytes or a negative status. */
 int64_t nq_job_device_bytes(const nq_job *job, int sms, int split_depth);
-/* Device bytes the batch holds, and host-to-device bytes its build copied
- * (records of count jobs, tasks of completion jobs). */
+/* Device bytes the batch holds, and host-to-device bytes its build copied (job
+ * tables and queries; records only where the device does not generate them). */
 int64_t nq_batch_device_bytes(const nq_batch *b);
 int64_t nq_batch_h2d_bytes(const nq_batch *b);
 /* All jobs in one persistent launch (use_graph: replay a captured CUDA graph). */

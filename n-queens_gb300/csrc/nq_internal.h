@@ -19,14 +19,15 @@ constexpr uint32_t DERR_FORMAT = 16u;    // a schedule op does not fit the compa
 // start row), which sets a task's work (about 7x per row).  Lanes of a warp share their work at the end of
 // the queue, so splitting only has to even out the warps and give a short list more items than lanes:
 // us of a whole call on GB300 at D = 0 / 1 / 2 / 3, m tasks:
-//   8 rows (N=12):    m=4300   60 / 59 / 60 / 70
-//   9 rows (N=13):    m=7731   75 / 72 / 68 / 79
-//   10 rows (N=14):   m=1000   73 / 65 / 61 / 76       m=13233 100 / 87 / 86 / 129
-//   12 rows (N=16):   m=4000  178 / 149 / 138 / 175    m=33046 593 / 441 / 381 / 471
-//   13 rows (N=18):   m=16000 898 / 761 / 493 / 550    m=200000 5761 / 4056 / 4326 / 5343
-//   14 rows (N=19):   m=100   915 / 247 / 144 / 180    m=4000 1747 / 1115 / 789 / 658
-//                     m=50000 10.5 / 5.4 / 4.7 / 5.2 ms   m=897071 79.1 / 74.3 / 78.8 ms
-//   15 rows (N=20):   m=1000  4.9 / 2.1 / 1.7 / 1.0 ms    m=16000 21.8 / 14.6 / 8.4 / 7.9 ms
+//   8 rows (N=12):    m=4300   48 / 46 / 46 / 52
+//   9 rows (N=13):    m=7731   62 / 54 / 55 / 62
+//   10 rows (N=14):   m=1000   57 / 47 / 46 / 62       m=13233 80 / 67 / 70 / 127
+//   12 rows (N=16):   m=4000  161 / 126 / 113 / 145    m=33046 601 / 343 / 322 / 421
+//   13 rows (N=17):   m=49207 3326 / 1570 / 1450 / 1655
+//   13 rows (N=18):   m=16000 903 / 696 / 420 / 475    m=200000 4864 / 3522 / 3661 / 4390
+//   14 rows (N=19):   m=100   749 / 192 / 122 / 149    m=4000 1544 / 1161 / 703 / 543
+//                     m=50000 9.9 / 4.7 / 4.0 / 4.4 ms    m=897071 67.2 / 64.4 / 67.4 ms
+//   15 rows (N=20):   m=1000  4.1 / 1.7 / 1.5 / 0.75 ms   m=16000 20.6 / 12.4 / 7.4 / 6.7 ms
 // Each level makes about 7 times the items (measured: 6.2x at N=16 to 8x at N=20), and an item costs its
 // loading; lists of 10^5 tasks and more are balanced at D = 1.
 inline int choose_split(int64_t m, int rows) {

@@ -22,9 +22,10 @@
 //   reference's packed stack) sit in shared memory, interleaved by lane so
 //   every access is conflict-free, above a sentinel frame whose candidates
 //   all die, which a finished lane works on until the next check.
-//   Bound by the issue slots and the integer pipes: N=18 takes 35.7 warp
-//   instructions a step of 32 lanes (16.7 on the ALU pipe, 14.0 on FMA, 8.5
-//   shared-memory wavefronts) at 77 % issue.
+//   Bound by shared-memory bandwidth: N=19 takes 8.85 wavefronts a step of
+//   32 lanes (a 16-byte frame out, one in, a word), 93 % of that pipe's rate,
+//   and 27.0 warp instructions (11.2 on the ALU pipe, 11.4 on FMA) at 72 %
+//   issue.
 //   Counts are summed per lane in u64 and flushed per job with one atomicAdd
 //   per warp (shuffle tree) at exit or per task when the job id changes.
 #include <algorithm>
@@ -41,8 +42,8 @@ constexpr unsigned FULL = 0xFFFFFFFFu;
 // refill), unrolled.  A lane that runs dry mid-round idles for the rest of the
 // round; a check costs two ballots, so checking less often wins until that
 // idle time dominates.  At most 30: the sentinel frame holds 31 candidates.
-// N=19 / N=17, ms: 30 steps unrolled 30 75.1 / 1.92, 15 76.1 / 1.93, 10 76.5 /
-// 1.91, 6 77.4 / 1.97; 20 steps 76.7 / 2.01; 15 steps 75.6 / 1.99.
+// N=19 / N=17, ms: 30 steps 63.29 / 1.334 (unrolled 10 63.55 / 1.332), 20 63.90 /
+// 1.362, 16 64.22 / 1.380, 10 65.12 / 1.434.
 constexpr int kStepsPerCheck = 30;
 // Searches of at most kShortDepth rows (2 to 40 steps an item) check twice as often, so lanes wait less for their
 // next item: us of 256 jobs of N=10..13 replayed 262 -> 258, of the counts N=6..13 300 -> 292.  At 7 rows 64 jobs of
@@ -52,12 +53,13 @@ constexpr int kShortDepth = 6, kShortSteps = 15;
 
 // A warp takes 32 queue items at a time (one atomic and one coalesced load round for the 32), less towards
 // the end of the queue: 1/8 of its even share of what is left, at least 8, so the warps end together.
-// Taking the items one by one instead took 74.1 ms at N=19, 1.715 at N=17 (73.2 and 1.675 with the pool);
-// a share of 1/4 1.71 at N=17; at least 1: 0.375 ms at N=16 against 0.365, 16: 1.725 at N=17.
+// Taking the items one by one took 74.1 ms at N=19 and 1.715 at N=17 where the pool took 73.2 and 1.675.  Now
+// N=14 / 16 / 17, ms: 0.0247 / 0.261 / 1.334; a share of 1/4 0.0245 / 0.257 / 1.364 (N=19 63.66 against 63.29); at
+// least 1 0.0492 / 0.286 / 1.362, at least 16 0.0227 / 0.259 / 1.329 (N=19 63.46).
 constexpr float kChunkShare = 8.0f;
 constexpr unsigned kMinChunk = 8;
 // A frame is given to a lane without work when it is at least this many levels above the terminal depth
-// (fewer: not worth the exchange; 3 and 7 measured the same from N=16 on, 7 is 25 % slower at N=14).
+// (3 / 5 / 7: N=14 0.0244 / 0.0247 / 0.0262 ms, N=16 0.262 / 0.261 / 0.265, N=17 1.335 / 1.334 / 1.326).
 constexpr int kGiveRows = 5;
 // What a pool entry needs besides its frame, ready when it is loaded: terminal depth (5 bits), weight (2),
 // root count (1), N (5), depth of its first word (5) and what to do with it.
@@ -759,8 +761,8 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
         // The queue is empty: a lane without work takes the bottom saved frame (the largest subtree left) of
         // a busy lane of its warp, or all but one candidate of that lane's current frame.  It reads the
         // giver's schedule words in place: only loading a queue item overwrites words, and none is left.
-        // Without this the last items of a warp left 7 of 32 lanes idle at N=17 (1.92 ms, 1.715 with it),
-        // N=16 0.404 -> 0.352, N=18 10.9 -> 10.4, N=19 75.1 -> 74.1.
+        // Without this the last items of a warp leave 7 of 32 lanes idle at N=17: 1.475 ms, 1.334 with it; N=16
+        // 0.304 / 0.261, N=19 64.4 / 63.3.
         const unsigned starved = __ballot_sync(FULL, !have);
         if (starved) {
           const bool saved = L.sp != top;

@@ -60,7 +60,7 @@ class _InFlight:
 # GPU milliseconds of a whole-board count, the starting point of each server's table: measured on
 # GB300 with bench-style timing; a server replaces an entry with the run time it measures for a
 # single-request batch of that board (exponential average), so another GPU recalibrates itself.
-_COUNT_MS = {16: 0.5, 17: 2.2, 18: 13.0, 19: 86.0, 20: 670.0, 21: 5600.0}
+_COUNT_MS = {16: 0.35, 17: 1.5, 18: 8.9, 19: 64.0, 20: 513.0, 21: 4500.0}
 
 
 def estimate_ms(job, table: Optional[dict] = None) -> float:
@@ -147,8 +147,8 @@ class Server:
             raise TypeError("submit a CountJob or a CompletionJob")
         f: Future = Future()
         now = time.perf_counter()
-        # Size the request here, on the caller's thread and outside the server's lock: the first sizing of a
-        # large board generates its constellations (about a second at N=22), which must not stall the scheduler.
+        # Size the request here, on the caller's thread and outside the server's lock: the sizing of a large
+        # board generates its constellations, which must not stall the scheduler.
         try:
             nbytes = self._job_bytes(job)
         except NQError as exc:
