@@ -95,32 +95,98 @@ __device__ __forceinline__ int jasmin(int x, int N) {                // 356Py:27
   return x;
 }
 
+// Thread q's candidate of a board; true if the reference's loops insert it.
+__device__ __forceinline__ bool board_candidate(int q, int N, Quad& x) {
+  const int corners = N * N;
+  if (q < corners) {                               // a queen in the corner: (0, j, 0, l), j < l
+    x = Quad{0, q / N, 0, q % N};
+    return x.j >= 1 && x.j < N - 2 && x.l > x.j && x.l <= N - 2;
+  }
+  q -= corners;
+  x.j = q % N; q /= N;
+  x.i = q % N; q /= N;
+  x.l = q % N; x.k = q / N + 1;
+  bool take = start_candidate(x, N);
+  if (take) {
+    const int rank = start_rank(x, N);
+    const Quad r[3] = {{N - 1 - x.k, N - 1 - x.l, x.j, x.i}, {N - 1 - x.j, N - 1 - x.i, N - 1 - x.l, N - 1 - x.k},
+                       {x.l, x.k, N - 1 - x.i, N - 1 - x.j}};
+#pragma unroll
+    for (int t = 0; t < 3; t++) take = take && !(start_candidate(r[t], N) && start_rank(r[t], N) < rank);
+  }
+  return take;
+}
+
 __global__ void __launch_bounds__(128) gen_board_kernel(int N, uint4* __restrict__ out, unsigned cap, unsigned* gn) {
   chain_next();
   chain_wait();
-  int q = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-  const int corners = N * N;
   Quad x;
-  bool take;
-  if (q < corners) {                               // a queen in the corner: (0, j, 0, l), j < l
-    x = Quad{0, q / N, 0, q % N};
-    take = x.j >= 1 && x.j < N - 2 && x.l > x.j && x.l <= N - 2;
-  } else {
-    q -= corners;
-    x.j = q % N; q /= N;
-    x.i = q % N; q /= N;
-    x.l = q % N; x.k = q / N + 1;
-    take = start_candidate(x, N);
-    if (take) {
-      const int rank = start_rank(x, N);
-      const Quad r[3] = {{N - 1 - x.k, N - 1 - x.l, x.j, x.i}, {N - 1 - x.j, N - 1 - x.i, N - 1 - x.l, N - 1 - x.k},
-                         {x.l, x.k, N - 1 - x.i, N - 1 - x.j}};
-#pragma unroll
-      for (int t = 0; t < 3; t++) take = take && !(start_candidate(r[t], N) && start_rank(r[t], N) < rank);
-    }
-  }
+  const bool take = board_candidate((int)(blockIdx.x * blockDim.x + threadIdx.x), N, x);
   const unsigned at = take_slots(&gn[0], take ? 1u : 0u);
   if (take && at < cap) out[at] = start_state(N, jasmin((x.i << 15) + (x.j << 10) + (x.k << 5) + x.l, N));
+}
+
+// The free columns of a state's row, with the side queens' diagonals.
+__device__ __forceinline__ uint32_t free_row(const uint4 s, int N, unsigned* err) {
+  const int ijkl = (int)(s.w & 0xFFFFFu), sh = N - 1 - ((int)(s.w >> 20) & 31);
+  if (sh < 0) { atomicOr(err, DERR_SHIFT); return 0u; }  // the reference raises on a negative shift here
+  const uint32_t L = 1u << (N - 1), Lj = L >> getj(ijkl);
+  const uint32_t LD = Lj | (L >> getl(ijkl)), RD = Lj | (1u << getk(ijkl));
+  return ~(s.x | s.y | s.z | (LD >> sh) | (RD << sh)) & ((1u << N) - 1u);
+}
+__device__ __forceinline__ uint4 state_child(const uint4 s, uint32_t bit) {
+  return settle((s.x | bit) << 1, (s.y | bit) >> 1, s.z | bit, (int)((s.w >> 20) & 31u) + 1, (int)(s.w >> kQueens) + 1, s.w & 0xFFFFFu);
+}
+
+// Presets 4 and 5 in one launch: a start constellation is at most kFused queens short, and its thread writes its
+// records (of a whole board, the corner constellations, which hold a queen less, have a thread a column).  us of a
+// count of N=6 / 10 / 13 / 16 with a launch a queen 30.8 / 35.2 / 47.6 / 319, so
+// 26.5 / 31.7 / 44.2 / 315.  A third level (preset 6)
+// keeps a launch a queen: N=14 70 us and N=16 328 with three in a thread.
+constexpr int kFused = 2;
+template <int DEPTH, class F>
+__device__ __forceinline__ void each_record(const uint4 s, int N, int preset, unsigned* err, F&& f) {
+  if constexpr (DEPTH > 0) {
+    if ((int)(s.w >> kQueens) < preset) {
+      for (uint32_t fr = free_row(s, N, err); fr; fr &= fr - 1u) each_record<DEPTH - 1>(state_child(s, fr & (0u - fr)), N, preset, err, f);
+      return;
+    }
+  }
+  f(make_uint4(s.x, s.y, s.z, s.w & ((1u << kQueens) - 1u)));
+}
+__global__ void __launch_bounds__(128) gen_records_kernel(int N, int preset, unsigned n, const int* __restrict__ starts,
+                                                          uint4* __restrict__ out, unsigned cap, unsigned* count, unsigned* err) {
+  chain_next();
+  chain_wait();
+  const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
+  bool take = q < n;
+  int sc = 0, column = -1;               // column: of a corner constellation's fourth queen
+  if (starts) {
+    if (take) sc = starts[q];
+  } else {
+    const unsigned corners = (unsigned)(N * N * N);
+    column = q < corners ? (int)(q % (unsigned)N) : -1;
+    Quad x;
+    take = board_candidate(column >= 0 ? (int)(q / (unsigned)N) : (int)(q - corners) + N * N, N, x) && q < n;
+    if (take) sc = jasmin((x.i << 15) + (x.j << 10) + (x.k << 5) + x.l, N);
+  }
+  uint4 s = make_uint4(0, 0, 0, 0);
+  unsigned c = 0;
+  if (take) {
+    s = start_state(N, sc);
+    if (column >= 0) {
+      const uint32_t bit = 1u << column;
+      take = (free_row(s, N, err) & bit) != 0u;
+      if (take) s = state_child(s, bit);
+    }
+  }
+  if (take) each_record<kFused>(s, N, preset, err, [&](uint4) { c++; });
+  unsigned at = take_slots(count, c);
+  if (take)
+    each_record<kFused>(s, N, preset, err, [&](uint4 r) {
+      if (at < cap) out[at] = r;
+      at++;
+    });
 }
 
 // One queen more for every state below the preset; the others move on (last: as records).
@@ -135,21 +201,10 @@ __global__ void __launch_bounds__(128) gen_level_kernel(int N, int preset, bool 
     uint4 s = make_uint4(0, 0, 0, 0);
     uint32_t fr = 0;
     bool keep = false;
-    int row = 0, queens = 0;
-    uint32_t ijkl = 0;
     if (q < n) {
       s = in[q];
-      ijkl = s.w & 0xFFFFFu; row = (int)(s.w >> 20) & 31; queens = (int)(s.w >> kQueens);
-      keep = queens >= preset;
-      if (!keep) {
-        const int sh = N - 1 - row;
-        if (sh < 0) atomicOr(err, DERR_SHIFT);           // the reference raises on a negative shift here
-        else {
-          const uint32_t L = 1u << (N - 1), Lj = L >> getj((int)ijkl);
-          const uint32_t LD = Lj | (L >> getl((int)ijkl)), RD = Lj | (1u << getk((int)ijkl));
-          fr = ~(s.x | s.y | s.z | (LD >> sh) | (RD << sh)) & ((1u << N) - 1u);
-        }
-      }
+      keep = (int)(s.w >> kQueens) >= preset;
+      if (!keep) fr = free_row(s, N, err);
     }
     unsigned at = take_slots(&gn[level + 1], keep ? 1u : (unsigned)__popc(fr));
     const uint32_t mask = last ? (1u << kQueens) - 1u : ~0u;
@@ -159,7 +214,7 @@ __global__ void __launch_bounds__(128) gen_level_kernel(int N, int preset, bool 
       while (fr) {
         const uint32_t bit = fr & (0u - fr);
         fr ^= bit;
-        uint4 c = settle((s.x | bit) << 1, (s.y | bit) >> 1, s.z | bit, row + 1, queens + 1, ijkl);
+        uint4 c = state_child(s, bit);
         c.w &= mask;
         if (at < cap) out[at] = c;
         at++;
@@ -307,13 +362,17 @@ cudaError_t launch_generate(int N, int preset, unsigned n_starts, const int* sta
   const int levels = gen_levels(preset);
   uint4* buf[2] = {buf0, buf1};
   const unsigned full = 8u * (unsigned)sms;
+  if (starts && n_starts == 0) return cudaSuccess;
+  const unsigned board = (unsigned)(N * N * (1 + ((N + 1) / 2 - 1) * N));      // a board's candidates
+  if (levels <= kFused) {
+    const unsigned n = starts ? n_starts : board + (unsigned)(N * N * (N - 1));      // corner ones: a thread a column
+    return launch_after(gen_records_kernel, (n + 127) / 128, 128, 0, st, N, preset, n, starts, buf[levels & 1], cap, gn + levels, err);
+  }
   if (starts) {
-    if (n_starts == 0) return cudaSuccess;
     const cudaError_t e = launch_after(gen_start_kernel, (n_starts + 127) / 128, 128, 0, st, N, n_starts, starts, buf[0], gn);
     if (e != cudaSuccess) return e;
   } else {
-    const unsigned n = (unsigned)(N * N * (1 + ((N + 1) / 2 - 1) * N));
-    const cudaError_t e = launch_after(gen_board_kernel, (n + 127) / 128, 128, 0, st, N, buf[0], cap, gn);
+    const cudaError_t e = launch_after(gen_board_kernel, (board + 127) / 128, 128, 0, st, N, buf[0], cap, gn);
     if (e != cudaSuccess) return e;
   }
   for (int l = 0; l < levels; l++) {
