@@ -176,17 +176,20 @@ int read_ctrl(nq_handle* h, cudaStream_t st, uint64_t* total) {
   return NQ_OK;
 }
 
-// Queue of a completion query: one block expands it to kQueryTarget frames and more, then the whole GPU by
-// another one to three levels where the rows left make the frames large.  us of a query (mean of six), levels
-// over the GPU: 10 rows (N=12, two queens) 0 / 1 level 36 / 42; 13 rows (N=14, one) 1 / 2 60 / 53; 14 rows (N=15,
-// one) 1 / 2 / 3 88 / 80 / 98; 15 rows (N=17, two) 143 / 122 / 129; 16 and more, 2 / 3: N=19 two queens 2118 / 1630,
-// N=20 three 1110 / 965.  A target of 1024 / 2048 / 4096 frames: N=19 three queens 366 / 256 / 257, N=13 one 44 /
-// 45 / 52.
+// Queue of a completion query: one block expands it to a target of frames and more, then the whole GPU by another
+// one to three levels where the rows left make the frames large.  One block writes its 2,000 to 20,000 frames no
+// faster than the whole GPU writes ten times as many, so it stops early where three levels are enough for the lanes.
+// us of a query (mean of six), target 2048 and levels 0 / 1 / 2 / 3 from 0 / 11 / 13 / 16 rows against target 512 and
+// 0 / 10 / 11 / 13 rows: N=12 two queens (10 rows) 35 / 35, N=14 one (13) 52 / 51, N=15 one 80 / 75, N=16 two 66 / 62,
+// N=17 two (15) 122 / 120, N=18 four 54 / 51; with 16 rows and more 2048 stays: N=19 three 250 / 258, N=20 three 965 /
+// 985.  Two levels there took 2118 us at N=19 with two queens (three 1630), one level
+// 42 us at N=12 with two queens where none took 36 (from the target of 2048).
 constexpr unsigned kQueryCap = 65536;
-constexpr unsigned kQueryTarget = 2048;
+constexpr unsigned kQueryTarget = 2048;      // ... and of each query of a batch
+unsigned query_target(int rows) { return rows >= 16 ? kQueryTarget : 512u; }
 constexpr unsigned kQueryCap2 = 4 << 20;     // queue after two levels (never reached: 7 children a frame on average)
 constexpr unsigned kQueryCap3 = 5 << 20;     // ... after three (0.5 to 4.5 10^6 measured for N=18..25; some of N=27 are longer)
-int query_levels(int rows) { return rows >= 16 ? 3 : rows >= 13 ? 2 : rows >= 11 ? 1 : 0; }
+int query_levels(int rows) { return rows >= 13 ? 3 : rows >= 11 ? 2 : rows >= 10 ? 1 : 0; }
 // A batch's queries share the lanes with its other jobs, so the same need not be cut as fine.
 int batch_query_levels(int rows) { return rows >= 15 ? 2 : rows >= 12 ? 1 : 0; }
 
@@ -1302,7 +1305,7 @@ int nq_count_completions(nq_handle* h, int N, int k, const int* rows, const int*
   if (!h->q_stream) NQ_CUDA(h, cudaStreamCreateWithFlags(&h->q_stream, cudaStreamNonBlocking));
   if (!h->h_query) NQ_CUDA(h, cudaMallocHost((void**)&h->h_query, QueryCtl::kWords * 8));
   cudaStream_t st = h->q_stream;
-  p.target = std::min(kQueryTarget, kQueryCap / (unsigned)N);
+  p.target = std::min(query_target((int)p.T + 2), kQueryCap / (unsigned)N);
   for (int levels = query_levels((int)p.T + 2);; levels--) {      // a level less where the queue did not fit
     QueryBuffers b{};
     b.cap[0] = kQueryCap; b.cap[1] = kQueryCap * (unsigned)N; b.cap[2] = kQueryCap2; b.cap[3] = kQueryCap3;
