@@ -447,6 +447,10 @@ int nq_exec_solutions_device(nq_handle* h, int N, const nq_record* d_records, in
     NQ_CUDA(h, cudaMemsetAsync(d_total, 0, 8, st));
     return NQ_OK;
   }
+  // A captured call would have no run for nq_sync to wait for, and long lists synchronise: none is captured.
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  NQ_CUDA(h, cudaStreamIsCapturing(st, &cap));
+  if (cap != cudaStreamCaptureStatusNone) return h->cuda_fail(cudaErrorStreamCaptureUnsupported, "exec_solutions_device");
   if (int s = run_records(h, N, (const uint4*)d_records, m, start_min, (unsigned long long*)d_solutions, st)) return s;
   NQ_CUDA(h, cudaMemcpyAsync(d_total, h->ctrl.p, 8, cudaMemcpyDeviceToDevice, st));
   NQ_CUDA(h, cudaEventRecord(h->done, st));

@@ -47,3 +47,27 @@ def test_calls_of_every_kind_in_turn(oracle_mod):
             assert eng.exec_records(12, r)[0] == total[12]
     finally:
         eng.close()
+
+
+def test_a_capturing_stream_is_refused(oracle_mod):
+    """A call on a stream under capture fails with a status, short lists included, and the handle goes on."""
+    import nqueens
+    import torch
+    r = nqueens.gen_records(10)
+    start = int((r["startijkl"] >> 20).min())
+    d_rec = torch.from_numpy(r.view(np.int32).copy()).cuda()
+    d_total = torch.zeros(1, dtype=torch.int64, device="cuda")
+    side = torch.cuda.Stream()
+    eng = nqueens.Engine(0, auto_tune=False)
+    try:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            with pytest.raises(nqueens.NQError) as e:
+                eng.exec_device(10, d_rec.data_ptr(), len(r), start, d_total.data_ptr(), 0, side.cuda_stream)
+            d_total.add_(1)
+        assert e.value.status == -4
+        eng.exec_device(10, d_rec.data_ptr(), len(r), start, d_total.data_ptr(), 0, side.cuda_stream)
+        eng.sync()
+        assert int(d_total.item()) == oracle_mod.EXPECTED_TOTAL[10]
+    finally:
+        eng.close()
