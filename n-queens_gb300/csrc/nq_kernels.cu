@@ -55,8 +55,10 @@ constexpr int kShortDepth = 6, kShortSteps = 15;
 // the end of the queue: 1/8 of its even share of what is left, at least 8, so the warps end together.
 // Taking the items one by one took 74.1 ms at N=19 and 1.715 at N=17 where the pool took 73.2 and 1.675.  Now
 // N=14 / 16 / 17, ms: 0.0247 / 0.261 / 1.334; a share of 1/4 0.0245 / 0.257 / 1.364 (N=19 63.66 against 63.29); at
-// least 1 0.0492 / 0.286 / 1.362, at least 16 0.0227 / 0.259 / 1.329 (N=19 63.46).
-constexpr float kChunkShare = 8.0f;
+// least 1 0.0492 / 0.286 / 1.362, at least 16 0.0227 / 0.259 / 1.340 (N=19 63.46).  Short searches (kShortDepth) take
+// the whole even share, their items are small enough: 256 jobs of N=9..12, share 1/8 / 1/4 / 1/2 / 1: 66.7 / 61.5 / 56.2
+// / 54.6 us, of N=10..14 784 / 778 / 780 / 770; 32 throughout 55.8 and 759, but 64 jobs of N=9..12 37.0 for 33.6.
+constexpr float kChunkShare = 8.0f, kShortShare = 1.0f;
 constexpr unsigned kMinChunk = 8;
 // A frame is given to a lane without work when it is at least this many levels above the terminal depth
 // (3 / 5 / 7: N=14 0.0244 / 0.0247 / 0.0262 ms, N=16 0.262 / 0.261 / 0.265, N=17 1.335 / 1.334 / 1.326).
@@ -657,7 +659,7 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
   // queue items a warp takes first: 32, or its share of a queue smaller than the grid
   const unsigned warps = gridDim.x * (BLOCK / 32);
   const unsigned chunk0 = m >= 32ull * warps ? 32u : ((unsigned)m + warps - 1u) / warps;
-  const float share = 1.0f / (kChunkShare * (float)warps);
+  const float share = 1.0f / ((STEPS == kShortSteps ? kShortShare : kChunkShare) * (float)warps);
   unsigned chunk = chunk0, pool_n = 0, pool_at = 0;
   uint4 p_root = make_uint4(0, 0, 0, 0);
   uint32_t p_task = 0, p_meta = 0, p_job = 0;
