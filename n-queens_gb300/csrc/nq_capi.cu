@@ -11,6 +11,7 @@
 #include <map>
 #include <mutex>
 #include <cstdarg>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <new>
@@ -922,6 +923,17 @@ void nq_batch_destroy(nq_batch* b) {
   delete b;
 }
 
+// A board's tasks in a batch go unsplit where the batch's counts give every lane at least a quarter of such a task:
+// splitting then only adds items (the queue's end is evened out by the other jobs and within the warps).  us of a
+// replay, split once (as any list above 10^5 tasks) / so: 64 jobs of N=12..15 1212 / 938, of N=10..14 271 / 174, 256
+// 760 / 429, 16 of N=13..16 1012 / 978.  With an eighth 4 jobs of N=13..15 173 for 125.  Up to 11 rows left: at 12
+// (N=16) an unsplit list saves 1 % in large batches, and the same job launched alone takes 550 us for 340.
+double task_nodes(int rows) { return 100.0 * std::pow(4.0, rows - 9); }   // about: N=13..16 at preset 5 100, 350, 1300, 5500
+constexpr double kLanes = 1024.0;                                          // resident an SM, about
+bool unsplit_in_batch(int rows, double work, int sms) {
+  return rows <= 11 && work >= 0.25 * task_nodes(rows) * kLanes * sms;
+}
+
 // Build, one synchronisation in all: the boards' records are generated on the device and prepared, each
 // query is expanded by one block (queries and tables are the only uploads), every
 // list's split is counted, the queue is allocated, and the jobs' items are written job after job.  Jobs of
@@ -951,6 +963,7 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
   std::vector<int> job_list(njobs, -1);
   std::map<std::pair<int, int>, uint32_t> board_list;
   uint64_t sources = 0;                          // all jobs' sources, roughly
+  double work = 0.0;                             // and the counts' search nodes
   for (int j = 0; j < njobs; j++) {
     const nq_job& J = jobs[j];
     if (J.N < 1 || J.N > kMaxN || J.k < 0 || J.k > 8) return bad(NQ_EINVAL, "bad N or k", j);
@@ -977,6 +990,7 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
       }
       job_list[j] = (int)it->second;
       sources += lists[it->second].cap / 4;      // the bound is about four times the records
+      work += (double)(lists[it->second].cap / 4) * task_nodes(lists[it->second].rows);
     } else {
       int rows[8], cols[8];
       const int k = (J.kind == NQ_JOB_COUNT) ? 0 : J.k;
@@ -1014,7 +1028,8 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
     ntask += l.query ? 1 : l.cap;
     words = std::max<uint64_t>(words, l.query ? l.T + 1 : l.rows + 1);
     const int levels = l.query ? batch_query_levels(l.rows) : choose_split((int64_t)std::max(sources, l.cap), l.rows);
-    l.D = l.N <= 12 ? 0 : h->split >= 0 ? h->split : l.query && sources > 100000 ? std::min(levels, 1) : levels;
+    const bool whole = !l.query && unsplit_in_batch(l.rows, work, h->sms);
+    l.D = l.N <= 12 ? 0 : h->split >= 0 ? h->split : whole ? 0 : l.query && sources > 100000 ? std::min(levels, 1) : levels;
   }
   for (const Board& bd : boards) {
     rec_cap = std::max(rec_cap, lists[bd.list].cap);

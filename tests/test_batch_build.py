@@ -104,3 +104,20 @@ def test_batches_from_two_threads_give_their_memory_back(oracle_mod):
 
     first = cycle()
     assert cycle() >= first - (8 << 20) and not wrong
+
+
+@pytest.mark.parametrize("sizes", [[13, 14, 15], [15] * 9 + [13], [16, 15] * 12, [14] * 40 + [16], [17, 16, 14, 13]])
+def test_unsplit_boards_in_a_batch(oracle_mod, sizes):
+    """Batches on both sides of the rule for unsplit boards, mixed with boards that are split."""
+    import nqueens
+    eng = nqueens.Engine(0, auto_tune=False)
+    try:
+        b = eng.batch([nqueens.CountJob(N) for N in sizes])
+        try:
+            want = [oracle_mod.EXPECTED_TOTAL[N] for N in sizes]
+            assert list(b.run(use_graph=False)) == want and list(b.run_plain()) == want
+            assert b.device_bytes <= sum(eng.job_device_bytes(nqueens.CountJob(N)) for N in sizes)
+        finally:
+            b.close()
+    finally:
+        eng.close()
