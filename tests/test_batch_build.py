@@ -121,3 +121,25 @@ def test_unsplit_boards_in_a_batch(oracle_mod, sizes):
             b.close()
     finally:
         eng.close()
+
+
+@pytest.mark.parametrize("n", [64, 65])
+def test_many_queries_with_counts(n):
+    """On both sides of the number of queries from which each starts from fewer frames and is split further."""
+    import random
+    import nqueens
+    rng = random.Random(7)
+    jobs = [nqueens.CountJob(N) for N in (16, 15, 16)]
+    for _ in range(n):
+        N, k = rng.randint(9, 16), rng.randint(1, 3)
+        jobs.append(nqueens.CompletionJob(N, list(zip(rng.sample(range(N), k), rng.sample(range(N), k)))))
+    eng = nqueens.Engine(0, auto_tune=False)
+    try:
+        want = [eng.count(j.N).total if isinstance(j, nqueens.CountJob) else eng.count_completions(j.N, j.queens) for j in jobs]
+        b = eng.batch(jobs)
+        try:
+            assert list(b.run(use_graph=False)) == want and list(b.run(use_graph=True)) == want
+        finally:
+            b.close()
+    finally:
+        eng.close()
