@@ -1308,9 +1308,9 @@ int nq_batch_run_plain(nq_batch* b, uint64_t* totals) {
   return NQ_OK;
 }
 
-// One launch builds the query's queue from its root frame (a parameter, so nothing is uploaded), larger
-// boards take another over the whole GPU, one counts, one read-back.  Building the tasks on the host and
-// running them as a batch of one took 340 us at N=10 and 990 us of 1.1 ms at N=17 (two queens).
+// One launch builds the query's queue from its root frame (a parameter, so nothing is uploaded), larger boards
+// take one to three more over the whole GPU, one counts and hands the count over.  Building the tasks on the host
+// and running them as a batch of one took 340 us at N=10 and 990 us of 1.1 ms at N=17 (two queens).
 int nq_count_completions(nq_handle* h, int N, int k, const int* rows, const int* cols, uint64_t* count) {
   if (!h || !count || k < 0 || k > 8 || (k > 0 && (!rows || !cols))) return h ? h->fail(NQ_EINVAL, "bad arguments") : NQ_EINVAL;
   if (N < 1 || N > kMaxN) return h->fail(NQ_EINVAL, "N=%d outside 1..27", N);

@@ -28,8 +28,7 @@ constexpr uint32_t DERR_FORMAT = 16u;    // a schedule op does not fit the compa
 //   14 rows (N=19):   m=100   749 / 192 / 122 / 149    m=4000 1544 / 1161 / 703 / 543
 //                     m=50000 9.9 / 4.7 / 4.0 / 4.4 ms    m=897071 67.2 / 64.4 / 67.4 ms
 //   15 rows (N=20):   m=1000  4.1 / 1.7 / 1.5 / 0.75 ms   m=16000 20.6 / 12.4 / 7.4 / 6.7 ms
-// Each level makes about 7 times the items (measured: 6.2x at N=16 to 8x at N=20), and an item costs its
-// loading; lists of 10^5 tasks and more are balanced at D = 1.
+// A level makes 4.5 (N=14) to 8 (N=20 and more) times the items, and an item costs its loading; lists of 10^5 tasks and more are balanced at D = 1.
 inline int choose_split(int64_t m, int rows) {
   if (rows <= 8) return 0;
   if (m > 100000) return m > 400000000 ? 0 : 1;   // ~7 subtasks a task stay within the u32 subtask queue
