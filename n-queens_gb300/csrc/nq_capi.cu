@@ -99,7 +99,7 @@ int run_records(nq_handle* h, int N, const uint4* d_rec, int64_t m, int start_mi
   P.err = (unsigned int*)(c + ctl::kErr); P.tmax = (unsigned int*)(c + ctl::kTmax);
   P.per_task = d_per_task; P.qn = (unsigned long long*)(c + ctl::kSplit); P.total = (unsigned long long*)(c + ctl::kTotal);
   // Queue capacity: a bound (each level places a queen in one of at most N - 2, N - 3, ... columns) where that
-  // is small, else 8 a level (measured: 6.2 to 8), built again if it was too small.
+  // is small, else 8 a level (measured: up to 8), built again if it was too small.
   uint64_t bound = (uint64_t)m, guess = (uint64_t)m + 1024;
   for (int d = 0; d < D; d++) { bound *= (uint64_t)(N - 2 - d); guess *= 8; }
   const bool read_back = (m > no_read_back(maxt) && !m_dev) || h->queue_order == 1 || (D > 0 && bound * sizeof(uint4) > (uint64_t)kQueueBytes);

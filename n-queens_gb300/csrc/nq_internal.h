@@ -16,7 +16,7 @@ constexpr uint32_t DERR_BADN = 8u;       // N outside 6..27 in a task
 constexpr uint32_t DERR_FORMAT = 16u;    // a schedule op does not fit the compact word's fields
 
 // Levels every task is expanded by before the DFS.  `rows`: rows left below the shallowest start (N - 2 -
-// start row), which sets a task's work (about 7x per row).  Lanes of a warp share their work at the end of
+// start row), which sets a task's work (about 4x per row).  Lanes of a warp share their work at the end of
 // the queue, so splitting only has to even out the warps and give a short list more items than lanes:
 // us of a whole call on GB300 at D = 0 / 1 / 2 / 3, m tasks:
 //   8 rows (N=12):    m=4300   48 / 46 / 46 / 52
