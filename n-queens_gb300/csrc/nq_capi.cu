@@ -830,7 +830,7 @@ struct nq_batch {
   int maxt = 1, sw = 2, grid = 0, block = 128;
   bool big = false;                        // some job's queue items may count 2^32: u64 per-lane counters
   bool wide = false;                       // 8-byte schedule words (a query with far-reaching steps); compact otherwise
-  bool ra_words = false;                   // compact words carry RA (a board too large to keep it in rd)
+  bool ra_words = false;                   // some board's compact words carry RA (too large to keep it in rd)
   std::vector<int64_t> sub_off, sub_m;     // queue range per job
   std::vector<int> job_maxt;
   std::vector<uint64_t> fixed_total;       // counts settled at build time (small tasks, full boards)
@@ -1111,12 +1111,15 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
         b->h2d_bytes += (int64_t)(l.cap * sizeof(nq_record));
       }
       ta.root = (uint4*)frames.p + ((int64_t)l.src0 - (int64_t)l.task0);      // task t's root is its list's source
+      // Each board by its own size, whatever the search's form: a board with RA in rd has none in its words, and where
+      // the step looks for it there it finds nothing.  In the words of a small board RA would meet the count flag.
+      ta.ra_words = !ra_in_rd(l.N, bd.p - 3, 0);
       if (e == cudaSuccess)
         e = launch_prepare(l.N, (int64_t)l.cap, dn, drec, ta, l.task0, derr + 1, st, (unsigned int*)(ds + o_tmax) + i, &dstate[bd.list].n);
       if (e == cudaSuccess && !packed.empty()) e = cudaStreamSynchronize(st);   // the host list goes out of scope
     }
     if (e != cudaSuccess) break;
-    ta.root = nullptr;
+    ta.root = nullptr; ta.ra_words = b->ra_words;
     if ((e = launch_batch_queries((int)nq, (const BatchQuery*)(dt + o_q), (uint4*)frames.p, (uint4*)tmp.p, dstate, ta, st)) !=
         cudaSuccess) break;
     // ---- count every list's items, read the sizes back

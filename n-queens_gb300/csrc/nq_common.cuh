@@ -55,7 +55,7 @@ constexpr int kMaxDepth = 28;    // schedule words per task (depths 0..T)
 // compact word fields
 constexpr uint32_t C_S = 0x1Fu;
 constexpr uint32_t C_FC = 1u << 28;
-NQ_HD uint32_t compact_ra_mask(int N) { return 3u << (N - 1); }   // where RA << s may sit
+NQ_HD constexpr uint32_t compact_ra_mask(int N) { return 3u << (N - 1); }   // where RA << s may sit
 // wide word fields (x)
 constexpr uint32_t W_S = 0x1Fu;
 constexpr uint32_t W_FC = 1u << 5;
@@ -344,7 +344,8 @@ constexpr uint32_t C_COUNT = 1u << 5;            // below RA's bits wherever RA 
 constexpr uint32_t W_COUNT = W_TERM;             // device words carry neither TERM nor TALL
 constexpr uint32_t kCountWord = 0xFFFFFFFFu;     // shift 31, every column of the child blocked
 // RA stands at most at bit N - 3 of a child row, at most N - 2 - start - D rows below a depth-D frame.
-NQ_HD bool ra_in_rd(int N, int start_min, int D) { return 2 * N - 5 - (start_min < 0 ? 1 : start_min) - D <= 31; }
+NQ_HD constexpr bool ra_in_rd(int N, int start_min, int D) { return 2 * N - 5 - (start_min < 0 ? 1 : start_min) - D <= 31; }
+static_assert(ra_in_rd(18, -1, 0) && !(compact_ra_mask(19) & C_COUNT), "no list whose words carry RA has it in the count flag's bit");
 NQ_HD uint32_t device_compact(Op o, bool with_ra) {
   if (!with_ra) o.ra = 0;
   return pack_compact(o) ^ C_NOLOOK;
