@@ -202,6 +202,12 @@ int nq_count_completions(nq_handle *h, int N, int k, const int *rows, const int 
  * of words (T+1), 0 for a task without DFS work, or a negative status. */
 int nq_debug_task_schedule(int N, nq_record rec, uint32_t root[4], uint32_t *info, uint32_t *words, int cap);
 
+/* Diagnostic: the row rules of the unique counter's start configuration `conf`
+ * (0 <= conf < N - 3 + (N - 2) / 2) as its search reads them, words[left] for
+ * a frame with `left` rows left (0..N): the columns its child's row may use,
+ * with flags above bit 26.  NQ_OK or NQ_EINVAL. */
+int nq_debug_unique_words(int N, int conf, uint32_t *words);
+
 /* Diagnostic: the host-built tasks of a completion query (see
  * nq_count_completions), wide format: per task root {ld, rd, col, avail},
  * info word and (T+1) word pairs {x, RA} at words + task * 2 * stride.

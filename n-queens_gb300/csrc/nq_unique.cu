@@ -153,15 +153,16 @@ constexpr uint32_t U_COUNT = 1u << 27;      // part 1, last row: a solution, x8
 constexpr uint32_t U_CLASSIFY = 1u << 28;   // part 2, last row: a board to classify
 constexpr uint32_t U_NOLOOK = 1u << 29;     // the child's row is the last one: there is none behind it
 constexpr uint32_t U_SIDES = 1u << 31;      // part 2, row bound2 + 1: dead while a side column is free
-__device__ __forceinline__ uint32_t row_word(const UConf& c, int N, int left) {
+__host__ __device__ __forceinline__ uint32_t row_word(const UConf& c, int N, int left) {
   if (left == 0) return 0u;                 // the sentinel: every child dies
   if (left == 1) return c.part == 1 ? U_COUNT : U_CLASSIFY;
   const uint32_t child = (uint32_t)(N - left + 1);
-  uint32_t w = (1u << N) - 1u;
+  const uint32_t columns = (1u << N) - 1u;
+  uint32_t w = columns;
   if (left == 2) w |= U_NOLOOK;
   if (child < c.bound1) w &= c.part == 1 ? ~2u : ~c.sidemask;
   if (c.part != 1) {
-    if (child == (uint32_t)N - 1u) w &= ~c.lastmask;
+    if (child == (uint32_t)N - 1u) w &= ~(c.lastmask & columns);   // lastmask has grown past the board, onto the flags
     // Row bound2 must take the last free side column (backTrack2, :126-151): after it both are behind.  Its
     // own candidates go unfiltered and die one step on: 5 % more steps (N=15 39.7 10^6 against 37.6, N=16 259
     // against 246, before the look-ahead), each about four instructions shorter.
@@ -342,7 +343,7 @@ __global__ void __launch_bounds__(BLOCK) unique_kernel(const UArgs a) {
 // at N=12; the same expansion on one host thread and its upload took 0.8 ms at
 // N=12, 6 ms at N=14 and 25 ms at N=16.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ UConf make_conf(int N, int i) {
+__host__ __device__ __forceinline__ UConf make_conf(int N, int i) {
   const uint32_t topbit = 1u << (N - 1);
   const int n1 = N - 3;                                 // part 1: bound1 = 2..N-2
   if (i < n1) return UConf{1, (uint32_t)(i + 2), 0, 0, 0};
@@ -436,6 +437,12 @@ __global__ void __launch_bounds__(128) unique_expand_kernel(int N, int level, un
 }  // namespace nq
 
 using namespace nq;
+
+extern "C" int nq_debug_unique_words(int N, int conf, uint32_t* words) {
+  if (N < 4 || N > kMaxN || conf < 0 || conf >= (N - 3) + (N - 2) / 2 || !words) return NQ_EINVAL;
+  for (int left = 0; left <= N; left++) words[left] = row_word(make_conf(N, conf), N, left);
+  return NQ_OK;
+}
 
 extern "C" int nq_count_unique(nq_handle* h, int N, uint64_t* unique, uint64_t* total) {
   if (!h) return NQ_EINVAL;
