@@ -649,18 +649,22 @@ int count_start_range(nq_handle* h, int N, int p, const std::vector<int>& starts
 constexpr uint64_t kGenRecords = 8 << 20;         // records a chunk may have (bound), 128 MiB a buffer
 constexpr int64_t kGenNoReadBack = 65536;         // bound up to which the list's length stays on the device
 
-// At most this many records from one start constellation: it holds 3 or 4 queens, and its first free row has
-// N - 3 or N - 4 columns left, the next one fewer, ...
+// At most this many states on any level from one start constellation to its records: it holds 3 or 4 queens, and its
+// first free row has N - 3 or N - 4 columns left, the next one fewer, ...  Where the columns run out (N=7 at preset 8)
+// a level before has more states than the records' own bound.
 uint64_t start_bound(int N, int preset, int start) {
   const uint32_t col = 1u | (1u << (N - 1)) | ((1u << (N - 1)) >> geti(start)) | ((1u << (N - 1)) >> getj(start));
-  uint64_t b = 1;
+  uint64_t b = 1, most = 1;
   int c = N - __builtin_popcount(col);
-  for (int q = getj(start) == N - 1 ? 3 : 4; q < preset; q++) b *= (uint64_t)std::max(0, c--);
-  return b;
+  for (int q = getj(start) == N - 1 ? 3 : 4; q < preset; q++) {
+    b *= (uint64_t)std::max(0, c--);
+    most = std::max(most, b);
+  }
+  return most;
 }
 
 // A bound on a board's start constellations (about twice their number: every candidate of the reference's
-// loops, before rotations are dropped, and the corner ones) and on its records.
+// loops, before rotations are dropped, and the corner ones) and on the states of any level up to its records.
 uint64_t board_starts(int N) {
   uint64_t n = 0;
   for (int k = 1; k < (N + 1) / 2; k++) {
@@ -672,10 +676,13 @@ uint64_t board_starts(int N) {
   return n + (uint64_t)(N - 2) * (N - 3) / 2;
 }
 uint64_t board_bound(int N, int p) {
-  uint64_t side = board_starts(N) - (uint64_t)(N - 2) * (N - 3) / 2, corner = (uint64_t)(N - 2) * (N - 3) / 2;
-  for (int q = 4; q < p; q++) side *= (uint64_t)std::max(0, N - q);
-  for (int q = 3; q < p; q++) corner *= (uint64_t)std::max(0, N - q);
-  return std::max(side + corner, board_starts(N));
+  uint64_t corner = (uint64_t)(N - 2) * (N - 3) / 2, side = board_starts(N) - corner, most = side + corner;
+  for (int q = 4; q <= p; q++) {                 // a level: a queen more, the corner ones are one behind
+    if (q < p) side *= (uint64_t)std::max(0, N - q);
+    corner *= (uint64_t)std::max(0, N - q + 1);
+    most = std::max(most, side + corner);
+  }
+  return most;
 }
 
 // One generated chunk on the handle's stream: starts (host list, or null: the whole board), counted.
@@ -726,7 +733,7 @@ int count_generated(nq_handle* h, int N, int p, const std::vector<int>& starts, 
   for (size_t s0 = s_begin; s0 < s_end;) {
     size_t s1 = s0;
     uint64_t bound = 0;
-    do { bound += std::max<uint64_t>(1, start_bound(N, p, starts[s1++])); }
+    do { bound += start_bound(N, p, starts[s1++]); }
     while (s1 < s_end && bound + start_bound(N, p, starts[s1]) <= kGenRecords);
     uint64_t t = 0;
     int64_t r = 0;

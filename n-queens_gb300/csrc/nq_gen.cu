@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(128) gen_level_kernel(int N, int preset, bool 
                                                         unsigned* err) {
   chain_next();
   chain_wait();
-  const unsigned n = gn[level];
+  const unsigned n = min(gn[level], cap);
   for (unsigned q0 = blockIdx.x * blockDim.x; q0 < n; q0 += gridDim.x * blockDim.x) {
     const unsigned q = q0 + threadIdx.x;
     uint4 s = make_uint4(0, 0, 0, 0);
