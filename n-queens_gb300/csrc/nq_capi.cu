@@ -188,7 +188,7 @@ int read_ctrl(nq_handle* h, cudaStream_t st, uint64_t* total) {
 constexpr unsigned kQueryCap = 65536;
 constexpr unsigned kQueryTarget = 2048;      // ... and of each query of a batch
 unsigned query_target(int rows) { return rows >= 16 ? kQueryTarget : 512u; }
-constexpr unsigned kQueryCap2 = 4 << 20;     // queue after two levels (never reached: 7 children a frame on average)
+constexpr unsigned kQueryCap2 = 4 << 20;     // queue after two levels (4.5 10^6 on the empty board of N=27, which take one)
 constexpr unsigned kQueryCap3 = 5 << 20;     // ... after three (0.5 to 4.5 10^6 measured for N=18..25; some of N=27 are longer)
 int query_levels(int rows) { return rows >= 13 ? 3 : rows >= 11 ? 2 : rows >= 10 ? 1 : 0; }
 // A batch's queries share the lanes with its other jobs, so the same need not be cut as fine.

@@ -327,7 +327,8 @@ __global__ void __launch_bounds__(512) batch_query_kernel(const BatchQuery* __re
   }
 }
 
-// The query's queue by another level (frames at the terminal depth move on).
+// The query's queue by another level (frames at the terminal depth move on).  A level that did not fit its buffer is
+// not read: the next one's length says that it did not fit either, so the search does nothing.
 template <bool WIDE>
 __global__ void __launch_bounds__(128) query_level_kernel(uint32_t N, uint32_t T, QueryBuffers b, int level) {
   using W = typename QueryWord<WIDE>::type;
@@ -335,6 +336,10 @@ __global__ void __launch_bounds__(128) query_level_kernel(uint32_t N, uint32_t T
   chain_wait();
   const unsigned n = b.ctl[QueryCtl::kQueue + level];
   const unsigned cap = b.cap[level + 1];
+  if (n > b.cap[level]) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) b.ctl[QueryCtl::kQueue + level + 1] = ~0u;
+    return;
+  }
   const uint4* __restrict__ in = b.sroot[level];
   uint4* __restrict__ out = b.sroot[level + 1];
   uint2* __restrict__ info = b.sinfo[level + 1];
