@@ -202,6 +202,11 @@ int nq_count_completions(nq_handle *h, int N, int k, const int *rows, const int 
  * of words (T+1), 0 for a task without DFS work, or a negative status. */
 int nq_debug_task_schedule(int N, nq_record rec, uint32_t root[4], uint32_t *info, uint32_t *words, int cap);
 
+/* Diagnostic: states on the widest level of a board's device generation (6 <= N
+ * <= 27, presets 4..8, else 0), which sizes its buffers: the records from N=12
+ * on, for smaller boards a level between may be wider. */
+int64_t nq_debug_board_states(int N, int preset);
+
 /* Diagnostic: the row rules of the unique counter's start configuration `conf`
  * (0 <= conf < N - 3 + (N - 2) / 2) as its search reads them, words[left] for
  * a frame with `left` rows left (0..N): the columns its child's row may use,

@@ -218,6 +218,18 @@ int query_task(int N, int k, const int* rows, const int* cols, QueryParam* p, bo
   return 1;
 }
 
+// The most frames a level of a query's expansion has: only levels below the target are expanded, and a frame of
+// depth d has at most as many candidates as columns are left there.
+uint64_t query_frames(const QueryParam& p) {
+  const uint64_t columns = (uint64_t)p.T + 2;      // left at the root
+  uint64_t n = 1, most = 1;
+  for (uint32_t d = 0; d < p.T; d++) {
+    n = std::min<uint64_t>(n, p.target) * (columns - d);
+    most = std::max(most, n);
+  }
+  return most;
+}
+
 // A compact query's words in the wide form.
 void widen_query(QueryParam* p) {
   for (uint32_t d = 0; d <= p->T; d++) {
@@ -491,6 +503,8 @@ int nq_debug_task_schedule(int N, nq_record rec, uint32_t root[4], uint32_t* inf
   return T + 1;
 }
 
+int64_t nq_debug_board_states(int N, int preset) { return (int64_t)board_states(N, preset); }
+
 int64_t nq_debug_completion_tasks(int N, int k, const int* rows, const int* cols, int min_tasks, uint32_t* roots,
                                   uint32_t* infos, uint32_t* words, int stride, int64_t cap, uint64_t* fixed_count) {
   if (k < 0 || k > 8 || (k > 0 && (!rows || !cols)) || stride < 1) return NQ_EINVAL;
@@ -647,7 +661,10 @@ int count_start_range(nq_handle* h, int N, int p, const std::vector<int>& starts
 // the device.  The host generator above spends 0.9 ms on its threads alone at N=9..13 (a count of N=13 took
 // 1.3 ms, 0.1 of it on the GPU) and 8 ms on N=19's 897,071 records.
 constexpr uint64_t kGenRecords = 8 << 20;         // records a chunk may have (bound), 128 MiB a buffer
-constexpr int64_t kGenNoReadBack = 65536;         // bound up to which the list's length stays on the device
+constexpr uint64_t kGenBoard = 2 << 20;           // states a board in one chunk may have
+// The list's length stays on the device up to this many records: by the bound of a range of start constellations
+// (2 to 4 times its records), or by a board's states.
+constexpr uint64_t kGenNoReadBack = 65536, kGenNoReadBackBoard = 32768;
 
 // At most this many states on any level from one start constellation to its records: it holds 3 or 4 queens, and its
 // first free row has N - 3 or N - 4 columns left, the next one fewer, ...  Where the columns run out (N=7 at preset 8)
@@ -663,29 +680,8 @@ uint64_t start_bound(int N, int preset, int start) {
   return most;
 }
 
-// A bound on a board's start constellations (about twice their number: every candidate of the reference's
-// loops, before rotations are dropped, and the corner ones) and on the states of any level up to its records.
-uint64_t board_starts(int N) {
-  uint64_t n = 0;
-  for (int k = 1; k < (N + 1) / 2; k++) {
-    const int j_max = N - k - 2;
-    for (int l = k + 1; l <= N - 2; l++)
-      for (int i = k + 1; i <= N - 2; i++)
-        if (i != N - 1 - l) n += (uint64_t)std::max(0, j_max - (i <= j_max) - (l <= j_max && l != i));
-  }
-  return n + (uint64_t)(N - 2) * (N - 3) / 2;
-}
-uint64_t board_bound(int N, int p) {
-  uint64_t corner = (uint64_t)(N - 2) * (N - 3) / 2, side = board_starts(N) - corner, most = side + corner;
-  for (int q = 4; q <= p; q++) {                 // a level: a queen more, the corner ones are one behind
-    if (q < p) side *= (uint64_t)std::max(0, N - q);
-    corner *= (uint64_t)std::max(0, N - q + 1);
-    most = std::max(most, side + corner);
-  }
-  return most;
-}
-
-// One generated chunk on the handle's stream: starts (host list, or null: the whole board), counted.
+// One generated chunk on the handle's stream: starts (host list, or null: the whole board of at most n), counted; no
+// level of it has more than `bound` states.
 int count_chunk(nq_handle* h, int N, int p, const int* starts, size_t n, uint64_t bound, uint64_t* total, int64_t* records) {
   cudaStream_t st = h->stream;
   NQ_CUDA(h, cudaSetDevice(h->device));
@@ -696,7 +692,7 @@ int count_chunk(nq_handle* h, int N, int p, const int* starts, size_t n, uint64_
   if (bound > 0x7FFFFFFFull) return h->fail(NQ_ENOMEM, "generator: too many records from one start constellation");
   const size_t cap = std::max<size_t>((size_t)bound, n);
   NQ_CUDA(h, h->rec.ensure(cap * sizeof(uint4)));
-  NQ_CUDA(h, h->gen.ensure(cap * sizeof(uint4)));
+  if (levels > kGenFused) NQ_CUDA(h, h->gen.ensure(cap * sizeof(uint4)));
   if (int e = h->ensure_pinned(kStage + (starts ? n * sizeof(int) : 0))) return e;
   if (starts) {
     NQ_CUDA(h, h->starts.ensure(n * sizeof(int)));
@@ -705,12 +701,12 @@ int count_chunk(nq_handle* h, int N, int p, const int* starts, size_t n, uint64_
   }
   NQ_CUDA(h, cudaMemsetAsync(c, 0, ctl::kAll, st));
   h->result_written = false;
-  uint4* buf[2] = {(uint4*)h->rec.p, (uint4*)h->gen.p};
+  uint4* buf[2] = {(uint4*)h->rec.p, (uint4*)(levels > kGenFused ? h->gen.p : h->rec.p)};
   NQ_CUDA(h, launch_generate(N, p, (unsigned)n, starts ? (const int*)h->starts.p : nullptr, buf[0], buf[1], (unsigned)cap, gn,
                              (unsigned int*)(c + ctl::kGenErr), h->sms, st));
   const uint4* rec = buf[levels & 1];
   const int t_max = std::max(1, N - p - 2);        // a queen a depth, one column left in the base row
-  const bool on_device = (int64_t)bound <= kGenNoReadBack && h->queue_order == 0;
+  const bool on_device = bound <= (starts ? kGenNoReadBack : kGenNoReadBackBoard) && h->queue_order == 0;
   int64_t m = (int64_t)bound;
   if (!on_device) {
     NQ_CUDA(h, cudaMemcpyAsync(h->h_ctrl, c, ctl::kAll, cudaMemcpyDeviceToHost, st));
@@ -759,9 +755,9 @@ int nq_count(nq_handle* h, int N, int preset, uint64_t* total) {
   if (N <= 5) return nq_count_completions(h, N, 0, nullptr, nullptr, total);
   const int p = preset > 0 ? preset : preset_for(N);
   if (p < 4) return h->fail(NQ_EPRESET, "generator: preset %d below 4", p);
-  if (h->chunk_records == 0 && p <= 8 && board_bound(N, p) <= kGenRecords) {
+  if (h->chunk_records == 0 && p <= 8 && board_states(N, p) <= kGenBoard) {
     int64_t records = 0;
-    if (int e = count_chunk(h, N, p, nullptr, board_starts(N), board_bound(N, p), total, &records)) return e;
+    if (int e = count_chunk(h, N, p, nullptr, board_states(N, 4), board_states(N, p), total, &records)) return e;
     h->last_chunks = records ? 1 : 0;
     h->last_records = records;
     return NQ_OK;
@@ -930,6 +926,9 @@ void nq_batch_destroy(nq_batch* b) {
   delete b;
 }
 
+// Boards whose list the device makes: the deeper presets' outgrow the generator's buffers.
+bool board_on_device(int N, int p) { return p <= 8 && board_states(N, p) <= kGenBoard; }
+
 // A board's tasks in a batch go unsplit where the batch's counts give every lane at least a quarter of such a task:
 // splitting then only adds items (the queue's end is evened out by the other jobs and within the warps).  us of a
 // replay, split once (as any list above 10^5 tasks) / so: 64 jobs of N=12..15 1212 / 938, of N=10..14 271 / 174, 256
@@ -962,7 +961,8 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
     return h->fail(status, "batch job %d: %s", j, what);
   };
   // ---- the lists: one per board (N, preset) and one per query
-  struct List { int N = 0, rows = 0, T = 0; uint64_t cap = 0; bool query = false; int D = 0; uint32_t src0 = 0, task0 = 0; };
+  // weight: the list's length as the rules below count it
+  struct List { int N = 0, rows = 0, T = 0; uint64_t cap = 0, weight = 0; bool query = false; int D = 0; uint32_t src0 = 0, task0 = 0; };
   struct Board { int p; uint32_t list; bool device; std::vector<GenRecord> recs; };
   std::vector<List> lists;
   std::vector<Board> boards;
@@ -983,21 +983,22 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
         Board bd;
         bd.p = p; bd.list = (uint32_t)lists.size();
         List l;
-        l.N = J.N; l.cap = board_bound(J.N, p); l.rows = maxt_for(J.N, p - 3);
+        l.N = J.N; l.cap = board_states(J.N, p); l.rows = maxt_for(J.N, p - 3);
         b->ra_words = b->ra_words || !ra_in_rd(J.N, p - 3, 0);
-        bd.device = p <= 8 && l.cap <= kGenRecords;
-        if (!bd.device) {                        // more than the device generator's buffers: the host's list
+        bd.device = board_on_device(J.N, p);
+        if (!bd.device) {                        // the host's list
           const int s = gen_constellations(J.N, p, bd.recs, 0);
           if (s != 0) return bad(s == -2 ? NQ_EPRESET : NQ_EINVAL, "generator failed", j);
           l.cap = bd.recs.size();
         }
+        l.weight = bd.device ? l.cap * (p == 4 ? 2 : 3) : l.cap;
         it = board_list.emplace(std::make_pair(J.N, p), bd.list).first;
         lists.push_back(l);
         boards.push_back(std::move(bd));
       }
       job_list[j] = (int)it->second;
-      sources += lists[it->second].cap / 4;      // the bound is about four times the records
-      work += (double)(lists[it->second].cap / 4) * task_nodes(lists[it->second].rows);
+      sources += lists[it->second].weight / 4;
+      work += (double)(lists[it->second].weight / 4) * task_nodes(lists[it->second].rows);
     } else {
       int rows[8], cols[8];
       const int k = (J.kind == NQ_JOB_COUNT) ? 0 : J.k;
@@ -1019,14 +1020,15 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
   const unsigned target = queries.size() > 64 ? kQueryTarget / 4 : kQueryTarget;
   for (BatchQuery& q : queries) {
     q.p.target = std::min(target, kQueryCap / q.p.N);
-    lists[q.list].cap = (uint64_t)q.p.target * q.p.N;
+    lists[q.list].cap = query_frames(q.p);
+    lists[q.list].weight = (uint64_t)q.p.target * q.p.N;
     sources += 4 * q.p.target;
     if (b->wide != (q.p.words_wide != 0)) widen_query(&q.p);
   }
   // ---- offsets, split depths, table sizes
   const size_t nl = lists.size(), nb = boards.size(), nq = queries.size();
   std::vector<unsigned long long> ends(nl);
-  uint64_t src = 0, ntask = 0, words = 1, rec_cap = 0, gen_cap = 0;
+  uint64_t src = 0, ntask = 0, words = 1, rec_cap = 0, gen_cap = 0, tmp_cap = 0;
   for (size_t i = 0; i < nl; i++) {
     List& l = lists[i];
     l.src0 = (uint32_t)src; l.task0 = (uint32_t)ntask;
@@ -1034,7 +1036,7 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
     ends[i] = src;
     ntask += l.query ? 1 : l.cap;
     words = std::max<uint64_t>(words, l.query ? l.T + 1 : l.rows + 1);
-    const int levels = l.query ? batch_query_levels(l.rows) : choose_split((int64_t)std::max(sources, l.cap), l.rows);
+    const int levels = l.query ? batch_query_levels(l.rows) : choose_split((int64_t)std::max(sources, l.weight), l.rows);
     const bool whole = !l.query && unsplit_in_batch(l.rows, work, h->sms);
     // queries of the larger target are cut once in a batch with that many sources, of the smaller one twice: 256 mixed
     // jobs of N=9..16 3628 us with one, 3070 so; 64 718 so, 986 uncut
@@ -1043,7 +1045,7 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
   }
   for (const Board& bd : boards) {
     rec_cap = std::max(rec_cap, lists[bd.list].cap);
-    if (bd.device) gen_cap = std::max(gen_cap, lists[bd.list].cap);
+    if (bd.device && gen_levels(bd.p) > kGenFused) gen_cap = std::max(gen_cap, lists[bd.list].cap);
   }
   if (src > 0xFFFFFFFFull || words > (uint64_t)kMaxDepth) { nq_batch_destroy(b); return h->fail(NQ_ENOMEM, "batch: too many tasks"); }
   b->sw = (int)words;
@@ -1076,8 +1078,7 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
         (e = frames.ensure(std::max<uint64_t>(src, 1) * sizeof(uint4))) != cudaSuccess ||
         (e = off.ensure(std::max<uint64_t>(src, 1) * 4)) != cudaSuccess ||
         (nb && (e = rec.ensure(std::max<uint64_t>(rec_cap, 1) * sizeof(uint4))) != cudaSuccess) ||
-        (gen_cap && (e = gen.ensure(gen_cap * sizeof(uint4))) != cudaSuccess) ||
-        (nq && (e = tmp.ensure(src * sizeof(uint4))) != cudaSuccess)) break;
+        (gen_cap && (e = gen.ensure(gen_cap * sizeof(uint4))) != cudaSuccess)) break;
     unsigned char *dt = (unsigned char*)tab.p, *ds = (unsigned char*)state.p;
     // ---- upload the lists and queries
     BatchList* hl = (BatchList*)(b->stage + o_lists);
@@ -1086,8 +1087,11 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
     BatchQuery* hq = (BatchQuery*)(b->stage + o_q);
     for (size_t i = 0; i < nq; i++) {
       hq[i] = queries[i];
-      hq[i].src0 = lists[queries[i].list].src0; hq[i].task = lists[queries[i].list].task0;
+      const List& l = lists[queries[i].list];
+      hq[i].src0 = l.src0; hq[i].task = l.task0; hq[i].cap = (uint32_t)l.cap; hq[i].tmp0 = (uint32_t)tmp_cap;
+      tmp_cap += l.cap;
     }
+    if (nq && (e = tmp.ensure(tmp_cap * sizeof(uint4))) != cudaSuccess) break;
     if ((e = cudaMemcpyAsync(dt, b->stage, o_jends, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
         (e = cudaMemsetAsync(ds, 0, state_bytes, st)) != cudaSuccess) break;
     b->h2d_bytes = (int64_t)o_jends;
@@ -1104,9 +1108,9 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
       std::vector<nq_record> packed;
       if (bd.device) {
         const int levels = gen_levels(bd.p);
-        uint4* buf[2] = {(uint4*)rec.p, (uint4*)gen.p};
+        uint4* buf[2] = {(uint4*)rec.p, (uint4*)(levels > kGenFused ? gen.p : rec.p)};
         unsigned int* gn = (unsigned int*)(ds + o_gn + i * 32);
-        e = launch_generate(l.N, bd.p, (unsigned)board_starts(l.N), nullptr, buf[0], buf[1],
+        e = launch_generate(l.N, bd.p, (unsigned)board_states(l.N, 4), nullptr, buf[0], buf[1],
                             (unsigned)l.cap, gn, derr, h->sms, st);
         drec = buf[levels & 1];
         dn = gn + levels;
@@ -1170,6 +1174,7 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
       items += s.items;
     }
     b->ms = (int64_t)items;
+    for (DevBuf* d : {&rec, &gen, &tmp}) d->release();       // the queue may take their place
     if ((e = b->sroot.ensure(std::max<uint64_t>(items, 1) * sizeof(uint4))) != cudaSuccess ||
         (e = b->sinfo.ensure(std::max<uint64_t>(items, 1) * sizeof(uint2))) != cudaSuccess) break;
     // ---- write the jobs' items
@@ -1194,22 +1199,23 @@ int64_t nq_job_device_bytes(const nq_job* job, int sms, int split_depth) {
   const nq_job& J = *job;
   if (J.N < 1 || J.N > kMaxN || J.k < 0 || J.k > 8) return NQ_EINVAL;
   int64_t m = 0, tasks = 1;
-  int rows = 1;
-  int levels = 0;
+  int rows = 1, levels = 0;
+  int64_t word = sizeof(uint2), list = sizeof(uint4);        // bytes a schedule word, and a source while its list is made
   if (J.kind == NQ_JOB_COUNT && J.N >= 6) {
-    // the record bound nq_batch_create builds the job with
     const int p = J.preset > 0 ? J.preset : preset_for(J.N);
     if (p < 4) return NQ_EPRESET;
-    m = (int64_t)board_bound(J.N, p);
-    if (p > 8 || (uint64_t)m > kGenRecords) {
+    m = (int64_t)board_states(J.N, p);
+    if (m == 0 || J.N < p) {               // no figure, or a preset that may be too deep
       std::vector<GenRecord> v;
       const int s = gen_constellations(J.N, p, v, 0);
       if (s != 0) return s == -2 ? NQ_EPRESET : NQ_EINVAL;
-      m = (int64_t)v.size();
+      m = std::max(m, (int64_t)v.size());
     }
     tasks = m;
     rows = maxt_for(J.N, p - 3);
-    levels = choose_split(m / 4, rows);
+    levels = choose_split(m, rows);
+    word = sizeof(uint32_t);
+    if (board_on_device(J.N, p) && gen_levels(p) > kGenFused) list *= 2;
   } else if (J.kind == NQ_JOB_COUNT || J.kind == NQ_JOB_COMPLETION) {
     int r[8], c[8];
     const int k = (J.kind == NQ_JOB_COUNT) ? 0 : J.k;
@@ -1220,20 +1226,21 @@ int64_t nq_job_device_bytes(const nq_job* job, int sms, int split_depth) {
     const int s = query_task(J.N, k, r, c, &p, &wide, &fixed);
     if (s < 0) return NQ_EINVAL;
     if (s > 0) {
-      m = (int64_t)std::min(kQueryTarget, kQueryCap / (unsigned)J.N) * J.N;
+      p.target = std::min(kQueryTarget, kQueryCap / (unsigned)J.N);
+      m = (int64_t)query_frames(p);
       rows = (int)p.T + 2;
       levels = batch_query_levels(rows);
     }
   } else {
     return NQ_EINVAL;
   }
-  // split queue: each level multiplies the items by at most ~8 (measured 6.2-8x)
+  // split queue: each level multiplies the items by at most ~8 (measured 6.2-8x); it takes the place of the list
   const int D = (J.N <= 12) ? 0 : (split_depth >= 0 ? split_depth : levels);
   int64_t ns = m;
   for (int d = 0; d < D; d++) ns *= 8;
-  const int64_t per_source = 16 /*record*/ + 16 /*generator*/ + 16 /*frame*/ + 4 /*slot*/;
-  return m * per_source + tasks * (4 /*info*/ + (int64_t)(rows + 1) * 8 /*widest words*/) + ns * (16 + 8) +
-         (int64_t)Ctrl::bytes(1) + 8192;
+  const int64_t per_source = 16 /*frame*/ + 4 /*slot*/;
+  return m * per_source + tasks * (4 /*info*/ + (int64_t)(rows + 1) * word) + std::max(m * list, ns * (16 + 8)) +
+         (int64_t)Ctrl::bytes(1) + 4096;
 }
 
 int nq_batch_set_grid(nq_batch* b, int grid) {

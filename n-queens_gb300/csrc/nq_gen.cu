@@ -138,12 +138,11 @@ __device__ __forceinline__ uint4 state_child(const uint4 s, uint32_t bit) {
   return settle((s.x | bit) << 1, (s.y | bit) >> 1, s.z | bit, (int)((s.w >> 20) & 31u) + 1, (int)(s.w >> kQueens) + 1, s.w & 0xFFFFFu);
 }
 
-// Presets 4 and 5 in one launch: a start constellation is at most kFused queens short, and its thread writes its
+// Presets 4 and 5 in one launch: a start constellation is at most kGenFused queens short, and its thread writes its
 // records (of a whole board, the corner constellations, which hold a queen less, have a thread a column).  us of a
 // count of N=6 / 10 / 13 / 16 with a launch a queen 30.8 / 35.2 / 47.6 / 319, so
 // 26.5 / 31.7 / 44.2 / 315.  A third level (preset 6)
 // keeps a launch a queen: N=14 70 us and N=16 328 with three in a thread.
-constexpr int kFused = 2;
 template <int DEPTH, class F>
 __device__ __forceinline__ void each_record(const uint4 s, int N, int preset, unsigned* err, F&& f) {
   if constexpr (DEPTH > 0) {
@@ -180,10 +179,10 @@ __global__ void __launch_bounds__(128) gen_records_kernel(int N, int preset, uns
       if (take) s = state_child(s, bit);
     }
   }
-  if (take) each_record<kFused>(s, N, preset, err, [&](uint4) { c++; });
+  if (take) each_record<kGenFused>(s, N, preset, err, [&](uint4) { c++; });
   unsigned at = take_slots(count, c);
   if (take)
-    each_record<kFused>(s, N, preset, err, [&](uint4 r) {
+    each_record<kGenFused>(s, N, preset, err, [&](uint4 r) {
       if (at < cap) out[at] = r;
       at++;
     });
@@ -247,9 +246,8 @@ __device__ __forceinline__ void each_child(const uint4 f, const QWord o, uint32_
   }
 }
 
-// The frames of one query, breadth-first from its root until there are `target` of them, the next level may
-// not fit, or they stand at the terminal depth: into (sroot, sinfo) from `slot` on.  Returns their number;
-// one block, buffers of `cap` frames.
+// The frames of one query, breadth-first from its root until there are `target` of them or they stand at the terminal
+// depth.  Returns their number; one block, buffers of `cap` frames, which no level exceeds.
 template <class W>
 __device__ unsigned expand_query(const uint4 root, uint32_t N, uint32_t T, const W* words, unsigned target, unsigned cap,
                                  uint4* buf0, uint4* buf1, unsigned& depth) {
@@ -259,7 +257,7 @@ __device__ unsigned expand_query(const uint4 root, uint32_t N, uint32_t T, const
   if (threadIdx.x == 0) in[0] = root;
   unsigned n = root.w ? 1u : 0u, d = 0;
   __syncthreads();
-  while (d < T && n && n < target && n * N <= cap) {
+  while (d < T && n && n < target) {
     if (threadIdx.x == 0) cnt = 0;
     __syncthreads();
     const QWord o = qword(words[d], N);
@@ -269,10 +267,10 @@ __device__ unsigned expand_query(const uint4 root, uint32_t N, uint32_t T, const
       unsigned c = 0;
       each_child(f, o, bm, [&](uint4) { c++; });
       unsigned at = take_slots(&cnt, c);
-      if (c) each_child(f, o, bm, [&](uint4 g) { out[at++] = g; });
+      if (c) each_child(f, o, bm, [&](uint4 g) { if (at < cap) out[at] = g; at++; });
     }
     __syncthreads();
-    n = cnt;
+    n = min(cnt, cap);
     uint4* t = in; in = out; out = t;
     d++;
     __syncthreads();
@@ -319,7 +317,7 @@ __global__ void __launch_bounds__(512) batch_query_kernel(const BatchQuery* __re
   }
   __syncthreads();
   unsigned d;
-  const unsigned n = expand_query<W>(q.p.root, q.p.N, q.p.T, words, q.p.target, q.p.target * q.p.N, src + q.src0, tmp + q.src0, d);
+  const unsigned n = expand_query<W>(q.p.root, q.p.N, q.p.T, words, q.p.target, q.cap, src + q.src0, tmp + q.tmp0, d);
   if (threadIdx.x == 0) {
     info[q.task] = info_pack(q.p.T, 0, 0, q.p.N, TS_OK);
     state[q.list].n = n;
@@ -369,7 +367,7 @@ cudaError_t launch_generate(int N, int preset, unsigned n_starts, const int* sta
   const unsigned full = 8u * (unsigned)sms;
   if (starts && n_starts == 0) return cudaSuccess;
   const unsigned board = (unsigned)(N * N * (1 + ((N + 1) / 2 - 1) * N));      // a board's candidates
-  if (levels <= kFused) {
+  if (levels <= kGenFused) {
     const unsigned n = starts ? n_starts : board + (unsigned)(N * N * (N - 1));      // corner ones: a thread a column
     return launch_after(gen_records_kernel, (n + 127) / 128, 128, 0, st, N, preset, n, starts, buf[levels & 1], cap, gn + levels, err);
   }

@@ -178,6 +178,35 @@ int gen_constellations(int N, int preset, std::vector<GenRecord>& out, int threa
   return expand_starts(N, preset, starts, 0, starts.size(), out, threads);
 }
 
+uint64_t board_states(int N, int preset) {
+  if (N < 6 || N > kMaxN || preset < 4 || preset > 8) return 0;
+  static constexpr uint32_t states[kMaxN - 5][5] = {      // N = 6.., preset 4..8
+      {16u, 16u, 16u, 16u, 16u},
+      {36u, 34u, 34u, 34u, 34u},
+      {92u, 134u, 121u, 121u, 121u},
+      {184u, 392u, 476u, 453u, 453u},
+      {346u, 1007u, 1722u, 1878u, 1837u},
+      {580u, 2161u, 5031u, 8100u, 8341u},
+      {932u, 4300u, 12943u, 27931u, 40943u},
+      {1404u, 7731u, 29043u, 79572u, 155925u},
+      {2054u, 13233u, 60127u, 204112u, 512539u},
+      {2884u, 21270u, 114209u, 466379u, 1444565u},
+      {3964u, 33046u, 205709u, 992487u, 3705028u},
+      {5296u, 49207u, 349418u, 1952839u, 8587857u},
+      {6962u, 71475u, 571705u, 3653940u, 18656800u},
+      {8964u, 100706u, 897071u, 6467354u, 37752890u},
+      {11396u, 139232u, 1369061u, 11029570u, 72820769u},
+      {14260u, 188147u, 2025282u, 18052162u, 133303405u},
+      {17662u, 250485u, 2932689u, 28719035u, 235271863u},
+      {21604u, 327606u, 4145833u, 44271796u, 399026853u},
+      {26204u, 423338u, 5762269u, 66737631u, 657666813u},
+      {31464u, 539335u, 7857828u, 98138478u, 1050644819u},
+      {37514u, 680311u, 10568809u, 141731791u, 1640320717u},
+      {44356u, 848242u, 13997139u, 200637190u, 2497629355u},
+  };
+  return states[N - 6][preset - 4];
+}
+
 // ---------------------------------------------------------------------------
 // completion queries
 // ---------------------------------------------------------------------------

@@ -36,6 +36,11 @@ int start_constellations(int N, std::vector<int>& starts);
 int expand_starts(int N, int preset, const std::vector<int>& starts, size_t s0, size_t s1,
                   std::vector<GenRecord>& out, int threads);
 
+// States on the widest level of a board's generation, 0 outside N 6..27 and presets 4..8: a level places one queen
+// more, from the start constellations on, and the last one is the list of records, which is the widest from N=12 on.
+// (Enumerated; a bound from the columns left is 2 times as much at preset 4, 3 at 5 and 100 for small boards at 8.)
+uint64_t board_states(int N, int preset);
+
 // The root frame {ld, rd, col, avail} and per-depth ops (the last one tall, n = free rows of them) of the
 // completions of k pre-placed queens; return values as build_completion_tasks.
 int completion_root(int N, int k, const int* rows, const int* cols, uint32_t root[4], Op* ops, int* n);

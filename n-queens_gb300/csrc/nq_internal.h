@@ -116,6 +116,7 @@ cudaError_t launch_dfs(const DfsLaunch& L, cudaStream_t st);
 // level, gn[gen_levels(preset)] the records, which end in buf0 when the level count is even, else in buf1
 // (`cap` records each; the caller bounds them).  gn zeroed before.
 inline int gen_levels(int preset) { return preset - 3; }     // start constellations hold 3 or 4 queens
+constexpr int kGenFused = 2;     // up to so many levels one launch makes the records: into the last buffer, the other stays untouched
 cudaError_t launch_generate(int N, int preset, unsigned n_starts, const int* starts, uint4* buf0, uint4* buf1, unsigned cap,
                             unsigned* gn, unsigned* err, int sms, cudaStream_t st);
 
@@ -171,8 +172,8 @@ struct ListArgs {
 };
 cudaError_t launch_list_count(const ListArgs& a, bool wide, cudaStream_t st);
 cudaError_t launch_list_write(const ListArgs& a, const BatchJob* jobs, uint4* sroot, uint2* sinfo, bool wide, cudaStream_t st);
-// The queries' tasks and frames (state n and depth), one block each; frames in src and tmp (cap = target * N).
-struct BatchQuery { QueryParam p; uint32_t list, src0, task, pad; };
+// The queries' tasks and frames (state n and depth), one block each; frames in src and tmp (no level has more than cap).
+struct BatchQuery { QueryParam p; uint32_t list, src0, tmp0, task, cap; };
 cudaError_t launch_batch_queries(int n, const BatchQuery* q, uint4* src, uint4* tmp, ListState* state, const TaskArrays& ta,
                                  cudaStream_t st);
 

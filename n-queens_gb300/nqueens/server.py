@@ -147,8 +147,8 @@ class Server:
             raise TypeError("submit a CountJob or a CompletionJob")
         f: Future = Future()
         now = time.perf_counter()
-        # Size the request here, on the caller's thread and outside the server's lock: the sizing of a large
-        # board generates its constellations, which must not stall the scheduler.
+        # Size the request here, on the caller's thread and outside the server's lock: the sizing of a board at a
+        # preset above 8 generates its constellations, which must not stall the scheduler.
         try:
             nbytes = self._job_bytes(job)
         except NQError as exc:
