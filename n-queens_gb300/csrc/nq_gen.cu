@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(128) gen_records_kernel(int N, int preset, uns
 }
 
 // One queen more for every state below the preset; the others move on (last: as records).
-__global__ void __launch_bounds__(128) gen_level_kernel(int N, int preset, bool last, const uint4* __restrict__ in,
+__global__ void __launch_bounds__(128) gen_level_kernel(int N, int preset, bool last, const uint4* in,
                                                         uint4* __restrict__ out, unsigned cap, unsigned* gn, int level,
                                                         unsigned* err) {
   chain_next();
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(128) query_level_kernel(uint32_t N, uint32_t T
     if (blockIdx.x == 0 && threadIdx.x == 0) b.ctl[QueryCtl::kQueue + level + 1] = ~0u;
     return;
   }
-  const uint4* __restrict__ in = b.sroot[level];
+  const uint4* in = b.sroot[level];
   uint4* __restrict__ out = b.sroot[level + 1];
   uint2* __restrict__ info = b.sinfo[level + 1];
   const uint32_t bm = (1u << N) - 1u;

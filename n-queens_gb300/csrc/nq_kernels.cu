@@ -124,8 +124,8 @@ struct RaInRd {
 };
 
 template <bool WIDE>
-__global__ void __launch_bounds__(256) prepare_kernel(int N, int64_t m, const unsigned* __restrict__ m_dev,
-                                                      const uint4* __restrict__ rec, uint4* __restrict__ root,
+__global__ void __launch_bounds__(256) prepare_kernel(int N, int64_t m, const unsigned* m_dev,
+                                                      const uint4* rec, uint4* __restrict__ root,
                                                       uint32_t* __restrict__ info,
                                                       typename WordT<WIDE>::type* __restrict__ sched, int sw, bool ra_words,
                                                       int64_t offset, unsigned int* err, unsigned int* tmax,
@@ -633,7 +633,7 @@ __global__ void __launch_bounds__(BLOCK) dfs_kernel(const DfsArgs a) {
   W* sch = reinterpret_cast<W*>(smem + (size_t)stack_slots(a.maxt) * BLOCK * sizeof(uint4)) + threadIdx.x;  // stride BLOCK
   const unsigned lane = threadIdx.x & 31u;
   const unsigned lt_mask = (1u << lane) - 1u;
-  const W* __restrict__ gsched = reinterpret_cast<const W*>(a.sched);
+  const W* gsched = reinterpret_cast<const W*>(a.sched);
   constexpr uint32_t ROW = BLOCK * (uint32_t)sizeof(W);
   constexpr uint32_t F = BLOCK * (uint32_t)sizeof(uint4);
   auto put_word = [&](uint32_t k, W w) { sch[k * BLOCK] = w; };

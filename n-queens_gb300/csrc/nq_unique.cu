@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(BLOCK) unique_kernel(const UArgs a) {
   auto arm = [&]() { sts_frame_u(top - F, 0u, 0u, 0u, kUSentinel); };
   arm();
   const int level = queue_level(a.ctl, a.cap);
-  const UTask* __restrict__ tasks = a.tasks[level & 1];
+  const UTask* tasks = a.tasks[level & 1];
   const unsigned m = a.ctl->n[level];
   // where the queue is smaller than the lanes, each warp takes its share and shares it among its lanes
   const unsigned warps = gridDim.x * (BLOCK / 32);
@@ -383,8 +383,8 @@ __global__ void __launch_bounds__(64) unique_init_kernel(int N, int nconf, UConf
 // Level l -> l + 1: one thread per state; its children with candidates left are counted, the warp reserves
 // their slots with one atomic, and they are written.  States that must not be expanded move on as they are.
 // n[l] <= 2^32: a level below the target (at most 2^21 states) has at most 27 children a state.
-__global__ void __launch_bounds__(128) unique_expand_kernel(int N, int level, unsigned target, unsigned cap, const UConf* __restrict__ confs,
-                                                            const UTask* __restrict__ in, UTask* __restrict__ out,
+__global__ void __launch_bounds__(128) unique_expand_kernel(int N, int level, unsigned target, unsigned cap, const UConf* confs,
+                                                            const UTask* in, UTask* __restrict__ out,
                                                             UCtl* ctl) {
   chain_next();
   chain_wait();
