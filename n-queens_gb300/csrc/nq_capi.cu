@@ -194,6 +194,18 @@ int query_levels(int rows) { return rows >= 13 ? 3 : rows >= 11 ? 2 : rows >= 10
 // A batch's queries share the lanes with its other jobs, so the same need not be cut as fine.
 int batch_query_levels(int rows) { return rows >= 15 ? 2 : rows >= 12 ? 1 : 0; }
 
+// The most frames a level of a query's expansion has: only levels below the target are expanded, and a frame of
+// depth d has at most as many candidates as columns are left there.
+uint64_t query_frames(const QueryParam& p) {
+  const uint64_t columns = (uint64_t)p.T + 2;      // left at the root
+  uint64_t n = 1, most = 1;
+  for (uint32_t d = 0; d < p.T; d++) {
+    n = std::min<uint64_t>(n, p.target) * (columns - d);
+    most = std::max(most, n);
+  }
+  return most;
+}
+
 // The query as a device task.  Returns 1, 0 when the count is settled here (*fixed), or -1 on bad arguments.
 // The last free row holds one column for every board, so its parent row is the task's terminal depth (count
 // the child if its row has a free square), as in constellation tasks.
@@ -216,18 +228,6 @@ int query_task(int N, int k, const int* rows, const int* cols, QueryParam* p, bo
   for (int d = 0; d <= n - 2; d++)
     p->words[d] = *wide ? make_uint2(device_wide_x(ops[d]), ops[d].ra) : make_uint2(device_compact(ops[d], false), 0u);
   return 1;
-}
-
-// The most frames a level of a query's expansion has: only levels below the target are expanded, and a frame of
-// depth d has at most as many candidates as columns are left there.
-uint64_t query_frames(const QueryParam& p) {
-  const uint64_t columns = (uint64_t)p.T + 2;      // left at the root
-  uint64_t n = 1, most = 1;
-  for (uint32_t d = 0; d < p.T; d++) {
-    n = std::min<uint64_t>(n, p.target) * (columns - d);
-    most = std::max(most, n);
-  }
-  return most;
 }
 
 // A compact query's words in the wide form.
@@ -284,6 +284,7 @@ void nq_destroy(nq_handle* h) {
   if (!h) return;
   cudaSetDevice(h->device);
   if (h->stream) cudaStreamSynchronize(h->stream);
+  for (QueryRun* q : h->q_free) h->query_free(q);
   h->rec.release(); h->root.release(); h->info.release(); h->sched.release(); h->per_task.release(); h->ctrl.release();
   h->sroot.release(); h->gen.release(); h->starts.release();
   h->okeys.release(); h->oorder.release(); h->ohist.release();
@@ -293,10 +294,7 @@ void nq_destroy(nq_handle* h) {
   for (auto& q : h->pinned_cap) cudaFreeHost(q.first);
   for (auto& e : h->ev) if (e) cudaEventDestroy(e);
   if (h->done) cudaEventDestroy(h->done);
-  h->qbuf.release();
   if (h->pool) cudaMemPoolDestroy(h->pool);
-  if (h->h_query) cudaFreeHost(h->h_query);
-  if (h->q_stream) cudaStreamDestroy(h->q_stream);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
 }
@@ -1339,22 +1337,26 @@ int nq_count_completions(nq_handle* h, int N, int k, const int* rows, const int*
   const int s = query_task(N, k, rows, cols, &p, &wide, &fixed);
   if (s < 0) return h->fail(NQ_EINVAL, "bad pre-placed queens");
   if (s == 0) { *count = fixed; return NQ_OK; }
-  std::lock_guard<std::mutex> lk(h->q_mu);
   NQ_CUDA(h, cudaSetDevice(h->device));
-  if (!h->q_stream) NQ_CUDA(h, cudaStreamCreateWithFlags(&h->q_stream, cudaStreamNonBlocking));
-  if (!h->h_query) NQ_CUDA(h, cudaMallocHost((void**)&h->h_query, QueryCtl::kWords * 8));
-  cudaStream_t st = h->q_stream;
+  struct Lease {                             // its stream and buffers are this call's alone
+    nq_handle* h;
+    QueryRun* q = nullptr;
+    ~Lease() { if (q) h->query_put(q); }
+  } lease{h};
+  NQ_CUDA(h, h->query_get(&lease.q));
+  QueryRun& q = *lease.q;
+  cudaStream_t st = q.stream;
   p.target = std::min(query_target((int)p.T + 2), kQueryCap / (unsigned)N);
   for (int levels = query_levels((int)p.T + 2);; levels--) {      // a level less where the queue did not fit
     QueryBuffers b{};
     b.cap[0] = kQueryCap; b.cap[1] = kQueryCap * (unsigned)N; b.cap[2] = kQueryCap2; b.cap[3] = kQueryCap3;
     size_t items = 0;
     for (int l = 0; l <= levels; l++) items += b.cap[l];
-    NQ_CUDA(h, h->qbuf.ensure(1024 + (kQueryCap + items) * sizeof(uint4) + items * sizeof(uint2)));
-    unsigned char* c = (unsigned char*)h->qbuf.p;
+    unsigned char* c = nullptr;
+    NQ_CUDA(h, q.ensure(1024 + (b.cap[0] + items) * sizeof(uint4) + items * sizeof(uint2), &c));
     b.ctl = (unsigned long long*)c; b.info = (uint32_t*)(c + 128); b.sched = c + 256;
     b.tmp = (uint4*)(c + 1024);
-    b.sroot[0] = b.tmp + kQueryCap;
+    b.sroot[0] = b.tmp + b.cap[0];
     b.sinfo[0] = (uint2*)(b.sroot[0] + items);
     for (int l = 1; l <= levels; l++) { b.sroot[l] = b.sroot[l - 1] + b.cap[l - 1]; b.sinfo[l] = b.sinfo[l - 1] + b.cap[l - 1]; }
     NQ_CUDA(h, launch_query(p, b, wide, levels, h->sms, st));
@@ -1368,16 +1370,18 @@ int nq_count_completions(nq_handle* h, int N, int k, const int* rows, const int*
     for (uint64_t f = 1; f < p.target; f *= (uint64_t)N) depth++;
     L.maxt = std::max(1, (int)p.T - depth); L.block = h->block; L.grid = h->grid;
     L.big = counts_need_u64(N, p.target);      // a queue below the target stands at its terminal depth
-    L.ctl = (const uint32_t*)b.ctl; L.ctl_words = QueryCtl::kWords; L.host_ctl = (uint32_t*)h->h_query;
+    L.ctl = (const uint32_t*)b.ctl; L.ctl_words = QueryCtl::kWords; L.host_ctl = (uint32_t*)q.host;
     L.blocks_done = (unsigned int*)(b.ctl + QueryCtl::kErr) + 1;
     L.chained = true;
     NQ_CUDA(h, launch_dfs(L, st));
     NQ_CUDA(h, cudaStreamSynchronize(st));
-    if (levels < 2 || (h->h_query[QueryCtl::kQueue + 2] <= b.cap[2] && (levels < 3 || h->h_query[QueryCtl::kQueue + 3] <= b.cap[3]))) break;
+    bool fits = true;
+    for (int l = 1; l <= levels; l++) fits = fits && q.host[QueryCtl::kQueue + l] <= b.cap[l];
+    if (fits) break;
   }
-  const uint32_t e = (uint32_t)h->h_query[QueryCtl::kErr];
+  const uint32_t e = (uint32_t)q.host[QueryCtl::kErr];
   if (e) return h->fail(derr_to_status(e), "device: %s", derr_text(e));
-  *count = h->h_query[QueryCtl::kTotal] + fixed;
+  *count = q.host[QueryCtl::kTotal] + fixed;
   return NQ_OK;
 }
 

@@ -267,7 +267,7 @@ __device__ unsigned expand_query(const uint4 root, uint32_t N, uint32_t T, const
       unsigned c = 0;
       each_child(f, o, bm, [&](uint4) { c++; });
       unsigned at = take_slots(&cnt, c);
-      if (c) each_child(f, o, bm, [&](uint4 g) { if (at < cap) out[at] = g; at++; });
+      if (c) each_child(f, o, bm, [&](uint4 g) { out[at++] = g; });
     }
     __syncthreads();
     n = min(cnt, cap);
@@ -326,18 +326,15 @@ __global__ void __launch_bounds__(512) batch_query_kernel(const BatchQuery* __re
 }
 
 // The query's queue by another level (frames at the terminal depth move on).  A level that did not fit its buffer is
-// not read: the next one's length says that it did not fit either, so the search does nothing.
+// not read: the levels behind it stay empty, so the search does nothing, and the host finds its length.
 template <bool WIDE>
 __global__ void __launch_bounds__(128) query_level_kernel(uint32_t N, uint32_t T, QueryBuffers b, int level) {
   using W = typename QueryWord<WIDE>::type;
   chain_next();
   chain_wait();
-  const unsigned n = b.ctl[QueryCtl::kQueue + level];
+  unsigned n = b.ctl[QueryCtl::kQueue + level];
+  if (n > b.cap[level]) n = 0;
   const unsigned cap = b.cap[level + 1];
-  if (n > b.cap[level]) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) b.ctl[QueryCtl::kQueue + level + 1] = ~0u;
-    return;
-  }
   const uint4* in = b.sroot[level];
   uint4* __restrict__ out = b.sroot[level + 1];
   uint2* __restrict__ info = b.sinfo[level + 1];

@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <map>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -55,6 +56,24 @@ constexpr size_t kTotal = 0, kCursor = 8, kErr = 16, kTmax = 20, kSplit = 24, kD
 constexpr size_t kGen = 64, kGenErr = 92, kAll = 96;
 }
 
+// What a completion query runs on: a stream, a buffer and a pinned block for its control block.  Up to kSmall bytes the
+// buffer is plain memory, in powers of two; what takes more comes from the handle's pool (which takes 32 MiB from the
+// device at a time) and is given back to it without waiting for other streams.
+struct QueryRun {
+  static constexpr size_t kSmall = 16ull << 20;
+  cudaStream_t stream = nullptr;
+  DevBuf small, large;
+  uint64_t* host = nullptr;
+  cudaError_t ensure(size_t n, unsigned char** p) {
+    size_t s = 256 << 10;
+    while (s < n && s <= kSmall) s *= 2;
+    DevBuf& b = s <= kSmall ? small : large;
+    const cudaError_t e = b.ensure(s <= kSmall ? s : n);
+    *p = (unsigned char*)b.p;
+    return e;
+  }
+};
+
 }  // namespace nq
 
 struct nq_handle {
@@ -66,11 +85,47 @@ struct nq_handle {
   nq::DevBuf rec, root, info, sched, per_task, ctrl, sroot;
   nq::DevBuf gen, starts;                // device generator: the other state buffer, the start list
   nq::DevBuf utasks, uconfs, uctl;       // unique counter (nq_count_unique)
-  // completion queries: a stream and buffers of their own, so a query may run beside an asynchronous count
-  cudaStream_t q_stream = nullptr;
-  nq::DevBuf qbuf;
-  uint64_t* h_query = nullptr;           // pinned read-back of a query's control block
+  // Completion queries: each runs on a stream and buffers of its own, so queries of several threads, and one beside an
+  // asynchronous count, do not wait for each other.  Up to kQueryRuns of them are kept for the next queries, one of
+  // them with what its largest query took.
+  static constexpr size_t kQueryRuns = 8;
+  std::vector<nq::QueryRun*> q_free;
   std::mutex q_mu;
+  cudaError_t query_get(nq::QueryRun** out) {
+    {
+      std::lock_guard<std::mutex> lk(q_mu);
+      if (!q_free.empty()) { *out = q_free.back(); q_free.pop_back(); return cudaSuccess; }
+    }
+    cudaError_t e = ensure_pool();
+    if (e != cudaSuccess) return e;
+    nq::QueryRun* q = new (std::nothrow) nq::QueryRun();
+    if (!q) return cudaErrorMemoryAllocation;
+    e = cudaStreamCreateWithFlags(&q->stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess && !(q->host = (uint64_t*)pin_get(256))) e = cudaErrorMemoryAllocation;
+    if (e != cudaSuccess) { query_free(q); return e; }
+    q->large.ordered = q->stream; q->large.pool = pool;
+    *out = q;
+    return cudaSuccess;
+  }
+  void query_put(nq::QueryRun* q) {
+    {
+      std::lock_guard<std::mutex> lk(q_mu);
+      if (q_free.empty()) { q_free.push_back(q); return; }
+      if (q_free.size() < kQueryRuns) {          // behind the one that may hold a large buffer
+        q->large.release();
+        q_free.insert(q_free.begin(), q);
+        return;
+      }
+    }
+    query_free(q);
+  }
+  void query_free(nq::QueryRun* q) {
+    q->large.release();
+    if (q->stream) { cudaStreamSynchronize(q->stream); cudaStreamDestroy(q->stream); }
+    q->small.release();
+    pin_put(q->host);
+    delete q;
+  }
   nq::DevBuf okeys, oorder, ohist;       // queue order (nq_set_queue_order)
   int queue_order = 0;                   // 0: generator / split order, 1: largest estimated subtree first
   int64_t chunk_records = 0;             // records per chunk of nq_count (0: the library default)

@@ -140,10 +140,10 @@ struct QueryBuffers {
   uint4* tmp;                   // cap[0] frames
   uint4* sroot[4];              // the queue from one block, and after one to three levels over the whole GPU
   uint2* sinfo[4];
-  unsigned cap[4];              // items each holds; cap[1] = cap[0] * N, so only the later ones can be too small
+  unsigned cap[4];              // items each holds; the block's own, [0], always fits
 };
 // Writes the task, its queue and the control block, the queue expanded by `levels` (0..3) more levels.  A
-// queue longer than its buffer leaves ctl[kQueue + levels] above cap[levels]: the DFS does nothing.
+// level longer than its buffer leaves its ctl[kQueue + ..] above its cap: what comes behind it does nothing.
 cudaError_t launch_query(const QueryParam& p, const QueryBuffers& b, bool wide, int levels, int sms, cudaStream_t st);
 
 // Batches.  A list holds sources: the tasks of a board's records (depth 0), or the frames a query was expanded
