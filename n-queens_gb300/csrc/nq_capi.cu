@@ -188,8 +188,10 @@ int read_ctrl(nq_handle* h, cudaStream_t st, uint64_t* total) {
 constexpr unsigned kQueryCap = 65536;
 constexpr unsigned kQueryTarget = 2048;      // ... and of each query of a batch
 unsigned query_target(int rows) { return rows >= 16 ? kQueryTarget : 512u; }
-constexpr unsigned kQueryCap2 = 4 << 20;     // queue after two levels (4.5 10^6 on the empty board of N=27, which take one)
-constexpr unsigned kQueryCap3 = 5 << 20;     // ... after three (0.5 to 4.5 10^6 measured for N=18..25; some of N=27 are longer)
+// The queue has room for the frames expected after each level (query_estimate), up to this many: a level less where
+// more come, or the device has no room.  After three levels 0.04 to 5 10^6 items of 24 bytes are in it for N=15..23, 8
+// to 20 10^6 for N=24..27 with two queens, and the level before them has a quarter at most.
+constexpr unsigned kQueryMost = 5 << 20, kQueryMost2 = kQueryMost / 4;
 int query_levels(int rows) { return rows >= 13 ? 3 : rows >= 11 ? 2 : rows >= 10 ? 1 : 0; }
 // A batch's queries share the lanes with its other jobs, so the same need not be cut as fine.
 int batch_query_levels(int rows) { return rows >= 15 ? 2 : rows >= 12 ? 1 : 0; }
@@ -204,6 +206,44 @@ uint64_t query_frames(const QueryParam& p) {
     most = std::max(most, n);
   }
   return most;
+}
+
+// Frames expected at each depth 0..T of a query's expansion: a row's squares off the pre-placed queens' lines, less
+// those that each queen of the rows above takes at random (its column and, on the board, two diagonals).  Diagonals that
+// meet on a square count twice, so the product stands a little above the frames there are: from the first depth with
+// the target's number on, 5,572 queries of N=8..27 had at most 0.88 / 0.78 / 0.66 of it after one / two / three levels.
+void query_estimate(const QueryParam& p, double est[kMaxDepth]) {
+  const double inv = 1.0 / p.N;
+  double left[kMaxN];                        // of a row's squares, after a queen so many rows above
+  for (uint32_t r = 1; r < p.N; r++) left[r] = 1.0 - (3.0 - 2.0 * r * inv) * inv;
+  const uint32_t bm = (1u << p.N) - 1u;
+  uint32_t ld = p.root.x, rd = p.root.y, row = 0, at[kMaxDepth];
+  est[0] = 1.0;
+  for (uint32_t d = 0; d < p.T; d++) {
+    at[d] = row;
+    double a = __builtin_popcount(bm & ~(ld | rd | p.root.z));
+    for (uint32_t j = 0; j < d; j++) a *= left[row - at[j]];
+    est[d + 1] = est[d] * a;
+    const uint32_t x = p.words[d].x, step = x & W_S;         // both forms of the words hold the step and LA alike
+    ld = (ld << step) | (x >> (32 - step));
+    rd = (rd >> step) | p.words[d].y;
+    row += step;
+  }
+}
+
+// Room for the queue after 0..levels levels over the GPU.  The block stops at the first depth with `target` frames: the
+// first with that many expected or, where fewer come there, the next, from less than the target.
+void query_caps(const QueryParam& p, const double est[kMaxDepth], int levels, unsigned cap[4]) {
+  uint32_t d = 0;
+  while (d < p.T && est[d] < p.target) d++;
+  cap[0] = (unsigned)query_frames(p);
+  for (int l = 1; l <= levels; l++) {
+    double n = 0.0;                    // at the terminal depth, which frames do not pass, the ones before it
+    for (uint32_t k = d; k <= std::min(d + l, p.T); k++) n = std::max(n, est[k]);
+    for (uint32_t k = d; k <= std::min(d + l + 1, p.T); k++) n = std::max(n, est[k] * std::min(1.0, p.target / est[d]));
+    const double most = l == 2 && levels == 3 ? kQueryMost2 : kQueryMost;
+    cap[l] = (unsigned)std::min(n + 512.0, most);
+  }
 }
 
 // The query as a device task.  Returns 1, 0 when the count is settled here (*fixed), or -1 on bad arguments.
@@ -1347,13 +1387,18 @@ int nq_count_completions(nq_handle* h, int N, int k, const int* rows, const int*
   QueryRun& q = *lease.q;
   cudaStream_t st = q.stream;
   p.target = std::min(query_target((int)p.T + 2), kQueryCap / (unsigned)N);
-  for (int levels = query_levels((int)p.T + 2);; levels--) {      // a level less where the queue did not fit
+  int levels = query_levels((int)p.T + 2);
+  double est[kMaxDepth] = {0.0};
+  if (levels > 0) query_estimate(p, est);
+  for (;; levels--) {                        // a level less where the queue did not fit
     QueryBuffers b{};
-    b.cap[0] = kQueryCap; b.cap[1] = kQueryCap * (unsigned)N; b.cap[2] = kQueryCap2; b.cap[3] = kQueryCap3;
+    query_caps(p, est, levels, b.cap);
     size_t items = 0;
     for (int l = 0; l <= levels; l++) items += b.cap[l];
     unsigned char* c = nullptr;
-    NQ_CUDA(h, q.ensure(1024 + (b.cap[0] + items) * sizeof(uint4) + items * sizeof(uint2), &c));
+    const cudaError_t room = q.ensure(1024 + (b.cap[0] + items) * sizeof(uint4) + items * sizeof(uint2), &c);
+    if (room == cudaErrorMemoryAllocation && levels > 0) { cudaGetLastError(); continue; }
+    NQ_CUDA(h, room);
     b.ctl = (unsigned long long*)c; b.info = (uint32_t*)(c + 128); b.sched = c + 256;
     b.tmp = (uint4*)(c + 1024);
     b.sroot[0] = b.tmp + b.cap[0];
