@@ -186,7 +186,9 @@ int nq_last_count_info(const nq_handle *h, int64_t *chunks, int64_t *records);
 /* Unique (distinct under rotation and reflection) and total counts by the
  * symmetry method (11Bit_Python/07Py_bit_symmetry.py:65-200; GPU form
  * 10Bit_CUDA/01CUDA_Bit_Symmetry.cu:627-960).  4 <= N <= 27.  Runs on the
- * handle's device and stream with buffers the handle keeps between calls;
+ * handle's device and stream with buffers the handle keeps between calls: up to
+ * 1.4 MiB for N <= 12, 23 MiB for N <= 15, 48 MiB at N=16, 172 MiB at N=18 and
+ * 298 MiB at N=19, which is the most (less where the device has not that much);
  * failures are reported through nq_last_error like every other call. */
 int nq_count_unique(nq_handle *h, int N, uint64_t *unique, uint64_t *total);
 
@@ -210,6 +212,10 @@ int nq_debug_task_schedule(int N, nq_record rec, uint32_t root[4], uint32_t *inf
  * <= 27, presets 4..8, else 0), which sizes its buffers: the records from N=12
  * on, for smaller boards a level between may be wider. */
 int64_t nq_debug_board_states(int N, int preset);
+
+/* Diagnostic: states of the unique counter's start configurations after
+ * `level` rows were expanded (4 <= N <= 27, 0..6), which size its buffers. */
+int64_t nq_debug_unique_states(int N, int level);
 
 /* Diagnostic: the row rules of the unique counter's start configuration `conf`
  * (0 <= conf < N - 3 + (N - 2) / 2) as its search reads them, words[left] for

@@ -110,12 +110,14 @@ struct UCtl {
   unsigned int cursor, done;    // done: blocks of unique_kernel that have ended
   unsigned int n[kLevels + 1];
 };
-// The queue is the last level with states in it that its buffer holds (levels alternate between two
-// buffers; a level that was large enough, or whose states all died, leaves the next one empty).
-__host__ __device__ __forceinline__ int queue_level(const UCtl* c, unsigned cap) {
+// Levels alternate between two buffers of cap[0] and cap[1] tasks.
+struct UCap { unsigned cap[2]; };
+// The queue is the last level with states in it that its buffer holds (a level that was large enough, or whose states
+// all died, leaves the next one empty).
+__host__ __device__ __forceinline__ int queue_level(const UCtl* c, const UCap& b) {
   int f = 0;
   for (int l = 1; l <= kLevels; l++)
-    if (c->n[l] && c->n[l] <= cap) f = l;
+    if (c->n[l] && c->n[l] <= b.cap[l & 1]) f = l;
   return f;
 }
 
@@ -125,7 +127,7 @@ struct UArgs {
   int N;
   int nconf;
   int maxf;                     // stack frames per lane: the sentinel's and one per row from the smallest task row
-  unsigned cap;                 // tasks a buffer holds
+  UCap cap;
   UCtl* ctl;
   uint32_t* host;               // pinned: receives the control block
 };
@@ -382,14 +384,16 @@ __global__ void __launch_bounds__(64) unique_init_kernel(int N, int nconf, UConf
 
 // Level l -> l + 1: one thread per state; its children with candidates left are counted, the warp reserves
 // their slots with one atomic, and they are written.  States that must not be expanded move on as they are.
-// n[l] <= 2^32: a level below the target (at most 2^21 states) has at most 27 children a state.
-__global__ void __launch_bounds__(128) unique_expand_kernel(int N, int level, unsigned target, unsigned cap, const UConf* confs,
+// n[l] <= 2^32: a level below the target (at most 2^21 states) has at most 27 children a state.  A level that did not
+// fit its buffer is not expanded: the queue stays the level before it.
+__global__ void __launch_bounds__(128) unique_expand_kernel(int N, int level, unsigned target, UCap room, const UConf* confs,
                                                             const UTask* in, UTask* __restrict__ out,
                                                             UCtl* ctl) {
   chain_next();
   chain_wait();
   const unsigned n = ctl->n[level];
-  if (n >= target) return;
+  if (n >= target || n > room.cap[level & 1]) return;
+  const unsigned cap = room.cap[(level + 1) & 1];
   const uint32_t mask = (1u << N) - 1u;
   const unsigned lane = threadIdx.x & 31u;
   for (unsigned i0 = blockIdx.x * blockDim.x; i0 < n; i0 += gridDim.x * blockDim.x) {
@@ -424,7 +428,7 @@ __global__ void __launch_bounds__(128) unique_expand_kernel(int N, int level, un
     unsigned base = 0;
     if (lane == 31 && incl) base = atomicAdd(&ctl->n[level + 1], incl);
     base = __shfl_sync(FULLM, base, 31) + incl - cnt;
-    if (base + cnt > cap) continue;      // the level does not fit: the queue stays the level before it
+    if (base + cnt > cap) continue;
     if (keep) out[base] = s;
     else if (cnt) each_child([&](UTask& t, uint32_t bit) {
       board_set(t, s.row, bit);
@@ -433,10 +437,45 @@ __global__ void __launch_bounds__(128) unique_expand_kernel(int N, int level, un
   }
 }
 
+// States after each level, which sizes the buffers (enumerated; a board whose rows end before holds its states).
+uint32_t level_states(int N, int level) {
+  static constexpr uint32_t n[kMaxN - 3][kLevels + 1] = {       // N = 4..
+      {1, 1, 1, 1, 1, 1, 1},
+      {2, 3, 3, 3, 3, 3, 3},
+      {4, 7, 7, 5, 5, 5, 5},
+      {6, 12, 21, 24, 17, 17, 17},
+      {8, 23, 50, 92, 80, 48, 48},
+      {9, 35, 97, 243, 358, 308, 174},
+      {11, 53, 183, 541, 1107, 1503, 1286},
+      {12, 69, 290, 1054, 2903, 5578, 6964},
+      {14, 94, 469, 1985, 6608, 16453, 27662},
+      {15, 115, 670, 3293, 13070, 41743, 87139},
+      {17, 147, 983, 5520, 25294, 95196, 230022},
+      {18, 173, 1310, 8349, 43935, 192828, 540547},
+      {20, 212, 1797, 12840, 76218, 380680, 1168189},
+      {21, 243, 2282, 18161, 121116, 686457, 2272413},
+      {23, 289, 2983, 26204, 194112, 1228927, 4388380},
+      {24, 325, 3658, 35253, 288698, 2035297, 7724564},
+      {26, 378, 4613, 48444, 434896, 3377711, 13757078},
+      {27, 419, 5510, 62721, 614466, 5238820, 22456135},
+      {29, 479, 6759, 82968, 881352, 8185547, 37537711},
+      {30, 525, 7910, 104237, 1195780, 12054968, 57765474},
+      {32, 592, 9493, 133760, 1648896, 17937511, 91713177},
+      {33, 643, 10930, 164049, 2165344, 25336316, 134614515},
+      {35, 717, 12887, 205380, 2891344, 36219683, 204807695},
+      {36, 773, 14642, 246981, 3696940, 49438122, 289262952},
+  };
+  return n[N - 4][level];
+}
+
 }  // namespace
 }  // namespace nq
 
 using namespace nq;
+
+extern "C" int64_t nq_debug_unique_states(int N, int level) {
+  return N < 4 || N > kMaxN || level < 0 || level > kLevels ? NQ_EINVAL : (int64_t)level_states(N, level);
+}
 
 extern "C" int nq_debug_unique_words(int N, int conf, uint32_t* words) {
   if (N < 4 || N > kMaxN || conf < 0 || conf >= (N - 3) + (N - 2) / 2 || !words) return NQ_EINVAL;
@@ -458,17 +497,26 @@ extern "C" int nq_count_unique(nq_handle* h, int N, uint64_t* unique, uint64_t* 
   // with a target of 512 / 1024 / 4096 / 13824 tasks per SM, N=15 235 / 235 / 186 / 187, N=16 620 / 626 / 575 /
   // 582, N=17 7770 / 3088 / 3090 / 3077, N=18 37772 / 37105 / 21139 / 19606 (now 170, 540, 2900 and 18208).
   const unsigned target = (unsigned)sms * (N <= 17 ? 4096u : 13824u);
-  const size_t cap = (size_t)target * 5;
-  NQ_CUDA(h, h->utasks.ensure(2 * cap * sizeof(UTask)));
+  int levels = 0;                               // N <= 9: a launch costs more than it balances
+  for (const int most = N <= 9 ? 1 : std::min(kLevels, N - 3);
+       levels < most && level_states(N, levels) < target && level_states(N, levels + 1) <= 5ull * target;) levels++;
+  UCap room{};
+  for (;; levels--) {                           // a level less where the device has no room for it
+    room = UCap{};
+    for (int l = 0; l <= levels; l++) room.cap[l & 1] = std::max(room.cap[l & 1], level_states(N, l));
+    const cudaError_t e = h->utasks.ensure(((size_t)room.cap[0] + room.cap[1]) * sizeof(UTask));
+    if (e == cudaErrorMemoryAllocation && levels > 0) { cudaGetLastError(); continue; }
+    NQ_CUDA(h, e);
+    break;
+  }
   NQ_CUDA(h, h->uconfs.ensure((size_t)nconf * sizeof(UConf)));
   NQ_CUDA(h, h->uctl.ensure(sizeof(UCtl)));
   UCtl* ctl = (UCtl*)h->uctl.p;
   UConf* confs = (UConf*)h->uconfs.p;
-  UTask* buf[2] = {(UTask*)h->utasks.p, (UTask*)h->utasks.p + cap};
+  UTask* buf[2] = {(UTask*)h->utasks.p, (UTask*)h->utasks.p + room.cap[0]};
   unique_init_kernel<<<1, 64, 0, st>>>(N, nconf, confs, buf[0], ctl);
-  const int levels = N <= 9 ? 1 : std::min(kLevels, N - 3);   // N <= 9: a launch costs more than it balances
   for (int l = 0; l < levels; l++)
-    NQ_CUDA(h, launch_after(unique_expand_kernel, l < 2 ? 1 : l == 2 ? sms : 4 * sms, 128, 0, st, N, l, target, (unsigned)cap, confs,
+    NQ_CUDA(h, launch_after(unique_expand_kernel, l < 2 ? 1 : l == 2 ? sms : 4 * sms, 128, 0, st, N, l, target, room, confs,
                             buf[l & 1], buf[(l + 1) & 1], ctl));
   NQ_CUDA(h, cudaGetLastError());
   if (int s = h->ensure_pinned(sizeof(UCtl))) return s;
@@ -478,7 +526,7 @@ extern "C" int nq_count_unique(nq_handle* h, int N, uint64_t* unique, uint64_t* 
   if (N >= kReadBackN) {
     NQ_CUDA(h, cudaMemcpyAsync(h->h_ctrl, ctl, sizeof(UCtl), cudaMemcpyDeviceToHost, st));
     NQ_CUDA(h, cudaStreamSynchronize(st));
-    row = 1 + queue_level((const UCtl*)h->h_ctrl, (unsigned)cap);
+    row = 1 + queue_level((const UCtl*)h->h_ctrl, room);
   }
   const int maxf = N - row + 1;
   constexpr int B = 128;   // N=18: 64 / 128 / 256 threads 20.3 / 19.6 / 19.9 ms
@@ -491,7 +539,7 @@ extern "C" int nq_count_unique(nq_handle* h, int N, uint64_t* unique, uint64_t* 
   NQ_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, unique_kernel<B>, B, smem));
   if (per <= 0) return h->fail(NQ_ECUDA, "count_unique: N=%d does not fit on an SM", N);
   UArgs a;
-  a.tasks[0] = buf[0]; a.tasks[1] = buf[1]; a.confs = confs; a.nconf = nconf; a.N = N; a.maxf = maxf; a.cap = (unsigned)cap; a.ctl = ctl;
+  a.tasks[0] = buf[0]; a.tasks[1] = buf[1]; a.confs = confs; a.nconf = nconf; a.N = N; a.maxf = maxf; a.cap = room; a.ctl = ctl;
   a.host = (uint32_t*)h->h_ctrl;
   NQ_CUDA(h, launch_after(unique_kernel<B>, sms * per, B, smem, st, a));
   NQ_CUDA(h, cudaStreamSynchronize(st));

@@ -87,6 +87,7 @@ SIGNATURES = {
     "nq_count_unique": (ctypes.c_int, [_vp, ctypes.c_int, _u64p, _u64p]),
     "nq_count_completions": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, _ip, _ip, _u64p]),
     "nq_debug_task_schedule": (ctypes.c_int, [ctypes.c_int, nq_record, _u32p, _u32p, _u32p, ctypes.c_int]),
+    "nq_debug_unique_states": (ctypes.c_int64, [ctypes.c_int, ctypes.c_int]),
     "nq_debug_board_states": (ctypes.c_int64, [ctypes.c_int, ctypes.c_int]),
     "nq_debug_unique_words": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _u32p]),
     "nq_debug_completion_tasks": (ctypes.c_int64, [ctypes.c_int, ctypes.c_int, _ip, _ip, ctypes.c_int, _u32p,
