@@ -99,13 +99,16 @@ int run_records(nq_handle* h, int N, const uint4* d_rec, int64_t m, int start_mi
   P.err = (unsigned int*)(c + ctl::kErr); P.tmax = (unsigned int*)(c + ctl::kTmax);
   P.per_task = d_per_task; P.qn = (unsigned long long*)(c + ctl::kSplit); P.total = (unsigned long long*)(c + ctl::kTotal);
   // Queue capacity: a bound (each level places a queen in one of at most N - 2, N - 3, ... columns) where that
-  // is small, else 8 a level (measured: up to 8), built again if it was too small.
+  // is small, else 8 a level (measured: up to 8), built again if it was too small.  Where the device has not that
+  // much, the first launch only counts the queue, and it is built at its length.
   uint64_t bound = (uint64_t)m, guess = (uint64_t)m + 1024;
   for (int d = 0; d < D; d++) { bound *= (uint64_t)(N - 2 - d); guess *= 8; }
-  const bool read_back = (m > no_read_back(maxt) && !m_dev) || h->queue_order == 1 || (D > 0 && bound * sizeof(uint4) > (uint64_t)kQueueBytes);
+  bool read_back = (m > no_read_back(maxt) && !m_dev) || h->queue_order == 1 || (D > 0 && bound * sizeof(uint4) > (uint64_t)kQueueBytes);
   if (D > 0) {
     const uint64_t q = std::max(read_back ? std::min(bound, guess) : bound, (uint64_t)(h->sroot.cap / sizeof(uint4)));
-    NQ_CUDA(h, h->sroot.ensure((size_t)q * sizeof(uint4)));
+    cudaError_t e = h->sroot.ensure((size_t)q * sizeof(uint4));
+    if (e == cudaErrorMemoryAllocation) { cudaGetLastError(); read_back = true; e = cudaSuccess; }
+    NQ_CUDA(h, e);
   } else {
     NQ_CUDA(h, h->root.ensure((size_t)m * sizeof(uint4)));
     P.root = (uint4*)h->root.p;
