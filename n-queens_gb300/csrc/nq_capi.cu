@@ -1186,6 +1186,9 @@ int nq_batch_create(nq_handle* h, const nq_job* jobs, int njobs, nq_batch** out)
     if (herr[0]) { status = h->fail(NQ_EPRESET, "batch: generator failed (preset too deep)"); break; }
     if (herr[1]) { status = h->fail(derr_to_status(herr[1]), "batch prepare: %s", derr_text(herr[1])); break; }
     const ListState* hst = (const ListState*)hs;
+    for (size_t i = 0; i < nl; i++)          // a source's first slot is kept in 32 bits
+      if (hst[i].items > 0xFFFFFFFFull) status = h->fail(NQ_ENOMEM, "batch: %llu items of one list", hst[i].items);
+    if (status != NQ_OK) break;
     // Stacks sized to the deepest item: items start `depth` + D down, so they need (deepest T) less that.
     std::vector<int> deep(nl, 1);
     for (size_t i = 0; i < nb; i++)
