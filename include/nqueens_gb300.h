@@ -109,7 +109,8 @@ int nq_sync(nq_handle *h);
  * read-back); waits for them. */
 int nq_last_kernel_ms(nq_handle *h, float *prepare_ms, float *dfs_ms);
 /* Split depth used by the last exec_solutions call and the length of the
- * DFS queue it built (records, or subtasks when split). */
+ * DFS queue it built (records, or subtasks when split); waits for the call
+ * where it is still queued and built the queue's length on the device. */
 int nq_last_run_info(const nq_handle *h, int *split_depth, int64_t *queued);
 
 /* exec_solutions for callers that cannot allocate device memory -- no

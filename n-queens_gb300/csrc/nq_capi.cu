@@ -370,7 +370,12 @@ int nq_int32_peak(nq_handle* h, int kind, double* ops_per_s) {
 int nq_last_run_info(const nq_handle* h, int* split_depth, int64_t* queued) {
   if (!h) return NQ_EINVAL;
   if (split_depth) *split_depth = h->last_split;
-  if (queued) *queued = h->last_queue;
+  if (!queued) return NQ_OK;
+  *queued = h->last_queue;
+  if (h->pending && h->queue_on_device) {      // its length comes with the run's result
+    if (cudaSetDevice(h->device) != cudaSuccess || cudaEventSynchronize(h->done) != cudaSuccess) return NQ_ECUDA;
+    *queued = (int64_t)*(const uint64_t*)((const unsigned char*)h->h_result + ctl::kSplit);
+  }
   return NQ_OK;
 }
 
