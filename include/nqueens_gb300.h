@@ -93,9 +93,12 @@ int nq_exec_solutions(nq_handle *h, int N, const nq_record *records, int64_t m, 
  * or -1 to use the bound 1.  d_total (device, 1 x u64) is overwritten.  Long
  * lists (from 16,385 records, 65,537 where at most 12 rows follow start_min)
  * wait once for a 64-byte read-back (the subtask count and the deepest
- * schedule, which size the DFS queue and stacks) before launching the DFS;
- * shorter ones are only queued.  Call nq_sync() to wait for the result and
- * collect the status. */
+ * schedule, which size the DFS queue and stacks) before launching the DFS, and
+ * so do shorter ones whose queue is bounded by more than 256 MiB (split 3: from
+ * some thousand records of N=19), for whose bound the device has no room, or
+ * that are sorted (nq_set_queue_order); the others are only queued.  A stream
+ * under capture is refused with NQ_ECUDA.  Call nq_sync() to wait for the
+ * result and collect the status. */
 int nq_exec_solutions_device(nq_handle *h, int N, const nq_record *d_records, int64_t m, int start_min,
                              uint64_t *d_solutions, uint64_t *d_total, void *stream);
 /* Waits for the handle's last nq_exec_solutions_device call (an event
@@ -124,8 +127,9 @@ int nq_last_run_info(const nq_handle *h, int *split_depth, int64_t *queued);
  * scratch is one fixed __device__ array of about 15 MiB inside the library,
  * held by every GPU that loads it until exit.  Limit: m <= 131072 records and
  * schedules up to 24 depths (N - start_min <= 25); larger inputs are rejected
- * with NQ_EINVAL, never truncated.  Tasks are split as far as the array holds
- * the queue; one that does not fit is counted unsplit.  The first call on each
+ * with NQ_EINVAL, never truncated.  Tasks are split as far as the array is
+ * expected to hold the queue; one that does not fit is built again with a level
+ * less, unsplit at the end.  The first call on each
  * device looks the array's address up (cudaGetSymbolAddress) with that device
  * current; with lazy module loading that first call is also when the array
  * and the kernels are loaded onto the device, so make it once at start-up --

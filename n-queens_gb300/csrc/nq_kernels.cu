@@ -281,7 +281,6 @@ cudaError_t launch_prepare_split(int D, int64_t m_max, const PrepareSplit& a, cu
     case 3: return launch_after(prepare_split_kernel<3>, G, B, 0, st, a);
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------

@@ -33,10 +33,9 @@ namespace {
 
 constexpr unsigned FULLM = 0xFFFFFFFFu;
 constexpr int kBoardRows = 8;    // rows of the board prefix carried by a task
-// Steps per lane between checks for finished lanes, a multiple of the steps unrolled.  Unrolled far the loop and
-// the classification in it outgrow the instruction cache (a whole count at N=18, unrolled by 1 / 2 / 5 / 10 / 15 /
-// 30 with every board classified by the warp: 24.5 / 23.4 / 23.4 / 23.3 / 24.0 / 28.9 ms; as it is now, by 2 / 5 /
-// 10: 18.7 / 18.2 / 18.1), and 20 steps a check gave 21.7 ms where 30 gave 21.5.
+// Steps per lane between checks for finished lanes, a multiple of the steps unrolled.  A whole count at N=18,
+// unrolled by 2 / 5 / 10: 18.7 / 18.2 / 18.1 ms; by 30 the loop and the classification in it outgrow the instruction
+// cache (a quarter slower), and 20 steps a check are 1 % slower than 30.
 constexpr int kUniqueSteps = 30, kUniqueUnroll = 5;
 // Boards from here on size the stacks to the tasks' rows (N=14 96 us without the read-back, 111 with; N=15 187
 // against 190, and the search grows sixfold a size from there).
@@ -493,9 +492,9 @@ extern "C" int nq_count_unique(nq_handle* h, int N, uint64_t* unique, uint64_t* 
   cudaStream_t st = h->stream;
   const int nconf = (N - 3) + (N - 2) / 2;      // part 1: bound1 2..N-2; part 2: bound1 < N - 1 - bound1
   // Rows are expanded until the queue holds `target` tasks, unless the next row does not fit the buffer.
-  // Lanes share work within a warp only, so the warps' sums have to even out: us of a whole count on GB300
-  // with a target of 512 / 1024 / 4096 / 13824 tasks per SM, N=15 235 / 235 / 186 / 187, N=16 620 / 626 / 575 /
-  // 582, N=17 7770 / 3088 / 3090 / 3077, N=18 37772 / 37105 / 21139 / 19606 (now 170, 540, 2900 and 18208).
+  // Lanes share work within a warp only, so the warps' sums have to even out: relative time of a whole count on GB300
+  // with a target of 512 / 1024 / 4096 / 13824 tasks per SM, N=15 1.26 / 1.26 / 1 / 1.01 (of 170 us), N=16 1.08 / 1.09 /
+  // 1 / 1.01 (540 us), N=17 2.52 / 1 / 1 / 1 (2.90 ms), N=18 1.93 / 1.89 / 1.08 / 1 (18.2 ms).
   const unsigned target = (unsigned)sms * (N <= 17 ? 4096u : 13824u);
   int levels = 0;                               // N <= 9: a launch costs more than it balances
   for (const int most = N <= 9 ? 1 : std::min(kLevels, N - 3);
