@@ -110,10 +110,10 @@ struct nq_handle {
   void query_put(nq::QueryRun* q) {
     {
       std::lock_guard<std::mutex> lk(q_mu);
-      if (q_free.empty()) { q_free.push_back(q); return; }
-      if (q_free.size() < kQueryRuns) {          // behind the one that may hold a large buffer
-        q->large.release();
-        q_free.insert(q_free.begin(), q);
+      if (q_free.size() < kQueryRuns) {
+        for (nq::QueryRun* f : q_free)
+          if (f->large.p) q->large.release();
+        q_free.insert(q->large.p ? q_free.end() : q_free.begin(), q);     // the one with a large buffer is taken next
         return;
       }
     }
@@ -212,12 +212,6 @@ struct nq_handle {
     return NQ_OK;
   }
 };
-
-#define NQ_CUDA(h, call)                                     \
-  do {                                                       \
-    cudaError_t _e = (call);                                 \
-    if (_e != cudaSuccess) return (h)->cuda_fail(_e, #call); \
-  } while (0)
 
 #define NQ_CUDA(h, call)                                     \
   do {                                                       \

@@ -41,3 +41,28 @@ def test_queries_of_several_threads(oracle_mod):
     finally:
         eng.close()
     assert _free(torch) >= before - 8 * MIB
+
+
+def test_the_large_buffer_stays_with_the_next_query():
+    """After queries of several threads left their streams behind, large queries one by one reuse one buffer: what the
+    device has free does not change between them, nor with small ones in between."""
+    import nqueens
+    torch = pytest.importorskip("torch")
+    eng = nqueens.Engine(0, auto_tune=False)
+    large = (20, [(2, 2), (10, 7)])
+    try:
+        want = eng.count_completions(*large)
+        threads = [threading.Thread(target=lambda: [eng.count_completions(12, [(0, i)]) for i in range(12)]) for _ in range(4)]
+        threads += [threading.Thread(target=lambda: eng.count_completions(*large)) for _ in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert eng.count_completions(*large) == want
+        free = _free(torch)
+        for _ in range(4):
+            assert eng.count_completions(*large) == want
+            assert eng.count_completions(8, []) == 92
+            assert _free(torch) == free
+    finally:
+        eng.close()
